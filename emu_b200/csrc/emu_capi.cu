@@ -285,6 +285,25 @@ long long mesh_elems(const emu_context* c) { return c->P.ncells * c->ND; }
 // an int64 mesh of the mixed path with its diagonal slots
 long long qmesh_elems(const emu_context* c) { return c->P.ncells * (c->ND + emu::kDiagSlots); }
 
+long long cmesh_elems(const emu_context* c) { return c->P.ncells * ((c->nf == 3 ? emu::Comb<3>::NG : emu::Comb<2>::NG) + emu::kDiagSlots); }
+
+int ensure_cmesh(emu_context* ctx)
+{
+    for (int i = 0; i < 4; i++)
+        if (!ctx->cmesh[i]) CU(emu_ctx::dev_malloc(&ctx->cmesh[i], sizeof(double) * cmesh_elems(ctx)));
+    return EMU_OK;
+}
+
+// nsteps steps of k_steps_1d (dt_mode as launch_steps_1d)
+int run_steps_1d(emu_context* ctx, int nsteps, int dt_mode)
+{
+    const cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, ctx->S[ctx->cur], ctx->cmesh, ctx->mesh[3], ctx->ctl,
+                                               nsteps, dt_mode, ctx->stream);
+    if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("cooperative steps: ") + cudaGetErrorString(e));
+    ctx->cur_mesh = 3;
+    return EMU_OK;
+}
+
 int zero_mesh(emu_context* ctx, int i)
 {
     if (ctx->mixed) CU(cudaMemsetAsync(ctx->qmesh[i], 0, sizeof(long long) * mesh_elems(ctx), ctx->stream));
@@ -340,6 +359,11 @@ int deposit_current(emu_context* ctx)
         emu::launch_deposit(ctx->nf, ctx->P, S, S.f0, ctx->mesh[0], ctx->stream);
         if ((r = check_launch(ctx, "deposit"))) return r;
         if ((r = emu_ctx::reduce_mesh(ctx, ctx->mesh[0], false, ctx->stream))) return r;
+        if (ctx->steps1d) {
+            emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh[0], ctx->stream);
+            if ((r = check_launch(ctx, "combined mesh"))) return r;
+            CU(cudaMemsetAsync(ctx->cmesh[1], 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
+        }
     }
     ctx->cur_mesh = 0;
     ctx->fused_ready = true;
@@ -543,7 +567,9 @@ bool rk4_fused(const emu_context* ctx)
 int emu_ctx::step_device(emu_context* ctx, bool last_stage_deposit)
 {
     int r;
-    if (ctx->coop) {
+    if (ctx->steps1d) {
+        return run_steps_1d(ctx, 1, emu::DT_ADVANCE);
+    } else if (ctx->coop) {
         double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
         cudaError_t e = emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx), ctx->ctl,
                                                   emu::DT_ADVANCE, ctx->stream);
@@ -633,6 +659,10 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     // (a sharded run reduces every deposit between stages: per-stage kernels)
     ctx->coop = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 2 && rk4_fused(ctx) &&
                 emu::coop_step_fits(ctx->nf, ctx->P, n);
+    // fused == 1, 1D along z, the grid fits: several steps per launch
+    ctx->steps1d = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
+                   emu::steps_1d_fit(ctx->nf, ctx->P, n);
+    if (ctx->steps1d && (r = ensure_cmesh(ctx))) return r;
     ctx->loaded = true;
     ctx->adj_valid = false;
     ctx->steps_since_sort = 0;
@@ -746,6 +776,7 @@ void emu_destroy(emu_context* ctx)
     if (ctx->tblock) emu_ctx::dev_free(ctx->tblock);
     if (ctx->S[0].kgen) emu_ctx::dev_free(ctx->S[0].kgen);
     for (int i = 0; i < 4; i++) if (ctx->mesh[i]) emu_ctx::dev_free(ctx->mesh[i]);
+    for (int i = 0; i < 4; i++) if (ctx->cmesh[i]) emu_ctx::dev_free(ctx->cmesh[i]);
     for (int i = 0; i < 2; i++) if (ctx->qmesh[i]) emu_ctx::dev_free(ctx->qmesh[i]);
     if (ctx->qfull) emu_ctx::dev_free(ctx->qfull);
     if (ctx->qfull_part) emu_ctx::dev_free(ctx->qfull_part);
@@ -942,7 +973,9 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
     emu::launch_ctl_set(ctx->ctl, dt, 0.0, INFINITY, 1, 1, ctx->stream);
     if (rk4_fused(ctx)) {
         if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
-        if (ctx->coop) {
+        if (ctx->steps1d) {
+            r = run_steps_1d(ctx, 1, -1);
+        } else if (ctx->coop) {
             double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
             cudaError_t e = emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx), ctx->ctl,
                                                       -1, ctx->stream);
@@ -982,6 +1015,7 @@ int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int m
         }
         emu::launch_dt_q(ctx->nf, ctx->P, ctx->qfull, nullptr, ctx->ctl, emu::DT_INIT, ctx->stream);
     }
+    else if (ctx->steps1d) emu::launch_dt_comb64(ctx->nf, ctx->P, ctx->cmesh[0], ctx->ctl, emu::DT_INIT, ctx->stream);
     else emu::launch_dt(ctx->nf, ctx->P, ctx->mesh[0], ctx->ctl, emu::DT_INIT, ctx->stream);
     return check_launch(ctx, "initial compute_dt");
 }
@@ -992,7 +1026,20 @@ int emu_evolve_steps(emu_context* ctx, int nsteps)
     int r;
     // the last of these steps deposits the full stage-4 mesh (the one a
     // caller can read after the call)
-    if (ctx->mixed && ctx->P.m4_reduced && nsteps > 0) emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
+    if (((ctx->mixed && ctx->P.m4_reduced) || ctx->steps1d) && nsteps > 0)
+        emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
+    if (ctx->steps1d) {
+        // one launch up to the next re-sort
+        const int ri = ctx->prm.resort_interval;
+        for (int i = 0; i < nsteps;) {
+            int len = std::min(nsteps - i, 256);
+            if (ri > 0) len = std::min(len, std::max(ri - ctx->steps_since_sort, 1));
+            if ((r = run_steps_1d(ctx, len, emu::DT_ADVANCE))) return r;
+            i += len;
+            if (ri > 0 && (ctx->steps_since_sort += len) >= ri && (r = resort(ctx))) return r;
+        }
+        return EMU_OK;
+    }
     for (int i = 0; i < nsteps; i++) {
         // when a re-sort follows this step, its gather makes the deposit of
         // the new state (in cell order) instead of the last stage
@@ -1052,7 +1099,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
 {
     if (!ctx || !kernel_ms || !nkernels) return EMU_ERR_ARG;
     if (!rk4_fused(ctx)) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: requires fused RK4");
-    if (ctx->coop) {
+    if (ctx->coop || ctx->steps1d) {
         // one cooperative kernel per step
         if (max_kernels < 1) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: kernel_ms too small");
         cudaEvent_t a, b;
@@ -1060,8 +1107,12 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
         CU(cudaEventCreate(&b));
         double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
         CU(cudaEventRecord(a, ctx->stream));
-        cudaError_t e = emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx), ctx->ctl,
-                                                  emu::DT_ADVANCE, ctx->stream);
+        if (ctx->steps1d) {
+            if (int rs = run_steps_1d(ctx, 1, emu::DT_ADVANCE)) return rs;
+        }
+        cudaError_t e = ctx->steps1d ? cudaSuccess
+                                     : emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx),
+                                                                 ctx->ctl, emu::DT_ADVANCE, ctx->stream);
         CU(cudaEventRecord(b, ctx->stream));
         if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("cooperative step: ") + cudaGetErrorString(e));
         CU(cudaEventSynchronize(b));

@@ -30,6 +30,10 @@ struct emu_context {
     void* tblock = nullptr;             // transient per-step arrays
     long long cap = 0;
     double* mesh[4] = {nullptr, nullptr, nullptr, nullptr};
+    // FP64 steps on combined meshes (steps1d): M_1..M_4 in the combined
+    // layout with the diagonal slots (kCombSlots per cell); mesh[0] and
+    // mesh[3] then hold the full deposit of a load and the full stage-4 mesh
+    double* cmesh[4] = {nullptr, nullptr, nullptr, nullptr};
     long long* qmesh[2] = {nullptr, nullptr};
     // mixed path: the full 8 NF^2 mesh of the state at the last deposit
     // (the step meshes M_1..M_3 hold only the combined self-interaction
@@ -61,6 +65,7 @@ struct emu_context {
     DevState graph_D[2][2];             // and the other buffer (the mixed stage 4 re-sorts into it)
     int steps_since_sort = 0;
     bool coop = false;                  // whole-step cooperative kernel (small FP64 problems)
+    bool steps1d = false;               // several steps per cooperative launch (k_steps_1d)
     emu_adjoint* adj = nullptr;         // allocated by the first adjoint call
     // particle sharding over ranks (emu_attach_comm): every deposit is summed
     // over the ranks before a stage reads it

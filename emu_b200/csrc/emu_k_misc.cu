@@ -3,6 +3,7 @@
 // emu_k_fp64_<nf>.cu and emu_k_mixed_<nf>.cu so that they compile in
 // parallel).
 #include "emu_kernels_impl.cuh"
+#include "emu_fp64.cuh"
 
 namespace emu {
 
@@ -178,6 +179,72 @@ void launch_finalize_mixed(int nf, const DevParams& P, const long long* qread, l
 void launch_dt(int nf, const DevParams& P, const double* mesh, StepCtl* ctl, int mode, cudaStream_t st)
 {
     EMU_NF_DISPATCH(nf, (k_dt<NFv, double><<<reduce_grid(P.ncells), kBlock, 0, st>>>(P, mesh, ctl, mode, nullptr)));
+}
+
+namespace {
+
+template <int NF>
+__global__ void __launch_bounds__(kBlock) k_full_to_comb64(DevParams P, const double* __restrict__ full,
+                                                           double* __restrict__ comb)
+{
+    using H = Herm<NF>;
+    using C = Comb<NF>;
+    constexpr int NH = NF * NF, ND = 8 * NH, NV = C::NV, NCS = kCombSlots<NF>;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < P.ncells * 4; i += stride) {
+        const long long cell = i / 4;
+        const int d = (int)(i - cell * 4);
+        const double* m = full + cell * ND;
+        double* out = comb + cell * NCS;
+        double c[NH], v[NV];
+#pragma unroll
+        for (int e = 0; e < NH; e++) {
+            const double a = m[2 * d * NH + e], b = m[(2 * d + 1) * NH + e];
+            c[e] = H::is_im(e) ? a + b : a - b;
+        }
+        C::values(c, v);
+#pragma unroll
+        for (int j = 0; j < NV; j++) out[d * NV + j] = v[j];
+        if (d == 0)
+            for (int k = 0; k < kDiagSlots; k++)
+                out[C::NG + k] = k < 2 * NF ? m[(k / NF) * NH + H::re(k % NF, k % NF)] : 0.0;
+    }
+}
+
+template <int NF>
+__global__ void __launch_bounds__(kBlock) k_dt_comb64(DevParams P, const double* __restrict__ comb, StepCtl* ctl,
+                                                      int mode)
+{
+    double vm = 0.0, unused = 0.0;
+    if (P.flavor_cfl_factor > 0.0) {
+        const long long stride = (long long)gridDim.x * blockDim.x;
+        for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < P.ncells; c += stride) {
+            const double* d = comb + c * kCombSlots<NF> + Comb<NF>::NG;
+            for (int i = 0; i < 2 * NF; i++) vm = fmax(vm, d[i]);
+        }
+        vm = fmax(vm, P.cell_volume * P.Ye * P.rho / kMp) * (2.0 * NF * M_SQRT2 * P.GF / P.cell_volume);
+    }
+    block_max2(vm, unused);
+    if (threadIdx.x == 0) {
+        atomicMax(&ctl->vmax_bits[1], (unsigned long long)__double_as_longlong(vm));
+        __threadfence();
+        if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            dt_finish(P, ctl, mode);
+        }
+    }
+}
+
+}  // namespace
+
+void launch_full_to_comb64(int nf, const DevParams& P, const double* full, double* comb, cudaStream_t st)
+{
+    EMU_NF_DISPATCH(nf, (k_full_to_comb64<NFv><<<reduce_grid(P.ncells * 4), kBlock, 0, st>>>(P, full, comb)));
+}
+
+void launch_dt_comb64(int nf, const DevParams& P, const double* comb, StepCtl* ctl, int mode, cudaStream_t st)
+{
+    EMU_NF_DISPATCH(nf, (k_dt_comb64<NFv><<<reduce_grid(P.ncells), kBlock, 0, st>>>(P, comb, ctl, mode)));
 }
 
 void launch_full_to_comb(int nf, const DevParams& P, const long long* qfull, long long* qcomb, cudaStream_t st)
