@@ -289,8 +289,7 @@ long long cmesh_elems(const emu_context* c) { return c->P.ncells * ((c->nf == 3 
 
 int ensure_cmesh(emu_context* ctx)
 {
-    for (int i = 0; i < 4; i++)
-        if (!ctx->cmesh[i]) CU(emu_ctx::dev_malloc(&ctx->cmesh[i], sizeof(double) * cmesh_elems(ctx)));
+    if (!ctx->cmesh) CU(emu_ctx::dev_malloc(&ctx->cmesh, sizeof(double) * 4 * cmesh_elems(ctx)));
     return EMU_OK;
 }
 
@@ -360,9 +359,9 @@ int deposit_current(emu_context* ctx)
         if ((r = check_launch(ctx, "deposit"))) return r;
         if ((r = emu_ctx::reduce_mesh(ctx, ctx->mesh[0], false, ctx->stream))) return r;
         if (ctx->steps1d) {
-            emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh[0], ctx->stream);
+            emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh, ctx->stream);
             if ((r = check_launch(ctx, "combined mesh"))) return r;
-            CU(cudaMemsetAsync(ctx->cmesh[1], 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
+            CU(cudaMemsetAsync(ctx->cmesh + cmesh_elems(ctx), 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
         }
     }
     ctx->cur_mesh = 0;
@@ -776,7 +775,7 @@ void emu_destroy(emu_context* ctx)
     if (ctx->tblock) emu_ctx::dev_free(ctx->tblock);
     if (ctx->S[0].kgen) emu_ctx::dev_free(ctx->S[0].kgen);
     for (int i = 0; i < 4; i++) if (ctx->mesh[i]) emu_ctx::dev_free(ctx->mesh[i]);
-    for (int i = 0; i < 4; i++) if (ctx->cmesh[i]) emu_ctx::dev_free(ctx->cmesh[i]);
+    if (ctx->cmesh) emu_ctx::dev_free(ctx->cmesh);
     for (int i = 0; i < 2; i++) if (ctx->qmesh[i]) emu_ctx::dev_free(ctx->qmesh[i]);
     if (ctx->qfull) emu_ctx::dev_free(ctx->qfull);
     if (ctx->qfull_part) emu_ctx::dev_free(ctx->qfull_part);
@@ -1015,7 +1014,7 @@ int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int m
         }
         emu::launch_dt_q(ctx->nf, ctx->P, ctx->qfull, nullptr, ctx->ctl, emu::DT_INIT, ctx->stream);
     }
-    else if (ctx->steps1d) emu::launch_dt_comb64(ctx->nf, ctx->P, ctx->cmesh[0], ctx->ctl, emu::DT_INIT, ctx->stream);
+    else if (ctx->steps1d) emu::launch_dt_comb64(ctx->nf, ctx->P, ctx->cmesh, ctx->ctl, emu::DT_INIT, ctx->stream);
     else emu::launch_dt(ctx->nf, ctx->P, ctx->mesh[0], ctx->ctl, emu::DT_INIT, ctx->stream);
     return check_launch(ctx, "initial compute_dt");
 }

@@ -31,9 +31,10 @@ struct emu_context {
     long long cap = 0;
     double* mesh[4] = {nullptr, nullptr, nullptr, nullptr};
     // FP64 steps on combined meshes (steps1d): M_1..M_4 in the combined
-    // layout with the diagonal slots (kCombSlots per cell); mesh[0] and
-    // mesh[3] then hold the full deposit of a load and the full stage-4 mesh
-    double* cmesh[4] = {nullptr, nullptr, nullptr, nullptr};
+    // layout with the diagonal slots (kCombSlots per cell), one after the
+    // other; mesh[0] and mesh[3] then hold the full deposit of a load and the
+    // full stage-4 mesh
+    double* cmesh = nullptr;
     long long* qmesh[2] = {nullptr, nullptr};
     // mixed path: the full 8 NF^2 mesh of the state at the last deposit
     // (the step meshes M_1..M_3 hold only the combined self-interaction

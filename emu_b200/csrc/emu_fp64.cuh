@@ -39,13 +39,17 @@ __device__ __forceinline__ void species_hamiltonian(const DevParams& P, const do
     }
 }
 
-// compute_dt without the adaptive branch from the largest diagonal number
-// (the operations of cell_potentials and dt_finish); st_dt: no limiter
+// compute_dt without the adaptive branch (the operations of cell_potentials
+// and dt_finish): the factor from a number per cell to V_stupid, and dt from
+// the largest number vmax (vacuum bound included); st_dt: no limiter
 template <int NF>
-__device__ __forceinline__ double next_dt_stupid(const DevParams& P, double vmax, int& st_dt)
+__device__ __forceinline__ double stupid_factor(const DevParams& P)
 {
-    double vs = fmax(vmax, P.cell_volume * P.Ye * P.rho / kMp);
-    vs = vs * (2.0 * NF * M_SQRT2 * P.GF / P.cell_volume) + P.vvac_max;
+    return 2.0 * NF * M_SQRT2 * P.GF / P.cell_volume;
+}
+__device__ __forceinline__ double next_dt_stupid(const DevParams& P, double vmax, double factor, int& st_dt)
+{
+    const double vs = vmax * factor + P.vvac_max;
     const double dtf = P.flavor_cfl_factor > 0.0 ? kHbar / vs * P.flavor_cfl_factor : 0.0;
     const double dtt = P.dt_translation;
     if (dtt != 0.0 && dtf != 0.0) return fmin(dtt, dtf);

@@ -7,51 +7,67 @@ namespace emu {
 namespace {
 
 // ---------------------------------------------------------------------------
-// A 1D problem of at most one wave of CTAs (128 particles each) is bound by
-// latency: the stage kernels of a graph step took 10-13 us each (2 flavors,
-// 128 cells x 80 directions: 40 us per step; 50 cells x 2 beams: 54 us), of
-// which the memory traffic accounts for well under 1 us.  Here one launch
-// takes all steps up to the next re-sort:
+// A 1D problem of at most one CTA per SM is bound by latency: the stage
+// kernels of a graph step took 10-13 us each (2 flavors, 128 cells x 80
+// directions: 40 us per step; 50 cells x 2 beams: 54 us), of which the memory
+// traffic accounts for well under 1 us.  Here one launch takes all steps up
+// to the next re-sort:
 //   - a thread pair per particle (one species each) keeps the RK state, the
 //     position and the stencil in registers; nothing but the mesh goes
-//     through memory between stages;
+//     through memory between stages.  The particles are spread evenly over
+//     the SMs (a multiple of 16 per CTA);
 //   - the stage mesh holds the combined self-interaction layout (Comb<NF>:
 //     all that a stage reads, half the values of the full mesh).  Each CTA
 //     copies its window, the cells that its particles touch, to shared
-//     memory and interpolates from there;
-//   - a warp deposits its 16 particles as a small matrix product on the FP64
-//     tensor cores (m8n8k4): window cells x particles times particles x
-//     values.  No ranking and no runs of equal stencils are needed, and a
-//     particle's weights are the sparse columns of the first factor;
+//     memory;
+//   - a warp interpolates and deposits its 16 particles as small matrix
+//     products on the FP64 tensor cores (m8n8k4): particles x cells times
+//     cells x values, and the transpose.  No ranking and no runs of equal
+//     stencils are needed, the weights are the sparse first factors, kept in
+//     registers for the four stages of a step.  (With scalar interpolation
+//     and the weights looked up per stage: 20.5 against 14.4 us per step for
+//     the two-flavor run above, 38 against 24 us for 256 cells x 92
+//     directions of three flavors.)
 //   - stages are separated by a grid barrier (measured 2350 clocks with the
 //     mesh reductions it waits for; a kernel boundary cost about the same,
-//     plus the reload of the state);
+//     plus the reload of the state).  What the next stage does not wait for
+//     (zeroing, the timestep) runs between arrival and wait;
 //   - every CTA reduces compute_dt over the stage-4 mesh by itself, so the
 //     step control needs no further exchange.
 // ONE: a problem of one CTA (at most kOneCells cells) keeps the meshes in
-// shared memory and needs no grid barrier; a warp then owns 8 x 8 tiles of
-// the mesh, whose sums are complete without reductions.
+// shared memory and needs no grid barrier: each warp leaves the rows of its
+// cells in shared memory, and a thread per mesh value adds the rows of its
+// cell (50 cells x 2 beams: 15.0 us per step when a warp owned 8 x 8 tiles of
+// the mesh and looked for their particles, 11.0 now).
+// What is left per stage (two flavors, 128 x 80, of 7200 clocks): the barrier
+// about 2500, the window's load after it 900, products and their reductions
+// 1200, the FP64 chains of the commutator, the update and Renormalize 1500.
 // ---------------------------------------------------------------------------
 constexpr int kWin = 160;        // cells of a window staged in shared memory
 constexpr int kOneCells = 128;
+constexpr int kOnePart = 128;    // particles of a one-CTA problem
+constexpr int kNarrow = 16;      // cells of a warp's particles on the matrix path
 
 template <int NF>
 struct Rec1D {
-    // w[3], cells (3 x int16 + pad), v4[4] = (1, vx, vy, vz), c[NV], diag[2 NF]
-    static constexpr int NV = Comb<NF>::NV;
-    static constexpr int W = 0, CELLS = 3, V = 4, CV = 8, DG = 8 + NV;
+    // w[3], 0, v4[4] = (1, vx, vy, vz), c[NV], diag[2 NF], first stencil cell
+    // (an int: window index, or a one-CTA problem's cell)
+    static constexpr int NV = Comb<NF>::NV, NG = Comb<NF>::NG;
+    static constexpr int W = 0, V = 4, CV = 8, DG = 8 + NV, FIRST = DG + 2 * NF;
     // (row lengths that put four particles' words into different banks)
-    static constexpr int RW = NF == 2 ? 18 : 22;
+    static constexpr int RW = NF == 2 ? 18 : 26;
     static constexpr int FW = 2 * NF * NF + 1;   // f N of both species (full deposit)
-    static_assert(DG + 2 * NF <= RW, "record");
+    static constexpr int MR = NG + 4;            // row of a staged mesh
+    static_assert(FIRST < RW, "record");
 };
 
 template <int NF, bool ONE>
-constexpr int steps1d_smem()
+int steps1d_smem(int npart)
 {
     using R = Rec1D<NF>;
-    constexpr int mesh = ONE ? kOneCells * (2 * Comb<NF>::NG + kDiagSlots) : kWin * Comb<NF>::NG;
-    return 8 * (mesh + kBlock * (R::RW + R::FW));
+    const int mesh = ONE ? 2 * kOneCells * R::MR + kOneCells * kDiagSlots + (kOnePart + 1) * kCombSlots<NF>
+                         : (kWin + 4) * R::MR;
+    return 8 * (mesh + npart * (R::RW + R::FW));
 }
 
 // values of a deposit: the combined layout, the diagonal slots, the full one
@@ -74,110 +90,101 @@ __device__ __forceinline__ double dep_value(const double* rec, const double* fn,
     else if constexpr (D == DEP_DIAG) return q < 2 * NF ? rec[R::DG + (q < 2 * NF ? q : 0)] : 0.0;
     else return fn[q % (2 * NF * NF)] * rec[R::V + q / (2 * NF * NF)];
 }
+// the weight of a particle on window cell `cell` (its stencil starts at its
+// first cell; weights past the stencil's width are zero)
+template <int NF>
 __device__ __forceinline__ double dep_weight(const double* rec, int cell)
 {
-    const int2 c = *reinterpret_cast<const int2*>(rec + 3);
-    const int c0 = (short)(c.x & 0xffff), c1 = (short)(c.x >> 16), c2 = (short)(c.y & 0xffff);
-    return (c0 == cell ? rec[0] : 0.0) + (c1 == cell ? rec[1] : 0.0) + (c2 == cell ? rec[2] : 0.0);
+    const unsigned i = (unsigned)(cell - *reinterpret_cast<const int*>(rec + Rec1D<NF>::FIRST));
+    return rec[i < 3u ? i : 3u];
+}
+// on cell `cell` of nz periodic cells
+template <int NF>
+__device__ __forceinline__ double dep_weight_periodic(const double* rec, int cell, int nz)
+{
+    int i = cell - *reinterpret_cast<const int*>(rec + Rec1D<NF>::FIRST);
+    if (i < 0) i += nz;
+    double w = 0.0;
+    for (; i < 3; i += nz) w += rec[i];
+    return w;
 }
 
-// the warp's own 16 particles (records r0..r0+15) into the global mesh
+// the warp's own 16 particles (records r0..r0+15) into the global mesh:
+// particles spread over any range [lo, hi] of window cells
 template <int NF, int D>
-__device__ __forceinline__ void deposit_warp(const DevParams& P, double* mesh, const double* srec, const double* sfn,
-                                             int r0, int klo, int khi, int c0)
+__device__ __noinline__ void deposit_spread(int nz, double* mesh, const double* srec, const double* sfn, int r0,
+                                            int lo, int hi, int c0)
 {
     using R = Rec1D<NF>;
     constexpr int NT = DepN<NF, D>::NT;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3;
-    const int lo = __reduce_min_sync(kFull, klo), hi = __reduce_max_sync(kFull, khi);
-    if (hi < 0) return;   // no particle in this warp
-    const double* rec[4];
-    const double* fn[4];
-    int kl[4], kh[4];
+    for (int base = lo; base <= hi; base += 8) {
+        double a[4];
+        bool any = false;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        rec[k] = srec + (r0 + 4 * k + col) * R::RW;
-        fn[k] = sfn + (r0 + 4 * k + col) * R::FW;
-        kl[k] = __shfl_sync(kFull, klo, 8 * k);
-        kh[k] = __shfl_sync(kFull, khi, 8 * k);
-    }
-    for (int mt = lo >> 3; mt <= hi >> 3; mt++) {
-        const int wl = 8 * mt + row;
-        // (six tiles at a time: the full layout of three flavors has nine)
-        constexpr int G = NT > 5 ? 3 : NT;
-#pragma unroll 1
-        for (int g = 0; g < NT; g += G) {
-            double acc[G][2];
-#pragma unroll
-            for (int i = 0; i < G; i++) acc[i][0] = acc[i][1] = 0.0;
+        for (int k = 0; k < 4; k++) {
+            a[k] = dep_weight<NF>(srec + (r0 + 4 * k + col) * R::RW, base + row);
+            any = any || a[k] != 0.0;
+        }
+        if (!__any_sync(kFull, any)) continue;
+        const int cell = (c0 + base + row) % nz;
+        double* m = mesh + (long long)cell * DepN<NF, D>::STRIDE + DepN<NF, D>::OFF;
+        for (int nt = 0; nt < NT; nt++) {
+            double x = 0.0, y = 0.0;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                if (kh[k] < 8 * mt || kl[k] > 8 * mt + 7) continue;   // (uniform)
-                const double a = dep_weight(rec[k], wl);
-#pragma unroll
-                for (int i = 0; i < G; i++) dmma(acc[i][0], acc[i][1], a, dep_value<NF, D>(rec[k], fn[k], g + i, row));
+                const int i = r0 + 4 * k + col;
+                dmma(x, y, a[k], dep_value<NF, D>(srec + i * R::RW, sfn + i * R::FW, nt, row));
             }
-            int cell = c0 + wl;
-            cell = cell % P.n[2];
-            if (cell < 0) cell += P.n[2];
-            double* m = mesh + (long long)cell * DepN<NF, D>::STRIDE + DepN<NF, D>::OFF;
-#pragma unroll
-            for (int i = 0; i < G; i++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int q = 8 * (g + i) + col + 4 * h;
-                    if (acc[i][h] != 0.0) atomic_add_mesh(m + q, acc[i][h]);
-                }
+            if (x != 0.0) atomic_add_mesh(m + 8 * nt + col, x);
+            if (y != 0.0) atomic_add_mesh(m + 8 * nt + col + 4, y);
         }
     }
 }
 
 // ONE: mesh tiles (8 cells x 8 values) summed over all particles by one warp
-// each and stored: mesh[cell * stride + q]
+// each and stored: mesh[cell * stride + q] (particles in any order; the full
+// layout of a run's last step, and warps that are not narrow)
 template <int NF, int D>
-__device__ __forceinline__ void deposit_tiles(int ncells, double* mesh, int stride, const double* srec,
-                                              const double* sfn, const int2* krange)
+__device__ __noinline__ void deposit_tiles(int ncells, double* mesh, int stride, const double* srec,
+                                           const double* sfn)
 {
     using R = Rec1D<NF>;
     constexpr int NT = DepN<NF, D>::NT;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3, w = threadIdx.x >> 5;
-    const int nmt = (ncells + 7) >> 3;
-    const int2 kr = krange[lane];
-    for (int tile = w; tile < nmt * NT; tile += 2 * kBlock / 32) {
+    const int nmt = (ncells + 7) >> 3, nwarps = blockDim.x >> 5;
+    for (int tile = w; tile < nmt * NT; tile += nwarps) {
         const int mt = tile / NT, nt = tile - mt * NT;
-        unsigned todo = __ballot_sync(kFull, kr.y >= 8 * mt && kr.x <= 8 * mt + 7);
-        double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-        while (todo) {
-            const int k = __ffs(todo) - 1;
-            todo &= todo - 1;
+        double x = 0.0, y = 0.0;
+        for (int k = 0; k < kOnePart / 4; k++) {
             const double* r = srec + (4 * k + col) * R::RW;
-            dmma(a0, a1, dep_weight(r, 8 * mt + row), dep_value<NF, D>(r, sfn + (4 * k + col) * R::FW, nt, row));
-            if (todo) {   // (two chains)
-                const int k2 = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const double* r2 = srec + (4 * k2 + col) * R::RW;
-                dmma(b0, b1, dep_weight(r2, 8 * mt + row), dep_value<NF, D>(r2, sfn + (4 * k2 + col) * R::FW, nt, row));
-            }
+            const double a = dep_weight_periodic<NF>(r, 8 * mt + row, ncells);
+            if (__any_sync(kFull, a != 0.0))
+                dmma(x, y, a, dep_value<NF, D>(r, sfn + (4 * k + col) * R::FW, nt, row));
         }
         const int cell = 8 * mt + row;
         if (cell < ncells) {
             double* m = mesh + cell * stride + 8 * nt + col;
-            m[0] = a0 + b0;
-            m[4] = a1 + b1;
+            m[0] = x;
+            m[4] = y;
         }
     }
 }
 
-// grid barrier: arrivals counted up from 0 over the launch (the last CTA to
-// leave the kernel sets the count back).  The wait is bounded; false: it gave
-// up (ST_TIMEOUT is set, the CTA leaves the kernel).
-__device__ __forceinline__ bool steps_barrier(StepCtl* ctl, unsigned target)
+// Grid barrier in two halves: arrivals counted up from 0 over the launch (the
+// last CTA to leave the kernel sets the count back).  The wait is bounded;
+// false: it gave up (ST_TIMEOUT is set, the CTA leaves the kernel).
+__device__ __forceinline__ void steps_arrive(StepCtl* ctl)
+{
+    __syncthreads();
+    if (threadIdx.x == 0)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
+}
+__device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target)
 {
     __shared__ int ok;
-    __syncthreads();
     if (threadIdx.x == 0) {
         int good = 1;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
         unsigned v;
         long long it = 0;
         for (;;) {
@@ -195,26 +202,32 @@ __device__ __forceinline__ bool steps_barrier(StepCtl* ctl, unsigned target)
     return ok != 0;
 }
 
-struct Meshes4 {
-    double* m[4];   // combined meshes, kCombSlots per cell: M_1, M_2, M_3, M_4
-};
-
-template <int NF, bool ONE>
-__global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
-    k_steps_1d(DevParams P, DevState S, Meshes4 M, double* __restrict__ full, StepCtl* ctl, int nsteps, int dt_mode)
+// cmesh: four combined meshes (kCombSlots per cell) one after the other, M_1
+// to M_4.  npart particles per CTA (a multiple of 16), 2 npart threads.
+template <int NF, bool ONE, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_steps_1d(DevParams P, DevState S, double* __restrict__ cmesh, double* __restrict__ full, StepCtl* ctl,
+               int npart, int nsteps, int dt_mode)
 {
     using H = Herm<NF>;
     using C = Comb<NF>;
     using R = Rec1D<NF>;
     constexpr int NH = NF * NF, NV = C::NV, NG = C::NG, NCS = kCombSlots<NF>, ND = 8 * NH, HV = NV / 2;
+    constexpr int NT = NG / 8, MR = R::MR, KI = kNarrow / 4;
     extern __shared__ __align__(16) double smem[];
-    double* const smesh = smem;                                              // ONE: [2][cells][NG], [cells][8]
-    double* const srec = smem + (ONE ? kOneCells * (2 * NG + kDiagSlots) : kWin * NG);
-    double* const sfn = srec + kBlock * R::RW;
-    double* const sdiag = smesh + 2 * kOneCells * NG;                        // (ONE)
-    __shared__ int2 krange[32];
-    __shared__ int swin[2][8];
-    __shared__ double sred[8];
+    double* const smesh = smem;                                  // ONE: two meshes, then the diagonal slots
+    constexpr int kHalf = kOneCells * MR;
+    double* const sdiag = smesh + 2 * kHalf;                     // (ONE)
+    double* const spart = sdiag + kOneCells * kDiagSlots;        // (ONE) 16 rows of a mesh per warp
+    double* const srec = ONE ? spart + (kOnePart + 1) * NCS : smesh + (kWin + 4) * MR;
+    double* const sfn = srec + npart * R::RW;
+    __shared__ int2 srange[2 * kOnePart / 32];                   // (ONE) first cell and cells of each warp
+    // (ONE) the rows of spart that hold parts of a cell's sums: their count,
+    // the first four (row kOnePart: zeros)
+    __shared__ int scount[ONE ? kOneCells : 1];
+    __shared__ __align__(4) unsigned char srows[ONE ? kOneCells : 1][4];
+    __shared__ int swin[2][16];
+    __shared__ double sred[16];
     __shared__ int sref;
 
     if (ctl->done) return;
@@ -224,13 +237,15 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
     const int max_step = ctl->max_step, full_from = ctl->m4_full_from;
     double* const hist = ctl->dt_hist;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int row = lane >> 2, col = lane & 3;
     const int pl = tid >> 1, sp = tid & 1;
-    const long long p = (long long)blockIdx.x * kBlock + pl;
+    const long long p = (long long)blockIdx.x * npart + pl;
     const bool active = p < S.n;
     const long long cap = S.cap;
     const int nz = P.n[2], ncells = (int)P.ncells;
     const int nthreads = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + tid;
+    const int msize = ncells * NCS;
 
     // the particle (both threads of its pair), this thread's species
     double x = 0, y = 0, z = 0, tp = 0, v[3] = {0, 0, 0}, vs = 0, Ns = 0, Ls = 1;
@@ -249,183 +264,233 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
         for (int e = 0; e < NH; e++) f[e] = y0[e] = S.f0[(sp * NH + e) * cap + p];
     }
     double* const rec = srec + pl * R::RW;
+    double* const wrec = srec + warp * 16 * R::RW;   // the warp's 16 records
     if (sp == 0) {
-        rec[R::V] = active ? 1.0 : 0.0;
+        rec[3] = 0.0;
+        rec[R::V] = 1.0;
 #pragma unroll
         for (int d = 0; d < 3; d++) rec[R::V + 1 + d] = v[d];
     }
     if constexpr (ONE) {
-        for (int i = tid; i < ncells * NG; i += blockDim.x)
-            smesh[i] = M.m[0][(long long)(i / NG) * NCS + i % NG];
+        for (int i = tid; i < kHalf; i += blockDim.x) {
+            const int c = i / MR, q = i - c * MR;
+            if (c < ncells && q < NG) smesh[i] = cmesh[c * NCS + q];
+        }
+        if (tid < NCS) spart[kOnePart * NCS + tid] = 0.0;
+    } else {
+        // (M_2's mesh is clean at a step boundary)
+        for (int i = gtid; i < msize; i += nthreads) cmesh[2 * msize + i] = 0.0;
     }
     int c0 = 0, win = 0;        // window: cells c0 .. c0 + win - 1 (wrapped)
     bool wide = false;          // the window exceeds the staging area
-    int ci[3] = {0, 0, 0};      // stencil cells (window index; wide, ONE: cell)
+    int ci0 = 0;                // first stencil cell (window index; wide, ONE: cell)
     double wz[3] = {0, 0, 0};
-    int klo = 0, khi = -1;      // cells that this lane group's four particles touch
-    unsigned nbar = 0;
-    int cur = 0;                // ONE: which half of smesh holds the stage mesh
+    int wlo = 0, whi = -1;      // window cells that the warp's particles touch
+    bool narrow = false;        // at most kNarrow of them: the matrix path (ONE: in every warp)
+    double ai[2][KI], ad[2][4]; // its weights: interpolation, deposit
+    int mrow_of[KI] = {};       // (ONE) mesh rows of the interpolation's cells
+    int gcell[2] = {0, 0};      // deposit rows: mesh offset of cell wlo + 8 i + row
 
-    // stencil, window and the weight part of the record, at the position z
+    // r in [-nz/2, nz/2) of cell c relative to cell ref
+    auto relative = [&](int c, int ref) {
+        const int half = nz >> 1;
+        int r = c - ref + half;
+        if (r < 0) r += nz;
+        if (r >= nz) r -= nz;
+        return r - half;
+    };
+    // stencil, window, weights and the weight part of the record, at the
+    // position z
     auto locate = [&]() {
         int first = 0;
         if (active) {
             shape<double>(z * P.dxi[2], P.ord[2], first, wz);
             first = wrapi(first, nz);
         }
+        int r = 0;
         if constexpr (!ONE) {
-            if (tid == 0) sref = first;   // (thread 0's particle exists)
-            __syncthreads();
-            // cells relative to the first particle's, in [-nz/2, nz/2)
-            const int half = nz >> 1;
-            int r = first - sref + half;
-            if (r < 0) r += nz;
-            if (r >= nz) r -= nz;
-            r -= half;
+            // relative to the first particle's cell at the launch
+            r = relative(first, sref);
             const int mn = __reduce_min_sync(kFull, active ? r : INT_MAX);
             const int mx = __reduce_max_sync(kFull, active ? r : INT_MIN);
             if (lane == 0) { swin[0][warp] = mn; swin[1][warp] = mx; }
             __syncthreads();
-            int lo = swin[0][0], hi = swin[1][0];
-#pragma unroll
-            for (int w = 1; w < 8; w++) {
-                lo = min(lo, swin[0][w]);
-                hi = max(hi, swin[1][w]);
-            }
+            const int lo = __reduce_min_sync(kFull, swin[0][lane < nwarps ? lane : 0]);
+            const int hi = __reduce_max_sync(kFull, swin[1][lane < nwarps ? lane : 0]);
             c0 = sref + lo;
             if (c0 < 0) c0 += nz;
             if (c0 >= nz) c0 -= nz;
             win = hi - lo + P.w[2];
             wide = win > kWin;
-            ci[0] = wide ? first : r - lo;
+            r -= lo;
+            ci0 = wide ? first : r;
+            wlo = mn - lo;
+            whi = mx - lo + P.w[2] - 1;
+            narrow = !wide && mx >= mn && whi - wlo < kNarrow;
         } else {
-            ci[0] = first;
-        }
+            // relative to the warp's first cell
+            const int ref = __shfl_sync(kFull, first, 0);
+            r = relative(first, ref);
+            wlo = __reduce_min_sync(kFull, active ? r : INT_MAX);
+            whi = __reduce_max_sync(kFull, active ? r : INT_MIN) + P.w[2] - 1;
+            const bool any = __any_sync(kFull, active);
+            narrow = !any || whi - wlo < kNarrow;
+            if (tid < kOneCells) {
+                scount[tid] = 0;
+                *reinterpret_cast<unsigned*>(srows[tid]) = 0x01010101u * kOnePart;
+            }
+            narrow = __syncthreads_and(narrow);
+            if (!any) { wlo = 0; whi = -1; }
+            c0 = wrapi(ref + wlo, nz);
+            r -= wlo;
+            whi -= wlo;
+            wlo = 0;
+            ci0 = first;
+            if (lane == 0) srange[warp] = make_int2(c0, whi + 1);
+            if (narrow && lane <= whi) {
+                const int c = (c0 + lane) % nz, k = atomicAdd(&scount[c], 1);
+                if (k < 4) srows[c][k] = (unsigned char)(warp * 16 + lane);
+            }
 #pragma unroll
-        for (int i = 1; i < 3; i++) {
-            int c = ci[0] + i;
-            if (ONE || wide) c = c >= nz ? c % nz : c;
-            ci[i] = i < P.w[2] ? c : ci[0];
-        }
-        // the range of each group of four particles (eight lanes)
-        int a = min(ci[0], min(ci[1], ci[2])), b = max(ci[0], max(ci[1], ci[2]));
-        if (!active) { a = INT_MAX; b = -1; }
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            a = min(a, __shfl_xor_sync(kFull, a, o));
-            b = max(b, __shfl_xor_sync(kFull, b, o));
-        }
-        klo = a;
-        khi = b;
-        if constexpr (ONE) {
-            if ((lane & 7) == 0) krange[tid >> 3] = make_int2(a, b);
+            for (int k = 0; k < KI; k++) mrow_of[k] = (c0 + 4 * k + col) % nz * MR;
         }
         if (sp == 0) {
 #pragma unroll
             for (int i = 0; i < 3; i++) rec[R::W + i] = wz[i];
-            *reinterpret_cast<int2*>(rec + R::CELLS) =
-                make_int2((ci[0] & 0xffff) | (ci[1] << 16), ci[2] & 0xffff);
+            *reinterpret_cast<int*>(rec + R::FIRST) = narrow ? r : ci0;
+        }
+        __syncwarp();
+        if (narrow) {
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+#pragma unroll
+                for (int k = 0; k < KI; k++) ai[m][k] = dep_weight<NF>(wrec + (8 * m + row) * R::RW, wlo + 4 * k + col);
+#pragma unroll
+                for (int k = 0; k < 4; k++) ad[m][k] = dep_weight<NF>(wrec + (4 * k + col) * R::RW, wlo + 8 * m + row);
+                if constexpr (!ONE) {
+                    int c = c0 + wlo + 8 * m + row;
+                    c = c >= nz ? c % nz : c;
+                    gcell[m] = c * NCS;
+                }
+            }
         }
     };
+    if constexpr (!ONE) {
+        if (tid == 0) {   // (the CTA's first particle exists)
+            int first;
+            shape<double>(z * P.dxi[2], P.ord[2], first, wz);
+            sref = wrapi(first, nz);
+        }
+    }
+    __syncthreads();
     locate();
+    const double dt_fac = stupid_factor<NF>(P), dt_vmin = P.cell_volume * P.Ye * P.rho / kMp;
     bool alive = true;
+    unsigned nbar = 0;
+    int cur = 0;   // ONE: which half of smesh holds the stage mesh
 
     for (int it = 0; it < nsteps && alive; it++) {
         if (hist && gtid == 0) hist[step] = dt;
         const bool want_full = step >= full_from || last || step + 1 >= max_step;
-        const bool final_step = it + 1 == nsteps;   // (or the run ends: see below)
+        const bool final_step = it + 1 == nsteps;
         double dt_next = dt, t_next = t_run;
         int last_next = last, step_next = step;
 #pragma unroll 1
         for (int s = 1; s <= 4; s++) {
-            double* const min_ = M.m[s - 1];
-            double* const mout = M.m[s & 3];
+            const double* const mesh_in = cmesh + (s - 1) * msize;
+            double* const mesh_out = cmesh + (s & 3) * msize;
             const double* mrow = smesh;
             if constexpr (!ONE) {
-                // the mesh deposited two stages on, and the full mesh
-                double* mz = M.m[(s + 1) & 3];
-                for (int i = gtid; i < ncells * NCS; i += nthreads) mz[i] = 0.0;
-                if (s == 1 && want_full)
-                    for (int i = gtid; i < ncells * ND; i += nthreads) full[i] = 0.0;
+                // M_4's mesh: here, since a CTA may still read the last
+                // step's for its timestep until it arrives at barrier 1
+                if (s == 2)
+                    for (int i = gtid; i < msize; i += nthreads) cmesh[3 * msize + i] = 0.0;
                 if (!wide) {
-                    for (int i = tid; i < win * (NG / 2); i += blockDim.x) {
-                        int c = c0 + i / (NG / 2);
+                    // (four further rows of zeros: the last product's depth)
+                    for (int i = tid; i < (win + 4) * (NG / 2); i += blockDim.x) {
+                        const int wl = i / (NG / 2), q = i - wl * (NG / 2);
+                        int c = c0 + wl;
                         c = c >= nz ? c % nz : c;
-                        reinterpret_cast<double2*>(smesh)[i] =
-                            __ldcg(reinterpret_cast<const double2*>(min_ + (long long)c * NCS) + i % (NG / 2));
+                        double2 t2 = make_double2(0.0, 0.0);
+                        if (wl < win) t2 = __ldcg(reinterpret_cast<const double2*>(mesh_in + c * NCS) + q);
+                        *reinterpret_cast<double2*>(smesh + wl * MR + 2 * q) = t2;
                     }
+                }
+                __syncthreads();
+            } else {
+                mrow = smesh + cur * kHalf;
+            }
+            // interpolation: u_j = G_0j - v . G_dj of the pair's particle
+            double hv[NV];
+            if (narrow) {
+                double g[2][NT][2];
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int nt = 0; nt < NT; nt++) g[m][nt][0] = g[m][nt][1] = 0.0;
+#pragma unroll
+                for (int k = 0; k < KI; k++) {
+                    if (wlo + 4 * k > whi) break;   // (uniform)
+                    const double* b = mrow + (ONE ? mrow_of[k] : (wlo + 4 * k + col) * MR);
+#pragma unroll
+                    for (int nt = 0; nt < NT; nt++) {
+                        // two flavors: column 2 e + i holds d = 2 nt + i of
+                        // value e, so that a lane's two columns are one value
+                        const double bv = b[NF == 2 ? (2 * nt + (row & 1)) * NV + (row >> 1) : nt * NV + row];
+#pragma unroll
+                        for (int m = 0; m < 2; m++) dmma(g[m][nt][0], g[m][nt][1], ai[m][k], bv);
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    double* r = wrec + (8 * m + row) * R::RW;
+                    const double vx = r[R::V + 1], vy = r[R::V + 2], vz = r[R::V + 3];
+                    if constexpr (NF == 2) {
+                        r[R::CV + col] = ((g[m][0][0] - vx * g[m][0][1]) - vy * g[m][1][0]) - vz * g[m][1][1];
+                    } else {
+                        double2 t2;
+                        t2.x = ((g[m][0][0] - vx * g[m][1][0]) - vy * g[m][2][0]) - vz * g[m][3][0];
+                        t2.y = ((g[m][0][1] - vx * g[m][1][1]) - vy * g[m][2][1]) - vz * g[m][3][1];
+                        *reinterpret_cast<double2*>(r + R::CV + 2 * col) = t2;
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < NV; j += 2) {
+                    const double2 t2 = *reinterpret_cast<const double2*>(rec + R::CV + j);
+                    hv[j] = t2.x;
+                    hv[j + 1] = t2.y;
                 }
             } else {
-                mrow = smesh + cur * kOneCells * NG;
-            }
-            if (s == 4 && dt_mode == DT_ADVANCE) {
-                // compute_dt on the stage-4 mesh (Evolve.cpp:22-89 with
-                // max_adaptive_speedup <= 1: V_stupid of the diagonal)
-                double vm = 0.0;
-                if (P.flavor_cfl_factor > 0.0)
-                    for (int c = tid; c < ncells; c += blockDim.x) {
-                        const double* dg = ONE ? sdiag + c * kDiagSlots : min_ + (long long)c * NCS + NG;
+                double u[HV];
 #pragma unroll
-                        for (int i = 0; i < 2 * NF; i++) vm = fmax(vm, ONE ? dg[i] : __ldcg(dg + i));
-                    }
+                for (int j = 0; j < HV; j++) u[j] = 0.0;
+                if (active) {
+#pragma unroll 1
+                    for (int i = 0; i < P.w[2]; i++) {
+                        int cc = ci0 + i;
+                        if (ONE || wide) cc = cc % nz;
+                        const double wi = i == 0 ? wz[0] : i == 1 ? wz[1] : wz[2];
 #pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) vm = fmax(vm, __shfl_xor_sync(kFull, vm, o));
-                if (lane == 0) sred[warp] = vm;
-            }
-            __syncthreads();
-            if (s == 4 && dt_mode == DT_ADVANCE) {
-                double vm = sred[0];
+                        for (int j = 0; j < HV; j++) {
+                            double g[4];
 #pragma unroll
-                for (int w = 1; w < 8; w++) vm = fmax(vm, sred[w]);
-                dt_next = next_dt_stupid<NF>(P, vm, st_dt);
-                t_next = t_run + dt;
-                step_next = step + 1;
-                if (last || step_next >= max_step) done = 1;
-                if (end_time - t_next < dt_next) {
-                    dt_next = end_time - t_next;
-                    last_next = 1;
-                }
-                if (st_dt) done = 1;
-            }
-            // interpolation: this thread's half of the NV values
-            double u[HV];
-#pragma unroll
-            for (int j = 0; j < HV; j++) u[j] = 0.0;
-            if (active) {
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    double g[4][HV];
-                    if (!ONE && wide) {
-#pragma unroll
-                        for (int d = 0; d < 4; d++)
-#pragma unroll
-                            for (int j = 0; j < HV; j++)
-                                g[d][j] = __ldcg(min_ + (long long)ci[i] * NCS + d * NV + sp * HV + j);
-                    } else {
-#pragma unroll
-                        for (int d = 0; d < 4; d++)
-#pragma unroll
-                            for (int j = 0; j < HV; j += 2) {
-                                const double2 t2 = *reinterpret_cast<const double2*>(mrow + ci[i] * NG + d * NV +
-                                                                                     sp * HV + j);
-                                g[d][j] = t2.x;
-                                g[d][j + 1] = t2.y;
-                            }
-                    }
-#pragma unroll
-                    for (int j = 0; j < HV; j++) {
-                        const double a = ((g[0][j] - g[1][j] * v[0]) - g[2][j] * v[1]) - g[3][j] * v[2];
-                        u[j] += wz[i] * a;
+                            for (int d = 0; d < 4; d++)
+                                g[d] = !ONE && wide ? __ldcg(mesh_in + cc * NCS + d * NV + sp * HV + j)
+                                                    : mrow[cc * MR + d * NV + sp * HV + j];
+                            u[j] += wi * (((g[0] - g[1] * v[0]) - g[2] * v[1]) - g[3] * v[2]);
+                        }
                     }
                 }
-            }
-            double hv[NV];
 #pragma unroll
-            for (int j = 0; j < HV; j++) {
-                const double own = u[j] * P.sqrt2GF_inv_vol, other = __shfl_xor_sync(kFull, own, 1);
-                hv[j] = sp == 0 ? own : other;
-                hv[HV + j] = sp == 0 ? other : own;
+                for (int j = 0; j < HV; j++) {
+                    const double other = __shfl_xor_sync(kFull, u[j], 1);
+                    hv[j] = sp == 0 ? u[j] : other;
+                    hv[HV + j] = sp == 0 ? other : u[j];
+                }
             }
+#pragma unroll
+            for (int j = 0; j < NV; j++) hv[j] *= P.sqrt2GF_inv_vol;
             double h[NH], K[NH];
             C::hermitian(hv, h);
             species_hamiltonian<NF>(P, h, vs, sp, h);
@@ -447,7 +512,7 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
                     // (the reference's order: four contributions per step)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        const double w = dt * kRK4B[i];
+                        const double w = dt * (i == 0 || i == 3 ? 1. / 6. : 1. / 3.);
                         x = __dadd_rn(__dmul_rn(w, v[0] * kC), x);
                         y = __dadd_rn(__dmul_rn(w, v[1] * kC), y);
                         z = __dadd_rn(__dmul_rn(w, v[2] * kC), z);
@@ -459,79 +524,218 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
                 }
 #pragma unroll
                 for (int e = 0; e < NH; e++) y0[e] = f[e];
-                __syncthreads();   // (every thread has read this stage's window)
+                __syncwarp();
                 locate();
             }
             // the record: the NV combined values (each thread of the pair
             // half of them), and the species' diagonal and f N where wanted
-            double fN[NH], fo[NH], cc[NH], cv[NV];
-#pragma unroll
-            for (int e = 0; e < NH; e++) {
-                fN[e] = f[e] * Ns;
-                fo[e] = __shfl_xor_sync(kFull, fN[e], 1);
-            }
-#pragma unroll
-            for (int e = 0; e < NH; e++) {
-                const double a = sp == 0 ? fN[e] : fo[e], b = sp == 0 ? fo[e] : fN[e];
-                cc[e] = H::is_im(e) ? a + b : a - b;
-            }
-            C::values(cc, cv);
-#pragma unroll
-            for (int j = 0; j < HV; j++) rec[R::CV + sp * HV + j] = sp == 0 ? cv[j] : cv[HV + j];
-            const bool diag = s == 3 || s == 4;
+            const bool diag = s >= 3;
             const bool fdep = s == 3 && want_full;
-            if (diag) {
+            {
+                double fN[NH], cc[NH], cv[NV];
 #pragma unroll
-                for (int i = 0; i < NF; i++) rec[R::DG + sp * NF + i] = fN[H::re(i, i)];
-            }
-            if (fdep) {
+                for (int e = 0; e < NH; e++) fN[e] = f[e] * Ns;
 #pragma unroll
-                for (int e = 0; e < NH; e++) sfn[pl * R::FW + sp * NH + e] = fN[e];
+                for (int e = 0; e < NH; e++) {
+                    const double o = __shfl_xor_sync(kFull, fN[e], 1);
+                    cc[e] = H::is_im(e) ? fN[e] + o : (sp == 0 ? fN[e] - o : o - fN[e]);
+                }
+                C::values(cc, cv);
+                __syncwarp();   // (the pair's reads of the interpolated values)
+#pragma unroll
+                for (int j = 0; j < HV; j++) rec[R::CV + sp * HV + j] = sp == 0 ? cv[j] : cv[HV + j];
+                if (diag) {
+#pragma unroll
+                    for (int i = 0; i < NF; i++) rec[R::DG + sp * NF + i] = fN[H::re(i, i)];
+                }
+                if (fdep) {
+#pragma unroll
+                    for (int e = 0; e < NH; e++) sfn[pl * R::FW + sp * NH + e] = fN[e];
+                }
             }
-            if constexpr (ONE) {
-                __syncthreads();
-                double* const out = smesh + (1 - cur) * kOneCells * NG;
-                deposit_tiles<NF, DEP_COMB>(ncells, out, NG, srec, sfn, krange);
-                if (diag) deposit_tiles<NF, DEP_DIAG>(ncells, sdiag, kDiagSlots, srec, sfn, krange);
-                if (fdep) deposit_tiles<NF, DEP_FULL>(ncells, full, ND, srec, sfn, krange);
-                cur = 1 - cur;
-                // (the barrier at the head of the next stage follows)
-            } else if (!wide) {
+            if (narrow) {
                 __syncwarp();   // (a warp reads only its own records)
-                const int r0 = warp * 16;
-                deposit_warp<NF, DEP_COMB>(P, mout, srec, sfn, r0, klo, khi, c0);
-                if (diag) deposit_warp<NF, DEP_DIAG>(P, mout, srec, sfn, r0, klo, khi, c0);
-                if (fdep) deposit_warp<NF, DEP_FULL>(P, full, srec, sfn, r0, klo, khi, c0);
-            } else if (active) {
-#pragma unroll 1
-                for (int i = 0; i < P.w[2]; i++) {
-                    double* m = mout + (long long)ci[i] * NCS;
+                double cval[4];
+                const int q0 = (row >> 1) + 4 * (row & 1);
 #pragma unroll
-                    for (int d = 0; d < 4; d++) {
-                        const double wd = d == 0 ? wz[i] : wz[i] * v[d - 1];
+                for (int k = 0; k < 4; k++) cval[k] = wrec[(4 * k + col) * R::RW + R::CV + q0 % NV];
 #pragma unroll
-                        for (int j = 0; j < HV; j++)
-                            atomic_add_mesh(m + d * NV + sp * HV + j, wd * (sp == 0 ? cv[j] : cv[HV + j]));
-                        if (fdep) {
+                for (int m = 0; m < 2; m++) {
+                    if (wlo + 8 * m > whi) break;   // (uniform)
+                    double g[NT][2], gd[2] = {0.0, 0.0};
 #pragma unroll
-                            for (int e = 0; e < NH; e++)
-                                atomic_add_mesh(full + (long long)ci[i] * ND + (2 * d + sp) * NH + e, wd * fN[e]);
+                    for (int nt = 0; nt < NT; nt++) g[nt][0] = g[nt][1] = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const double* r = wrec + (4 * k + col) * R::RW;
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++) {
+                            const int d = (8 * nt + q0) / NV;
+                            dmma(g[nt][0], g[nt][1], ad[m][k], cval[k] * r[R::V + d]);
+                        }
+                        if (diag) dmma(gd[0], gd[1], ad[m][k], q0 < 2 * NF ? r[R::DG + (q0 < 2 * NF ? q0 : 0)] : 0.0);
+                    }
+                    if constexpr (ONE) {
+                        // the warp's rows, summed over the warps below
+                        double* o = spart + (warp * 16 + 8 * m + row) * NCS + col;
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++) {
+                            o[8 * nt] = g[nt][0];
+                            o[8 * nt + 4] = g[nt][1];
+                        }
+                        if (diag) {
+                            o[NG] = gd[0];
+                            o[NG + 4] = gd[1];
+                        }
+                    } else if (wlo + 8 * m + row <= whi) {
+                        double* o = mesh_out + gcell[m] + col;
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++) {
+                            atomic_add_mesh(o + 8 * nt, g[nt][0]);
+                            atomic_add_mesh(o + 8 * nt + 4, g[nt][1]);
+                        }
+                        if (diag) {
+                            atomic_add_mesh(o + NG, gd[0]);
+                            if (NF == 3 && col < 2) atomic_add_mesh(o + NG + 4, gd[1]);
                         }
                     }
-                    if (diag) {
+                }
+            }
+            if constexpr (ONE) {
+                double* const out = smesh + (1 - cur) * kHalf;
+                __syncthreads();
+                if (narrow) {
+                    const int nq = diag ? NCS : NG;
+                    for (int i = tid; i < ncells * nq; i += blockDim.x) {
+                        const int c = diag ? i / NCS : i / NG, q = i - c * nq;
+                        const uchar4 r4 = *reinterpret_cast<const uchar4*>(srows[c]);
+                        double t2 = (spart[r4.x * NCS + q] + spart[r4.y * NCS + q]) +
+                                    (spart[r4.z * NCS + q] + spart[r4.w * NCS + q]);
+                        if (scount[c] > 4) {
+                            t2 = 0.0;
+                            for (int w = 0; w < 2 * kOnePart / 32; w++) {
+                                const int2 rg = srange[w];
+                                int k = c - rg.x;
+                                if (k < 0) k += nz;
+                                for (; k < rg.y; k += nz) t2 += spart[(w * 16 + k) * NCS + q];
+                            }
+                        }
+                        if (q < NG) out[c * MR + q] = t2;
+                        else sdiag[c * kDiagSlots + q - NG] = t2;
+                    }
+                } else {
+                    deposit_tiles<NF, DEP_COMB>(ncells, out, MR, srec, sfn);
+                    if (diag) deposit_tiles<NF, DEP_DIAG>(ncells, sdiag, kDiagSlots, srec, sfn);
+                }
+                if (fdep) {
+                    // (cells in place of rows relative to the warp's first)
+                    if (narrow) {
+                        __syncthreads();
+                        if (sp == 0) *reinterpret_cast<int*>(rec + R::FIRST) = ci0;
+                        __syncthreads();
+                    }
+                    deposit_tiles<NF, DEP_FULL>(ncells, full, ND, srec, sfn);
+                }
+                cur = 1 - cur;
+                if (s == 3 && dt_mode == DT_ADVANCE) {
+                    // the largest diagonal number, for the next step's dt
+                    __syncthreads();
+                    double vm = 0.0;
+                    for (int i = tid; i < ncells * 2 * NF; i += blockDim.x)
+                        vm = fmax(vm, sdiag[i / (2 * NF) * kDiagSlots + i % (2 * NF)]);
 #pragma unroll
-                        for (int k = 0; k < NF; k++)
-                            atomic_add_mesh(m + NG + sp * NF + k, wz[i] * fN[H::re(k, k)]);
+                    for (int o = 16; o >= 1; o >>= 1) vm = fmax(vm, __shfl_xor_sync(kFull, vm, o));
+                    if (lane == 0) sred[warp] = vm;
+                }
+                __syncthreads();
+            } else {
+                if (narrow) {
+                    if (fdep) deposit_spread<NF, DEP_FULL>(nz, full, srec, sfn, warp * 16, wlo, whi, c0);
+                } else if (!wide) {
+                    if (whi >= wlo) {
+                        deposit_spread<NF, DEP_COMB>(nz, mesh_out, srec, sfn, warp * 16, wlo, whi, c0);
+                        if (diag) deposit_spread<NF, DEP_DIAG>(nz, mesh_out, srec, sfn, warp * 16, wlo, whi, c0);
+                        if (fdep) deposit_spread<NF, DEP_FULL>(nz, full, srec, sfn, warp * 16, wlo, whi, c0);
+                    }
+                } else if (active) {
+#pragma unroll 1
+                    for (int i = 0; i < P.w[2]; i++) {
+                        const int cell = (ci0 + i) % nz;
+                        const double wi = i == 0 ? wz[0] : i == 1 ? wz[1] : wz[2];
+                        double* m = mesh_out + cell * NCS;
+                        for (int d = 0; d < 4; d++) {
+                            const double wd = wi * rec[R::V + d];
+                            for (int j = 0; j < HV; j++)
+                                atomic_add_mesh(m + d * NV + sp * HV + j, wd * rec[R::CV + sp * HV + j]);
+                            if (fdep)
+                                for (int e = 0; e < NH; e++)
+                                    atomic_add_mesh(full + (long long)cell * ND + (2 * d + sp) * NH + e,
+                                                    wd * sfn[pl * R::FW + sp * NH + e]);
+                        }
+                        if (diag)
+                            for (int k = 0; k < NF; k++) atomic_add_mesh(m + NG + sp * NF + k, wi * rec[R::DG + sp * NF + k]);
+                    }
+                }
+                const bool wait = !(s == 4 && (final_step || last || step + 1 >= max_step) && dt_mode == DT_ADVANCE) &&
+                                  !(s == 4 && final_step);
+                if (wait) steps_arrive(ctl);
+                // the mesh deposited two stages on (its last readers are past
+                // the previous barrier)
+                {
+                    double* mz = cmesh + ((s + 2) & 3) * msize;
+                    if (s == 2 || s == 3 || (s == 4 && wait))
+                        for (int i = gtid; i < msize; i += nthreads) mz[i] = 0.0;
+                    if (s == 1 && want_full)
+                        for (int i = gtid; i < ncells * ND; i += nthreads) full[i] = 0.0;
+                }
+                if (s == 4 && dt_mode == DT_ADVANCE) {
+                    // (eight loads in flight: one pass over 512 cells or so)
+                    double vm = 0.0;
+                    const int nv = ncells * NF, bd = blockDim.x;
+                    for (int i0 = tid; i0 < nv; i0 += 8 * bd) {
+                        double2 t2[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            const int i = min(i0 + k * bd, nv - 1);
+                            t2[k] = __ldcg(reinterpret_cast<const double2*>(mesh_in + i / NF * NCS + NG) + i % NF);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 8; k++) vm = fmax(vm, fmax(t2[k].x, t2[k].y));
+                    }
+#pragma unroll
+                    for (int o = 16; o >= 1; o >>= 1) vm = fmax(vm, __shfl_xor_sync(kFull, vm, o));
+                    if (lane == 0) sred[warp] = vm;
+                    __syncthreads();
+                }
+                if (s == 4 && dt_mode == DT_ADVANCE) {
+                    // compute_dt on the stage-4 mesh (Evolve.cpp:22-89 with
+                    // max_adaptive_speedup <= 1: V_stupid of the diagonal)
+                    double vm = sred[0];
+                    for (int w = 1; w < nwarps; w++) vm = fmax(vm, sred[w]);
+                    dt_next = next_dt_stupid(P, fmax(P.flavor_cfl_factor > 0.0 ? vm : 0.0, dt_vmin), dt_fac, st_dt);
+                }
+                if (wait) {
+                    nbar++;
+                    if (!steps_wait(ctl, nbar * gridDim.x)) {
+                        alive = false;
+                        break;
                     }
                 }
             }
-            if constexpr (ONE) __syncthreads();
-            else if (!(s == 4 && (final_step || done))) {
-                nbar++;
-                if (!steps_barrier(ctl, nbar * gridDim.x)) {
-                    alive = false;
-                    break;
+            if (s == 4 && dt_mode == DT_ADVANCE) {
+                if constexpr (ONE) {
+                    double vm = sred[0];
+                    for (int w = 1; w < nwarps; w++) vm = fmax(vm, sred[w]);
+                    dt_next = next_dt_stupid(P, fmax(P.flavor_cfl_factor > 0.0 ? vm : 0.0, dt_vmin), dt_fac, st_dt);
                 }
+                t_next = t_run + dt;
+                step_next = step + 1;
+                if (last || step_next >= max_step) done = 1;
+                if (end_time - t_next < dt_next) {
+                    dt_next = end_time - t_next;
+                    last_next = 1;
+                }
+                if (st_dt) done = 1;
             }
         }
         t_run = t_next;
@@ -554,10 +758,10 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
     }
     if constexpr (ONE) {
         // the new state's mesh and a clean next one, as a step leaves them
-        for (int i = tid; i < ncells * NCS; i += blockDim.x) {
+        for (int i = tid; i < msize; i += blockDim.x) {
             const int c = i / NCS, q = i - c * NCS;
-            M.m[0][i] = q < NG ? smesh[cur * kOneCells * NG + c * NG + q] : sdiag[c * kDiagSlots + q - NG];
-            M.m[1][i] = 0.0;
+            cmesh[i] = q < NG ? smesh[cur * kHalf + c * MR + q] : sdiag[c * kDiagSlots + q - NG];
+            cmesh[msize + i] = 0.0;
         }
     }
     // the last CTA to leave writes the step control (all hold the same)
@@ -579,55 +783,72 @@ __global__ void __launch_bounds__(2 * kBlock, ONE ? 1 : 2)
     }
 }
 
-template <int NF, bool ONE>
-bool fits(long long n)
+// particles per CTA: spread over the SMs, whole warps of 16, at least 64 (a
+// smaller CTA only adds barrier arrivals) and at most 256 (512 threads)
+int particles_per_cta(long long n, int nsm)
 {
-    auto kern = k_steps_1d<NF, ONE>;
-    constexpr int bytes = steps1d_smem<NF, ONE>();
-    smem_optin(kern, bytes);
-    int per_sm = 0, dev = 0, nsm = 0;
-    const bool ok = cudaGetDevice(&dev) == cudaSuccess &&
-                    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 2 * kBlock, bytes) == cudaSuccess &&
-                    (long long)per_sm * nsm >= (long long)grid_for(n);
-    cudaGetLastError();
-    return ok;
+    const long long per = (n + nsm - 1) / nsm;
+    return (int)std::max<long long>(64, (per + 15) / 16 * 16);
 }
 
-template <int NF, bool ONE>
-cudaError_t launch(const DevParams& P, const DevState& S, double* const cmesh[4], double* full, StepCtl* ctl,
-                   int nsteps, int dt_mode, cudaStream_t st)
+bool one_cta(const DevParams& P, long long n) { return n <= kOnePart && P.ncells <= kOneCells; }
+
+int device_sms()
 {
-    constexpr int bytes = steps1d_smem<NF, ONE>();
-    smem_optin(k_steps_1d<NF, ONE>, bytes);
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        nsm = 0;
+    cudaGetLastError();
+    return nsm;
+}
+
+// the kernel for a CTA of npart particles: the fewer threads, the more
+// registers each (three flavors spill at 128)
+using Steps1DKernel = void (*)(DevParams, DevState, double*, double*, StepCtl*, int, int, int);
+template <int NF>
+Steps1DKernel steps1d_kernel(bool one, int npart)
+{
+    if (one) return k_steps_1d<NF, true, 256>;
+    if (npart <= 128) return k_steps_1d<NF, false, 256>;
+    if (npart <= 192) return k_steps_1d<NF, false, 384>;
+    return k_steps_1d<NF, false, 512>;
+}
+
+template <int NF>
+cudaError_t launch_t(const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl, int nsteps,
+                     int dt_mode, cudaStream_t st)
+{
+    const bool one = one_cta(P, S.n);
+    int npart = one ? kOnePart : particles_per_cta(S.n, device_sms());
+    const Steps1DKernel kern = steps1d_kernel<NF>(one, npart);
+    const int bytes = one ? steps1d_smem<NF, true>(npart) : steps1d_smem<NF, false>(npart);
+    smem_optin(kern, bytes);
     DevParams Pc = P;
     DevState Sc = S;
-    Meshes4 M{{cmesh[0], cmesh[1], cmesh[2], cmesh[3]}};
-    void* args[] = {&Pc, &Sc, &M, &full, &ctl, &nsteps, &dt_mode};
-    return cudaLaunchCooperativeKernel((const void*)k_steps_1d<NF, ONE>, dim3(grid_for(S.n)), dim3(2 * kBlock), args,
-                                       bytes, st);
+    void* args[] = {&Pc, &Sc, &cmesh, &full, &ctl, &npart, &nsteps, &dt_mode};
+    return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid_for(S.n, npart)), dim3(2 * npart), args, bytes, st);
 }
-
-bool one_cta(const DevParams& P, long long n) { return n <= kBlock && P.ncells <= kOneCells; }
 
 }  // namespace
 
+// one-dimensional along z, at most 256 particles per SM (two flavors, 128 x
+// 80: 40 -> 15 us per step; past one CTA per SM the stage kernels, which
+// keep several CTAs in flight on each, take over)
 bool steps_1d_fit(int nf, const DevParams& P, long long n)
 {
     if (P.n[0] != 1 || P.n[1] != 1 || P.max_adaptive_speedup > 1.0) return false;
-    if (P.ncells > (1 << 20)) return false;   // (mesh indices are ints)
-    if (one_cta(P, n)) return nf == 2 ? fits<2, true>(n) : fits<3, true>(n);
-    return nf == 2 ? fits<2, false>(n) : fits<3, false>(n);
+    if (P.ncells > (1 << 20)) return false;   // (mesh offsets are ints)
+    if (one_cta(P, n)) return true;
+    const int nsm = device_sms();
+    return nsm > 0 && particles_per_cta(n, nsm) <= 256;
 }
 
-cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* const cmesh[4], double* full,
-                            StepCtl* ctl, int nsteps, int dt_mode, cudaStream_t st)
+cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl,
+                            int nsteps, int dt_mode, cudaStream_t st)
 {
-    if (one_cta(P, S.n))
-        return nf == 2 ? launch<2, true>(P, S, cmesh, full, ctl, nsteps, dt_mode, st)
-                       : launch<3, true>(P, S, cmesh, full, ctl, nsteps, dt_mode, st);
-    return nf == 2 ? launch<2, false>(P, S, cmesh, full, ctl, nsteps, dt_mode, st)
-                   : launch<3, false>(P, S, cmesh, full, ctl, nsteps, dt_mode, st);
+    return nf == 2 ? launch_t<2>(P, S, cmesh, full, ctl, nsteps, dt_mode, st)
+                   : launch_t<3>(P, S, cmesh, full, ctl, nsteps, dt_mode, st);
 }
 
 }  // namespace emu

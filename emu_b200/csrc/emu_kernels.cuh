@@ -146,11 +146,12 @@ bool coop_step_fits(int nf, const DevParams& P, long long n);
 cudaError_t launch_rk4_step_coop(int nf, const DevParams& P, const DevState& S, double* const mesh[4], long long nmesh,
                                  StepCtl* ctl, int dt_mode, cudaStream_t st);
 // nsteps FP64 RK4 steps of a small 1D problem in one cooperative launch on
-// combined meshes (cmesh: M_1 deposited, M_2 zeroed; full: target of the full
+// combined meshes (cmesh: M_1..M_4 one after the other, M_1 deposited, M_2
+// zeroed; full: target of the full
 // stage-4 mesh); dt_mode DT_ADVANCE, or -1 for one step of the control's dt
 bool steps_1d_fit(int nf, const DevParams& P, long long n);
-cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* const cmesh[4], double* full,
-                            StepCtl* ctl, int nsteps, int dt_mode, cudaStream_t st);
+cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl,
+                            int nsteps, int dt_mode, cudaStream_t st);
 // a full FP64 mesh in the combined layout with its diagonal slots
 void launch_full_to_comb64(int nf, const DevParams& P, const double* full, double* comb, cudaStream_t st);
 // compute_dt from the diagonal slots of a combined FP64 mesh
