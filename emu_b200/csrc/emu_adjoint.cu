@@ -1231,7 +1231,7 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
     CU(cudaMemcpyAsync(ctx->mesh[3], a->mst + (size_t)(nsteps - 1) * G.mst_stride + 3 * nm, sizeof(double) * nm,
                        cudaMemcpyDeviceToDevice, st));
     ctx->cur_mesh = 3;
-    if (ctx->steps1d) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
+    if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
     return EMU_OK;
 }
 

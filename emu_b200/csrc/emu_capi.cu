@@ -358,7 +358,7 @@ int deposit_current(emu_context* ctx)
         emu::launch_deposit(ctx->nf, ctx->P, S, S.f0, ctx->mesh[0], ctx->stream);
         if ((r = check_launch(ctx, "deposit"))) return r;
         if ((r = emu_ctx::reduce_mesh(ctx, ctx->mesh[0], false, ctx->stream))) return r;
-        if (ctx->steps1d) {
+        if (ctx->steps1d || ctx->comb64) {
             emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh, ctx->stream);
             if ((r = check_launch(ctx, "combined mesh"))) return r;
             CU(cudaMemsetAsync(ctx->cmesh + cmesh_elems(ctx), 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
@@ -384,6 +384,55 @@ int enqueue_rk4_fp64(emu_context* ctx, cudaStream_t st, bool with_dt, bool dep4 
         if (dep && (r = emu_ctx::reduce_mesh(ctx, ctx->mesh[s % 4], false, st))) return r;
     }
     return check_launch(ctx, "rk4 stage");
+}
+
+// FP64 RK4 on combined meshes: stage s reads cmesh s-1, deposits cmesh s%4,
+// zeroes cmesh (s+1)%4; the full stage-4 mesh (mesh[3], on the steps after
+// which it can be read) by a kernel between stages 3 and 4.  dep4 = false: a
+// re-sort follows, made by stage 4's stores (enqueue_sc_before), then the
+// deposit of the re-sorted state.  stage_event(i, end): before and after each
+// timed kernel (emu_profile_step), i = 0..3 the stages, 4 and 5 the re-sort's
+// parts.
+template <class Ev>
+int enqueue_rk4_comb64(emu_context* ctx, cudaStream_t st, bool with_dt, bool dep4, Ev stage_event)
+{
+    const DevState& S = ctx->S[ctx->cur];
+    const long long ms = cmesh_elems(ctx);
+    auto cm = [&](int i) { return ctx->cmesh + (i & 3) * ms; };
+    const int dt_mode = with_dt ? emu::DT_ADVANCE : -1;
+    int r;
+    for (int s = 1; s <= 3; s++) {
+        const bool keys = s == 3 && !dep4;
+        stage_event(s - 1, 0);
+        emu::launch_stage64(ctx->nf, ctx->P, S, s, cm(s - 1), cm(s), cm(s + 1), s == 2 ? ctx->mesh[3] : nullptr,
+                            ctx->ctl, dt_mode, st, nullptr, nullptr, keys ? ctx->keys : nullptr,
+                            keys ? ctx->idx : nullptr);
+        if (s == 3) emu::launch_deposit_full64(ctx->nf, ctx->P, S, S.f0, ctx->mesh[3], ctx->ctl, st);
+        stage_event(s - 1, 1);
+    }
+    if (dep4) {
+        stage_event(3, 0);
+        emu::launch_stage64(ctx->nf, ctx->P, S, 4, cm(3), cm(0), cm(1), nullptr, ctx->ctl, dt_mode, st);
+        stage_event(3, 1);
+    } else {
+        DevState& D = ctx->S[1 - ctx->cur];
+        D.n = S.n;
+        stage_event(4, 0);
+        if ((r = sort_perm(ctx, S.n, st))) return r;
+        emu::launch_sc_invert(ctx->idx2, ctx->idx, S.n, st);
+        stage_event(4, 1);
+        stage_event(3, 0);
+        emu::launch_stage64(ctx->nf, ctx->P, S, 4, cm(3), nullptr, cm(1), nullptr, ctx->ctl, dt_mode, st, &D, ctx->idx);
+        stage_event(3, 1);
+        stage_event(5, 0);
+        emu::launch_deposit_comb64(ctx->nf, ctx->P, D, cm(0), ctx->ctl, st);
+        stage_event(5, 1);
+    }
+    return check_launch(ctx, "rk4 stage");
+}
+int enqueue_rk4_comb64(emu_context* ctx, cudaStream_t st, bool with_dt, bool dep4 = true)
+{
+    return enqueue_rk4_comb64(ctx, st, with_dt, dep4, [](int, int) {});
 }
 
 // mixed RK4: finalize(q[a] -> g, zero q[b]); stage deposits into q[b]; swap
@@ -486,7 +535,7 @@ int step_generic(emu_context* ctx, double dt)
 // mesh instead (mesh[0] / qmesh[0], zeroed here first)
 int resort(emu_context* ctx, bool deposit = false)
 {
-    if (deposit && ctx->mixed) {
+    if (deposit && (ctx->mixed || ctx->comb64)) {
         // (the step's stage 4 has made it, into the other buffer)
         ctx->cur = 1 - ctx->cur;
         ctx->steps_since_sort = 0;
@@ -525,6 +574,7 @@ int resort(emu_context* ctx, bool deposit = false)
 
 int enqueue_step_body(emu_context* ctx, cudaStream_t st, bool dep4)
 {
+    if (ctx->comb64) return enqueue_rk4_comb64(ctx, st, true, dep4);
     return ctx->mixed ? enqueue_rk4_mixed(ctx, st, true, dep4) : enqueue_rk4_fp64(ctx, st, true, dep4);
 }
 
@@ -661,7 +711,11 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     // fused == 1, 1D along z, the grid fits: several steps per launch
     ctx->steps1d = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                    emu::steps_1d_fit(ctx->nf, ctx->P, n);
-    if (ctx->steps1d && (r = ensure_cmesh(ctx))) return r;
+    // any other FP64 RK4 context of one rank without the adaptive timestep:
+    // stage kernels on combined meshes
+    ctx->comb64 = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
+                  !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d;
+    if ((ctx->steps1d || ctx->comb64) && (r = ensure_cmesh(ctx))) return r;
     ctx->loaded = true;
     ctx->adj_valid = false;
     ctx->steps_since_sort = 0;
@@ -981,7 +1035,9 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
             r = e == cudaSuccess ? EMU_OK : fail(ctx, EMU_ERR_CUDA, std::string("cooperative step: ") +
                                                                       cudaGetErrorString(e));
         } else {
-            r = ctx->mixed ? enqueue_rk4_mixed(ctx, ctx->stream, false) : enqueue_rk4_fp64(ctx, ctx->stream, false);
+            r = ctx->mixed    ? enqueue_rk4_mixed(ctx, ctx->stream, false)
+                : ctx->comb64 ? enqueue_rk4_comb64(ctx, ctx->stream, false)
+                              : enqueue_rk4_fp64(ctx, ctx->stream, false);
         }
         if (r) return r;
         if (ctx->mixed && (r = sum_full_parts(ctx))) return r;
@@ -1014,7 +1070,7 @@ int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int m
         }
         emu::launch_dt_q(ctx->nf, ctx->P, ctx->qfull, nullptr, ctx->ctl, emu::DT_INIT, ctx->stream);
     }
-    else if (ctx->steps1d) emu::launch_dt_comb64(ctx->nf, ctx->P, ctx->cmesh, ctx->ctl, emu::DT_INIT, ctx->stream);
+    else if (ctx->steps1d || ctx->comb64) emu::launch_dt_comb64(ctx->nf, ctx->P, ctx->cmesh, ctx->ctl, emu::DT_INIT, ctx->stream);
     else emu::launch_dt(ctx->nf, ctx->P, ctx->mesh[0], ctx->ctl, emu::DT_INIT, ctx->stream);
     return check_launch(ctx, "initial compute_dt");
 }
@@ -1025,7 +1081,7 @@ int emu_evolve_steps(emu_context* ctx, int nsteps)
     int r;
     // the last of these steps deposits the full stage-4 mesh (the one a
     // caller can read after the call)
-    if (((ctx->mixed && ctx->P.m4_reduced) || ctx->steps1d) && nsteps > 0)
+    if (((ctx->mixed && ctx->P.m4_reduced) || ctx->steps1d || ctx->comb64) && nsteps > 0)
         emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
     if (ctx->steps1d) {
         // one launch up to the next re-sort
@@ -1128,7 +1184,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
     const int nk = ctx->mixed ? 8 : 4;
     // timed as a step inside a longer run: the stage-4 mesh stays in the
     // combined layout (DevParams::m4_reduced) unless the run ends here
-    if (ctx->mixed && ctx->P.m4_reduced) emu::launch_ctl_m4(ctx->ctl, 2, ctx->stream);
+    if ((ctx->mixed && ctx->P.m4_reduced) || ctx->comb64) emu::launch_ctl_m4(ctx->ctl, 2, ctx->stream);
     const bool resort_due = ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
     if (max_kernels < nk + (resort_due ? 1 : 0))
         return fail(ctx, EMU_ERR_ARG, "emu_profile_step: kernel_ms too small");
@@ -1141,8 +1197,14 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
     // (mixed: the re-sort made around stage 4, timed as one entry after the
     // stages: its keys (unless stage 3 stores them) and sort before stage 4
     // plus its deposit after it)
-    const bool sc = ctx->mixed && resort_due;
-    if (ctx->mixed) {
+    const bool sc = (ctx->mixed || ctx->comb64) && resort_due;
+    if (ctx->comb64) {
+        const int rc = enqueue_rk4_comb64(ctx, st, true, !resort_due, [&](int i, int end) {
+            rec(i < 4 ? 2 * i + end : 2 * nk + 2 * (i - 4) + end);
+        });
+        if (rc) return rc;
+        k = 4;
+    } else if (ctx->mixed) {
         int a = 0;
         for (int s = 1; s <= 4; s++) {
             const int b = 1 - a;

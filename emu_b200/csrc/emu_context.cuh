@@ -30,7 +30,7 @@ struct emu_context {
     void* tblock = nullptr;             // transient per-step arrays
     long long cap = 0;
     double* mesh[4] = {nullptr, nullptr, nullptr, nullptr};
-    // FP64 steps on combined meshes (steps1d): M_1..M_4 in the combined
+    // FP64 steps on combined meshes (steps1d, comb64): M_1..M_4 in the combined
     // layout with the diagonal slots (kCombSlots per cell), one after the
     // other; mesh[0] and mesh[3] then hold the full deposit of a load and the
     // full stage-4 mesh
@@ -67,6 +67,7 @@ struct emu_context {
     int steps_since_sort = 0;
     bool coop = false;                  // whole-step cooperative kernel (small FP64 problems)
     bool steps1d = false;               // several steps per cooperative launch (k_steps_1d)
+    bool comb64 = false;                // FP64 stages on combined meshes (k_stage64)
     emu_adjoint* adj = nullptr;         // allocated by the first adjoint call
     // particle sharding over ranks (emu_attach_comm): every deposit is summed
     // over the ranks before a stage reads it

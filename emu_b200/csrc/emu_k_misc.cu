@@ -2,16 +2,20 @@
 // dispatch of the large ones (whose instantiations live in
 // emu_k_fp64_<nf>.cu and emu_k_mixed_<nf>.cu so that they compile in
 // parallel).
-#include "emu_kernels_impl.cuh"
-#include "emu_fp64.cuh"
+#include "emu_fp64_impl.cuh"
 
 namespace emu {
 
 #define EMU_EXTERN(NF)                                                                                          \
     extern template void launch_rk4_stage_t<NF>(const DevParams&, const DevState&, int, const double*, double*,  \
                                                 double*, long long, StepCtl*, int, cudaStream_t);                \
-    extern template void launch_deposit_t<NF>(const DevParams&, const DevState&, const double*, double*,         \
-                                              cudaStream_t);                                                     \
+    extern template void launch_stage64_t<NF>(const DevParams&, const DevState&, int, const double*, double*,    \
+                                              double*, double*, StepCtl*, int, cudaStream_t, const DevState*,    \
+                                              const unsigned*, unsigned*, unsigned*);                            \
+    extern template void launch_deposit_comb64_t<NF>(const DevParams&, const DevState&, double*, const StepCtl*, \
+                                                     cudaStream_t);                                              \
+    extern template void launch_deposit_full64_t<NF>(const DevParams&, const DevState&, const double*, double*,  \
+                                                     StepCtl*, cudaStream_t);                                    \
     extern template void launch_rhs_t<NF>(const DevParams&, const DevState&, const double*, const double*,       \
                                           double*, cudaStream_t);                                                \
     extern template void launch_rk4_stage_mixed_t<NF>(const DevParams&, const DevState&, int, const float*,      \
@@ -83,7 +87,31 @@ void launch_gather_deposit(int nf, bool mixed, const DevParams& P, const DevStat
 
 void launch_deposit(int nf, const DevParams& P, const DevState& S, const double* f, double* mesh, cudaStream_t st)
 {
-    if (nf == 2) launch_deposit_t<2>(P, S, f, mesh, st); else launch_deposit_t<3>(P, S, f, mesh, st);
+    launch_deposit_full64(nf, P, S, f, mesh, nullptr, st);
+}
+
+void launch_deposit_full64(int nf, const DevParams& P, const DevState& S, const double* f, double* mesh, StepCtl* ctl,
+                           cudaStream_t st)
+{
+    if (nf == 2) launch_deposit_full64_t<2>(P, S, f, mesh, ctl, st);
+    else launch_deposit_full64_t<3>(P, S, f, mesh, ctl, st);
+}
+
+void launch_deposit_comb64(int nf, const DevParams& P, const DevState& S, double* mesh, const StepCtl* ctl,
+                           cudaStream_t st)
+{
+    if (nf == 2) launch_deposit_comb64_t<2>(P, S, mesh, ctl, st);
+    else launch_deposit_comb64_t<3>(P, S, mesh, ctl, st);
+}
+
+void launch_stage64(int nf, const DevParams& P, const DevState& S, int s, const double* mesh_in, double* mesh_out,
+                    double* mesh_zero, double* full_zero, StepCtl* ctl, int dt_mode, cudaStream_t st,
+                    const DevState* D, const unsigned* inv, unsigned* kout, unsigned* iout)
+{
+    if (nf == 2)
+        launch_stage64_t<2>(P, S, s, mesh_in, mesh_out, mesh_zero, full_zero, ctl, dt_mode, st, D, inv, kout, iout);
+    else
+        launch_stage64_t<3>(P, S, s, mesh_in, mesh_out, mesh_zero, full_zero, ctl, dt_mode, st, D, inv, kout, iout);
 }
 
 void launch_deposit_q(int nf, const DevParams& P, const DevState& S, const double* f, long long* mesh,

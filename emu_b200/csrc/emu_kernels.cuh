@@ -108,7 +108,8 @@ struct StepCtl {
     // m4_full_from on and on the final step of a run, and otherwise only the
     // combined layout stage 4 interpolates; the diagonal N_ii compute_dt
     // reads are deposited apart in both cases.  m4_full: whether the latest
-    // stage-3 deposit was the full one.
+    // stage-3 deposit was the full one.  (FP64 steps on combined meshes: the
+    // same; 2: the run had ended before the latest step)
     int m4_full_from;
     int m4_full;
 };
@@ -152,6 +153,20 @@ cudaError_t launch_rk4_step_coop(int nf, const DevParams& P, const DevState& S, 
 bool steps_1d_fit(int nf, const DevParams& P, long long n);
 cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl,
                             int nsteps, int dt_mode, cudaStream_t st);
+// one FP64 RK4 stage on combined meshes; full_zero: stage 2 zeroes it on the
+// steps that deposit the full stage-4 mesh; D, inv, kout, iout as
+// launch_rk4_stage_mixed
+void launch_stage64(int nf, const DevParams& P, const DevState& S, int s, const double* mesh_in, double* mesh_out,
+                    double* mesh_zero, double* full_zero, StepCtl* ctl, int dt_mode, cudaStream_t st,
+                    const DevState* D = nullptr, const unsigned* inv = nullptr, unsigned* kout = nullptr,
+                    unsigned* iout = nullptr);
+// the combined deposit of a cell-sorted state after a re-sorting step
+void launch_deposit_comb64(int nf, const DevParams& P, const DevState& S, double* mesh, const StepCtl* ctl,
+                           cudaStream_t st);
+// the full deposit of state f into mesh (zeroed); with ctl only on the steps
+// whose stage-4 mesh can be read (between stages 3 and 4)
+void launch_deposit_full64(int nf, const DevParams& P, const DevState& S, const double* f, double* mesh, StepCtl* ctl,
+                           cudaStream_t st);
 // a full FP64 mesh in the combined layout with its diagonal slots
 void launch_full_to_comb64(int nf, const DevParams& P, const double* full, double* comb, cudaStream_t st);
 // compute_dt from the diagonal slots of a combined FP64 mesh

@@ -19,7 +19,7 @@
 //                            FP64 state, int64 fixed-point deposit
 //   k_finalize_mixed<NF>     int64 mesh -> FP32 potential mesh
 //   k_dt<NF>                 compute_dt reduction (host-driven calls)
-//   k_deposit / k_rhs / k_stage_state / k_combine: unfused building blocks
+//   k_rhs / k_stage_state / k_combine: unfused building blocks
 //                            for the C ABI calls and FE/trapezoid/SSPRK3
 // W = stencil widths (WX,WY,WZ): (1,1,3) for 1D runs along z, (3,3,3) for 3D
 // TSC, (0,0,0) generic runtime widths.
@@ -1072,33 +1072,6 @@ __global__ void __launch_bounds__(2 * kBlock, 2) k_rk4_step_coop_split(DevParams
 // ===========================================================================
 // unfused building blocks (FP64)
 // ===========================================================================
-template <int NF, int WX, int WY, int WZ>
-__global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, const double* __restrict__ f,
-                                                    double* __restrict__ mesh)
-{
-    using SWt = SW<WX, WY, WZ>;
-    constexpr int NH = NF * NF, NS = 2 * NH;
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < S.n;
-    Stencil<double> st{};
-    double fN[NS] = {};
-    double vx = 0, vy = 0, vz = 0;
-    if (active) {
-        make_stencil<double>(P, S.pos[0][p], S.pos[1][p], S.pos[2][p], st);
-        vx = S.vhat[0][p];
-        vy = S.vhat[1][p];
-        vz = S.vhat[2][p];
-        const double N0 = S.Nn[0][p], N1 = S.Nn[1][p];
-#pragma unroll
-        for (int e = 0; e < NH; e++) {
-            fN[e] = f[e * S.cap + p] * N0;
-            fN[NH + e] = f[(NH + e) * S.cap + p] * N1;
-        }
-    }
-    tile_deposit_block<NF, SWt, double>(P, mesh, active, st, fN, vx, vy, vz,
-                                        [](double a, int) -> double { return a; }, true);
-}
-
 template <int NF, int WX, int WY, int WZ>
 __global__ void __launch_bounds__(kBlock) k_rhs(DevParams P, DevState S, const double* __restrict__ f,
                                                 const double* __restrict__ mesh, double* __restrict__ K)
@@ -2340,16 +2313,6 @@ void launch_gather_deposit_t(bool mixed, const DevParams& P, const DevState& src
             k_gather_deposit<NF, WXv, WYv, WZv, false><<<grid_for(src.n), kBlock, bytes, st>>>(P, src, dst, perm,
                                                                                               mesh, qmesh);
         }
-    });
-}
-
-template <int NF>
-void launch_deposit_t(const DevParams& P, const DevState& S, const double* f, double* mesh, cudaStream_t st)
-{
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        smem_optin(k_deposit<NF, WXv, WYv, WZv>, bytes);
-        k_deposit<NF, WXv, WYv, WZv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, f, mesh);
     });
 }
 
