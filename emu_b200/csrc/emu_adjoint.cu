@@ -31,7 +31,7 @@
 // backward.  Particles keep their slot order for the whole recorded run (no
 // re-sort).
 #include "emu_context.cuh"
-#include "emu_kernels_impl.cuh"
+#include "emu_fp64_impl.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -96,29 +96,29 @@ namespace {
 
 // ---- per-particle adjoint pieces ------------------------------------------
 
-// VJP of K = C(H, F) = -i/hbar [H, F] (bilinear in H and F):
-//   lamF_b = sum_c lam_c C_c(H, e_b),  lamH_a = sum_c lam_c C_c(e_a, F)
+// VJP of K = C(H, F) = -i/hbar [H, F].  With the Hermitian matrix L whose
+// trace product is the contraction with lam, Tr(L K) = sum_c lam_c K_c (L_ii =
+// lam_ii, L_ij = (lam_re + i lam_im) / 2), cyclic permutation of the trace
+// gives Tr(L C(H, F)) = Tr(C(L, H) F) = Tr(C(F, L) H): two commutators (the
+// sums over unit vectors they replace were 18 of them for three flavors, half
+// of the adjoint stage's arithmetic).
 template <int NF>
 __device__ __forceinline__ void commutator_vjp(const double* h, const double* f, const double* lam, double* lamH,
                                                double* lamF, double inv_hbar)
 {
+    using H = Herm<NF>;
     constexpr int NH = NF * NF;
+    double l[NH];
 #pragma unroll
-    for (int b = 0; b < NH; b++) {
-        double e[NH], o[NH];
+    for (int e = 0; e < NH; e++) l[e] = H::is_diag(e) ? lam[e] : 0.5 * lam[e];
+    commutator_lean<NF, double>(l, h, lamF, inv_hbar);
+    commutator_lean<NF, double>(f, l, lamH, inv_hbar);
 #pragma unroll
-        for (int k = 0; k < NH; k++) e[k] = (k == b) ? 1.0 : 0.0;
-        commutator<NF, double>(h, e, o, inv_hbar);
-        double sf = 0.0;
-#pragma unroll
-        for (int c = 0; c < NH; c++) sf += lam[c] * o[c];
-        lamF[b] = sf;
-        commutator<NF, double>(e, f, o, inv_hbar);
-        double sh = 0.0;
-#pragma unroll
-        for (int c = 0; c < NH; c++) sh += lam[c] * o[c];
-        lamH[b] = sh;
-    }
+    for (int e = 0; e < NH; e++)
+        if (!H::is_diag(e)) {
+            lamF[e] *= 2.0;
+            lamH[e] *= 2.0;
+        }
 }
 
 // VJP of renormalize<NF>() at input fin (one species): replays the forward
@@ -213,97 +213,185 @@ __device__ __forceinline__ void gather_deposit_adjoint(const DevParams& P, const
 
 // ---- kernels ----------------------------------------------------------------
 
-// Stage recompute: K = RHS(Yin, M_s); s < 4: acc, Y_{s+1} = Y0 + a dt K and
-// its deposit; s == 4: Y_n = acc + b4 dt K.  Same arithmetic as the forward
-// stage kernel.
-template <int NF, class SWt>
-__device__ __forceinline__ void adj_fwd_stage_body(const DevParams& P, const DevState& S, int s, double dt,
-                                                   const double* __restrict__ Yin, const double* __restrict__ Y0,
-                                                   double* __restrict__ acc, double* __restrict__ Yout,
-                                                   const double* __restrict__ mesh_in, double* __restrict__ mesh_out)
+// The meshes of the sweep and of the recompute are combined ones (Comb<NF>,
+// kCombSlots per cell): the forward stages read no more, and the adjoint mesh
+// has the same structure (the transpose of the interpolation scatters lam_H
+// of nu and nubar with the potential's signs; lam_H is traceless, like every
+// commutator).  Interpolations and deposits are the FP64 matrix products of
+// emu_fp64_impl.cuh.
+
+// a tile's weights, keys and velocities in key order; returns this thread's
+// slot.  x, v, st: the particle's
+template <int NF, class T, int WX, int WY, int WZ, int RW>
+__device__ __forceinline__ int adj_tile(const DevParams& P, const Smem64<NF, T, RW>& sm, bool active, const double* x,
+                                        const double* v, Stencil<double>& st)
 {
-    constexpr int NH = NF * NF, NS = 2 * NH;
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int key = -1;
+    if (active) {
+        make_stencil<double>(P, x[0], x[1], x[2], st);
+        key = stencil_key(P, st.b);
+    }
+    const int slot = rank_slots(P, key, sm.rec, sm.rank);
+    write_weights<T, WX, WY, WZ>(P, sm.rec + slot * RW, active, st);
+    sm.key[slot] = key;
+#pragma unroll
+    for (int d = 0; d < 3; d++) sm.v[d * T::VS + slot] = v[d];
+    __syncthreads();
+    run_starts(sm.key, sm.starts);
+    __syncthreads();
+    return slot;
+}
+
+// the values c_j of a record (zeros for an inactive thread)
+template <int NF, int WP>
+__device__ __forceinline__ void adj_record(double* rec, bool active, const double* c)
+{
+#pragma unroll
+    for (int j = 0; j < Comb<NF>::NV; j += 2)
+        *reinterpret_cast<double2*>(rec + WP + j) = make_double2(active ? c[j] : 0.0, active ? c[j + 1] : 0.0);
+}
+// and of the interpolated sums, expanded to the Hermitian components
+template <int NF, int WP>
+__device__ __forceinline__ void adj_sums(const double* rec, double scale, double* h)
+{
+    double u[Comb<NF>::NV];
+#pragma unroll
+    for (int j = 0; j < Comb<NF>::NV; j += 2) {
+        const double2 t2 = *reinterpret_cast<const double2*>(rec + WP + j);
+        u[j] = t2.x * scale;
+        u[j + 1] = t2.y * scale;
+    }
+    Comb<NF>::hermitian(u, h);
+}
+
+struct AdjFwdPtrs {
+    const double* Yin;      // Y_s
+    const double* Y0;
+    double* acc;
+    double* Yout;           // Y_{s+1}; s = 4: Y_n (before Renormalize)
+    const double* mesh_in;  // M_s
+    double* mesh_out;       // M_{s+1} (null: given), s = 4: the next step's M_1 (null: none)
+    double* Ynext;          // s = 4: the renormalised state (null: not wanted)
+    double* xnext;          // s = 4: the positions after the step (null: not wanted)
+    StepCtl* report;        // s = 4: Renormalize's findings go here (null: nowhere)
+    int diag;               // s = 3: deposit the diagonal slots too (recorded runs: compute_dt)
+};
+
+// Stage recompute: K = RHS(Yin, M_s); s < 4: acc, Y_{s+1} = Y0 + a dt K and
+// its deposit; s == 4: Y_n = acc + b4 dt K, and the step's completion: Y_new =
+// Renormalize(Y_n), positions advanced and wrapped, the deposit of Y_new at
+// the new positions.  Same operations as the forward stage kernel.
+template <int NF, int WX, int WY, int WZ, int KS>
+__device__ __forceinline__ void adj_fwd_body(const DevParams& P, const DevState& S, int s, double dt,
+                                             const AdjFwdPtrs& A)
+{
+    using T = Tile64<NF, WX, WY, WZ, KS>;
+    using H = Herm<NF>;
+    using C = Comb<NF>;
+    constexpr int NH = NF * NF, NV = C::NV, WP = T::WP, VS = T::VS, RW = T::template row<NV>();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    const Smem64<NF, T, RW> sm(tile_smem);
+    const long long p = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = p < S.n;
     const long long cap = S.cap;
     Stencil<double> st{};
-    double fN[NS] = {};
-    double vx = 0, vy = 0, vz = 0;
+    double x[3] = {0, 0, 0}, v[3] = {0, 0, 0}, vsc = 0.0;
     if (active) {
-        make_stencil<double>(P, S.pos[0][p], S.pos[1][p], S.pos[2][p], st);
-        vx = S.vhat[0][p];
-        vy = S.vhat[1][p];
-        vz = S.vhat[2][p];
-        double V[NS];
-        potential_fp64<NF, SWt>(P, mesh_in, st, vx, vy, vz, S.vscale[p], V);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            x[d] = S.pos[d][p];
+            v[d] = S.vhat[d][p];
+        }
+        vsc = S.vscale[p];
+    }
+    int slot = adj_tile<NF, T, WX, WY, WZ, RW>(P, sm, active, x, v, st);
+    interp64<NF, T, WX, WY, RW>(P, A.mesh_in, sm.rec, sm.key, sm.v);
+    __syncthreads();
+    double* rec = sm.rec + slot * RW;
+    double hs[NH], c[NV];
+    adj_sums<NF, WP>(rec, P.sqrt2GF_inv_vol, hs);
+    double dnum[2 * NF];
+#pragma unroll
+    for (int i = 0; i < 2 * NF; i++) dnum[i] = 0.0;
+    if (active) {
         const double bw = dt * kRK4B[s - 1];
         const double aw = s < 4 ? dt * kRK4A[s] : 0.0;
+        int stt = 0;
+        double cc[NH];
 #pragma unroll
         for (int sp = 0; sp < 2; sp++) {
-            double f[NH], K[NH];
+            double f[NH], K[NH], h[NH];
 #pragma unroll
-            for (int e = 0; e < NH; e++) f[e] = Yin[(sp * NH + e) * cap + p];
-            commutator<NF, double>(V + sp * NH, f, K, P.inv_hbar);
+            for (int e = 0; e < NH; e++) f[e] = A.Yin[(sp * NH + e) * cap + p];
+            species_hamiltonian<NF>(P, hs, vsc, sp, h);
+            commutator_lean<NF, double>(h, f, K, P.inv_hbar);
+            if (s < 4) {
+#pragma unroll
+                for (int e = 0; e < NH; e++) {
+                    const long long o = (sp * NH + e) * cap + p;
+                    const double y0 = (s == 1) ? f[e] : A.Y0[o];
+                    const double a0 = (s == 1) ? y0 : A.acc[o];
+                    A.acc[o] = __dadd_rn(__dmul_rn(bw, K[e]), a0);
+                    f[e] = __dadd_rn(__dmul_rn(aw, K[e]), y0);
+                    A.Yout[o] = f[e];
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < NH; e++) {
+                    const long long o = (sp * NH + e) * cap + p;
+                    f[e] = __dadd_rn(__dmul_rn(bw, K[e]), A.acc[o]);
+                    A.Yout[o] = f[e];
+                }
+                if (A.Ynext) {
+                    stt |= renormalize<NF>(f, S.Ll[sp][p], P.maxError);
+#pragma unroll
+                    for (int e = 0; e < NH; e++) A.Ynext[(sp * NH + e) * cap + p] = f[e];
+                }
+            }
             const double Ns = S.Nn[sp][p];
 #pragma unroll
             for (int e = 0; e < NH; e++) {
-                const long long o = (sp * NH + e) * cap + p;
-                if (s < 4) {
-                    const double y0 = (s == 1) ? f[e] : Y0[o];
-                    const double a0 = (s == 1) ? y0 : acc[o];
-                    acc[o] = __dadd_rn(__dmul_rn(bw, K[e]), a0);
-                    const double fn = __dadd_rn(__dmul_rn(aw, K[e]), y0);
-                    Yout[o] = fn;
-                    fN[sp * NH + e] = fn * Ns;
-                } else {
-                    Yout[o] = __dadd_rn(__dmul_rn(bw, K[e]), acc[o]);
-                }
+                const double a = f[e] * Ns;
+                cc[e] = sp == 0 ? a : (H::is_im(e) ? cc[e] + a : cc[e] - a);
+                if (H::is_diag(e)) dnum[sp * NF + (e == 0 ? 0 : e == NH - 1 ? NF - 1 : 1)] = a;
             }
         }
-    }
-    if (s < 4 && mesh_out)   // (null: the stage meshes are stored)
-        tile_deposit_block<NF, SWt, double>(P, mesh_out, active, st, fN, vx, vy, vz,
-                                            [](double a, int) -> double { return a; });
-}
-
-template <int NF, int WX, int WY, int WZ>
-__global__ void __launch_bounds__(kBlock) k_adj_fwd_stage(DevParams P, DevState S, int s, double dt,
-                                                          const double* __restrict__ Yin, const double* __restrict__ Y0,
-                                                          double* __restrict__ acc, double* __restrict__ Yout,
-                                                          const double* __restrict__ mesh_in,
-                                                          double* __restrict__ mesh_out)
-{
-    adj_fwd_stage_body<NF, SW<WX, WY, WZ>>(P, S, s, dt, Yin, Y0, acc, Yout, mesh_in, mesh_out);
-}
-
-// deposit of (f N) at S.pos (k_deposit's body)
-template <int NF, class SWt>
-__device__ __forceinline__ void adj_deposit_body(const DevParams& P, const DevState& S, const double* __restrict__ f,
-                                                 double* __restrict__ mesh)
-{
-    constexpr int NH = NF * NF, NS = 2 * NH;
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < S.n;
-    Stencil<double> st{};
-    double fN[NS] = {};
-    double vx = 0, vy = 0, vz = 0;
-    if (active) {
-        make_stencil<double>(P, S.pos[0][p], S.pos[1][p], S.pos[2][p], st);
-        vx = S.vhat[0][p];
-        vy = S.vhat[1][p];
-        vz = S.vhat[2][p];
+        C::values(cc, c);
+        if (s == 4 && A.xnext) {
+            double tn = 0.0;
+            rk4_push64(P, dt, v, x, tn);
 #pragma unroll
-        for (int c = 0; c < NS; c++) fN[c] = f[c * S.cap + p] * S.Nn[c / NH][p];
+            for (int d = 0; d < 3; d++) A.xnext[d * cap + p] = x[d];
+        }
+        if (A.report && stt) report_bad(A.report, stt, S.id[p]);
     }
-    tile_deposit_block<NF, SWt, double>(P, mesh, active, st, fN, vx, vy, vz,
-                                        [](double a, int) -> double { return a; }, true);
+    if (!A.mesh_out) return;
+    if (s == 4) {
+        __syncthreads();
+        slot = adj_tile<NF, T, WX, WY, WZ, RW>(P, sm, active, x, v, st);
+        rec = sm.rec + slot * RW;
+    }
+    adj_record<NF, WP>(rec, active, c);
+    if (A.diag) {
+#pragma unroll
+        for (int i = 0; i < 2 * NF; i++) sm.d[i * VS + slot] = dnum[i];
+    }
+    __syncthreads();
+    if (A.diag) deposit_comb64<NF, T, WX, WY, RW, true>(P, A.mesh_out, sm.rec, sm.key, sm.starts, sm.v, sm.d);
+    else deposit_comb64<NF, T, WX, WY, RW, false>(P, A.mesh_out, sm.rec, sm.key, sm.starts, sm.v, sm.d);
+}
+
+template <int NF, int WX, int WY, int WZ, int KS>
+__global__ void __launch_bounds__(kBlock, 4) k_adj_fwd_stage(DevParams P, DevState S, int s, double dt, AdjFwdPtrs A)
+{
+    adj_fwd_body<NF, WX, WY, WZ, KS>(P, S, s, dt, A);
 }
 
 struct AdjStagePtrs {
     const double* Ys;       // stage state Y_s (s >= 1)
     const double* Ynext;    // Y_{s+1} (Y_0 for s = 0), gathered stage
     const double* Yn;       // pre-Renormalize state (s = 4)
-    const double* mesh_s;   // forward mesh M_s (s >= 1)
+    const double* mesh_s;   // forward mesh M_s (s >= 1), combined like all meshes here
     const double* lm_in;    // adjoint mesh of stage s+1 (s < 4)
     double* lm_out;         // adjoint mesh of stage s (s >= 1), zeroed
     double* lm_zero;        // adjoint mesh zeroed for the next launch
@@ -317,177 +405,114 @@ struct AdjStagePtrs {
 // One backward launch: (s < 4) finish stage s+1 by gathering its adjoint
 // mesh, (s >= 1) start stage s: commutator VJP and the scatter of lam_H.
 // s = 4 starts from the Renormalize VJP.
-template <int NF, class SWt>
+template <int NF, int WX, int WY, int WZ, int KS>
 __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevState& S, int s, double dt,
                                                const AdjStagePtrs& A)
 {
+    using T = Tile64<NF, WX, WY, WZ, KS>;
     using H = Herm<NF>;
-    constexpr int NH = NF * NF, NS = 2 * NH;
+    using C = Comb<NF>;
+    constexpr int NH = NF * NF, NS = 2 * NH, NV = C::NV, WP = T::WP, RW = T::template row<NV>();
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    const Smem64<NF, T, RW> sm(tile_smem);
     zero_slice(A.lm_zero, A.nmesh);
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long p = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = p < S.n;
     const long long cap = S.cap;
     Stencil<double> st{};
-    double g[NS] = {};
-    double vx = 0, vy = 0, vz = 0;
+    double x[3] = {0, 0, 0}, v[3] = {0, 0, 0};
     if (active) {
-        make_stencil<double>(P, S.pos[0][p], S.pos[1][p], S.pos[2][p], st);
-        vx = S.vhat[0][p];
-        vy = S.vhat[1][p];
-        vz = S.vhat[2][p];
-        const double Nsp[2] = {S.Nn[0][p], S.Nn[1][p]};
-        double lamK[NS], ln[NS];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            x[d] = S.pos[d][p];
+            v[d] = S.vhat[d][p];
+        }
+    }
+    const int slot = adj_tile<NF, T, WX, WY, WZ, RW>(P, sm, active, x, v, st);
+    double* const rec = sm.rec + slot * RW;
+    double g[NH];
+    if (s < 4) {
+        // D^T (the transpose of the N / F deposit): G_c of nu; of nubar with
+        // the opposite sign for real components
+        interp64<NF, T, WX, WY, RW, true>(P, A.lm_in, sm.rec, sm.key, sm.v);
+        __syncthreads();
+        adj_sums<NF, WP>(rec, 1.0, g);
+        __syncthreads();
+    }
+    double lamK[NS];
+    if (active) {
         if (s == 4) {
+            const double b4 = dt * kRK4B[3];
 #pragma unroll
             for (int sp = 0; sp < 2; sp++) {
-                double y[NH], lr[NH];
+                double y[NH], lr[NH], ln[NH];
 #pragma unroll
                 for (int e = 0; e < NH; e++) {
                     y[e] = A.Yn[(sp * NH + e) * cap + p];
                     lr[e] = A.lamY0[(sp * NH + e) * cap + p];
                 }
-                renormalize_vjp<NF>(y, S.Ll[sp][p], P.maxError, lr, ln + sp * NH);
-            }
-            const double b4 = dt * kRK4B[3];
-#pragma unroll
-            for (int c = 0; c < NS; c++) {
-                A.lamn[c * cap + p] = ln[c];
-                A.lamY0[c * cap + p] = ln[c];
-                lamK[c] = b4 * ln[c];
-            }
-        } else {
-            double G[NS];
-            gather_deposit_adjoint<NF, SWt>(P, A.lm_in, st, vx, vy, vz, G);
-            double dN[2] = {0.0, 0.0};
-#pragma unroll
-            for (int c = 0; c < NS; c++) {
-                const int sp = c / NH;
-                const long long o = c * cap + p;
-                const double ly = A.lamYd[o] + Nsp[sp] * G[c];   // lam of Y_{s+1}
-                dN[sp] += A.Ynext[o] * G[c];
-                A.lamY0[o] += ly;
-                if (s >= 1) lamK[c] = dt * kRK4B[s - 1] * A.lamn[o] + dt * kRK4A[s] * ly;
-            }
-            A.lamN[p] += dN[0];
-            A.lamN[cap + p] += dN[1];
-        }
-        if (s >= 1) {
-            double V[NS];
-            potential_fp64<NF, SWt>(P, A.mesh_s, st, vx, vy, vz, S.vscale[p], V);
-            double lH[NS];
-#pragma unroll
-            for (int sp = 0; sp < 2; sp++) {
-                double y[NH], ly[NH];
-#pragma unroll
-                for (int e = 0; e < NH; e++) y[e] = A.Ys[(sp * NH + e) * cap + p];
-                commutator_vjp<NF>(V + sp * NH, y, lamK + sp * NH, lH + sp * NH, ly, P.inv_hbar);
-#pragma unroll
-                for (int e = 0; e < NH; e++) A.lamYd[(sp * NH + e) * cap + p] = ly[e];
-            }
-            // I^T: V[e] += coef inside_e, V[NH+e] += (im ? +1 : -1) coef inside_e,
-            // inside_e = SI_e (+/-) Sb_e with SI from the N/F fields of nu and
-            // Sb from those of nubar (velocity terms enter with a minus sign)
-#pragma unroll
-            for (int e = 0; e < NH; e++) {
-                const double li = P.sqrt2GF_inv_vol * (H::is_im(e) ? lH[e] + lH[NH + e] : lH[e] - lH[NH + e]);
-                g[e] = li;
-                g[NH + e] = H::is_im(e) ? li : -li;
-            }
-        }
-    }
-    if (s >= 1)
-        tile_deposit_block<NF, SWt, double>(P, A.lm_out, active, st, g, -vx, -vy, -vz,
-                                            [](double a, int) -> double { return a; });
-}
-
-template <int NF, int WX, int WY, int WZ>
-__global__ void __launch_bounds__(kBlock) k_adj_stage(DevParams P, DevState S, int s, double dt, AdjStagePtrs A)
-{
-    adj_stage_body<NF, SW<WX, WY, WZ>>(P, S, s, dt, A);
-}
-
-// Stage 4 of a recorded step with the step's completion: Y_n = acc + b4 dt K
-// (stored), Y_new = Renormalize(Y_n), positions advanced and wrapped, and
-// the deposit of Y_new at the new positions (the next step's M_1).  Same
-// arithmetic as the forward stage kernel.
-template <int NF, class SWt>
-__device__ __forceinline__ void adj_fwd_stage4_next_body(const DevParams& P, const DevState& S, double dt,
-                                                         const double* __restrict__ Y4, const double* __restrict__ acc,
-                                                         double* __restrict__ Yn, double* __restrict__ Ynext,
-                                                         double* __restrict__ xnext, const double* __restrict__ mesh_in,
-                                                         double* __restrict__ mesh_next, StepCtl* report = nullptr)
-{
-    constexpr int NH = NF * NF, NS = 2 * NH;
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < S.n;
-    const long long cap = S.cap;
-    Stencil<double> st{};
-    double fN[NS] = {};
-    double vx = 0, vy = 0, vz = 0;
-    if (active) {
-        const double x = S.pos[0][p], y = S.pos[1][p], z = S.pos[2][p];
-        make_stencil<double>(P, x, y, z, st);
-        vx = S.vhat[0][p];
-        vy = S.vhat[1][p];
-        vz = S.vhat[2][p];
-        double V[NS];
-        potential_fp64<NF, SWt>(P, mesh_in, st, vx, vy, vz, S.vscale[p], V);
-        const double bw = dt * kRK4B[3];
-        int stt = 0;
-#pragma unroll
-        for (int sp = 0; sp < 2; sp++) {
-            double f[NH], K[NH];
-#pragma unroll
-            for (int e = 0; e < NH; e++) f[e] = Y4[(sp * NH + e) * cap + p];
-            commutator<NF, double>(V + sp * NH, f, K, P.inv_hbar);
-#pragma unroll
-            for (int e = 0; e < NH; e++) {
-                const long long o = (sp * NH + e) * cap + p;
-                f[e] = __dadd_rn(__dmul_rn(bw, K[e]), acc[o]);
-                Yn[o] = f[e];
-            }
-            if (Ynext) {
-                stt |= renormalize<NF>(f, S.Ll[sp][p], P.maxError);
-                const double Ns = S.Nn[sp][p];
+                renormalize_vjp<NF>(y, S.Ll[sp][p], P.maxError, lr, ln);
 #pragma unroll
                 for (int e = 0; e < NH; e++) {
-                    Ynext[(sp * NH + e) * cap + p] = f[e];
-                    fN[sp * NH + e] = f[e] * Ns;
+                    const int q = sp * NH + e;
+                    A.lamn[q * cap + p] = ln[e];
+                    A.lamY0[q * cap + p] = ln[e];
+                    lamK[q] = b4 * ln[e];
                 }
             }
-        }
-        if (xnext) {
-            double xn[3] = {x, y, z};
-            const double kxv[3] = {vx * kC, vy * kC, vz * kC};
+        } else {
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const double w = dt * kRK4B[i];
+            for (int sp = 0; sp < 2; sp++) {
+                const double Ns = S.Nn[sp][p];
+                double dN = 0.0;
 #pragma unroll
-                for (int d = 0; d < 3; d++) xn[d] = __dadd_rn(__dmul_rn(w, kxv[d]), xn[d]);
+                for (int e = 0; e < NH; e++) {
+                    const int q = sp * NH + e;
+                    const long long o = q * cap + p;
+                    const double G = sp == 0 || H::is_im(e) ? g[e] : -g[e];
+                    const double ly = A.lamYd[o] + Ns * G;   // lam of Y_{s+1}
+                    dN += A.Ynext[o] * G;
+                    A.lamY0[o] += ly;
+                    if (s >= 1) lamK[q] = dt * kRK4B[s - 1] * A.lamn[o] + dt * kRK4A[s] * ly;
+                }
+                A.lamN[sp * cap + p] += dN;
             }
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                xn[d] = wrap_coord(xn[d], P.L[d]);
-                xnext[d * cap + p] = xn[d];
-            }
-            make_stencil<double>(P, xn[0], xn[1], xn[2], st);
         }
-        if (report) report_bad(report, stt, S.id[p]);
     }
-    if (mesh_next)
-        tile_deposit_block<NF, SWt, double>(P, mesh_next, active, st, fN, vx, vy, vz,
-                                            [](double a, int) -> double { return a; }, true);
+    if (s < 1) return;
+    interp64<NF, T, WX, WY, RW>(P, A.mesh_s, sm.rec, sm.key, sm.v);
+    __syncthreads();
+    double hs[NH], c[NV];
+    adj_sums<NF, WP>(rec, P.sqrt2GF_inv_vol, hs);
+    if (active) {
+        double li[NH];
+        const double vsc = S.vscale[p];
+#pragma unroll
+        for (int sp = 0; sp < 2; sp++) {
+            double y[NH], ly[NH], lH[NH], h[NH];
+#pragma unroll
+            for (int e = 0; e < NH; e++) y[e] = A.Ys[(sp * NH + e) * cap + p];
+            species_hamiltonian<NF>(P, hs, vsc, sp, h);
+            commutator_vjp<NF>(h, y, lamK + sp * NH, lH, ly, P.inv_hbar);
+            // I^T: V[e] += coef inside_e, V[NH+e] += (im ? +1 : -1) coef
+            // inside_e (velocity terms enter with a minus sign)
+#pragma unroll
+            for (int e = 0; e < NH; e++) {
+                A.lamYd[(sp * NH + e) * cap + p] = ly[e];
+                li[e] = sp == 0 ? lH[e] : P.sqrt2GF_inv_vol * (H::is_im(e) ? li[e] + lH[e] : li[e] - lH[e]);
+            }
+        }
+        C::values(li, c);
+    }
+    adj_record<NF, WP>(rec, active, c);
+    __syncthreads();
+    deposit_comb64<NF, T, WX, WY, RW, false, true>(P, A.lm_out, sm.rec, sm.key, sm.starts, sm.v, sm.d);
 }
 
-template <int NF, int WX, int WY, int WZ>
-__global__ void __launch_bounds__(kBlock) k_adj_fwd_stage4_next(DevParams P, DevState S, double dt,
-                                                                const double* __restrict__ Y4,
-                                                                const double* __restrict__ acc, double* __restrict__ Yn,
-                                                                double* __restrict__ Ynext, double* __restrict__ xnext,
-                                                                const double* __restrict__ mesh_in,
-                                                                double* __restrict__ mesh_next)
+template <int NF, int WX, int WY, int WZ, int KS>
+__global__ void __launch_bounds__(kBlock, 3) k_adj_stage(DevParams P, DevState S, int s, double dt, AdjStagePtrs A)
 {
-    adj_fwd_stage4_next_body<NF, SW<WX, WY, WZ>>(P, S, dt, Y4, acc, Yn, Ynext, xnext, mesh_in, mesh_next);
+    adj_stage_body<NF, WX, WY, WZ, KS>(P, S, s, dt, A);
 }
 
 // One checkpoint segment of len steps, stored step by step:
@@ -552,13 +577,30 @@ __host__ __device__ inline AdjStagePtrs seg_stage_ptrs(const SegPtrs& G, int j, 
     return A;
 }
 
+// stage s of the recompute of segment step j
+__host__ __device__ inline AdjFwdPtrs seg_fwd_ptrs(const SegPtrs& G, int j, int s, long long cap, bool next, bool more,
+                                                   StepCtl* report)
+{
+    AdjFwdPtrs A{};
+    A.Y0 = seg_f(G, j);
+    A.Yin = s == 1 ? A.Y0 : seg_y(G, j, s, cap);
+    A.acc = G.acc;
+    A.Yout = seg_y(G, j, s + 1, cap);
+    A.mesh_in = seg_m(G, j, s - 1);
+    A.mesh_out = s < 4 ? seg_m(G, j, s) : more ? seg_m(G, j + 1, 0) : nullptr;
+    A.Ynext = s == 4 && next ? seg_f(G, j + 1) : nullptr;
+    A.xnext = s == 4 && next ? seg_f(G, j + 1) + (long long)G.NS * cap : nullptr;
+    A.report = s == 4 ? report : nullptr;
+    A.diag = s == 3 && G.record;
+    return A;
+}
+
 // Forward over a whole segment in one cooperative launch (Y_0 and x of step
 // 0 and its deposit M_1 are in place; every stored mesh starts at zero):
 // four phases per step separated by bounded grid barriers.
-template <int NF, int WX, int WY, int WZ>
+template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_fwd_coop(DevParams P, DevState S, SegPtrs G, StepCtl* ctl)
 {
-    using SWt = SW<WX, WY, WZ>;
     const long long cap = S.cap;
 #pragma unroll 1
     for (int j = 0; j < G.len; j++) {
@@ -567,24 +609,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_fwd_coop(DevParams P, Dev
         // reads it before any block can reach the reduction that replaces it)
         const double dt = G.record ? __ldcg(&ctl->dt) : G.dts[G.k0 + j];
         if (G.record && blockIdx.x == 0 && threadIdx.x == 0) G.dts_out[G.k0 + j] = dt;
-        const double* Y0 = seg_f(G, j);
-#pragma unroll 1
-        for (int s = 1; s <= 3; s++) {
-            adj_fwd_stage_body<NF, SWt>(P, Q, s, dt, s == 1 ? Y0 : seg_y(G, j, s, cap), Y0, G.acc,
-                                        seg_y(G, j, s + 1, cap), seg_m(G, j, s - 1), seg_m(G, j, s));
-            grid_barrier(ctl, P.wait_polls);
-        }
-        // recording: compute_dt on the stage-4 mesh (main.cpp:193-198), the
-        // next step's dt; M_4 is complete and every block holds this step's
-        // dt, so it overlaps stage 4 and shares its barrier
-        if (G.record) dt_reduce_and_finish<NF, double>(P, seg_m(G, j, 3), ctl, DT_ADVANCE, reduce_blocks(P));
         // (recording: the state after the segment goes to slot len too)
         const bool more = j + 1 < G.len, next = more || G.record;
-        adj_fwd_stage4_next_body<NF, SWt>(P, Q, dt, seg_y(G, j, 4, cap), G.acc, seg_y(G, j, 5, cap),
-                                          next ? seg_f(G, j + 1) : nullptr,
-                                          next ? seg_f(G, j + 1) + (long long)G.NS * cap : nullptr, seg_m(G, j, 3),
-                                          more ? seg_m(G, j + 1, 0) : nullptr, G.record ? ctl : nullptr);
-        grid_barrier(ctl, P.wait_polls);
+#pragma unroll 1
+        for (int s = 1; s <= 4; s++) {
+            // recording: compute_dt on the stage-4 mesh (main.cpp:193-198), the
+            // next step's dt; M_4 is complete and every block holds this step's
+            // dt, so it overlaps stage 4 and shares its barrier
+            if (s == 4 && G.record) dt_reduce_comb64<NF>(P, seg_m(G, j, 3), ctl, reduce_blocks(P));
+            adj_fwd_body<NF, WX, WY, WZ, KS>(P, Q, s, dt, seg_fwd_ptrs(G, j, s, cap, next, more, G.record ? ctl : nullptr));
+            grid_barrier(ctl, P.wait_polls);
+        }
         if (G.record && __ldcg(&ctl->done) && more) break;   // (uniform: read after the barrier)
     }
 }
@@ -618,10 +653,9 @@ __global__ void k_time_advance(DevState S, const double* __restrict__ dts, int k
 
 // Backward over a whole segment in one cooperative launch: five phases per
 // step, last step first.
-template <int NF, int WX, int WY, int WZ>
+template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_bwd_coop(DevParams P, DevState S, SegPtrs G, StepCtl* ctl)
 {
-    using SWt = SW<WX, WY, WZ>;
     const long long cap = S.cap;
 #pragma unroll 1
     for (int j = G.len - 1; j >= 0; j--) {
@@ -629,7 +663,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_bwd_coop(DevParams P, Dev
         const double dt = G.dts[G.k0 + j];
 #pragma unroll 1
         for (int s = 4; s >= 0; s--) {
-            adj_stage_body<NF, SWt>(P, Q, s, dt, seg_stage_ptrs(G, j, s, cap));
+            adj_stage_body<NF, WX, WY, WZ, KS>(P, Q, s, dt, seg_stage_ptrs(G, j, s, cap));
             grid_barrier(ctl, P.wait_polls);
         }
     }
@@ -759,15 +793,13 @@ __global__ void k_rows_to_soa(const long long* __restrict__ id, const double* __
 
 // ---- launchers ----------------------------------------------------------------
 template <int NF>
-void launch_adj_fwd_stage_t(const DevParams& P, const DevState& S, int s, double dt, const double* Yin,
-                            const double* Y0, double* acc, double* Yout, const double* mesh_in, double* mesh_out,
+void launch_adj_fwd_stage_t(const DevParams& P, const DevState& S, int s, double dt, const AdjFwdPtrs& A,
                             cudaStream_t st)
 {
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        smem_optin(k_adj_fwd_stage<NF, WXv, WYv, WZv>, bytes);
-        k_adj_fwd_stage<NF, WXv, WYv, WZv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, s, dt, Yin, Y0, acc, Yout,
-                                                                                 mesh_in, mesh_out);
+    EMU_W64_DISPATCH(P, {
+        constexpr int bytes = stage64_smem<NF, Tile64<NF, WXv, WYv, WZv, KSv>>();
+        smem_optin(k_adj_fwd_stage<NF, WXv, WYv, WZv, KSv>, bytes);
+        k_adj_fwd_stage<NF, WXv, WYv, WZv, KSv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, s, dt, A);
     });
 }
 
@@ -775,10 +807,10 @@ template <int NF>
 void launch_adj_stage_t(const DevParams& P, const DevState& S, int s, double dt, const AdjStagePtrs& A,
                         cudaStream_t st)
 {
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        smem_optin(k_adj_stage<NF, WXv, WYv, WZv>, bytes);
-        k_adj_stage<NF, WXv, WYv, WZv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, s, dt, A);
+    EMU_W64_DISPATCH(P, {
+        constexpr int bytes = stage64_smem<NF, Tile64<NF, WXv, WYv, WZv, KSv>>();
+        smem_optin(k_adj_stage<NF, WXv, WYv, WZv, KSv>, bytes);
+        k_adj_stage<NF, WXv, WYv, WZv, KSv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, s, dt, A);
     });
 }
 
@@ -806,10 +838,10 @@ template <int NF>
 bool adj_coop_fits_t(const DevParams& P, long long n)
 {
     bool ok = false;
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        ok = coop_fits<NF>(k_adj_seg_fwd_coop<NF, WXv, WYv, WZv>, bytes, n) &&
-             coop_fits<NF>(k_adj_seg_bwd_coop<NF, WXv, WYv, WZv>, bytes, n);
+    EMU_W64_DISPATCH(P, {
+        constexpr int bytes = stage64_smem<NF, Tile64<NF, WXv, WYv, WZv, KSv>>();
+        ok = coop_fits<NF>(k_adj_seg_fwd_coop<NF, WXv, WYv, WZv, KSv>, bytes, n) &&
+             coop_fits<NF>(k_adj_seg_bwd_coop<NF, WXv, WYv, WZv, KSv>, bytes, n);
     });
     return ok;
 }
@@ -819,12 +851,12 @@ cudaError_t launch_adj_seg_coop_t(bool forward, const DevParams& P, const DevSta
                                   StepCtl* ctl, cudaStream_t st)
 {
     cudaError_t err = cudaSuccess;
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        smem_optin(k_adj_seg_fwd_coop<NF, WXv, WYv, WZv>, bytes);
-        smem_optin(k_adj_seg_bwd_coop<NF, WXv, WYv, WZv>, bytes);
-        const void* kern = forward ? (const void*)k_adj_seg_fwd_coop<NF, WXv, WYv, WZv>
-                                   : (const void*)k_adj_seg_bwd_coop<NF, WXv, WYv, WZv>;
+    EMU_W64_DISPATCH(P, {
+        constexpr int bytes = stage64_smem<NF, Tile64<NF, WXv, WYv, WZv, KSv>>();
+        smem_optin(k_adj_seg_fwd_coop<NF, WXv, WYv, WZv, KSv>, bytes);
+        smem_optin(k_adj_seg_bwd_coop<NF, WXv, WYv, WZv, KSv>, bytes);
+        const void* kern = forward ? (const void*)k_adj_seg_fwd_coop<NF, WXv, WYv, WZv, KSv>
+                                   : (const void*)k_adj_seg_bwd_coop<NF, WXv, WYv, WZv, KSv>;
         DevParams Pc = P;
         DevState Sc = S;
         SegPtrs Gc = G;
@@ -833,19 +865,6 @@ cudaError_t launch_adj_seg_coop_t(bool forward, const DevParams& P, const DevSta
         err = cudaLaunchCooperativeKernel(kern, dim3(grid_for(S.n)), dim3(kBlock), args, bytes, st);
     });
     return err;
-}
-
-template <int NF>
-void launch_adj_fwd_stage4_next_t(const DevParams& P, const DevState& S, double dt, const double* Y4,
-                                  const double* acc, double* Yn, double* Ynext, double* xnext, const double* mesh_in,
-                                  double* mesh_next, cudaStream_t st)
-{
-    EMU_W_DISPATCH(P, {
-        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        smem_optin(k_adj_fwd_stage4_next<NF, WXv, WYv, WZv>, bytes);
-        k_adj_fwd_stage4_next<NF, WXv, WYv, WZv><<<grid_for(S.n), kBlock, bytes, st>>>(P, S, dt, Y4, acc, Yn, Ynext,
-                                                                                       xnext, mesh_in, mesh_next);
-    });
 }
 
 // two flavors only: the three-flavor backward body needs more than the
@@ -871,20 +890,11 @@ cudaError_t launch_adj_seg_coop(int nf, bool forward, const DevParams& P, const 
     return nf == 2 ? launch_adj_seg_coop_t<2>(forward, P, S, G, ctl, st) : cudaErrorInvalidValue;
 }
 
-void launch_adj_fwd_stage4_next(int nf, const DevParams& P, const DevState& S, double dt, const double* Y4,
-                                const double* acc, double* Yn, double* Ynext, double* xnext, const double* mesh_in,
-                                double* mesh_next, cudaStream_t st)
-{
-    if (nf == 2) launch_adj_fwd_stage4_next_t<2>(P, S, dt, Y4, acc, Yn, Ynext, xnext, mesh_in, mesh_next, st);
-    else launch_adj_fwd_stage4_next_t<3>(P, S, dt, Y4, acc, Yn, Ynext, xnext, mesh_in, mesh_next, st);
-}
-
-void launch_adj_fwd_stage(int nf, const DevParams& P, const DevState& S, int s, double dt, const double* Yin,
-                          const double* Y0, double* acc, double* Yout, const double* mesh_in, double* mesh_out,
+void launch_adj_fwd_stage(int nf, const DevParams& P, const DevState& S, int s, double dt, const AdjFwdPtrs& A,
                           cudaStream_t st)
 {
-    if (nf == 2) launch_adj_fwd_stage_t<2>(P, S, s, dt, Yin, Y0, acc, Yout, mesh_in, mesh_out, st);
-    else launch_adj_fwd_stage_t<3>(P, S, s, dt, Yin, Y0, acc, Yout, mesh_in, mesh_out, st);
+    if (nf == 2) launch_adj_fwd_stage_t<2>(P, S, s, dt, A, st);
+    else launch_adj_fwd_stage_t<3>(P, S, s, dt, A, st);
 }
 
 void launch_adj_stage(int nf, const DevParams& P, const DevState& S, int s, double dt, const AdjStagePtrs& A,
@@ -916,6 +926,11 @@ void launch_adj_nex(int nf, const DevParams& P, const double* mesh, double* lm, 
 namespace {
 
 long long mesh_elems(const emu_context* c) { return c->P.ncells * c->ND; }
+// a combined mesh of the recompute and the sweep
+long long cmesh_elems(const emu_context* c)
+{
+    return c->P.ncells * (c->nf == 3 ? emu::kCombSlots<3> : emu::kCombSlots<2>);
+}
 
 void free_adj(emu_adjoint* a)
 {
@@ -986,7 +1001,7 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
     const long long cap = ctx->cap;
     const int NS = ctx->NS;
     const int nck = (nsteps + interval - 1) / interval;
-    const long long nm = mesh_elems(ctx);
+    const long long nm = cmesh_elems(ctx);
     emu_adjoint* a = ctx->adj;
     if (a && (a->cap != cap || a->NS != NS || a->ck_slots < nck || a->interval_cap < interval ||
               (int)a->dts.size() < nsteps || (a->full && a->full_steps < nsteps))) {
@@ -1013,7 +1028,9 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         const size_t per_step = sizeof(double) * ((size_t)4 * NS * cap + (size_t)4 * nm);
         a->store = (size_t)interval * per_step <= budget;
         const char* fenv = std::getenv("EMU_ADJOINT_FULL_STORE");
-        a->full = a->store && (!fenv || std::atoi(fenv) != 0) &&
+        // (the recorded forward takes dt from combined meshes: no adaptive
+        // timestep there)
+        a->full = a->store && (!fenv || std::atoi(fenv) != 0) && !(ctx->prm.max_adaptive_speedup > 1.0) &&
                   emu::adj_coop_fits(ctx->nf, ctx->P, ctx->S[ctx->cur].n) &&
                   (size_t)nsteps * (per_step + sizeof(double) * slot) <= budget;
         a->full_steps = a->full ? nsteps : 0;
@@ -1066,7 +1083,8 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         CU(alloc(&a->mst, sizeof(double) * st_steps * 4 * nm));
         // acc, lamY0, lamn, lamYd, wf, lamtmp: 6 NS; lamN 2, lamtmp 2; wpos 3; wtime 1
         CU(alloc(&a->work, sizeof(double) * (size_t)(6 * NS + 8) * cap));
-        for (int i = 0; i < 4; i++) CU(alloc(&a->lmesh[i], sizeof(double) * nm));
+        // (full size: the objective's deposit and gather are in the full layout)
+        for (int i = 0; i < 4; i++) CU(alloc(&a->lmesh[i], sizeof(double) * mesh_elems(ctx)));
         CU(alloc(&a->nex, sizeof(double) * 2 * ctx->P.ncells));
         CU(alloc(&a->rows, sizeof(double) * (size_t)NS * cap));
         for (int i = 0; i < 2; i++) CU(alloc(&a->map[i], sizeof(unsigned) * cap));
@@ -1127,11 +1145,20 @@ int check_ready(emu_context* ctx, const char* who)
     return EMU_OK;
 }
 
-// deposit of (f, x) into mesh (zeroed first)
+// full deposit of (f, x) into mesh (zeroed first)
 int deposit_into(emu_context* ctx, const DevState& S, const double* f, double* mesh)
 {
     CU(cudaMemsetAsync(mesh, 0, sizeof(double) * mesh_elems(ctx), ctx->stream));
     emu::launch_deposit(ctx->nf, ctx->P, S, f, mesh, ctx->stream);
+    return check_launch(ctx, "adjoint deposit");
+}
+
+// combined deposit of (f, x) into mesh
+int deposit_comb_into(emu_context* ctx, DevState S, const double* f, double* mesh)
+{
+    CU(cudaMemsetAsync(mesh, 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
+    S.f0 = const_cast<double*>(f);
+    emu::launch_deposit_comb64(ctx->nf, ctx->P, S, mesh, nullptr, ctx->stream);
     return check_launch(ctx, "adjoint deposit");
 }
 
@@ -1146,7 +1173,7 @@ int segment_sweep(emu_context* ctx, const DevState& W, const emu::SegPtrs& G, bo
     cudaStream_t st = ctx->stream;
     int r;
     if (!meshes_given &&
-        (r = deposit_into(ctx, emu::seg_state(W, G, 0), emu::seg_f(G, 0), emu::seg_m(G, 0, 0))))
+        (r = deposit_comb_into(ctx, emu::seg_state(W, G, 0), emu::seg_f(G, 0), emu::seg_m(G, 0, 0))))
         return r;
     if (coop) {
         cudaError_t e = emu::launch_adj_seg_coop(nf, true, ctx->P, W, G, ctx->ctl, st);
@@ -1157,16 +1184,12 @@ int segment_sweep(emu_context* ctx, const DevState& W, const emu::SegPtrs& G, bo
     for (int j = 0; j < G.len; j++) {
         const DevState Q = emu::seg_state(W, G, j);
         const double dt = ctx->adj->dts[G.k0 + j];
-        const double* Y0 = emu::seg_f(G, j);
-        for (int s = 1; s <= 3; s++)
-            emu::launch_adj_fwd_stage(nf, ctx->P, Q, s, dt, s == 1 ? Y0 : emu::seg_y(G, j, s, cap), Y0, G.acc,
-                                      emu::seg_y(G, j, s + 1, cap), emu::seg_m(G, j, s - 1),
-                                      meshes_given ? nullptr : emu::seg_m(G, j, s), st);
         const bool more = j + 1 < G.len;
-        emu::launch_adj_fwd_stage4_next(nf, ctx->P, Q, dt, emu::seg_y(G, j, 4, cap), G.acc, emu::seg_y(G, j, 5, cap),
-                                        more ? emu::seg_f(G, j + 1) : nullptr,
-                                        more ? emu::seg_f(G, j + 1) + (long long)G.NS * cap : nullptr,
-                                        emu::seg_m(G, j, 3), more ? emu::seg_m(G, j + 1, 0) : nullptr, st);
+        for (int s = 1; s <= 4; s++) {
+            emu::AdjFwdPtrs A = emu::seg_fwd_ptrs(G, j, s, cap, more, more, nullptr);
+            if (meshes_given) A.mesh_out = nullptr;
+            emu::launch_adj_fwd_stage(nf, ctx->P, Q, s, dt, A, st);
+        }
     }
     for (int j = G.len - 1; j >= 0; j--) {
         const DevState Q = emu::seg_state(W, G, j);
@@ -1185,7 +1208,7 @@ int segment_sweep(emu_context* ctx, const DevState& W, const emu::SegPtrs& G, bo
 int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
 {
     const int NS = ctx->NS;
-    const long long cap = ctx->cap, nm = mesh_elems(ctx);
+    const long long cap = ctx->cap, nm = cmesh_elems(ctx);
     cudaStream_t st = ctx->stream;
     int r;
     emu::SegPtrs G{};
@@ -1214,7 +1237,7 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
         G.k0 = k0;
         G.len = len;
         CU(cudaMemsetAsync(G.mst, 0, sizeof(double) * (size_t)len * 4 * nm, st));
-        if ((r = deposit_into(ctx, emu::seg_state(S, G, 0), emu::seg_f(G, 0), emu::seg_m(G, 0, 0)))) return r;
+        if ((r = deposit_comb_into(ctx, emu::seg_state(S, G, 0), emu::seg_f(G, 0), emu::seg_m(G, 0, 0)))) return r;
         cudaError_t e = emu::launch_adj_seg_coop(ctx->nf, true, ctx->P, S, G, ctx->ctl, st);
         if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("recorded segment: ") + cudaGetErrorString(e));
         emu::launch_time_advance(S, a->dts_dev, k0, len, st);
@@ -1226,10 +1249,11 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
     }
     // the context as after the step loop: the new state's deposit in mesh 0,
     // the last step's stage-4 mesh as the current mesh
-    if ((r = deposit_into(ctx, ctx->S[ctx->cur], ctx->S[ctx->cur].f0, ctx->mesh[0]))) return r;
-    CU(cudaMemsetAsync(ctx->mesh[1], 0, sizeof(double) * nm, st));
-    CU(cudaMemcpyAsync(ctx->mesh[3], a->mst + (size_t)(nsteps - 1) * G.mst_stride + 3 * nm, sizeof(double) * nm,
-                       cudaMemcpyDeviceToDevice, st));
+    const DevState& S = ctx->S[ctx->cur];
+    const int last = nsteps - (nseg - 1) * interval - 1;   // (the last step in its segment)
+    if ((r = deposit_into(ctx, S, S.f0, ctx->mesh[0]))) return r;
+    CU(cudaMemsetAsync(ctx->mesh[1], 0, sizeof(double) * mesh_elems(ctx), st));
+    if ((r = deposit_into(ctx, emu::seg_state(S, G, last), emu::seg_y(G, last, 4, cap), ctx->mesh[3]))) return r;
     ctx->cur_mesh = 3;
     if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
     return EMU_OK;
@@ -1388,7 +1412,7 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     const int NS = ctx->NS, nf = ctx->nf;
     cudaStream_t st = ctx->stream;
     const unsigned g = (unsigned)((n + emu::kBlock - 1) / emu::kBlock);
-    const long long nm = mesh_elems(ctx);
+    const long long nm = cmesh_elems(ctx);
 
     // adjoint state of the final (renormalised) state, in the final slot order
     CU(cudaMemcpyAsync(a->rows, lam_f_final, sizeof(double) * (size_t)n * NS, cudaMemcpyHostToDevice, st));
@@ -1523,14 +1547,14 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
                 CU(cudaMemcpyAsync(rp, slot + (size_t)NS * cap, sizeof(double) * 3 * cap, cudaMemcpyDeviceToDevice,
                                    st));
                 CU(cudaMemsetAsync(m2, 0, sizeof(double) * nm, st));
-                return deposit_into(ctx, Rv(), rf, m1);
+                return deposit_comb_into(ctx, Rv(), rf, m1);
             };
             // one step: stage s reads q[s-1], deposits into q[s] and zeroes
             // q[s+1] (q[4], q[5]: M_1 and M_2 of the next step)
             auto advance_q = [&](double* const q[6]) {
                 const DevState R = Rv();
                 for (int s = 1; s <= 4; s++)
-                    emu::launch_rk4_stage(nf, ctx->P, R, s, q[s - 1], q[s], q[s + 1], nm, ctx->ctl, -1, st);
+                    emu::launch_stage64(nf, ctx->P, R, s, q[s - 1], q[s], q[s + 1], nullptr, ctx->ctl, -1, st);
             };
             double* const Mr[6] = {M[0], M[1], M[2], M[3], M[0], M[1]};   // the context's rotating meshes
             auto advance = [&]() { advance_q(Mr); };
@@ -1631,11 +1655,11 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
                 CU(cudaMemcpyAsync(a->wpos, slot + (size_t)NS * cap, sizeof(double) * 3 * cap,
                                    cudaMemcpyDeviceToDevice, st));
                 CU(cudaMemsetAsync(M[1], 0, sizeof(double) * nm, st));
-                return deposit_into(ctx, R, R.f0, M[0]);
+                return deposit_comb_into(ctx, R, R.f0, M[0]);
             };
             auto advance = [&]() {
                 for (int s = 1; s <= 4; s++)
-                    emu::launch_rk4_stage(nf, ctx->P, R, s, M[s - 1], M[s % 4], M[(s + 1) % 4], nm, ctx->ctl, -1, st);
+                    emu::launch_stage64(nf, ctx->P, R, s, M[s - 1], M[s % 4], M[(s + 1) % 4], nullptr, ctx->ctl, -1, st);
             };
             if (nsub > 1) {
                 if ((r = restore(slot_f(a, a->ck, seg)))) return r;
@@ -1691,7 +1715,7 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     CU(cudaMemcpyAsync(lam_N0, a->rows, sizeof(double) * (size_t)n * 2, cudaMemcpyDeviceToHost, st));
     // the forward meshes were reused: restore the current state's deposit
     double* const* M = ctx->mesh;
-    CU(cudaMemsetAsync(M[1], 0, sizeof(double) * nm, st));
+    CU(cudaMemsetAsync(M[1], 0, sizeof(double) * mesh_elems(ctx), st));
     if ((r = deposit_into(ctx, S, S.f0, M[0]))) return r;
     ctx->cur_mesh = 0;
     CU(cudaStreamSynchronize(st));

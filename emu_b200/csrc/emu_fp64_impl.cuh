@@ -127,8 +127,9 @@ __device__ __forceinline__ void run_starts(const int* skey, unsigned* starts)
 
 // The interpolated, velocity-weighted sums u_j = G_0j - v . G_dj of the
 // warp's 32 slots, from the combined mesh, into the records' values
-// (rec + WP + j).  sv: v per slot and dimension, rows of VS.
-template <int NF, class T, int WX, int WY, int RW>
+// (rec + WP + j).  sv: v per slot and dimension, rows of VS.  PLUS: G_0 + v . G_d
+// (the transpose of a deposit, see emu_adjoint.cu).
+template <int NF, class T, int WX, int WY, int RW, bool PLUS = false>
 __device__ __forceinline__ void interp64(const DevParams& P, const double* __restrict__ mesh, double* srec,
                                          const int* skey, const double* sv)
 {
@@ -182,7 +183,8 @@ __device__ __forceinline__ void interp64(const DevParams& P, const double* __res
             // (the rows of other stencils: not theirs)
             if ((mine >> (8 * g + row)) & 1u) {
                 const int s = base + 8 * g + row;
-                const double vx = sv[s], vy = sv[VS + s], vz = sv[2 * VS + s];
+                const double sg = PLUS ? -1.0 : 1.0;
+                const double vx = sg * sv[s], vy = sg * sv[VS + s], vz = sg * sv[2 * VS + s];
                 if constexpr (NF == 2) {
                     r[WP + col] = ((c[0][0] - vx * c[0][1]) - vy * c[1][0]) - vz * c[1][1];
                 } else {
@@ -281,8 +283,9 @@ struct NoAdd {
 };
 
 // the combined deposit of the CTA's records (values c_j at rec + WP + j; sv:
-// v per slot; sd: with DIAG the 2 NF diagonal numbers per slot, rows of VS)
-template <int NF, class T, int WX, int WY, int RW, bool DIAG>
+// v per slot; sd: with DIAG the 2 NF diagonal numbers per slot, rows of VS).
+// MINUS: fluxes with -v (the transpose of an interpolation)
+template <int NF, class T, int WX, int WY, int RW, bool DIAG, bool MINUS = false>
 __device__ __forceinline__ void deposit_comb64(const DevParams& P, double* mesh, const double* srec, const int* skey,
                                                const unsigned* starts, const double* sv, const double* sd)
 {
@@ -294,7 +297,8 @@ __device__ __forceinline__ void deposit_comb64(const DevParams& P, double* mesh,
         const int q = (n >> 1) + 4 * (n & 1);
         const double c = srec[s * RW + WP + q % NV];
         const int d = (8 * nt + q) / NV;   // (three flavors: uniform over the warp)
-        return d == 0 ? c : c * sv[(d - 1) * VS + s];
+        const double f = sv[(d > 0 ? d - 1 : 0) * VS + s];
+        return d == 0 ? c : MINUS ? -(c * f) : c * f;
     };
     auto add = [&](long long cell, int q, double x) { atomic_add_mesh(mesh + cell * NCS + 8 * nt + q, x); };
     if constexpr (DIAG) {
@@ -661,11 +665,11 @@ __global__ void __launch_bounds__(kBlock, 4)
     constexpr int NH = NF * NF, NV = C::NV, WP = T::WP, VS = T::VS, RW = T::template row<NV>();
     extern __shared__ __align__(16) unsigned char tile_smem[];
     Smem64<NF, T, RW> sm(tile_smem);
-    const int mode = ctl->m4_full;
+    const int mode = ctl ? ctl->m4_full : 0;
     const int t = threadIdx.x;
     const long long p = (long long)blockIdx.x * kBlock + t;
     const bool active = p < S.n;
-    if (active) S.rslot[p] = t;   // in cell order: the identity rank
+    if (active && ctl) S.rslot[p] = t;   // in cell order: the identity rank
     if (mode == 2) return;        // (the run had ended before this step: the mesh stands)
     Stencil<double> st{};
     int key = -1;

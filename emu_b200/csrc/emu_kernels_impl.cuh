@@ -993,35 +993,39 @@ __global__ void __launch_bounds__(kBlock, 4) k_rk4_stage(DevParams P, DevState S
     rk4_stage_body<NF, SW<WX, WY, WZ>>(P, S, s, mesh_in, mesh_out, mesh_zero, nzero, ctl, dt, dt_mode);
 }
 
-// Grid-wide barrier of the cooperative step kernel (its CTAs are co-resident
-// by cooperative launch).  The wait is bounded: after `polls` polls (64 ns
-// sleeps; DevParams::wait_polls, kBarrierSpins unless a caller set another
-// limit) the CTA records ST_TIMEOUT in the step status and continues, so a
-// failure can never hang the GPU.  The results of a step that timed out are
-// invalid; every memory index of the step is computed from wrapped
-// positions and CTA-local ranks, so they stay in bounds whatever the data.
+// Grid-wide barrier of the cooperative kernels (their CTAs are co-resident
+// by cooperative launch).  The wait is bounded: after `polls` polls
+// (DevParams::wait_polls, kBarrierSpins unless a caller set another limit)
+// the CTA records ST_TIMEOUT in the step status and continues, so a failure
+// can never hang the GPU.  The results of a step that timed out are invalid;
+// every memory index of the step is computed from wrapped positions and
+// CTA-local ranks, so they stay in bounds whatever the data.  (Release and
+// acquire on the counter and the generation, no fences and no sleep between
+// polls: 2450 clocks over 148 CTAs where fences took 3060.)
 __device__ __forceinline__ void grid_barrier(StepCtl* ctl, long long polls)
 {
+    unsigned g = 0;
+    // (the generation cannot change before this CTA arrives)
+    if (threadIdx.x == 0) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(&ctl->bar_gen) : "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* genp = &ctl->bar_gen;
-        const unsigned g = *genp;
-        __threadfence();
-        if (atomicAdd(&ctl->bar_count, 1u) == gridDim.x - 1) {
-            ctl->bar_count = 0u;
-            __threadfence();
-            atomicAdd(&ctl->bar_gen, 1u);
+        unsigned n;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(n) : "l"(&ctl->bar_count) : "memory");
+        if (n == gridDim.x - 1) {
+            asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(&ctl->bar_count) : "memory");
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_gen) : "memory");
         } else {
             long long it = 0;
-            while (*genp == g) {
+            for (;;) {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->bar_gen) : "memory");
+                if (v != g) break;
                 if (++it > polls) {
                     atomicOr(&ctl->status, ST_TIMEOUT);
                     break;
                 }
-                __nanosleep(64);
             }
         }
-        __threadfence();
     }
     __syncthreads();
 }
