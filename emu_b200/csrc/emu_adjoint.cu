@@ -1306,6 +1306,8 @@ int emu_adjoint_forward(emu_context* ctx, int nsteps, int checkpoint_interval, d
         if ((r = record_full(ctx, a, nsteps, checkpoint_interval))) return r;
     } else {
     emu::launch_ctl_hist(ctx->ctl, a->dts_dev, ctx->stream);   // the step kernels record their dt
+    // (only the last step's stage-4 mesh can be read)
+    if (ctx->steps1d || ctx->comb64) emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
     // cell re-sorts on the step loop's schedule; the backward recomputes each
     // segment in its start order, so a segment's re-sorts are composed into
     // one map (slot -> slot at the segment start) that the backward undoes at

@@ -716,6 +716,18 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     ctx->comb64 = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                   !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d;
     if ((ctx->steps1d || ctx->comb64) && (r = ensure_cmesh(ctx))) return r;
+    if (ctx->auto_resort) {
+        // a 27-cell stencil loses its per-CTA cell runs within a step or two
+        // once particles leave their cells, a 1D stencil within several.  FP64
+        // stages in a plane re-sort every step too, since the re-sort is made
+        // by stage 4's stores (90 x 77 cells x 60 directions: 445 us per step
+        // at 1, 457 at 2, 498 at 4, 577 at 16)
+        const int cells = ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2];
+        ctx->prm.resort_interval = cells > (ctx->comb64 ? 3 : 9) ? 1 : 16;
+    }
+    // with a re-sort after every step, the deposits of stages 1-3 see
+    // cell-sorted particles; otherwise every deposit ranks its keys
+    ctx->P.rank_stages = ctx->prm.resort_interval != 1;
     ctx->loaded = true;
     ctx->adj_valid = false;
     ctx->steps_since_sort = 0;
@@ -760,16 +772,7 @@ int emu_create(const emu_params* p, emu_context** out)
     ctx->nreal = emu_nreal(ctx->nf);
     ctx->mixed = p->precision == EMU_PREC_MIXED;
     emu::make_devparams(*p, ctx->P);
-    if (ctx->prm.resort_interval < 0) {
-        // automatic: a 27-cell stencil loses its per-CTA cell runs within a
-        // step or two once particles leave their cells, a 1D stencil within
-        // several
-        const int cells = ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2];
-        ctx->prm.resort_interval = cells > 9 ? 1 : 16;
-    }
-    // with a re-sort after every step, the deposits of stages 1-3 see
-    // cell-sorted particles; otherwise every deposit ranks its keys
-    ctx->P.rank_stages = ctx->prm.resort_interval != 1;
+    ctx->auto_resort = ctx->prm.resort_interval < 0;
     int r = EMU_OK;
     auto bail = [&](int code) {
         g_host_err = ctx->err;
@@ -1023,9 +1026,12 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
     if (!ctx->loaded) return fail(ctx, EMU_ERR_STATE, "emu_step: no particles loaded");
     if (!(dt >= 0.0) || !std::isfinite(dt)) return fail(ctx, EMU_ERR_ARG, "emu_step: dt must be finite and >= 0");
     int r;
+    bool fuse = false;
     emu::launch_ctl_set(ctx->ctl, dt, 0.0, INFINITY, 1, 1, ctx->stream);
     if (rk4_fused(ctx)) {
         if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+        // (FP64 stages: a re-sort due after the step is made by its stage 4)
+        fuse = ctx->comb64 && ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
         if (ctx->steps1d) {
             r = run_steps_1d(ctx, 1, -1);
         } else if (ctx->coop) {
@@ -1036,7 +1042,7 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
                                                                       cudaGetErrorString(e));
         } else {
             r = ctx->mixed    ? enqueue_rk4_mixed(ctx, ctx->stream, false)
-                : ctx->comb64 ? enqueue_rk4_comb64(ctx, ctx->stream, false)
+                : ctx->comb64 ? enqueue_rk4_comb64(ctx, ctx->stream, false, !fuse)
                               : enqueue_rk4_fp64(ctx, ctx->stream, false);
         }
         if (r) return r;
@@ -1048,7 +1054,7 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
         if ((r = step_generic(ctx, dt))) return r;
     }
     if (++ctx->steps_since_sort >= ctx->prm.resort_interval && ctx->prm.resort_interval > 0)
-        if ((r = resort(ctx))) return r;
+        if ((r = resort(ctx, fuse))) return r;
     if ((r = sync_ctl(ctx))) return r;
     return status_of(ctx, bad);
 }

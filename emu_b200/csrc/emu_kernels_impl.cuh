@@ -25,8 +25,7 @@
 // TSC, (0,0,0) generic runtime widths.
 #pragma once
 #include "emu_kernels.cuh"
-
-#include <cub/block/block_radix_sort.cuh>
+#include "emu_tile64.cuh"
 
 #include <climits>
 #include <cstdio>
@@ -446,103 +445,6 @@ __device__ __forceinline__ void combine_species(const float* fN, float* v)
 #pragma unroll
     for (int e = 0; e < NH; e++) c[e] = Herm<NF>::is_im(e) ? fN[e] + fN[NH + e] : fN[e] - fN[NH + e];
     Comb<NF>::values(c, v);
-}
-
-// Stable rank of the stencil keys held by the first NW warps of the block
-// (key -1 = inactive, ranked last): the permutation a stable sort of the
-// keys gives, by a counting sort over the distinct keys when the warps hold
-// at most 32 (warp, key) groups (cell-sorted particles that moved a few
-// cells: the usual case).  Group leaders list their keys, one warp sorts the
-// list (bitonic, shuffles) and drops repeats, every thread finds its key's
-// bucket by binary search, and one warp scans the (bucket, warp) counts.
-// Every thread of the block calls it; the result is uniform over the block:
-// false (nothing ranked, the caller sorts; the scratch is free again) when
-// there are more groups.  scratch: 66 + 32 NW ints; on success it is read
-// after the last barrier here, so the caller waits at a barrier before it
-// writes there.
-template <int NW>
-__device__ __forceinline__ bool distinct_key_rank(int key, int* scratch, int& slot)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const bool part = w < NW;
-    const unsigned lt = (1u << lane) - 1u;
-    int* ngroups = scratch;                                      // (warp, key) groups listed
-    int* nkeys = scratch + 1;                                    // distinct keys
-    unsigned* list = reinterpret_cast<unsigned*>(scratch + 2);   // [32] group keys
-    unsigned* ukey = list + 32;                                  // [32] sorted distinct keys
-    int* cnt = scratch + 66;                                     // [NW][32] counts, then bases
-    if (threadIdx.x == 0) *ngroups = 0;
-    if (part) cnt[w * 32 + lane] = 0;
-    __syncthreads();
-    const unsigned k = key >= 0 ? (unsigned)key : 0xffffffffu;   // inactive last
-    unsigned peers = 0u;
-    if (part) {
-        peers = __match_any_sync(kFull, k);
-        if ((peers & lt) == 0u) {
-            const int i = atomicAdd(ngroups, 1);
-            if (i < 32) list[i] = k;
-        }
-    }
-    __syncthreads();
-    const int ng = *ngroups;
-    if (ng > 32) {
-        __syncthreads();   // every thread has read the count before the caller's sort reuses the scratch
-        return false;
-    }
-    if (w == 0) {
-        unsigned v = lane < ng ? list[lane] : 0xffffffffu;
-#pragma unroll
-        for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                const unsigned o = __shfl_xor_sync(kFull, v, stride);
-                const bool up = (lane & size) == 0, lower = (lane & stride) == 0;
-                v = (lower == up) ? min(v, o) : max(v, o);
-            }
-        const unsigned prev = __shfl_up_sync(kFull, v, 1);
-        const bool first = lane == 0 || prev != v;
-        const unsigned fm = __ballot_sync(kFull, first);
-        if (first) ukey[__popc(fm & lt)] = v;
-        if (lane == 0) *nkeys = __popc(fm);
-    }
-    __syncthreads();
-    int b = 0, rank = 0;
-    if (part) {
-        int lo = 0, hi = *nkeys - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (ukey[mid] < k) lo = mid + 1;
-            else hi = mid;
-        }
-        b = lo;
-        rank = __popc(peers & lt);
-        if ((peers & lt) == 0u) cnt[w * 32 + b] = __popc(peers);
-    }
-    __syncthreads();
-    if (w == 0) {
-        // lane = bucket: base of each (bucket, warp) in bucket-major order
-        int c[NW], tot = 0;
-#pragma unroll
-        for (int i = 0; i < NW; i++) {
-            c[i] = cnt[i * 32 + lane];
-            tot += c[i];
-        }
-        int inc = tot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, inc, o);
-            if (lane >= o) inc += t;
-        }
-        int base = inc - tot;
-#pragma unroll
-        for (int i = 0; i < NW; i++) {
-            cnt[i * 32 + lane] = base;
-            base += c[i];
-        }
-    }
-    __syncthreads();
-    if (part) slot = cnt[w * 32 + b] + rank;
-    return true;
 }
 
 // sort_keys: the CTA's particles may not be in stencil order (particles
