@@ -692,7 +692,7 @@ __device__ __forceinline__ void tile_deposit_comb(const DevParams& P, T* mesh, c
 // value of slot c at SP + voff(c): the particle's f N in the full layout,
 // the values after the NV combinations in the combined one.  Eight threads
 // per record stream (BLOCK / 8 streams of NTILE / (BLOCK / 8) records), or
-// for 27-cell stencils a warp per stream with a lane per stencil cell: the
+// for 9- and 27-cell stencils a warp per stream with a lane per cell: the
 // grouping of the FP32 run sums, and so the int64 results, do not depend on
 // which layout the records have.
 template <int NF, int BLOCK, int NTILE, class SWt, class T, class Conv>
@@ -705,14 +705,14 @@ __device__ __forceinline__ void tile_deposit_diag(const DevParams& P, T* diag, c
     constexpr int NSTREAM = BLOCK / kDiagSlots;
     constexpr int CH = (NTILE + NSTREAM - 1) / NSTREAM;
     static_assert(2 * NF <= kDiagSlots, "diagonal slots");
-    if constexpr (S == 27) {
-        // 27-cell stencils: lane k of a record stream (one warp) owns stencil
-        // cell k and sums all 2 NF values there: one weight load per record
-        // and lane, one cell index per flush
+    if constexpr (S >= 9) {
+        // 9- and 27-cell stencils: lane k of a record stream (one warp) owns
+        // stencil cell k and sums all 2 NF values there: one weight load per
+        // record and lane, one cell index per flush
         constexpr int NW = BLOCK / 32, CW = (NTILE + NW - 1) / NW;
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         if (w >= NW || lane >= S) return;   // no block-wide barrier follows inside
-        const int kk = lane / 9, jj = (lane / 3) % 3, ii = lane % 3;
+        const int kk = lane / (SWt::MX * SWt::MY), jj = (lane / SWt::MX) % SWt::MY, ii = lane % SWt::MX;
         const bool on = SWt::on(P, ii, jj, kk);
         float2 acc[NF];
         auto flush = [&](int key) {
