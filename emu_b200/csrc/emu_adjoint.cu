@@ -30,6 +30,7 @@
 // states Y_2..Y_4, Y_n and meshes M_1..M_4 are recomputed before its
 // backward.  Particles keep their slot order for the whole recorded run (no
 // re-sort).
+#include "emu_adjoint.cuh"
 #include "emu_context.cuh"
 #include "emu_fp64_impl.cuh"
 
@@ -93,102 +94,6 @@ struct emu_adjoint {
 
 namespace emu {
 namespace {
-
-// ---- per-particle adjoint pieces ------------------------------------------
-
-// VJP of K = C(H, F) = -i/hbar [H, F].  With the Hermitian matrix L whose
-// trace product is the contraction with lam, Tr(L K) = sum_c lam_c K_c (L_ii =
-// lam_ii, L_ij = (lam_re + i lam_im) / 2), cyclic permutation of the trace
-// gives Tr(L C(H, F)) = Tr(C(L, H) F) = Tr(C(F, L) H): two commutators (the
-// sums over unit vectors they replace were 18 of them for three flavors, half
-// of the adjoint stage's arithmetic).
-template <int NF>
-__device__ __forceinline__ void commutator_vjp(const double* h, const double* f, const double* lam, double* lamH,
-                                               double* lamF, double inv_hbar)
-{
-    using H = Herm<NF>;
-    constexpr int NH = NF * NF;
-    double l[NH];
-#pragma unroll
-    for (int e = 0; e < NH; e++) l[e] = H::is_diag(e) ? lam[e] : 0.5 * lam[e];
-    commutator_lean<NF, double>(l, h, lamF, inv_hbar);
-    commutator_lean<NF, double>(f, l, lamH, inv_hbar);
-#pragma unroll
-    for (int e = 0; e < NH; e++)
-        if (!H::is_diag(e)) {
-            lamF[e] *= 2.0;
-            lamH[e] *= 2.0;
-        }
-}
-
-// VJP of renormalize<NF>() at input fin (one species): replays the forward
-// branch decisions with the same arithmetic.
-template <int NF>
-__device__ __forceinline__ void renormalize_vjp(const double* fin, double L, double maxError, const double* lam_out,
-                                                double* lam_in)
-{
-    using H = Herm<NF>;
-    constexpr int NH = NF * NF;
-    double f[NH];
-#pragma unroll
-    for (int e = 0; e < NH; e++) f[e] = fin[e];
-    double sumP = 0.0;
-#pragma unroll
-    for (int i = 0; i < NF; i++) sumP = __dadd_rn(sumP, f[H::re(i, i)]);
-    const double err = sumP - 1.0;
-    const bool trace_fix = fabs(err) > maxError;
-    if (trace_fix) {
-#pragma unroll
-        for (int i = 0; i < NF; i++) f[H::re(i, i)] = __dsub_rn(f[H::re(i, i)], __ddiv_rn(err, (double)NF));
-    }
-    bool clamped[NF];
-#pragma unroll
-    for (int i = 0; i < NF; i++) {
-        clamped[i] = f[H::re(i, i)] < -maxError;
-        if (clamped[i]) f[H::re(i, i)] = 0;
-    }
-    const double length = su_length<NF>(f);
-    const bool rescale = fabs(length - L) > maxError;
-    double lam[NH];
-#pragma unroll
-    for (int e = 0; e < NH; e++) lam[e] = lam_out[e];
-    if (rescale) {
-        // f' = f L / length(f):  lam_f = (L/len) lam - (L/len^2) (lam . f) grad len
-        double g[NH];
-#pragma unroll
-        for (int e = 0; e < NH; e++) g[e] = H::is_diag(e) ? 0.0 : f[e] / length;
-#pragma unroll
-        for (int l = 1; l < NF; l++) {
-            const double cl = (l == 1) ? 0.5 : 0.28867513459481287;
-            double t = 0.0;
-#pragma unroll
-            for (int i = 0; i < l; i++) t += cl * f[H::re(i, i)];
-            t -= cl * l * f[H::re(l, l)];
-#pragma unroll
-            for (int i = 0; i < l; i++) g[H::re(i, i)] += t * cl / length;
-            g[H::re(l, l)] -= t * cl * l / length;
-        }
-        double dot = 0.0;
-#pragma unroll
-        for (int e = 0; e < NH; e++) dot += lam[e] * f[e];
-        const double a = L / length, b = L / (length * length) * dot;
-#pragma unroll
-        for (int e = 0; e < NH; e++) lam[e] = a * lam[e] - b * g[e];
-    }
-#pragma unroll
-    for (int i = 0; i < NF; i++)
-        if (clamped[i]) lam[H::re(i, i)] = 0.0;
-    if (trace_fix) {
-        double m = 0.0;
-#pragma unroll
-        for (int i = 0; i < NF; i++) m += lam[H::re(i, i)];
-        m /= NF;
-#pragma unroll
-        for (int i = 0; i < NF; i++) lam[H::re(i, i)] -= m;
-    }
-#pragma unroll
-    for (int e = 0; e < NH; e++) lam_in[e] = lam[e];
-}
 
 // D^T: G_c = sum_cells w * (lm[c] + vx lm[NS+c] + vy lm[2NS+c] + vz lm[3NS+c])
 // (the transpose of the deposit's N / F layout)
@@ -939,8 +844,7 @@ void free_adj(emu_adjoint* a)
                     (void*)a->perm, (void*)a->stat, (void*)a->sst, (void*)a->mst, (void*)a->map[0], (void*)a->map[1],
                     (void*)a->wf2, (void*)a->wpos2, (void*)a->gperm, (void*)a->smap, (void*)a->smesh})
         if (p) emu_ctx::dev_free(p);
-    for (int i = 0; i < 4; i++)
-        if (a->lmesh[i]) emu_ctx::dev_free(a->lmesh[i]);
+    if (a->lmesh[0]) emu_ctx::dev_free(a->lmesh[0]);   // (one block)
     delete a;
 }
 
@@ -1031,7 +935,7 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         // (the recorded forward takes dt from combined meshes: no adaptive
         // timestep there)
         a->full = a->store && (!fenv || std::atoi(fenv) != 0) && !(ctx->prm.max_adaptive_speedup > 1.0) &&
-                  emu::adj_coop_fits(ctx->nf, ctx->P, ctx->S[ctx->cur].n) &&
+                  (ctx->steps1d || emu::adj_coop_fits(ctx->nf, ctx->P, ctx->S[ctx->cur].n)) &&
                   (size_t)nsteps * (per_step + sizeof(double) * slot) <= budget;
         a->full_steps = a->full ? nsteps : 0;
         const size_t st_steps = a->full ? (size_t)nsteps : a->store ? (size_t)interval : 1;
@@ -1084,7 +988,8 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         // acc, lamY0, lamn, lamYd, wf, lamtmp: 6 NS; lamN 2, lamtmp 2; wpos 3; wtime 1
         CU(alloc(&a->work, sizeof(double) * (size_t)(6 * NS + 8) * cap));
         // (full size: the objective's deposit and gather are in the full layout)
-        for (int i = 0; i < 4; i++) CU(alloc(&a->lmesh[i], sizeof(double) * mesh_elems(ctx)));
+        CU(alloc(&a->lmesh[0], sizeof(double) * 4 * mesh_elems(ctx)));
+        for (int i = 1; i < 4; i++) a->lmesh[i] = a->lmesh[0] + i * mesh_elems(ctx);
         CU(alloc(&a->nex, sizeof(double) * 2 * ctx->P.ncells));
         CU(alloc(&a->rows, sizeof(double) * (size_t)NS * cap));
         for (int i = 0; i < 2; i++) CU(alloc(&a->map[i], sizeof(unsigned) * cap));
@@ -1230,13 +1135,22 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
         }
         const DevState& S = ctx->S[ctx->cur];
         if ((r = save_slot(ctx, a, a->ck, c, S.f0, S.pos))) return r;
-        if ((r = save_slot(ctx, a, a->seg, k0, S.f0, S.pos))) return r;
         G.seg = a->seg + (size_t)k0 * G.seg_stride;
         G.sst = a->sst + (size_t)k0 * G.sst_stride;
         G.mst = a->mst + (size_t)k0 * G.mst_stride;
         G.k0 = k0;
         G.len = len;
         CU(cudaMemsetAsync(G.mst, 0, sizeof(double) * (size_t)len * 4 * nm, st));
+        if (ctx->steps1d) {
+            if ((r = deposit_comb_into(ctx, S, S.f0, G.mst))) return r;
+            emu::Rec1DStore rec{G.seg, G.sst, G.mst, G.seg_stride, G.sst_stride, G.mst_stride};
+            cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, S, ctx->cmesh, ctx->mesh[3], ctx->ctl, len,
+                                                 emu::DT_ADVANCE, st, &rec);
+            if (e != cudaSuccess)
+                return fail(ctx, EMU_ERR_CUDA, std::string("recorded segment: ") + cudaGetErrorString(e));
+            continue;
+        }
+        if ((r = save_slot(ctx, a, a->seg, k0, S.f0, S.pos))) return r;
         if ((r = deposit_comb_into(ctx, emu::seg_state(S, G, 0), emu::seg_f(G, 0), emu::seg_m(G, 0, 0)))) return r;
         cudaError_t e = emu::launch_adj_seg_coop(ctx->nf, true, ctx->P, S, G, ctx->ctl, st);
         if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("recorded segment: ") + cudaGetErrorString(e));
@@ -1249,14 +1163,14 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
     }
     // the context as after the step loop: the new state's deposit in mesh 0,
     // the last step's stage-4 mesh as the current mesh
+    ctx->cur_mesh = 3;
+    if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
+    if (ctx->steps1d) return EMU_OK;   // (its last step deposits the full stage-4 mesh)
     const DevState& S = ctx->S[ctx->cur];
     const int last = nsteps - (nseg - 1) * interval - 1;   // (the last step in its segment)
     if ((r = deposit_into(ctx, S, S.f0, ctx->mesh[0]))) return r;
     CU(cudaMemsetAsync(ctx->mesh[1], 0, sizeof(double) * mesh_elems(ctx), st));
-    if ((r = deposit_into(ctx, emu::seg_state(S, G, last), emu::seg_y(G, last, 4, cap), ctx->mesh[3]))) return r;
-    ctx->cur_mesh = 3;
-    if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
-    return EMU_OK;
+    return deposit_into(ctx, emu::seg_state(S, G, last), emu::seg_y(G, last, 4, cap), ctx->mesh[3]);
 }
 
 }  // namespace
@@ -1302,12 +1216,12 @@ int emu_adjoint_forward(emu_context* ctx, int nsteps, int checkpoint_interval, d
     std::fill(a->resorted.begin(), a->resorted.end(), 0);
     a->final_mapped = false;
     if ((r = emu_evolve_begin(ctx, start_time, INFINITY, nsteps))) return r;
-    if (a->full) {
-        if ((r = record_full(ctx, a, nsteps, checkpoint_interval))) return r;
-    } else {
     emu::launch_ctl_hist(ctx->ctl, a->dts_dev, ctx->stream);   // the step kernels record their dt
     // (only the last step's stage-4 mesh can be read)
     if (ctx->steps1d || ctx->comb64) emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
+    if (a->full) {
+        if ((r = record_full(ctx, a, nsteps, checkpoint_interval))) return r;
+    } else {
     // cell re-sorts on the step loop's schedule; the backward recomputes each
     // segment in its start order, so a segment's re-sorts are composed into
     // one map (slot -> slot at the segment start) that the backward undoes at
@@ -1339,8 +1253,8 @@ int emu_adjoint_forward(emu_context* ctx, int nsteps, int checkpoint_interval, d
     if (nmap > 0)
         CU(cudaMemcpyAsync(a->perm + (size_t)a->nck * a->cap, a->map[mcur], sizeof(unsigned) * n,
                            cudaMemcpyDeviceToDevice, ctx->stream));
-    emu::launch_ctl_hist(ctx->ctl, nullptr, ctx->stream);
     }
+    emu::launch_ctl_hist(ctx->ctl, nullptr, ctx->stream);
     ctx->steps_since_sort = 0;
     emu_run_info ri{};
     r = emu_evolve_end(ctx, &ri);
@@ -1464,7 +1378,19 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
             G.mst = a->mst + (size_t)k0 * G.mst_stride;
             G.k0 = k0;
             G.len = len;
-            cudaError_t e = emu::launch_adj_seg_coop(nf, false, ctx->P, W, G, ctx->ctl, st);
+            cudaError_t e;
+            if (ctx->steps1d) {
+                emu::Adj1DStore A;
+                A.rec = emu::Rec1DStore{G.seg, G.sst, G.mst, G.seg_stride, G.sst_stride, G.mst_stride};
+                A.dts = a->dts_dev + k0;
+                A.lm = a->lmesh[0];
+                A.lm_stride = mesh_elems(ctx);
+                A.lamY0 = a->lamY0;
+                A.lamN = a->lamN;
+                e = emu::launch_adjoint_1d(nf, ctx->P, W, A, ctx->ctl, len, st);
+            } else {
+                e = emu::launch_adj_seg_coop(nf, false, ctx->P, W, G, ctx->ctl, st);
+            }
             if (e != cudaSuccess)
                 return fail(ctx, EMU_ERR_CUDA, std::string("adjoint segment: ") + cudaGetErrorString(e));
             if ((r = check_launch(ctx, "adjoint segment"))) return r;

@@ -1,7 +1,8 @@
 // emu_k_steps1d.cu -- whole runs of FP64 RK4 steps of small one-dimensional
 // problems in one cooperative launch (k_steps_1d).
-#include "emu_kernels_impl.cuh"
+#include "emu_adjoint.cuh"
 #include "emu_fp64.cuh"
+#include "emu_kernels_impl.cuh"
 
 namespace emu {
 namespace {
@@ -111,7 +112,7 @@ __device__ __forceinline__ double dep_weight_periodic(const double* rec, int cel
 
 // the warp's own 16 particles (records r0..r0+15) into the global mesh:
 // particles spread over any range [lo, hi] of window cells
-template <int NF, int D>
+template <int NF, int D, bool MINUS>
 __device__ __noinline__ void deposit_spread(int nz, double* mesh, const double* srec, const double* sfn, int r0,
                                             int lo, int hi, int c0)
 {
@@ -134,7 +135,9 @@ __device__ __noinline__ void deposit_spread(int nz, double* mesh, const double* 
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int i = r0 + 4 * k + col;
-                dmma(x, y, a[k], dep_value<NF, D>(srec + i * R::RW, sfn + i * R::FW, nt, row));
+                double b = dep_value<NF, D>(srec + i * R::RW, sfn + i * R::FW, nt, row);
+                if (MINUS && (8 * nt + (row >> 1) + 4 * (row & 1)) / R::NV > 0) b = -b;
+                dmma(x, y, a[k], b);
             }
             if (x != 0.0) atomic_add_mesh(m + 8 * nt + col, x);
             if (y != 0.0) atomic_add_mesh(m + 8 * nt + col + 4, y);
@@ -180,7 +183,7 @@ __device__ __forceinline__ void steps_arrive(StepCtl* ctl)
     if (threadIdx.x == 0)
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
 }
-__device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target)
+__device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target, long long polls)
 {
     __shared__ int ok;
     if (threadIdx.x == 0) {
@@ -190,7 +193,7 @@ __device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target)
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->bar_count) : "memory");
             if (v >= target) break;
-            if (++it > kBarrierSpins) {
+            if (++it > polls) {
                 atomicOr(&ctl->status, ST_TIMEOUT);
                 good = 0;
                 break;
@@ -202,18 +205,288 @@ __device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target)
     return ok != 0;
 }
 
+// Where a warp's 16 particles of a 1D problem sit, and the products' weights.
+struct Place1D {
+    int c0 = 0, win = 0;        // the CTA's window: cells c0 .. c0 + win - 1 (periodic)
+    bool wide = false;          // the window exceeds the staging area
+    int ci0 = 0;                // first stencil cell (window index; wide, one-CTA problems: the cell)
+    double wz[3] = {0, 0, 0};
+    int wlo = 0, whi = -1;      // window cells that the warp's particles touch
+    bool narrow = false;        // at most kNarrow of them: the matrix path (one CTA: in every warp)
+    double ai[2][kNarrow / 4], ad[2][4];   // its weights: interpolation, deposit
+    int gcell[2] = {0, 0};      // deposit rows: mesh offset of cell wlo + 8 i + row
+};
+
+// r in [-nz/2, nz/2) of cell c relative to cell ref
+__device__ __forceinline__ int relative_cell(int c, int ref, int nz)
+{
+    const int half = nz >> 1;
+    int r = c - ref + half;
+    if (r < 0) r += nz;
+    if (r >= nz) r -= nz;
+    return r - half;
+}
+
+// the record's weight part and the products' weights; r: the first stencil
+// cell in the numbering of wlo, whi
+template <int NF>
+__device__ __forceinline__ void place_weights(Place1D& L, double* rec, const double* wrec, int sp, int r)
+{
+    using R = Rec1D<NF>;
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3;
+    if (sp == 0) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) rec[R::W + i] = L.wz[i];
+        *reinterpret_cast<int*>(rec + R::FIRST) = L.narrow ? r : L.ci0;
+    }
+    __syncwarp();
+    if (L.narrow) {
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+#pragma unroll
+            for (int k = 0; k < kNarrow / 4; k++)
+                L.ai[m][k] = dep_weight<NF>(wrec + (8 * m + row) * R::RW, L.wlo + 4 * k + col);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                L.ad[m][k] = dep_weight<NF>(wrec + (4 * k + col) * R::RW, L.wlo + 8 * m + row);
+        }
+    }
+}
+
+// stencil, window and weights at the position z (barrier inside).  sref: a
+// cell near the CTA's particles
+template <int NF>
+__device__ __forceinline__ void place_particles(const DevParams& P, Place1D& L, double z, bool active, int sp, int sref,
+                                                int (*swin)[16], double* rec, const double* wrec)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, nz = P.n[2];
+    int first = 0;
+    if (active) {
+        shape<double>(z * P.dxi[2], P.ord[2], first, L.wz);
+        first = wrapi(first, nz);
+    }
+    int r = relative_cell(first, sref, nz);
+    const int mn = __reduce_min_sync(kFull, active ? r : INT_MAX);
+    const int mx = __reduce_max_sync(kFull, active ? r : INT_MIN);
+    if (lane == 0) { swin[0][warp] = mn; swin[1][warp] = mx; }
+    __syncthreads();
+    const int lo = __reduce_min_sync(kFull, swin[0][lane < nwarps ? lane : 0]);
+    const int hi = __reduce_max_sync(kFull, swin[1][lane < nwarps ? lane : 0]);
+    L.c0 = sref + lo;
+    if (L.c0 < 0) L.c0 += nz;
+    if (L.c0 >= nz) L.c0 -= nz;
+    L.win = hi - lo + P.w[2];
+    L.wide = L.win > kWin;
+    r -= lo;
+    L.ci0 = L.wide ? first : r;
+    L.wlo = mn - lo;
+    L.whi = mx - lo + P.w[2] - 1;
+    L.narrow = !L.wide && mx >= mn && L.whi - L.wlo < kNarrow;
+    place_weights<NF>(L, rec, wrec, sp, r);
+    if (L.narrow) {
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            int c = L.c0 + L.wlo + 8 * m + (lane >> 2);
+            c = c >= nz ? c % nz : c;
+            L.gcell[m] = c * kCombSlots<NF>;
+        }
+    }
+}
+
+// the window of a combined mesh into shared memory (four further rows of
+// zeros: the last product's depth)
+template <int NF>
+__device__ __forceinline__ void stage_window(const Place1D& L, double* smesh, const double* mesh, int nz)
+{
+    using R = Rec1D<NF>;
+    constexpr int NG = R::NG, NCS = kCombSlots<NF>;
+    if (L.wide) return;
+    for (int i = threadIdx.x; i < (L.win + 4) * (NG / 2); i += blockDim.x) {
+        const int wl = i / (NG / 2), q = i - wl * (NG / 2);
+        int c = L.c0 + wl;
+        c = c >= nz ? c % nz : c;
+        double2 t2 = make_double2(0.0, 0.0);
+        if (wl < L.win) t2 = __ldcg(reinterpret_cast<const double2*>(mesh + c * NCS) + q);
+        *reinterpret_cast<double2*>(smesh + wl * R::MR + 2 * q) = t2;
+    }
+}
+
+// The interpolated sums u_j = G_0j - v . G_dj (PLUS: + v . G_dj) of the pair's
+// particle, both threads.  ONE: mrow holds the whole mesh, mrow_of the rows of
+// this lane's cells.
+template <int NF, bool ONE, bool PLUS>
+__device__ __forceinline__ void interp_1d(const DevParams& P, const Place1D& L, const double* mrow, const int* mrow_of,
+                                          const double* mesh, double* rec, double* wrec, int sp, bool active, double* hv)
+{
+    using R = Rec1D<NF>;
+    constexpr int NV = R::NV, NT = R::NG / 8, HV = NV / 2, NCS = kCombSlots<NF>;
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3, nz = P.n[2];
+    const double sg = PLUS ? -1.0 : 1.0;
+    if (L.narrow) {
+        double g[2][NT][2];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) g[m][nt][0] = g[m][nt][1] = 0.0;
+#pragma unroll
+        for (int k = 0; k < kNarrow / 4; k++) {
+            if (L.wlo + 4 * k > L.whi) break;   // (uniform)
+            const double* b = mrow + (ONE ? mrow_of[k] : (L.wlo + 4 * k + col) * R::MR);
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                // two flavors: column 2 e + i holds d = 2 nt + i of value e, so
+                // that a lane's two columns are one value
+                const double bv = b[NF == 2 ? (2 * nt + (row & 1)) * NV + (row >> 1) : nt * NV + row];
+#pragma unroll
+                for (int m = 0; m < 2; m++) dmma(g[m][nt][0], g[m][nt][1], L.ai[m][k], bv);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            double* r = wrec + (8 * m + row) * R::RW;
+            const double vx = sg * r[R::V + 1], vy = sg * r[R::V + 2], vz = sg * r[R::V + 3];
+            if constexpr (NF == 2) {
+                r[R::CV + col] = ((g[m][0][0] - vx * g[m][0][1]) - vy * g[m][1][0]) - vz * g[m][1][1];
+            } else {
+                double2 t2;
+                t2.x = ((g[m][0][0] - vx * g[m][1][0]) - vy * g[m][2][0]) - vz * g[m][3][0];
+                t2.y = ((g[m][0][1] - vx * g[m][1][1]) - vy * g[m][2][1]) - vz * g[m][3][1];
+                *reinterpret_cast<double2*>(r + R::CV + 2 * col) = t2;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NV; j += 2) {
+            const double2 t2 = *reinterpret_cast<const double2*>(rec + R::CV + j);
+            hv[j] = t2.x;
+            hv[j + 1] = t2.y;
+        }
+    } else {
+        double u[HV];
+#pragma unroll
+        for (int j = 0; j < HV; j++) u[j] = 0.0;
+        if (active) {
+            const double vx = sg * rec[R::V + 1], vy = sg * rec[R::V + 2], vz = sg * rec[R::V + 3];
+#pragma unroll 1
+            for (int i = 0; i < P.w[2]; i++) {
+                int cc = L.ci0 + i;
+                if (ONE || L.wide) cc = cc % nz;
+                const double wi = i == 0 ? L.wz[0] : i == 1 ? L.wz[1] : L.wz[2];
+#pragma unroll
+                for (int j = 0; j < HV; j++) {
+                    double g[4];
+#pragma unroll
+                    for (int d = 0; d < 4; d++)
+                        g[d] = !ONE && L.wide ? __ldcg(mesh + cc * NCS + d * NV + sp * HV + j)
+                                              : mrow[cc * R::MR + d * NV + sp * HV + j];
+                    u[j] += wi * (((g[0] - g[1] * vx) - g[2] * vy) - g[3] * vz);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < HV; j++) {
+            const double other = __shfl_xor_sync(kFull, u[j], 1);
+            hv[j] = sp == 0 ? u[j] : other;
+            hv[HV + j] = sp == 0 ? other : u[j];
+        }
+    }
+}
+
+// the products of a narrow warp's deposit, window cells wlo + 8 m + row: g the
+// combined values, gd the diagonal ones (diag).  MINUS: fluxes with -v
+template <int NF, bool MINUS>
+__device__ __forceinline__ void products_1d(const Place1D& L, const double* wrec, int m, bool diag,
+                                            double (*g)[2], double* gd)
+{
+    using R = Rec1D<NF>;
+    constexpr int NT = R::NG / 8, NV = R::NV;
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3, q0 = (row >> 1) + 4 * (row & 1);
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) g[nt][0] = g[nt][1] = 0.0;
+    gd[0] = gd[1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const double* r = wrec + (4 * k + col) * R::RW;
+        const double c = r[R::CV + q0 % NV];
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) {
+            const int d = (8 * nt + q0) / NV;
+            double b = c * r[R::V + d];
+            if (MINUS && d > 0) b = -b;
+            dmma(g[nt][0], g[nt][1], L.ad[m][k], b);
+        }
+        if (diag) dmma(gd[0], gd[1], L.ad[m][k], q0 < 2 * NF ? r[R::DG + (q0 < 2 * NF ? q0 : 0)] : 0.0);
+    }
+}
+
+// the warp's particles into a global combined mesh (not wide)
+template <int NF, bool MINUS>
+__device__ __forceinline__ void deposit_1d(const Place1D& L, const double* srec, const double* sfn, const double* wrec,
+                                           double* mesh, int nz, bool diag)
+{
+    using R = Rec1D<NF>;
+    constexpr int NG = R::NG, NT = NG / 8;
+    const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3, r0 = (threadIdx.x >> 5) * 16;
+    if (L.narrow) {
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            if (L.wlo + 8 * m > L.whi) break;   // (uniform)
+            double g[NT][2], gd[2];
+            products_1d<NF, MINUS>(L, wrec, m, diag, g, gd);
+            if (L.wlo + 8 * m + row <= L.whi) {
+                double* o = mesh + L.gcell[m] + col;
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++) {
+                    atomic_add_mesh(o + 8 * nt, g[nt][0]);
+                    atomic_add_mesh(o + 8 * nt + 4, g[nt][1]);
+                }
+                if (diag) {
+                    atomic_add_mesh(o + NG, gd[0]);
+                    if (NF == 3 && col < 2) atomic_add_mesh(o + NG + 4, gd[1]);
+                }
+            }
+        }
+    } else if (L.whi >= L.wlo) {
+        deposit_spread<NF, DEP_COMB, MINUS>(nz, mesh, srec, sfn, r0, L.wlo, L.whi, L.c0);
+        if (diag) deposit_spread<NF, DEP_DIAG, false>(nz, mesh, srec, sfn, r0, L.wlo, L.whi, L.c0);
+    }
+}
+// and of a wide window, value by value: this thread's half of the pair's
+template <int NF, bool MINUS>
+__device__ __forceinline__ void deposit_1d_wide(const DevParams& P, const Place1D& L, const double* rec, int sp,
+                                                double* mesh, bool diag)
+{
+    using R = Rec1D<NF>;
+    constexpr int NV = R::NV, HV = NV / 2, NG = R::NG, NCS = kCombSlots<NF>;
+#pragma unroll 1
+    for (int i = 0; i < P.w[2]; i++) {
+        double* m = mesh + (L.ci0 + i) % P.n[2] * NCS;
+        const double wi = i == 0 ? L.wz[0] : i == 1 ? L.wz[1] : L.wz[2];
+        for (int d = 0; d < 4; d++) {
+            const double wd = MINUS && d > 0 ? -(wi * rec[R::V + d]) : wi * rec[R::V + d];
+            for (int j = 0; j < HV; j++) atomic_add_mesh(m + d * NV + sp * HV + j, wd * rec[R::CV + sp * HV + j]);
+        }
+        if (diag)
+            for (int k = 0; k < NF; k++) atomic_add_mesh(m + NG + sp * NF + k, wi * rec[R::DG + sp * NF + k]);
+    }
+}
+
 // cmesh: four combined meshes (kCombSlots per cell) one after the other, M_1
 // to M_4.  npart particles per CTA (a multiple of 16), 2 npart threads.
-template <int NF, bool ONE, int MAXT>
+// REC (not ONE): a recorded run (Rec1DStore): every step's state, stage states
+// and meshes are kept, the meshes where they are stored (zeroed; M_1 of the
+// first step deposited) instead of in cmesh; the last step's M_1 is not made.
+template <int NF, bool ONE, int MAXT, bool REC>
 __global__ void __launch_bounds__(MAXT, 1)
     k_steps_1d(DevParams P, DevState S, double* __restrict__ cmesh, double* __restrict__ full, StepCtl* ctl,
-               int npart, int nsteps, int dt_mode)
+               int npart, int nsteps, int dt_mode, Rec1DStore store)
 {
     using H = Herm<NF>;
     using C = Comb<NF>;
     using R = Rec1D<NF>;
     constexpr int NH = NF * NF, NV = C::NV, NG = C::NG, NCS = kCombSlots<NF>, ND = 8 * NH, HV = NV / 2;
     constexpr int NT = NG / 8, MR = R::MR, KI = kNarrow / 4;
+    static_assert(!(ONE && REC), "recorded runs keep global meshes");
     extern __shared__ __align__(16) double smem[];
     double* const smesh = smem;                                  // ONE: two meshes, then the diagonal slots
     constexpr int kHalf = kOneCells * MR;
@@ -248,11 +521,11 @@ __global__ void __launch_bounds__(MAXT, 1)
     const int msize = ncells * NCS;
 
     // the particle (both threads of its pair), this thread's species
-    double x = 0, y = 0, z = 0, tp = 0, v[3] = {0, 0, 0}, vs = 0, Ns = 0, Ls = 1;
+    double x = 0, yy = 0, z = 0, tp = 0, v[3] = {0, 0, 0}, vs = 0, Ns = 0, Ls = 1;
     double y0[NH] = {}, acc[NH] = {}, f[NH] = {};
     if (active) {
         x = S.pos[0][p];
-        y = S.pos[1][p];
+        yy = S.pos[1][p];
         z = S.pos[2][p];
         tp = S.time[p];
 #pragma unroll
@@ -277,108 +550,53 @@ __global__ void __launch_bounds__(MAXT, 1)
             if (c < ncells && q < NG) smesh[i] = cmesh[c * NCS + q];
         }
         if (tid < NCS) spart[kOnePart * NCS + tid] = 0.0;
-    } else {
+    } else if constexpr (!REC) {
         // (M_2's mesh is clean at a step boundary)
         for (int i = gtid; i < msize; i += nthreads) cmesh[2 * msize + i] = 0.0;
     }
-    int c0 = 0, win = 0;        // window: cells c0 .. c0 + win - 1 (wrapped)
-    bool wide = false;          // the window exceeds the staging area
-    int ci0 = 0;                // first stencil cell (window index; wide, ONE: cell)
-    double wz[3] = {0, 0, 0};
-    int wlo = 0, whi = -1;      // window cells that the warp's particles touch
-    bool narrow = false;        // at most kNarrow of them: the matrix path (ONE: in every warp)
-    double ai[2][KI], ad[2][4]; // its weights: interpolation, deposit
+    Place1D L;
     int mrow_of[KI] = {};       // (ONE) mesh rows of the interpolation's cells
-    int gcell[2] = {0, 0};      // deposit rows: mesh offset of cell wlo + 8 i + row
-
-    // r in [-nz/2, nz/2) of cell c relative to cell ref
-    auto relative = [&](int c, int ref) {
-        const int half = nz >> 1;
-        int r = c - ref + half;
-        if (r < 0) r += nz;
-        if (r >= nz) r -= nz;
-        return r - half;
-    };
     // stencil, window, weights and the weight part of the record, at the
     // position z
     auto locate = [&]() {
-        int first = 0;
-        if (active) {
-            shape<double>(z * P.dxi[2], P.ord[2], first, wz);
-            first = wrapi(first, nz);
-        }
-        int r = 0;
         if constexpr (!ONE) {
-            // relative to the first particle's cell at the launch
-            r = relative(first, sref);
-            const int mn = __reduce_min_sync(kFull, active ? r : INT_MAX);
-            const int mx = __reduce_max_sync(kFull, active ? r : INT_MIN);
-            if (lane == 0) { swin[0][warp] = mn; swin[1][warp] = mx; }
-            __syncthreads();
-            const int lo = __reduce_min_sync(kFull, swin[0][lane < nwarps ? lane : 0]);
-            const int hi = __reduce_max_sync(kFull, swin[1][lane < nwarps ? lane : 0]);
-            c0 = sref + lo;
-            if (c0 < 0) c0 += nz;
-            if (c0 >= nz) c0 -= nz;
-            win = hi - lo + P.w[2];
-            wide = win > kWin;
-            r -= lo;
-            ci0 = wide ? first : r;
-            wlo = mn - lo;
-            whi = mx - lo + P.w[2] - 1;
-            narrow = !wide && mx >= mn && whi - wlo < kNarrow;
+            // (cells relative to the first particle's at the launch)
+            place_particles<NF>(P, L, z, active, sp, sref, swin, rec, wrec);
         } else {
+            int first = 0;
+            if (active) {
+                shape<double>(z * P.dxi[2], P.ord[2], first, L.wz);
+                first = wrapi(first, nz);
+            }
             // relative to the warp's first cell
             const int ref = __shfl_sync(kFull, first, 0);
-            r = relative(first, ref);
-            wlo = __reduce_min_sync(kFull, active ? r : INT_MAX);
-            whi = __reduce_max_sync(kFull, active ? r : INT_MIN) + P.w[2] - 1;
+            int r = relative_cell(first, ref, nz);
+            const int mn = __reduce_min_sync(kFull, active ? r : INT_MAX);
+            const int mx = __reduce_max_sync(kFull, active ? r : INT_MIN);
             const bool any = __any_sync(kFull, active);
-            narrow = !any || whi - wlo < kNarrow;
             if (tid < kOneCells) {
                 scount[tid] = 0;
                 *reinterpret_cast<unsigned*>(srows[tid]) = 0x01010101u * kOnePart;
             }
-            narrow = __syncthreads_and(narrow);
-            if (!any) { wlo = 0; whi = -1; }
-            c0 = wrapi(ref + wlo, nz);
-            r -= wlo;
-            whi -= wlo;
-            wlo = 0;
-            ci0 = first;
-            if (lane == 0) srange[warp] = make_int2(c0, whi + 1);
-            if (narrow && lane <= whi) {
-                const int c = (c0 + lane) % nz, k = atomicAdd(&scount[c], 1);
+            L.narrow = __syncthreads_and(!any || mx - mn + P.w[2] <= kNarrow);
+            L.c0 = any ? wrapi(ref + mn, nz) : 0;
+            L.wlo = 0;
+            L.whi = any ? mx - mn + P.w[2] - 1 : -1;
+            L.ci0 = first;
+            if (lane == 0) srange[warp] = make_int2(L.c0, L.whi + 1);
+            if (L.narrow && lane <= L.whi) {
+                const int c = (L.c0 + lane) % nz, k = atomicAdd(&scount[c], 1);
                 if (k < 4) srows[c][k] = (unsigned char)(warp * 16 + lane);
             }
 #pragma unroll
-            for (int k = 0; k < KI; k++) mrow_of[k] = (c0 + 4 * k + col) % nz * MR;
-        }
-        if (sp == 0) {
-#pragma unroll
-            for (int i = 0; i < 3; i++) rec[R::W + i] = wz[i];
-            *reinterpret_cast<int*>(rec + R::FIRST) = narrow ? r : ci0;
-        }
-        __syncwarp();
-        if (narrow) {
-#pragma unroll
-            for (int m = 0; m < 2; m++) {
-#pragma unroll
-                for (int k = 0; k < KI; k++) ai[m][k] = dep_weight<NF>(wrec + (8 * m + row) * R::RW, wlo + 4 * k + col);
-#pragma unroll
-                for (int k = 0; k < 4; k++) ad[m][k] = dep_weight<NF>(wrec + (4 * k + col) * R::RW, wlo + 8 * m + row);
-                if constexpr (!ONE) {
-                    int c = c0 + wlo + 8 * m + row;
-                    c = c >= nz ? c % nz : c;
-                    gcell[m] = c * NCS;
-                }
-            }
+            for (int k = 0; k < KI; k++) mrow_of[k] = (L.c0 + 4 * k + col) % nz * MR;
+            place_weights<NF>(L, rec, wrec, sp, r - mn);
         }
     };
     if constexpr (!ONE) {
         if (tid == 0) {   // (the CTA's first particle exists)
             int first;
-            shape<double>(z * P.dxi[2], P.ord[2], first, wz);
+            shape<double>(z * P.dxi[2], P.ord[2], first, L.wz);
             sref = wrapi(first, nz);
         }
     }
@@ -397,98 +615,35 @@ __global__ void __launch_bounds__(MAXT, 1)
         int last_next = last, step_next = step;
 #pragma unroll 1
         for (int s = 1; s <= 4; s++) {
-            const double* const mesh_in = cmesh + (s - 1) * msize;
-            double* const mesh_out = cmesh + (s & 3) * msize;
+            const double* mesh_in = cmesh + (s - 1) * msize;
+            double* mesh_out = cmesh + (s & 3) * msize;
+            if constexpr (REC) {
+                mesh_in = store.mst + it * store.mst_stride + (s - 1) * msize;
+                mesh_out = s < 4 ? store.mst + it * store.mst_stride + s * msize : store.mst + (it + 1) * store.mst_stride;
+                if (s == 1 && active) {
+                    double* y = store.seg + it * store.seg_stride;
+#pragma unroll
+                    for (int e = 0; e < NH; e++) y[(sp * NH + e) * cap + p] = y0[e];
+                    if (sp == 0) {
+                        y[(2 * NH) * cap + p] = x;
+                        y[(2 * NH + 1) * cap + p] = yy;
+                        y[(2 * NH + 2) * cap + p] = z;
+                    }
+                }
+            }
             const double* mrow = smesh;
             if constexpr (!ONE) {
                 // M_4's mesh: here, since a CTA may still read the last
                 // step's for its timestep until it arrives at barrier 1
-                if (s == 2)
+                if (!REC && s == 2)
                     for (int i = gtid; i < msize; i += nthreads) cmesh[3 * msize + i] = 0.0;
-                if (!wide) {
-                    // (four further rows of zeros: the last product's depth)
-                    for (int i = tid; i < (win + 4) * (NG / 2); i += blockDim.x) {
-                        const int wl = i / (NG / 2), q = i - wl * (NG / 2);
-                        int c = c0 + wl;
-                        c = c >= nz ? c % nz : c;
-                        double2 t2 = make_double2(0.0, 0.0);
-                        if (wl < win) t2 = __ldcg(reinterpret_cast<const double2*>(mesh_in + c * NCS) + q);
-                        *reinterpret_cast<double2*>(smesh + wl * MR + 2 * q) = t2;
-                    }
-                }
+                stage_window<NF>(L, smesh, mesh_in, nz);
                 __syncthreads();
             } else {
                 mrow = smesh + cur * kHalf;
             }
-            // interpolation: u_j = G_0j - v . G_dj of the pair's particle
             double hv[NV];
-            if (narrow) {
-                double g[2][NT][2];
-#pragma unroll
-                for (int m = 0; m < 2; m++)
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++) g[m][nt][0] = g[m][nt][1] = 0.0;
-#pragma unroll
-                for (int k = 0; k < KI; k++) {
-                    if (wlo + 4 * k > whi) break;   // (uniform)
-                    const double* b = mrow + (ONE ? mrow_of[k] : (wlo + 4 * k + col) * MR);
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++) {
-                        // two flavors: column 2 e + i holds d = 2 nt + i of
-                        // value e, so that a lane's two columns are one value
-                        const double bv = b[NF == 2 ? (2 * nt + (row & 1)) * NV + (row >> 1) : nt * NV + row];
-#pragma unroll
-                        for (int m = 0; m < 2; m++) dmma(g[m][nt][0], g[m][nt][1], ai[m][k], bv);
-                    }
-                }
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    double* r = wrec + (8 * m + row) * R::RW;
-                    const double vx = r[R::V + 1], vy = r[R::V + 2], vz = r[R::V + 3];
-                    if constexpr (NF == 2) {
-                        r[R::CV + col] = ((g[m][0][0] - vx * g[m][0][1]) - vy * g[m][1][0]) - vz * g[m][1][1];
-                    } else {
-                        double2 t2;
-                        t2.x = ((g[m][0][0] - vx * g[m][1][0]) - vy * g[m][2][0]) - vz * g[m][3][0];
-                        t2.y = ((g[m][0][1] - vx * g[m][1][1]) - vy * g[m][2][1]) - vz * g[m][3][1];
-                        *reinterpret_cast<double2*>(r + R::CV + 2 * col) = t2;
-                    }
-                }
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < NV; j += 2) {
-                    const double2 t2 = *reinterpret_cast<const double2*>(rec + R::CV + j);
-                    hv[j] = t2.x;
-                    hv[j + 1] = t2.y;
-                }
-            } else {
-                double u[HV];
-#pragma unroll
-                for (int j = 0; j < HV; j++) u[j] = 0.0;
-                if (active) {
-#pragma unroll 1
-                    for (int i = 0; i < P.w[2]; i++) {
-                        int cc = ci0 + i;
-                        if (ONE || wide) cc = cc % nz;
-                        const double wi = i == 0 ? wz[0] : i == 1 ? wz[1] : wz[2];
-#pragma unroll
-                        for (int j = 0; j < HV; j++) {
-                            double g[4];
-#pragma unroll
-                            for (int d = 0; d < 4; d++)
-                                g[d] = !ONE && wide ? __ldcg(mesh_in + cc * NCS + d * NV + sp * HV + j)
-                                                    : mrow[cc * MR + d * NV + sp * HV + j];
-                            u[j] += wi * (((g[0] - g[1] * v[0]) - g[2] * v[1]) - g[3] * v[2]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < HV; j++) {
-                    const double other = __shfl_xor_sync(kFull, u[j], 1);
-                    hv[j] = sp == 0 ? u[j] : other;
-                    hv[HV + j] = sp == 0 ? other : u[j];
-                }
-            }
+            interp_1d<NF, ONE, false>(P, L, mrow, mrow_of, mesh_in, rec, wrec, sp, active, hv);
 #pragma unroll
             for (int j = 0; j < NV; j++) hv[j] *= P.sqrt2GF_inv_vol;
             double h[NH], K[NH];
@@ -506,6 +661,15 @@ __global__ void __launch_bounds__(MAXT, 1)
             } else {
 #pragma unroll
                 for (int e = 0; e < NH; e++) f[e] = __dadd_rn(__dmul_rn(bw, K[e]), acc[e]);
+            }
+            if constexpr (REC) {   // Y_2, Y_3, Y_4, Y_n
+                if (active) {
+                    double* y = store.sst + it * store.sst_stride + (s - 1) * (2 * NH) * cap;
+#pragma unroll
+                    for (int e = 0; e < NH; e++) y[(sp * NH + e) * cap + p] = f[e];
+                }
+            }
+            if (s == 4) {
                 if (active) {
                     const int stt = renormalize<NF>(f, Ls, P.maxError);
                     if (stt) report_bad(ctl, stt, S.id[p]);
@@ -514,12 +678,12 @@ __global__ void __launch_bounds__(MAXT, 1)
                     for (int i = 0; i < 4; i++) {
                         const double w = dt * (i == 0 || i == 3 ? 1. / 6. : 1. / 3.);
                         x = __dadd_rn(__dmul_rn(w, v[0] * kC), x);
-                        y = __dadd_rn(__dmul_rn(w, v[1] * kC), y);
+                        yy = __dadd_rn(__dmul_rn(w, v[1] * kC), yy);
                         z = __dadd_rn(__dmul_rn(w, v[2] * kC), z);
                         tp = __dadd_rn(w, tp);
                     }
                     x = wrap_coord(x, P.L[0]);
-                    y = wrap_coord(y, P.L[1]);
+                    yy = wrap_coord(yy, P.L[1]);
                     z = wrap_coord(z, P.L[2]);
                 }
 #pragma unroll
@@ -553,29 +717,14 @@ __global__ void __launch_bounds__(MAXT, 1)
                     for (int e = 0; e < NH; e++) sfn[pl * R::FW + sp * NH + e] = fN[e];
                 }
             }
-            if (narrow) {
-                __syncwarp();   // (a warp reads only its own records)
-                double cval[4];
-                const int q0 = (row >> 1) + 4 * (row & 1);
+            if constexpr (ONE) {
+                if (L.narrow) {
+                    __syncwarp();   // (a warp reads only its own records)
 #pragma unroll
-                for (int k = 0; k < 4; k++) cval[k] = wrec[(4 * k + col) * R::RW + R::CV + q0 % NV];
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    if (wlo + 8 * m > whi) break;   // (uniform)
-                    double g[NT][2], gd[2] = {0.0, 0.0};
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++) g[nt][0] = g[nt][1] = 0.0;
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const double* r = wrec + (4 * k + col) * R::RW;
-#pragma unroll
-                        for (int nt = 0; nt < NT; nt++) {
-                            const int d = (8 * nt + q0) / NV;
-                            dmma(g[nt][0], g[nt][1], ad[m][k], cval[k] * r[R::V + d]);
-                        }
-                        if (diag) dmma(gd[0], gd[1], ad[m][k], q0 < 2 * NF ? r[R::DG + (q0 < 2 * NF ? q0 : 0)] : 0.0);
-                    }
-                    if constexpr (ONE) {
+                    for (int m = 0; m < 2; m++) {
+                        if (8 * m > L.whi) break;   // (uniform)
+                        double g[NT][2], gd[2];
+                        products_1d<NF, false>(L, wrec, m, diag, g, gd);
                         // the warp's rows, summed over the warps below
                         double* o = spart + (warp * 16 + 8 * m + row) * NCS + col;
 #pragma unroll
@@ -587,24 +736,13 @@ __global__ void __launch_bounds__(MAXT, 1)
                             o[NG] = gd[0];
                             o[NG + 4] = gd[1];
                         }
-                    } else if (wlo + 8 * m + row <= whi) {
-                        double* o = mesh_out + gcell[m] + col;
-#pragma unroll
-                        for (int nt = 0; nt < NT; nt++) {
-                            atomic_add_mesh(o + 8 * nt, g[nt][0]);
-                            atomic_add_mesh(o + 8 * nt + 4, g[nt][1]);
-                        }
-                        if (diag) {
-                            atomic_add_mesh(o + NG, gd[0]);
-                            if (NF == 3 && col < 2) atomic_add_mesh(o + NG + 4, gd[1]);
-                        }
                     }
                 }
             }
             if constexpr (ONE) {
                 double* const out = smesh + (1 - cur) * kHalf;
                 __syncthreads();
-                if (narrow) {
+                if (L.narrow) {
                     const int nq = diag ? NCS : NG;
                     for (int i = tid; i < ncells * nq; i += blockDim.x) {
                         const int c = diag ? i / NCS : i / NG, q = i - c * nq;
@@ -629,9 +767,9 @@ __global__ void __launch_bounds__(MAXT, 1)
                 }
                 if (fdep) {
                     // (cells in place of rows relative to the warp's first)
-                    if (narrow) {
+                    if (L.narrow) {
                         __syncthreads();
-                        if (sp == 0) *reinterpret_cast<int*>(rec + R::FIRST) = ci0;
+                        if (sp == 0) *reinterpret_cast<int*>(rec + R::FIRST) = L.ci0;
                         __syncthreads();
                     }
                     deposit_tiles<NF, DEP_FULL>(ncells, full, ND, srec, sfn);
@@ -649,31 +787,25 @@ __global__ void __launch_bounds__(MAXT, 1)
                 }
                 __syncthreads();
             } else {
-                if (narrow) {
-                    if (fdep) deposit_spread<NF, DEP_FULL>(nz, full, srec, sfn, warp * 16, wlo, whi, c0);
-                } else if (!wide) {
-                    if (whi >= wlo) {
-                        deposit_spread<NF, DEP_COMB>(nz, mesh_out, srec, sfn, warp * 16, wlo, whi, c0);
-                        if (diag) deposit_spread<NF, DEP_DIAG>(nz, mesh_out, srec, sfn, warp * 16, wlo, whi, c0);
-                        if (fdep) deposit_spread<NF, DEP_FULL>(nz, full, srec, sfn, warp * 16, wlo, whi, c0);
-                    }
-                } else if (active) {
+                if (!(REC && s == 4 && final_step)) {
+                    __syncwarp();   // (a warp reads only its own records)
+                    if (!L.wide) {
+                        deposit_1d<NF, false>(L, srec, sfn, wrec, mesh_out, nz, diag);
+                        if (fdep && L.whi >= L.wlo)
+                            deposit_spread<NF, DEP_FULL, false>(nz, full, srec, sfn, warp * 16, L.wlo, L.whi, L.c0);
+                    } else if (active) {
+                        deposit_1d_wide<NF, false>(P, L, rec, sp, mesh_out, diag);
+                        if (fdep) {
 #pragma unroll 1
-                    for (int i = 0; i < P.w[2]; i++) {
-                        const int cell = (ci0 + i) % nz;
-                        const double wi = i == 0 ? wz[0] : i == 1 ? wz[1] : wz[2];
-                        double* m = mesh_out + cell * NCS;
-                        for (int d = 0; d < 4; d++) {
-                            const double wd = wi * rec[R::V + d];
-                            for (int j = 0; j < HV; j++)
-                                atomic_add_mesh(m + d * NV + sp * HV + j, wd * rec[R::CV + sp * HV + j]);
-                            if (fdep)
-                                for (int e = 0; e < NH; e++)
-                                    atomic_add_mesh(full + (long long)cell * ND + (2 * d + sp) * NH + e,
-                                                    wd * sfn[pl * R::FW + sp * NH + e]);
+                            for (int i = 0; i < P.w[2]; i++) {
+                                double* m = full + (long long)((L.ci0 + i) % nz) * ND;
+                                const double wi = i == 0 ? L.wz[0] : i == 1 ? L.wz[1] : L.wz[2];
+                                for (int d = 0; d < 4; d++)
+                                    for (int e = 0; e < NH; e++)
+                                        atomic_add_mesh(m + (2 * d + sp) * NH + e,
+                                                        wi * rec[R::V + d] * sfn[pl * R::FW + sp * NH + e]);
+                            }
                         }
-                        if (diag)
-                            for (int k = 0; k < NF; k++) atomic_add_mesh(m + NG + sp * NF + k, wi * rec[R::DG + sp * NF + k]);
                     }
                 }
                 const bool wait = !(s == 4 && (final_step || last || step + 1 >= max_step) && dt_mode == DT_ADVANCE) &&
@@ -683,7 +815,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                 // the previous barrier)
                 {
                     double* mz = cmesh + ((s + 2) & 3) * msize;
-                    if (s == 2 || s == 3 || (s == 4 && wait))
+                    if (!REC && (s == 2 || s == 3 || (s == 4 && wait)))
                         for (int i = gtid; i < msize; i += nthreads) mz[i] = 0.0;
                     if (s == 1 && want_full)
                         for (int i = gtid; i < ncells * ND; i += nthreads) full[i] = 0.0;
@@ -716,7 +848,8 @@ __global__ void __launch_bounds__(MAXT, 1)
                 }
                 if (wait) {
                     nbar++;
-                    if (!steps_wait(ctl, nbar * gridDim.x)) {
+                    // (the caller's limit is for fused = 2 and the adjoint)
+                    if (!steps_wait(ctl, nbar * gridDim.x, REC ? P.wait_polls : kBarrierSpins)) {
                         alive = false;
                         break;
                     }
@@ -751,7 +884,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         for (int e = 0; e < NH; e++) S.f0[(sp * NH + e) * cap + p] = y0[e];
         if (sp == 0) {
             S.pos[0][p] = x;
-            S.pos[1][p] = y;
+            S.pos[1][p] = yy;
             S.pos[2][p] = z;
             S.time[p] = tp;
         }
@@ -783,6 +916,164 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
 }
 
+// The backward sweep over recorded steps of a 1D run (emu_adjoint.cu: the
+// discrete adjoint), last step first, in one cooperative launch with the
+// means of k_steps_1d: the adjoint state in registers, the windows of the
+// adjoint mesh and of the recorded stage mesh in shared memory, matrix
+// products for the two gathers and the scatter, four grid barriers per step
+// (stage 0 only gathers).  The next stage's recorded mesh and state are
+// loaded between arrival and wait.  Two flavors, 128 x 80: a recorded step
+// 49 -> 17 us, a backward step 62 -> 22 us (against tiles of 128 particles
+// that reloaded their state and ranked their keys in every stage).
+template <int NF, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_adjoint_1d(DevParams P, DevState S, Adj1DStore A, StepCtl* ctl, int npart, int len)
+{
+    using H = Herm<NF>;
+    using C = Comb<NF>;
+    using R = Rec1D<NF>;
+    constexpr int NH = NF * NF, NV = C::NV, HV = NV / 2;
+    extern __shared__ __align__(16) double smem[];
+    double* const sm_lam = smem;                              // window of the adjoint mesh
+    double* const sm_fwd = smem + (kWin + 4) * R::MR;         // and of the recorded stage mesh
+    double* const srec = sm_fwd + (kWin + 4) * R::MR;
+    __shared__ int swin[2][16];
+    __shared__ int sref;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int pl = tid >> 1, sp = tid & 1;
+    const long long p = (long long)blockIdx.x * npart + pl;
+    const bool active = p < S.n;
+    const long long cap = S.cap;
+    const int nz = P.n[2], msize = (int)P.ncells * kCombSlots<NF>;
+    const int nthreads = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + tid;
+    double* const rec = srec + pl * R::RW;
+    double* const wrec = srec + warp * 16 * R::RW;
+
+    double vs = 0, Ns = 0, Ls = 1, dN = 0;
+    double lamY[NH] = {}, lamn[NH] = {}, lamYd[NH] = {}, ys[NH] = {}, yn[NH] = {};
+    if (active) {
+        vs = S.vscale[p];
+        Ns = S.Nn[sp][p];
+        Ls = S.Ll[sp][p];
+#pragma unroll
+        for (int e = 0; e < NH; e++) lamY[e] = A.lamY0[(sp * NH + e) * cap + p];
+    }
+    if (sp == 0) {
+        rec[3] = 0.0;
+        rec[R::V] = 1.0;
+#pragma unroll
+        for (int d = 0; d < 3; d++) rec[R::V + 1 + d] = active ? S.vhat[d][p] : 0.0;
+    }
+    // a recorded state's components of this thread
+    auto load = [&](const double* base, double* y) {
+        if (active)
+#pragma unroll
+            for (int e = 0; e < NH; e++) y[e] = __ldcg(base + (sp * NH + e) * cap + p);
+    };
+    auto stage_mesh = [&](int j, int s) { return A.rec.mst + j * A.rec.mst_stride + (s - 1) * msize; };
+    auto zpos = [&](int j) { return active ? __ldcg(A.rec.seg + j * A.rec.seg_stride + (2 * NH + 2) * cap + p) : 0.0; };
+    Place1D L;
+    if (tid == 0) {   // (the CTA's first particle exists)
+        int first;
+        shape<double>(zpos(len - 1) * P.dxi[2], P.ord[2], first, L.wz);
+        sref = wrapi(first, nz);
+    }
+    __syncthreads();
+    unsigned nbar = 0;
+    for (int j = len - 1; j >= 0; j--) {
+        const double* const sst = A.rec.sst + j * A.rec.sst_stride;
+        const double dt = A.dts[j];
+        load(sst + 3 * (2 * NH) * cap, yn);   // Y_n
+        load(sst + 2 * (2 * NH) * cap, ys);   // Y_4
+        place_particles<NF>(P, L, zpos(j), active, sp, sref, swin, rec, wrec);
+        stage_window<NF>(L, sm_fwd, stage_mesh(j, 4), nz);
+        __syncthreads();
+#pragma unroll 1
+        for (int s = 4; s >= 0; s--) {
+            double lamK[NH];
+            if (s == 4) {
+                double ln[NH];
+                renormalize_vjp<NF>(yn, Ls, P.maxError, lamY, ln);
+                const double b4 = dt * (1. / 6.);
+#pragma unroll
+                for (int e = 0; e < NH; e++) {
+                    lamn[e] = lamY[e] = ln[e];
+                    lamK[e] = b4 * ln[e];
+                    yn[e] = ys[e];
+                }
+            } else {
+                // the gather of stage s + 1's adjoint mesh: G of nu; of nubar
+                // with the opposite sign for real components
+                const double* const lm_in = A.lm + ((s + 1) & 3) * A.lm_stride;
+                stage_window<NF>(L, sm_lam, lm_in, nz);
+                __syncthreads();
+                double gv[NV], g[NH];
+                interp_1d<NF, false, true>(P, L, sm_lam, nullptr, lm_in, rec, wrec, sp, active, gv);
+                __syncwarp();
+                C::hermitian(gv, g);
+                const double b = dt * (s == 1 ? 1. / 6. : 1. / 3.), a = dt * (s == 3 ? 1.0 : 0.5);
+#pragma unroll
+                for (int e = 0; e < NH; e++) {
+                    const double G = sp == 0 || H::is_im(e) ? g[e] : -g[e];
+                    const double ly = lamYd[e] + Ns * G;   // lam of Y_{s+1}
+                    dN += yn[e] * G;
+                    lamY[e] += ly;
+                    lamK[e] = b * lamn[e] + a * ly;
+                    yn[e] = ys[e];   // (Y_s: the next gather's)
+                }
+                if (s == 0) break;
+            }
+            // commutator VJP and the scatter of lam_H
+            double hv[NV], h[NH], lH[NH], cc[NH], cv[NV];
+            interp_1d<NF, false, false>(P, L, sm_fwd, nullptr, stage_mesh(j, s), rec, wrec, sp, active, hv);
+#pragma unroll
+            for (int q = 0; q < NV; q++) hv[q] *= P.sqrt2GF_inv_vol;
+            C::hermitian(hv, h);
+            species_hamiltonian<NF>(P, h, vs, sp, h);
+            commutator_vjp<NF>(h, ys, lamK, lH, lamYd, P.inv_hbar);
+#pragma unroll
+            for (int e = 0; e < NH; e++) {
+                const double o = __shfl_xor_sync(kFull, lH[e], 1);
+                cc[e] = P.sqrt2GF_inv_vol * (H::is_im(e) ? lH[e] + o : (sp == 0 ? lH[e] - o : o - lH[e]));
+            }
+            C::values(cc, cv);
+            __syncwarp();   // (the pair's reads of the interpolated values)
+#pragma unroll
+            for (int q = 0; q < HV; q++) {
+                const double x = sp == 0 ? cv[q] : cv[HV + q];
+                rec[R::CV + sp * HV + q] = active ? x : 0.0;
+            }
+            __syncwarp();
+            double* const lm_out = A.lm + (s & 3) * A.lm_stride;
+            if (!L.wide) deposit_1d<NF, true>(L, srec, nullptr, wrec, lm_out, nz, false);
+            else if (active) deposit_1d_wide<NF, true>(P, L, rec, sp, lm_out, false);
+            // the next stage's target (last read three stages ago)
+            double* const lz = A.lm + ((s + 3) & 3) * A.lm_stride;
+            for (int i = gtid; i < msize; i += nthreads) lz[i] = 0.0;
+            steps_arrive(ctl);
+            if (s > 1) {
+                stage_window<NF>(L, sm_fwd, stage_mesh(j, s - 1), nz);
+                load(s == 2 ? A.rec.seg + j * A.rec.seg_stride : sst + (s - 3) * (2 * NH) * cap, ys);   // Y_{s-1}
+            }
+            nbar++;
+            if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) return;
+        }
+    }
+    if (active) {
+#pragma unroll
+        for (int e = 0; e < NH; e++) A.lamY0[(sp * NH + e) * cap + p] = lamY[e];
+        A.lamN[sp * cap + p] += dN;
+    }
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            ctl->blocks_done = 0u;
+            ctl->bar_count = 0u;
+        }
+    }
+}
+
 // particles per CTA: spread over the SMs, whole warps of 16, at least 64 (a
 // smaller CTA only adds barrier arrivals) and at most 256 (512 threads)
 int particles_per_cta(long long n, int nsm)
@@ -805,28 +1096,46 @@ int device_sms()
 
 // the kernel for a CTA of npart particles: the fewer threads, the more
 // registers each (three flavors spill at 128)
-using Steps1DKernel = void (*)(DevParams, DevState, double*, double*, StepCtl*, int, int, int);
-template <int NF>
+using Steps1DKernel = void (*)(DevParams, DevState, double*, double*, StepCtl*, int, int, int, Rec1DStore);
+template <int NF, bool REC>
 Steps1DKernel steps1d_kernel(bool one, int npart)
 {
-    if (one) return k_steps_1d<NF, true, 256>;
-    if (npart <= 128) return k_steps_1d<NF, false, 256>;
-    if (npart <= 192) return k_steps_1d<NF, false, 384>;
-    return k_steps_1d<NF, false, 512>;
+    if constexpr (!REC)
+        if (one) return k_steps_1d<NF, true, 256, false>;
+    if (npart <= 128) return k_steps_1d<NF, false, 256, REC>;
+    if (npart <= 192) return k_steps_1d<NF, false, 384, REC>;
+    return k_steps_1d<NF, false, 512, REC>;
 }
 
 template <int NF>
 cudaError_t launch_t(const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl, int nsteps,
-                     int dt_mode, cudaStream_t st)
+                     int dt_mode, cudaStream_t st, const Rec1DStore* rec)
 {
-    const bool one = one_cta(P, S.n);
+    const bool one = !rec && one_cta(P, S.n);
     int npart = one ? kOnePart : particles_per_cta(S.n, device_sms());
-    const Steps1DKernel kern = steps1d_kernel<NF>(one, npart);
+    const Steps1DKernel kern = rec ? steps1d_kernel<NF, true>(false, npart) : steps1d_kernel<NF, false>(one, npart);
     const int bytes = one ? steps1d_smem<NF, true>(npart) : steps1d_smem<NF, false>(npart);
     smem_optin(kern, bytes);
     DevParams Pc = P;
     DevState Sc = S;
-    void* args[] = {&Pc, &Sc, &cmesh, &full, &ctl, &npart, &nsteps, &dt_mode};
+    Rec1DStore store = rec ? *rec : Rec1DStore{};
+    void* args[] = {&Pc, &Sc, &cmesh, &full, &ctl, &npart, &nsteps, &dt_mode, &store};
+    return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid_for(S.n, npart)), dim3(2 * npart), args, bytes, st);
+}
+
+template <int NF>
+cudaError_t launch_adjoint_t(const DevParams& P, const DevState& S, const Adj1DStore& A, StepCtl* ctl, int len,
+                             cudaStream_t st)
+{
+    using R = Rec1D<NF>;
+    int npart = particles_per_cta(S.n, device_sms());
+    auto kern = npart <= 128 ? k_adjoint_1d<NF, 256> : npart <= 192 ? k_adjoint_1d<NF, 384> : k_adjoint_1d<NF, 512>;
+    const int bytes = 8 * (2 * (kWin + 4) * R::MR + npart * R::RW);
+    smem_optin(kern, bytes);
+    DevParams Pc = P;
+    DevState Sc = S;
+    Adj1DStore Ac = A;
+    void* args[] = {&Pc, &Sc, &Ac, &ctl, &npart, &len};
     return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid_for(S.n, npart)), dim3(2 * npart), args, bytes, st);
 }
 
@@ -845,10 +1154,16 @@ bool steps_1d_fit(int nf, const DevParams& P, long long n)
 }
 
 cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl,
-                            int nsteps, int dt_mode, cudaStream_t st)
+                            int nsteps, int dt_mode, cudaStream_t st, const Rec1DStore* rec)
 {
-    return nf == 2 ? launch_t<2>(P, S, cmesh, full, ctl, nsteps, dt_mode, st)
-                   : launch_t<3>(P, S, cmesh, full, ctl, nsteps, dt_mode, st);
+    return nf == 2 ? launch_t<2>(P, S, cmesh, full, ctl, nsteps, dt_mode, st, rec)
+                   : launch_t<3>(P, S, cmesh, full, ctl, nsteps, dt_mode, st, rec);
+}
+
+cudaError_t launch_adjoint_1d(int nf, const DevParams& P, const DevState& S, const Adj1DStore& A, StepCtl* ctl, int len,
+                              cudaStream_t st)
+{
+    return nf == 2 ? launch_adjoint_t<2>(P, S, A, ctl, len, st) : launch_adjoint_t<3>(P, S, A, ctl, len, st);
 }
 
 }  // namespace emu

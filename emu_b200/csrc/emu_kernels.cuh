@@ -150,9 +150,29 @@ cudaError_t launch_rk4_step_coop(int nf, const DevParams& P, const DevState& S, 
 // combined meshes (cmesh: M_1..M_4 one after the other, M_1 deposited, M_2
 // zeroed; full: target of the full
 // stage-4 mesh); dt_mode DT_ADVANCE, or -1 for one step of the control's dt
+// rec: a recorded run; step it of the launch stores its Y_0, x, y, z at seg +
+// it seg_stride (2 NF^2 + 3 arrays of the state's capacity), Y_2, Y_3, Y_4 and
+// Y_n at sst + it sst_stride, and keeps M_1..M_4 at mst + it mst_stride
+// (zeroed; M_1 of the first step deposited), in place of cmesh
+struct Rec1DStore {
+    double *seg = nullptr, *sst = nullptr, *mst = nullptr;
+    long long seg_stride = 0, sst_stride = 0, mst_stride = 0;
+};
 bool steps_1d_fit(int nf, const DevParams& P, long long n);
 cudaError_t launch_steps_1d(int nf, const DevParams& P, const DevState& S, double* cmesh, double* full, StepCtl* ctl,
-                            int nsteps, int dt_mode, cudaStream_t st);
+                            int nsteps, int dt_mode, cudaStream_t st, const Rec1DStore* rec = nullptr);
+// the backward sweep over len recorded steps (rec, dts: of the first one) in
+// one cooperative launch: four adjoint meshes of stride lm_stride at lm (the
+// first zeroed), dJ/d(state) lamY0 and dJ/d(N, Nbar) lamN in place
+struct Adj1DStore {
+    Rec1DStore rec;
+    const double* dts = nullptr;
+    double* lm = nullptr;
+    long long lm_stride = 0;
+    double *lamY0 = nullptr, *lamN = nullptr;
+};
+cudaError_t launch_adjoint_1d(int nf, const DevParams& P, const DevState& S, const Adj1DStore& A, StepCtl* ctl, int len,
+                              cudaStream_t st);
 // one FP64 RK4 stage on combined meshes; full_zero: stage 2 zeroes it on the
 // steps that deposit the full stage-4 mesh; D, inv, kout, iout as
 // launch_rk4_stage_mixed
