@@ -229,7 +229,7 @@ __device__ __forceinline__ void adj_fwd_body(const DevParams& P, const DevState&
 #pragma unroll
             for (int e = 0; e < NH; e++) f[e] = A.Yin[(sp * NH + e) * cap + p];
             species_hamiltonian<NF>(P, hs, vsc, sp, h);
-            commutator_lean<NF, double>(h, f, K, P.inv_hbar);
+            commutator<NF, double>(h, f, K, P.inv_hbar);
             if (s < 4) {
 #pragma unroll
                 for (int e = 0; e < NH; e++) {

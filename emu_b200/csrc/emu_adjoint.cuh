@@ -21,8 +21,8 @@ __device__ __forceinline__ void commutator_vjp(const double* h, const double* f,
     double l[NH];
 #pragma unroll
     for (int e = 0; e < NH; e++) l[e] = H::is_diag(e) ? lam[e] : 0.5 * lam[e];
-    commutator_lean<NF, double>(l, h, lamF, inv_hbar);
-    commutator_lean<NF, double>(f, l, lamH, inv_hbar);
+    commutator<NF, double>(l, h, lamF, inv_hbar);
+    commutator<NF, double>(f, l, lamH, inv_hbar);
 #pragma unroll
     for (int e = 0; e < NH; e++)
         if (!H::is_diag(e)) {

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kBlock, 4)
                 }
             }
             species_hamiltonian<NF>(P, hs, vsc, sp, h);
-            commutator_lean<NF, double>(h, f, K, P.inv_hbar);
+            commutator<NF, double>(h, f, K, P.inv_hbar);
             if constexpr (SG < 4) {
 #pragma unroll
                 for (int e = 0; e < NH; e++) {

@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             double h[NH], K[NH];
             C::hermitian(hv, h);
             species_hamiltonian<NF>(P, h, vs, sp, h);
-            commutator_lean<NF, double>(h, f, K, P.inv_hbar);
+            commutator<NF, double>(h, f, K, P.inv_hbar);
             const double bw = dt * (s == 1 || s == 4 ? 1. / 6. : 1. / 3.);
             if (s < 4) {
                 const double aw = dt * (s == 3 ? 1.0 : 0.5);
