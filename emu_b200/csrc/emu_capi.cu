@@ -724,6 +724,12 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
         // at 1, 457 at 2, 498 at 4, 577 at 16)
         const int cells = ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2];
         ctx->prm.resort_interval = cells > (ctx->comb64 ? 3 : 9) ? 1 : 16;
+        // several steps per launch: the re-sort's own launches weigh more and
+        // a window a few cells wider costs little (two flavors, 128 x 80: 15.5
+        // us per step at 16, 14.3 at 32, 13.9 at 64; 50 cells x 2 beams, whose
+        // warps outgrow the products past 40 steps: 11.0, 10.5, 23.1); one
+        // cell needs none
+        if (ctx->steps1d) ctx->prm.resort_interval = ctx->P.ncells > 1 ? 32 : 0;
     }
     // with a re-sort after every step, the deposits of stages 1-3 see
     // cell-sorted particles; otherwise every deposit ranks its keys
