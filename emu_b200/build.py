@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 
 SOURCES = ["emu_k_comb64_3.cu", "emu_k_comb64_2.cu", "emu_k_fp64_3.cu", "emu_k_mixed_3.cu", "emu_adjoint.cu", "emu_k_fp64_2.cu", "emu_k_mixed_2.cu",
-           "emu_k_misc.cu", "emu_k_steps1d.cu", "emu_capi.cu", "emu_comm.cu", "emu_noalloc.cu", "emu_init_device.cu", "emu_host.cpp",
+           "emu_k_misc.cu", "emu_k_steps1d.cu", "emu_capi.cu", "emu_comm.cu", "emu_hostcopy.cu", "emu_noalloc.cu", "emu_init_device.cu", "emu_host.cpp",
            "emu_init.cpp"]
 # the device initial-condition generator must round like the host one
 EXTRA = {"emu_init_device.cu": ["-fmad=false"]}

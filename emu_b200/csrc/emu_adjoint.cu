@@ -1296,14 +1296,12 @@ int emu_adjoint_objective(emu_context* ctx, double* J, double* lam_f, double* la
     const unsigned g = (unsigned)((n + emu::kBlock - 1) / emu::kBlock);
     if (lam_f) {
         emu::k_soa_to_rows<<<g, emu::kBlock, 0, ctx->stream>>>(S.id, lamf, ctx->NS, cap, n, a->rows);
-        CU(cudaMemcpyAsync(lam_f, a->rows, sizeof(double) * (size_t)n * ctx->NS, cudaMemcpyDeviceToHost,
-                           ctx->stream));
+        if ((r = emu_ctx::copy_to_host(ctx, lam_f, a->rows, sizeof(double) * (size_t)n * ctx->NS))) return r;
     }
     CU(cudaStreamSynchronize(ctx->stream));
     if (lam_N) {
         emu::k_soa_to_rows<<<g, emu::kBlock, 0, ctx->stream>>>(S.id, lamN, 2, cap, n, a->rows);
-        CU(cudaMemcpyAsync(lam_N, a->rows, sizeof(double) * (size_t)n * 2, cudaMemcpyDeviceToHost, ctx->stream));
-        CU(cudaStreamSynchronize(ctx->stream));
+        if ((r = emu_ctx::copy_to_host(ctx, lam_N, a->rows, sizeof(double) * (size_t)n * 2))) return r;
     }
     if ((r = check_launch(ctx, "adjoint objective output"))) return r;
     const double inv_vol = ctx->P.dxi[0] * ctx->P.dxi[1] * ctx->P.dxi[2];
@@ -1331,11 +1329,11 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     const long long nm = cmesh_elems(ctx);
 
     // adjoint state of the final (renormalised) state, in the final slot order
-    CU(cudaMemcpyAsync(a->rows, lam_f_final, sizeof(double) * (size_t)n * NS, cudaMemcpyHostToDevice, st));
+    if ((r = emu_ctx::copy_to_device(ctx, a->rows, lam_f_final, sizeof(double) * (size_t)n * NS))) return r;
     emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, NS, cap, n, a->lamY0);
     CU(cudaStreamSynchronize(st));
     if (lam_N_final) {
-        CU(cudaMemcpyAsync(a->rows, lam_N_final, sizeof(double) * (size_t)n * 2, cudaMemcpyHostToDevice, st));
+        if ((r = emu_ctx::copy_to_device(ctx, a->rows, lam_N_final, sizeof(double) * (size_t)n * 2))) return r;
         emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, 2, cap, n, a->lamN);
     } else {
         CU(cudaMemsetAsync(a->lamN, 0, sizeof(double) * 2 * cap, st));
@@ -1637,10 +1635,9 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     // outputs in load order (the order of the run's first segment)
     const DevState W0 = stat_view(a, w, S);
     emu::k_soa_to_rows<<<g, emu::kBlock, 0, st>>>(W0.id, a->lamY0, NS, cap, n, a->rows);
-    CU(cudaMemcpyAsync(lam_f0, a->rows, sizeof(double) * (size_t)n * NS, cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
+    if ((r = emu_ctx::copy_to_host(ctx, lam_f0, a->rows, sizeof(double) * (size_t)n * NS))) return r;
     emu::k_soa_to_rows<<<g, emu::kBlock, 0, st>>>(W0.id, a->lamN, 2, cap, n, a->rows);
-    CU(cudaMemcpyAsync(lam_N0, a->rows, sizeof(double) * (size_t)n * 2, cudaMemcpyDeviceToHost, st));
+    if ((r = emu_ctx::copy_to_host(ctx, lam_N0, a->rows, sizeof(double) * (size_t)n * 2))) return r;
     // the forward meshes were reused: restore the current state's deposit
     double* const* M = ctx->mesh;
     CU(cudaMemsetAsync(M[1], 0, sizeof(double) * mesh_elems(ctx), st));

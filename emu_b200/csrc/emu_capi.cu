@@ -847,6 +847,7 @@ void emu_destroy(emu_context* ctx)
     if (ctx->planes) emu_ctx::dev_free(ctx->planes);
     if (ctx->ctl) emu_ctx::dev_free(ctx->ctl);
     if (ctx->ctl_host) emu_ctx::host_free(ctx->ctl_host);
+    emu_ctx::ring_free(ctx);
     if (ctx->aos) emu_ctx::dev_free(ctx->aos);
     for (void* a : {(void*)ctx->keys, (void*)ctx->keys2, (void*)ctx->idx, (void*)ctx->idx2})
         if (a) emu_ctx::dev_free(a);
@@ -922,10 +923,7 @@ int emu_get_particles(emu_context* ctx, double* records, int64_t n)
     if ((r = ensure_aos(ctx, S.n))) return r;
     emu::launch_unpack(ctx->nf, S, ctx->aos, ctx->stream);
     if ((r = check_launch(ctx, "unpack"))) return r;
-    CU(cudaMemcpyAsync(records, ctx->aos, sizeof(double) * (size_t)S.n * ctx->nreal, cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
-    return EMU_OK;
+    return emu_ctx::copy_to_host(ctx, records, ctx->aos, sizeof(double) * (size_t)S.n * ctx->nreal);
 }
 
 int emu_num_particles(const emu_context* ctx, int64_t* n)
@@ -954,9 +952,7 @@ int emu_get_mesh(emu_context* ctx, double* out)
     else emu::launch_mesh_out(ctx->nf, ctx->P, ctx->mesh[ctx->cur_mesh], ctx->planes, ctx->stream);
     int r;
     if ((r = check_launch(ctx, "mesh out"))) return r;
-    CU(cudaMemcpyAsync(out + 3 * nc, ctx->planes + 3 * nc, sizeof(double) * nc * ctx->ND, cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
+    if ((r = emu_ctx::copy_to_host(ctx, out + 3 * nc, ctx->planes + 3 * nc, sizeof(double) * nc * ctx->ND))) return r;
     for (long long c = 0; c < nc; c++) {
         out[c] = ctx->prm.rho_in;
         out[nc + c] = ctx->prm.T_in;
@@ -990,10 +986,7 @@ int emu_interpolate_rhs(emu_context* ctx, double* rhs_records)
     if ((r = ensure_aos(ctx, S.n))) return r;
     emu::launch_unpack_rhs(ctx->nf, S, S.kgen, ctx->aos, ctx->stream);
     if ((r = check_launch(ctx, "rhs"))) return r;
-    CU(cudaMemcpyAsync(rhs_records, ctx->aos, sizeof(double) * (size_t)S.n * ctx->nreal, cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CU(cudaStreamSynchronize(ctx->stream));
-    return EMU_OK;
+    return emu_ctx::copy_to_host(ctx, rhs_records, ctx->aos, sizeof(double) * (size_t)S.n * ctx->nreal);
 }
 
 int emu_renormalize(emu_context* ctx, int64_t* bad)

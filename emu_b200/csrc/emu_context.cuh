@@ -79,6 +79,8 @@ struct emu_context {
     double* stats = nullptr;            // per-block record statistics of a load (device)
     double* stats_host = nullptr;       // and their pinned host copy
     bool adj_valid = false;             // a recorded run matches the slot order
+    char* ring = nullptr;               // pinned chunks of large copies (emu_hostcopy.cu), made by the first one
+    cudaEvent_t ring_event[8] = {};
     std::string err;
 };
 
@@ -117,6 +119,11 @@ inline cudaError_t host_free(void* p)
 int fail(emu_context* c, int code, const std::string& msg);
 // EMU_ERR_CUDA with what + the pending launch error, if any
 int check_launch(emu_context* ctx, const char* what);
+// bytes between device memory and the caller's host memory (pinned or not),
+// after the work of the context's stream; complete on return
+int copy_to_host(emu_context* ctx, void* dst, const void* src, size_t bytes);
+int copy_to_device(emu_context* ctx, void* dst, const void* src, size_t bytes);
+void ring_free(emu_context* ctx);
 // one device-resident step of the fused RK4 loop (cooperative kernel or
 // graph), without the periodic re-sort; dt comes from the device control.
 // last_stage_deposit = false leaves the deposit of the new state to a
