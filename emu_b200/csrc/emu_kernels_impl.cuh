@@ -173,49 +173,44 @@ __device__ __forceinline__ void zero_slice(T* buf, long long n)
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Bulk copies global -> shared on the TMA engine (cp.async.bulk, no
-// multicast) completing on an mbarrier: a CTA stages its particles' state
-// arrays (one contiguous 128-particle slice per component) while its threads
-// do other work.  Addresses and sizes are multiples of 16 bytes (particle
-// capacities are multiples of 128).
-__device__ __forceinline__ unsigned smem_u32(const void* ptr) { return (unsigned)__cvta_generic_to_shared(ptr); }
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
+// Asynchronous copies global -> shared, 16 bytes a lane: a CTA stages its
+// particles' state arrays while its threads do other work.  Addresses are
+// multiples of 16 bytes (particle capacities are multiples of 128).
+__device__ __forceinline__ void cp_async16(void* dst, const void* src)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
-// wait for phase `parity` of the barrier, at most kMbarPolls polls (each
-// try_wait may suspend the thread for a while); false when it gave up
-constexpr int kMbarPolls = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity)
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the last N committed groups of this thread are complete
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
 {
-    const unsigned a = smem_u32(bar);
-    for (int i = 0; i < kMbarPolls; i++) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ===========================================================================
-// compute_dt pieces (Evolve.cpp:22-89 + compute_dt fill)
-// ===========================================================================
+// ROWS rows of a state array (row r at src + r cap, from the CTA's first
+// particle on) into dst[ROWS][kBlock]: every warp copies the slices of its
+// own 32 particles, 512 bytes an instruction, and alone reads them, so no block
+// barrier follows.  (Bulk copies of one row each cost the warp that issued
+// them ~85 clocks apiece: 1500 to 6000 of a CTA's 28,000 clocks for a
+// stage's 18 to 63 rows.  With the control words, positions and these copies
+// now in flight together, 64^3 cells x 96 directions: stages of
+// 4801/5143/6683/4746 us -> 4215/4422/5667/4063; 1 x 1 x 1024 x 378:
+// 227 -> 209 us a step.)
+template <int ROWS, class E>
+__device__ __forceinline__ void stage_rows(E* dst, const E* src, long long cap)
+{
+    constexpr int PER = 16 / (int)sizeof(E);    // elements a lane copies
+    constexpr int LPR = 32 / PER, RPI = 32 / LPR;   // lanes of a row, rows an instruction
+    const int lane = threadIdx.x & 31, e = (threadIdx.x & ~31) + (lane % LPR) * PER;
+#pragma unroll
+    for (int r0 = 0; r0 < ROWS; r0 += RPI) {
+        const int r = r0 + lane / LPR;
+        if (r0 + RPI <= ROWS || r < ROWS) cp_async16(dst + r * kBlock + e, src + r * cap + e);
+    }
+}
+
 __device__ __forceinline__ void block_max2(double& a, double& b)
 {
     __shared__ double sa[32], sb[32];
@@ -1234,10 +1229,11 @@ __device__ __forceinline__ void potential_si32(const DevParams& P, const float* 
 }
 
 // The neighbourhood of a CTA's particles for 27-cell stencils: the box of
-// cells their stencils touch, staged in shared memory by bulk copies (the TMA
-// engine, no multicast) of the potential mesh's rows when it holds at most
+// cells their stencils touch, staged in shared memory by asynchronous copies
+// of the potential mesh's rows when it holds at most
 // kMeshTileCells cells.  Built from the smallest and largest stencil key of
-// the CTA: every key between them lies in one z plane and in one or two
+// the CTA (their cells: the warps' extremes, so no thread divides a key):
+// every key between them lies in one z plane and in one or two
 // consecutive y rows, so the box is x from the smallest key's x to the
 // largest's (+ nx when the rows differ), y over one or two rows, z one
 // plane, each grown by the stencil's two further cells.  Otherwise (keys
@@ -1250,18 +1246,20 @@ struct MeshBox {
     int nx, ny, nz;   // its extent; nx = 0: not staged
 };
 
-__device__ __forceinline__ MeshBox mesh_box(const DevParams& P, unsigned kmin, unsigned kmax)
+struct KeyCell {
+    int key, x, y, z;   // a stencil key and its cell
+};
+
+// lo, hi: the smallest and largest key (lo.key > hi.key: no particle)
+__device__ __forceinline__ MeshBox mesh_box(const DevParams& P, const KeyCell& lo, const KeyCell& hi)
 {
     MeshBox b{0, 0, 0, 0, 0, 0};
-    if (kmin > kmax) return b;   // no particle
-    const int n0 = P.n[0], n1 = P.n[1];
-    const int xa = (int)(kmin % n0), ya = (int)((kmin / n0) % n1), za = (int)(kmin / (n0 * n1));
-    const int xb = (int)(kmax % n0), yb = (int)((kmax / n0) % n1), zb = (int)(kmax / (n0 * n1));
-    if (za != zb || (yb != ya && yb != ya + 1)) return b;
-    const int lx = (yb == ya ? xb - xa : xb + n0 - xa) + 3;
-    const int ly = yb - ya + 3;
-    if (lx > n0 || ly > n1 || 3 > P.n[2] || lx * ly * 3 > kMeshTileCells) return b;
-    b.x0 = xa; b.y0 = ya; b.z0 = za;
+    if (lo.key > hi.key) return b;
+    if (lo.z != hi.z || (hi.y != lo.y && hi.y != lo.y + 1)) return b;
+    const int lx = (hi.y == lo.y ? hi.x - lo.x : hi.x + P.n[0] - lo.x) + 3;
+    const int ly = hi.y - lo.y + 3;
+    if (lx > P.n[0] || ly > P.n[1] || 3 > P.n[2] || lx * ly * 3 > kMeshTileCells) return b;
+    b.x0 = lo.x; b.y0 = lo.y; b.z0 = lo.z;
     b.nx = lx; b.ny = ly; b.nz = 3;
     return b;
 }
@@ -1297,12 +1295,10 @@ __host__ __device__ constexpr int mixed_mesh_tile_offset()
 // the step (the stage-4 push of its momentum with the step's dt; the key of
 // the unchanged position once the run has ended), with the identity index,
 // for the radix sort.
-__device__ __forceinline__ void sc_key(const DevParams& P, const DevState& S, long long p, double dt, bool push,
-                                       unsigned* keys, unsigned* idx)
+__device__ __forceinline__ void sc_key(const DevParams& P, long long p, double dt, bool push, double (&xn)[3],
+                                       const double* pq, unsigned* keys, unsigned* idx)
 {
-    double xn[3] = {__ldcg(S.pos[0] + p), __ldcg(S.pos[1] + p), __ldcg(S.pos[2] + p)};
     if (push) {
-        const double pq[4] = {__ldcg(S.pup[0] + p), __ldcg(S.pup[1] + p), __ldcg(S.pup[2] + p), __ldcg(S.pup[3] + p)};
         double tn = 0.0;
         rk4_push(P, dt, pq, xn, tn);
     }
@@ -1319,7 +1315,11 @@ __global__ void k_sc_keys(DevParams P, DevState S, const StepCtl* __restrict__ c
     const int done = __ldcg(&ctl->done);
     const double dt = __ldcg(&ctl->dt);
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < S.n) sc_key(P, S, p, dt, !done, keys, idx);
+    if (p < S.n) {
+        double xn[3] = {__ldcg(S.pos[0] + p), __ldcg(S.pos[1] + p), __ldcg(S.pos[2] + p)};
+        const double pq[4] = {__ldcg(S.pup[0] + p), __ldcg(S.pup[1] + p), __ldcg(S.pup[2] + p), __ldcg(S.pup[3] + p)};
+        sc_key(P, p, dt, !done, xn, pq, keys, idx);
+    }
 }
 
 // inverse of the sort's permutation: particle perm[i] goes to slot i
@@ -1379,25 +1379,104 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
     // stages 1-3 read the FP32 copy of the step-start state (mixed_f0_copy)
     constexpr bool F32C = mixed_f0_copy_w<WX, WY, WZ>() && s < 4;
     // without the register preload, the CTA's slices of f0, k32 and ksum32
-    // are staged in shared memory by bulk copies (the record area of the
-    // deposit, written only after the state is consumed)
+    // are staged in shared memory by asynchronous copies (the record area of
+    // the deposit, written only after the state is consumed)
     constexpr bool STAGE = !PRELOAD;
     // (programmatic dependent launch: see grid_dep_wait; the finalize
     // kernel before this stage has waited for the previous stage)
     static_assert(!SC || SG == 4, "the re-sort scatter is stage 4's");
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool active = p < S.n;
+    const long long cap = S.cap;
+    const int t = threadIdx.x;
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    // 27-cell stencils: the staged mesh neighbourhood (see mesh_box)
+    constexpr bool MTILE = STAGE && mixed_mesh_tile<NF, WX, WY, WZ>();
+    constexpr int NGC = Comb<NF>::NG;
+    __shared__ KeyCell key_ext[2][kBlock / 32];
+    float* const mtile = reinterpret_cast<float*>(tile_smem + mixed_mesh_tile_offset<NF, WX, WY, WZ>());
+    double* const sf0 = reinterpret_cast<double*>(tile_smem);        // [NS][kBlock]
+    float* const sf32 = reinterpret_cast<float*>(tile_smem);         // [NS][kBlock] (F32C)
+    float* const sk = reinterpret_cast<float*>(sf0 + NS * kBlock);   // [NS][kBlock]
+    float* const sks = sk + NS * kBlock;                             // [NS][kBlock]
+    double* const s4 = reinterpret_cast<double*>(sks + NS * kBlock); // stage 4: time, pup[4], L[2] x kBlock
+    const long long p0 = (long long)blockIdx.x * kBlock;
+
+    // prologue, in one memory round trip: the control words and the fields
+    // that no kernel of this step before this one writes (all of the state
+    // at the step start for two flavors in 1D, the per-species scalars
+    // otherwise); the step-start state on its way to shared memory
     const int done = __ldcg(&ctl->done);
-    const double dt = __ldcg(&ctl->dt);   // both control loads in one round trip
+    const double dt = __ldcg(&ctl->dt);
+    Stencil<float> st{};
+    float fN[NS] = {};
+    float vx = 0, vy = 0, vz = 0;
+    double x = 0, y = 0, z = 0, vs = 0, t_in = 0;
+    float Nsp[2] = {0.f, 0.f};
+    double Lsp[2] = {0, 0}, pu[4] = {0, 0, 0, 1};
+    const bool hoist = PRELOAD && s == 4;
+    // (a re-sort follows the step: stage 3 stores its keys)
+    constexpr bool KEYS = SG == 3 && sc_keys_in_stage3_w<WX, WY, WZ>();
+    constexpr int PRE = PRELOAD ? NS : 1;
+    double y0a[PRE];
+    float ka[PRE], ksa[PRE];
+    int given = -1;   // stages 1-3: the rank the last stage 4 stored, see rk4_stage_body
+    if (s < 4 && P.rank_stages) given = t;
+    if (active) {
+        x = __ldcg(S.pos[0] + p);
+        y = __ldcg(S.pos[1] + p);
+        z = __ldcg(S.pos[2] + p);
+        vx = __ldcg(S.vhat32[0] + p);
+        vy = __ldcg(S.vhat32[1] + p);
+        vz = __ldcg(S.vhat32[2] + p);
+        vs = __ldcg(S.vscale + p);
+        Nsp[0] = __ldcg(S.N32[0] + p);
+        Nsp[1] = __ldcg(S.N32[1] + p);
+        if (s < 4 && P.rank_stages) given = __ldcg(S.rslot + p);
+        if (hoist) {
+            Lsp[0] = __ldcg(S.Ll[0] + p);
+            Lsp[1] = __ldcg(S.Ll[1] + p);
+            t_in = __ldcg(S.time + p);
+        }
+        if (hoist || (KEYS && kout)) {
+#pragma unroll
+            for (int d = 0; d < 4; d++) pu[d] = __ldcg(S.pup[d] + p);
+        }
+        if constexpr (PRELOAD) {
+#pragma unroll
+            for (int c = 0; c < NS; c++) y0a[c] = F32C ? (double)__ldcg(S.f032 + c * cap + p) : __ldcg(S.f0 + c * cap + p);
+        }
+    }
+    if constexpr (STAGE) {
+        // f0, and stage 4's time, momentum and SU(n) lengths, are written
+        // only by the previous step: their copies start before the
+        // dependency wait, those of k32 and ksum32 (the previous stage's)
+        // after it
+        if constexpr (F32C) stage_rows<NS>(sf32, S.f032 + p0, cap);   // (in the first half of the FP64 slices' area)
+        else stage_rows<NS>(sf0, S.f0 + p0, cap);
+        if constexpr (s == 4) {
+            const int e = (t & ~31) + (t & 15) * 2;
+#pragma unroll
+            for (int r0 = 0; r0 < 7; r0 += 2) {
+                const int r = r0 + ((t >> 4) & 1);
+                if (r < 7) {
+                    const double* src = r == 0 ? S.time : r < 5 ? S.pup[r - 1] : S.Ll[r - 5];
+                    cp_async16(s4 + r * kBlock + e, src + p0 + e);
+                }
+            }
+        }
+    }
     if (done) {
-        if constexpr (SG == 3 && sc_keys_in_stage3_w<WX, WY, WZ>()) {
-            const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-            if (kout && p < S.n) sc_key(P, S, p, dt, false, kout, iout);
+        if constexpr (STAGE) cp_async_wait<0>();   // (no copy outlives its CTA)
+        if constexpr (KEYS) {
+            double xn[3] = {x, y, z};
+            if (kout && active) sc_key(P, p, dt, false, xn, pu, kout, iout);
         }
         if constexpr (SC) {
             // after the run's end the re-sort still moves the unchanged
             // state (its keys were those of the unchanged positions)
             grid_dep_wait();
-            const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-            if (p < S.n) {
+            if (active) {
                 const long long q = inv[p];
                 double pq[4], L2[2];
                 for (int d = 0; d < 4; d++) pq[d] = S.pup[d][p];
@@ -1413,153 +1492,73 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
         }
         return;
     }
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < S.n;
-    const long long cap = S.cap;
-    const int t = threadIdx.x;
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    __shared__ __align__(8) unsigned long long stage_bar;
-    // 27-cell stencils: the staged mesh neighbourhood (see mesh_box)
-    constexpr bool MTILE = STAGE && mixed_mesh_tile<NF, WX, WY, WZ>();
-    constexpr int NGC = Comb<NF>::NG;
-    __shared__ __align__(8) unsigned long long mesh_bar;
-    __shared__ unsigned key_ext[2][kBlock / 32];
-    __shared__ MeshBox mbox;
-    float* const mtile = reinterpret_cast<float*>(tile_smem + mixed_mesh_tile_offset<NF, WX, WY, WZ>());
-    double* const sf0 = reinterpret_cast<double*>(tile_smem);        // [NS][kBlock]
-    float* const sf32 = reinterpret_cast<float*>(tile_smem);         // [NS][kBlock] (F32C)
-    float* const sk = reinterpret_cast<float*>(sf0 + NS * kBlock);   // [NS][kBlock]
-    float* const sks = sk + NS * kBlock;                             // [NS][kBlock]
-    double* const s4 = reinterpret_cast<double*>(sks + NS * kBlock); // stage 4: time, pup[4], L[2] x kBlock
-    const long long p0 = (long long)blockIdx.x * kBlock;
-    // slices of k32 and ksum32 staged: none in stage 1; K_1 alone in stage
-    // 2 (after stage 1 the running sum K_1 + 2 K_2 + ... is K_1 itself, so
-    // stage 1 stores no ksum32); both in stages 3 and 4
-    constexpr int NKS = s == 1 ? 0 : (s == 2 ? NS : 2 * NS);
-    if constexpr (STAGE) {
-        // f0 is written only by the previous step: its copies start before
-        // the dependency wait, k32 and ksum32 (the previous stage's) after it
-        if (t < 32) {
-            if (t == 0) {
-                mbar_init(&stage_bar, 1);
-                mbar_expect_tx(&stage_bar, NS * kBlock * (F32C ? 4 : 8) + NKS * kBlock * 4 + (s == 4 ? 7 * kBlock * 8 : 0));
-                if constexpr (MTILE) mbar_init(&mesh_bar, 1);
-            }
-            __syncwarp();
-            // (F32C: the FP32 copy, in the first half of the FP64 slices' area)
-            for (int c = t; c < NS; c += 32) {
-                if (F32C) bulk_g2s(sf32 + c * kBlock, S.f032 + c * cap + p0, kBlock * 4, &stage_bar);
-                else bulk_g2s(sf0 + c * kBlock, S.f0 + c * cap + p0, kBlock * 8, &stage_bar);
-            }
-            // stage 4's time, momentum and SU(n) lengths (written only by
-            // the previous step too)
-            if (s == 4 && t < 7) {
-                const double* src = t == 0 ? S.time : t < 5 ? S.pup[t - 1] : S.Ll[t - 5];
-                bulk_g2s(s4 + t * kBlock, src + p0, kBlock * 8, &stage_bar);
-            }
-        }
-        __syncthreads();   // the barrier is initialised before anyone waits on it
-    }
-
-    // prologue: fields that no kernel of this step writes (one memory round
-    // trip with the control loads; all of the state at the step start for
-    // two flavors in 1D, the per-species scalars otherwise)
-    Stencil<float> st{};
-    float fN[NS] = {};
-    float vx = 0, vy = 0, vz = 0;
-    double x = 0, y = 0, z = 0, vs = 0, t_in = 0;
-    float Nsp[2] = {0.f, 0.f};
-    double Lsp[2] = {0, 0}, pu[4] = {0, 0, 0, 1};
-    const bool hoist = PRELOAD && s == 4;
-    constexpr int PRE = PRELOAD ? NS : 1;
-    double y0a[PRE];
-    float ka[PRE], ksa[PRE];
     if (active) {
-        x = __ldcg(S.pos[0] + p);
-        y = __ldcg(S.pos[1] + p);
-        z = __ldcg(S.pos[2] + p);
-        vx = __ldcg(S.vhat32[0] + p);
-        vy = __ldcg(S.vhat32[1] + p);
-        vz = __ldcg(S.vhat32[2] + p);
-        vs = __ldcg(S.vscale + p);
-        Nsp[0] = __ldcg(S.N32[0] + p);
-        Nsp[1] = __ldcg(S.N32[1] + p);
-        if (hoist) {
-            Lsp[0] = __ldcg(S.Ll[0] + p);
-            Lsp[1] = __ldcg(S.Ll[1] + p);
-            t_in = __ldcg(S.time + p);
-#pragma unroll
-            for (int d = 0; d < 4; d++) pu[d] = __ldcg(S.pup[d] + p);
-        }
-        if constexpr (PRELOAD) {
-#pragma unroll
-            for (int c = 0; c < NS; c++) y0a[c] = F32C ? (double)__ldcg(S.f032 + c * cap + p) : __ldcg(S.f0 + c * cap + p);
-        }
         make_stencil<float>(P, x, y, z, st);
-        // (a re-sort follows the step: its keys, from fields no kernel of
-        // the step writes)
-        if constexpr (SG == 3 && sc_keys_in_stage3_w<WX, WY, WZ>())
-            if (kout) sc_key(P, S, p, dt, true, kout, iout);
+        if constexpr (KEYS) {
+            double xn[3] = {x, y, z};
+            if (kout) sc_key(P, p, dt, true, xn, pu, kout, iout);
+        }
     }
     if constexpr (MTILE) {
-        // the CTA's smallest and largest stencil key
-        const unsigned key = active ? (unsigned)stencil_key(P, st.b) : 0u;
-        const unsigned kmin = __reduce_min_sync(kFull, active ? key : 0xffffffffu);
-        const unsigned kmax = __reduce_max_sync(kFull, key);
-        if ((t & 31) == 0) {
-            key_ext[0][t >> 5] = kmin;
-            key_ext[1][t >> 5] = kmax;
-        }
+        // each warp's smallest and largest stencil key, with their cells
+        const int key = stencil_key(P, st.b);
+        const int kmin = __reduce_min_sync(kFull, active ? key : INT_MAX);
+        const int kmax = __reduce_max_sync(kFull, active ? key : -1);
+        const KeyCell kc = active ? KeyCell{key, st.b[0], st.b[1], st.b[2]} : KeyCell{kmin, 0, 0, 0};
+        if (active ? key == kmin : kmax < 0) key_ext[0][t >> 5] = kc;   // (equal keys: the same words)
+        if (kmax < 0) key_ext[1][t >> 5] = KeyCell{-1, 0, 0, 0};
+        else if (active && key == kmax) key_ext[1][t >> 5] = kc;
         __syncthreads();
     }
     grid_dep_wait();
     grid_dep_launch();
-    bool live = active;   // false: this particle's staged state never arrived
     long long qsc = 0;    // SC: the particle's slot in D (the inverse, written before this stage)
     if constexpr (SC) qsc = active ? (long long)inv[p] : 0;
-    if constexpr (STAGE) {
-        if (s > 1 && t < 32)
-            for (int c = t; c < NKS; c += 32) {
-                const float* src = c < NS ? S.k32 + c * cap + p0 : S.ksum32 + (c - NS) * cap + p0;
-                bulk_g2s(sk + c * kBlock, src, kBlock * 4, &stage_bar);
-            }
-    }
+    MeshBox mb{};
     if constexpr (MTILE) {
         // the neighbourhood's rows of the potential mesh (written by the
-        // finalize kernel this stage waited for): one or two contiguous x
-        // segments per (y, z) row, one lane per row
-        if (t < 32) {
-            if (t == 0) {
-                unsigned kmin = key_ext[0][0], kmax = key_ext[1][0];
+        // finalize kernel this stage waited for): a warp per row (y, z)
+        KeyCell lo = key_ext[0][0], hi = key_ext[1][0];
 #pragma unroll
-                for (int w = 1; w < kBlock / 32; w++) {
-                    kmin = min(kmin, key_ext[0][w]);
-                    kmax = max(kmax, key_ext[1][w]);
-                }
-                const MeshBox b = mesh_box(P, kmin, kmax);
-                mbox = b;
-                mbar_expect_tx(&mesh_bar, (unsigned)(b.nx * b.ny * b.nz * NGC * 4));
-            }
-            __syncwarp();
-            const MeshBox b = mbox;
-            const int nrow = b.ny * b.nz;
-            for (int row = t; row < nrow; row += 32) {
-                const int yy = row % b.ny, zz = row / b.ny;
-                const int gy = (b.y0 + yy) % P.n[1], gz = (b.z0 + zz) % P.n[2];
-                const long long grow = ((long long)gz * P.n[1] + gy) * P.n[0];
-                float* dst = mtile + (long long)row * b.nx * NGC;
-                // x from b.x0 over b.nx cells, split where it wraps
-                const int first = min(b.nx, P.n[0] - b.x0);
-                bulk_g2s(dst, gmesh + (grow + b.x0) * NGC, (unsigned)(first * NGC * 4), &mesh_bar);
-                if (first < b.nx)
-                    bulk_g2s(dst + first * NGC, gmesh + grow * NGC, (unsigned)((b.nx - first) * NGC * 4), &mesh_bar);
+        for (int w = 1; w < kBlock / 32; w++) {
+            if (key_ext[0][w].key < lo.key) lo = key_ext[0][w];
+            if (key_ext[1][w].key > hi.key) hi = key_ext[1][w];
+        }
+        mb = mesh_box(P, lo, hi);
+        constexpr int CH = NGC / 4;   // 16-byte chunks of a cell
+        const int lane = t & 31, nch = mb.nx * CH;
+        for (int row = t >> 5; row < mb.ny * mb.nz; row += kBlock / 32) {
+            const int zz = row >= 2 * mb.ny ? 2 : row >= mb.ny ? 1 : 0, yy = row - zz * mb.ny;
+            int gy = mb.y0 + yy, gz = mb.z0 + zz;
+            if (gy >= P.n[1]) gy -= P.n[1];
+            if (gz >= P.n[2]) gz -= P.n[2];
+            const float* const g = gmesh + ((long long)gz * P.n[1] + gy) * P.n[0] * NGC;
+            float* const d = mtile + row * mb.nx * NGC;
+            for (int c = lane; c < nch; c += 32) {
+                int gx = mb.x0 + c / CH;
+                if (gx >= P.n[0]) gx -= P.n[0];
+                cp_async16(d + c * 4, g + gx * NGC + (c % CH) * 4);
             }
         }
+    }
+    if constexpr (STAGE) {
+        cp_async_commit();
+        // slices of k32 and ksum32: none in stage 1; K_1 alone in stage 2
+        // (after stage 1 the running sum K_1 + 2 K_2 + ... is K_1 itself, so
+        // stage 1 stores no ksum32); both in stages 3 and 4
+        if constexpr (s > 1) stage_rows<NS>(sk, S.k32 + p0, cap);
+        if constexpr (s > 2) stage_rows<NS>(sks, S.ksum32 + p0, cap);
+        cp_async_commit();
     }
     // compute_dt on the stage-4 mesh (every block has read this step's dt)
     if (dt_mode == DT_ADVANCE)
         dt_reduce_and_finish<NF, long long>(P, qdt, ctl, DT_ADVANCE, reduce_blocks(P),
                                             P.m4_reduced ? qdt + P.ncells * (8 * NH) : nullptr);
+    if constexpr (MTILE) {
+        cp_async_wait<1>();
+        __syncthreads();   // every warp's rows of the neighbourhood
+    }
+    float hs[NH];
     if (active) {
         // the state arrays never alias
         const float* __restrict__ k32p = S.k32;
@@ -1573,26 +1572,18 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
         }
         // FP32 self-interaction part, trace removed (it commutes; three
         // flavors: the combined mesh holds only the traceless part)
-        float hs[NH];
         bool tiled = false;
         if constexpr (MTILE) {
-            // (the wait also orders mbox, written before the arrival)
-            if (!mbar_wait(&mesh_bar, 0)) {
-                atomicOr(&ctl->status, ST_TIMEOUT);
-                live = false;
-            } else {
-                const MeshBox b = mbox;
-                const int lx = wrapi(st.b[0] - b.x0, P.n[0]), ly = wrapi(st.b[1] - b.y0, P.n[1]),
-                          lz = wrapi(st.b[2] - b.z0, P.n[2]);
-                if (b.nx > 0 && lx + 2 < b.nx && ly + 2 < b.ny && lz + 2 < b.nz) {
-                    tiled = true;
-                    const float4* base =
-                        reinterpret_cast<const float4*>(mtile + ((lz * b.ny + ly) * b.nx + lx) * NGC);
-                    const int sy = b.nx * NGC / 4, sz = b.ny * b.nx * NGC / 4;
-                    potential_si32_from<NF, SWt>(
-                        P, [&](int ii, int jj, int kk, int k) { return base[kk * sz + jj * sy + ii * (NGC / 4) + k]; },
-                        st, vx, vy, vz, hs);
-                }
+            int lx = st.b[0] - mb.x0, ly = st.b[1] - mb.y0;   // (an active particle's z is the box's)
+            if (lx < 0) lx += P.n[0];
+            if (ly < 0) ly += P.n[1];
+            if (mb.nx > 0 && lx + 2 < mb.nx && ly + 2 < mb.ny) {
+                tiled = true;
+                const float4* base = reinterpret_cast<const float4*>(mtile + (ly * mb.nx + lx) * NGC);
+                const int sy = mb.nx * NGC / 4, sz = mb.ny * mb.nx * NGC / 4;
+                potential_si32_from<NF, SWt>(
+                    P, [&](int ii, int jj, int kk, int k) { return base[kk * sz + jj * sy + ii * (NGC / 4) + k]; }, st,
+                    vx, vy, vz, hs);
             }
         }
         if (!tiled) potential_si32<NF, SWt>(P, gmesh, st, vx, vy, vz, hs);
@@ -1605,24 +1596,22 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             for (int e = 0; e < NH; e++)
                 if (H::is_diag(e)) hs[e] -= tr;
         }
+    }
+    if constexpr (STAGE) {
+        // the state of the warp's particles, copied by its lanes
+        cp_async_wait<0>();
+        __syncwarp();
+    }
+    if (active) {
         const float ih = (float)P.inv_hbar;
         const double mat = P.sqrt2GF_inv_vol * P.matter;
         const float awf = (float)(s > 1 ? dt * kRK4A[s - 1] : 0.0);
         const float anf = (float)(s < 4 ? dt * kRK4A[s] : 0.0);
         const double w6 = dt * (1.0 / 6.0);
         int stt = 0;
-        if constexpr (STAGE) {
-            // a thread whose wait gives up reads none of the staged state
-            // and writes nothing of its particle (the step is invalid)
-            if (!mbar_wait(&stage_bar, 0)) {
-                atomicOr(&ctl->status, ST_TIMEOUT);
-                live = false;
-            }
-        }
         // one species at a time keeps the live state small
 #pragma unroll
         for (int sp = 0; sp < 2; sp++) {
-            if (!live) break;
             // the stage state Y_s = y0 + aw K_{s-1} only enters the FP32
             // commutator and (stages 1-3) the FP32 deposit: formed in FP32
             // from the step-start state rounded to FP32 (with 1D stencils
@@ -1708,7 +1697,7 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
                 }
             }
         }
-        if (s == 4 && live) {
+        if (s == 4) {
             double xn[3] = {x, y, z};
             double tn = PRELOAD ? t_in : s4[t];
             const double pq[4] = {PRELOAD ? pu[0] : s4[kBlock + t], PRELOAD ? pu[1] : s4[2 * kBlock + t],
@@ -1729,24 +1718,13 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             make_stencil<float>(P, xn[0], xn[1], xn[2], st);
         }
     }
-    if constexpr (STAGE) {
-        // the staged state is consumed (and the copies complete) before the
-        // deposit records reuse the area; when the copies do not complete
-        // within the bounded wait the CTA deposits nothing
-        const bool drained =
-            __syncthreads_and(t != 0 || (mbar_wait(&stage_bar, 0) && (!MTILE || mbar_wait(&mesh_bar, 0))));
-        if (!drained) {
-            if (t == 0) atomicOr(&ctl->status, ST_TIMEOUT);
-            return;
-        }
-    }
+    // the staged state is consumed before the deposit records reuse its area
+    if constexpr (STAGE) __syncthreads();
     if (qout) {
-        // (stages 1-3: the rank the last stage 4 stored, see rk4_stage_body)
-        const int given = (s < 4 && P.rank_stages) ? (active ? S.rslot[p] : t) : -1;
         if (s == 3 && !P.m4_reduced) {
             // M_4 in the full layout (N, Nbar and the fluxes apart): compute_dt
             // reads more of it than the diagonal
-            tile_deposit_block<NF, SWt, float>(P, qout, live, st, fN, vx, vy, vz, QuantConv{P}, false, given);
+            tile_deposit_block<NF, SWt, float>(P, qout, active, st, fN, vx, vy, vz, QuantConv{P}, false, given);
         } else if (s == 3) {
             // M_4: the combined layout stage 4 interpolates, the diagonal N_ii
             // compute_dt reads apart, and the full layout (into qm4) only on
@@ -1764,11 +1742,11 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             if constexpr (NF == 3 && SWt::MX * SWt::MY * SWt::MZ == 27) {
                 // (27-cell stencils: the diagonal slots in the same walk)
                 sl = tile_deposit_block<NF, SWt, float, long long, QuantConvG, true, NV + 2 * NF>(
-                    P, qout, live, st, cN, vx, vy, vz, QuantConvG{P}, false, given,
+                    P, qout, active, st, cN, vx, vy, vz, QuantConvG{P}, false, given,
                     DiagOut<long long, QuantConv>{qdiag, QuantConv{P}});
             } else {
                 sl = tile_deposit_block<NF, SWt, float, long long, QuantConvG, true, NV + 2 * NF>(
-                    P, qout, live, st, cN, vx, vy, vz, QuantConvG{P}, false, given);
+                    P, qout, active, st, cN, vx, vy, vz, QuantConvG{P}, false, given);
                 // (the records the deposit above has read, still in place)
                 tile_deposit_diag<NF, kBlock, kBlock, SWt, long long>(
                     P, qdiag, reinterpret_cast<const int*>(tile_smem),
@@ -1777,7 +1755,7 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             const bool full = m4_full_step(ctl);   // uniform over the grid
             if (full) {
                 __syncthreads();   // every record has been read
-                tile_deposit_block<NF, SWt, float>(P, qm4, live, st, fN, vx, vy, vz, QuantConv{P}, false, sl);
+                tile_deposit_block<NF, SWt, float>(P, qm4, active, st, fN, vx, vy, vz, QuantConv{P}, false, sl);
             }
             if (blockIdx.x == 0 && t == 0) ctl->m4_full = full ? 1 : 0;
         } else {
@@ -1786,7 +1764,7 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             float cN[Comb<NF>::NV];
             combine_species<NF>(fN, cN);
             const int sl = tile_deposit_block<NF, SWt, float, long long, QuantConvG, true>(
-                P, qout, live, st, cN, vx, vy, vz, QuantConvG{P}, s == 4, given);
+                P, qout, active, st, cN, vx, vy, vz, QuantConvG{P}, s == 4, given);
             if (s == 4 && active) S.rslot[p] = sl;
         }
     }
