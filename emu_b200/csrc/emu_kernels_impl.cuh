@@ -1330,16 +1330,15 @@ __global__ void k_sc_invert(const unsigned* __restrict__ perm, unsigned* __restr
 }
 
 // the fields of particle p that no stage changes, into slot q of D
-__device__ __forceinline__ void sc_static_fields(const DevParams& P, const DevState& S, const DevState& D, long long p,
-                                                 long long q, const double* pq, const double* L2)
+__device__ __forceinline__ void sc_static_fields(const DevParams& P, const DevState& D, long long q, long long id,
+                                                 const double* nn2, const double* pq, const double* L2)
 {
     D.rslot[q] = (int)(q % kBlock);   // in cell order: the identity rank
-    D.id[q] = S.id[p];
+    D.id[q] = id;
 #pragma unroll
     for (int sp = 0; sp < 2; sp++) {
-        const double nn = S.Nn[sp][p];
-        D.Nn[sp][q] = nn;
-        D.N32[sp][q] = (float)nn;
+        D.Nn[sp][q] = nn2[sp];
+        D.N32[sp][q] = (float)nn2[sp];
         D.Ll[sp][q] = L2[sp];
     }
 #pragma unroll
@@ -1478,10 +1477,10 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
             grid_dep_wait();
             if (active) {
                 const long long q = inv[p];
-                double pq[4], L2[2];
+                double pq[4];
                 for (int d = 0; d < 4; d++) pq[d] = S.pup[d][p];
-                for (int sp = 0; sp < 2; sp++) L2[sp] = S.Ll[sp][p];
-                sc_static_fields(P, S, D, p, q, pq, L2);
+                const double nn[2] = {S.Nn[0][p], S.Nn[1][p]}, L2[2] = {S.Ll[0][p], S.Ll[1][p]};
+                sc_static_fields(P, D, q, S.id[p], nn, pq, L2);
                 for (int d = 0; d < 3; d++) D.pos[d][q] = S.pos[d][p];
                 D.time[q] = S.time[p];
                 for (int c = 0; c < 2 * NF * NF; c++) {
@@ -1597,6 +1596,18 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
                 if (H::is_diag(e)) hs[e] -= tr;
         }
     }
+    // (SC: the last fields to move, on their way during the commutators:
+    // 64^3 cells x 96 directions 4064 -> 3720 us, loaded where they are
+    // stored their latency was the CTA's)
+    long long id_sc = 0;
+    double nn_sc[2] = {0, 0};
+    if constexpr (SC) {
+        if (active) {
+            id_sc = __ldcg(S.id + p);
+            nn_sc[0] = __ldcg(S.Nn[0] + p);
+            nn_sc[1] = __ldcg(S.Nn[1] + p);
+        }
+    }
     if constexpr (STAGE) {
         // the state of the warp's particles, copied by its lanes
         cp_async_wait<0>();
@@ -1708,13 +1719,13 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
                 for (int d = 0; d < 3; d++) D.pos[d][qsc] = xn[d];
                 D.time[qsc] = tn;
                 const double L2[2] = {PRELOAD ? Lsp[0] : s4[5 * kBlock + t], PRELOAD ? Lsp[1] : s4[6 * kBlock + t]};
-                sc_static_fields(P, S, D, p, qsc, pq, L2);
+                sc_static_fields(P, D, qsc, id_sc, nn_sc, pq, L2);
             } else {
 #pragma unroll
                 for (int d = 0; d < 3; d++) S.pos[d][p] = xn[d];
                 S.time[p] = tn;
             }
-            report_bad(ctl, stt, S.id[p]);
+            if (stt) report_bad(ctl, stt, S.id[p]);
             make_stencil<float>(P, xn[0], xn[1], xn[2], st);
         }
     }
