@@ -154,6 +154,15 @@ __device__ __forceinline__ int stencil_key(const DevParams& P, const int b[3])
     return (b[2] * P.n[1] + b[1]) * P.n[0] + b[0];
 }
 
+// the cell of a stencil key (two unsigned divisions)
+__device__ __forceinline__ void key_cell(const DevParams& P, int key, int& bx, int& by, int& bz)
+{
+    const unsigned row = (unsigned)key / (unsigned)P.n[0], z = row / (unsigned)P.n[1];
+    bx = key - (int)row * P.n[0];
+    by = (int)(row - z * (unsigned)P.n[1]);
+    bz = (int)z;
+}
+
 __device__ __forceinline__ long long cell_of(const DevParams& P, int bx, int by, int bz, int ii, int jj, int kk)
 {
     int i = bx + ii; if (i >= P.n[0]) i -= P.n[0];
@@ -474,9 +483,8 @@ __device__ __forceinline__ void tile_deposit_pairs(const DevParams& P, T* mesh, 
     const int voff1 = SP + NS + dir0 + 1;
     RunAcc<float, S, SP> acc0, acc1;
     auto flush = [&](int key) {
-        const int bx = key % P.n[0];
-        const int by = (key / P.n[0]) % P.n[1];
-        const int bz = key / (P.n[0] * P.n[1]);
+        int bx, by, bz;
+        key_cell(P, key, bx, by, bz);
 #pragma unroll
         for (int kk = 0; kk < SWt::MZ; kk++)
 #pragma unroll
@@ -560,20 +568,31 @@ __device__ __forceinline__ void tile_deposit_comb(const DevParams& P, T* mesh, c
     float2 acc[NP];
     float2 dacc[WITH_DIAG ? NF : 1];
     auto flush = [&](int key) {
-        const int bx = key % P.n[0];
-        const int by = (key / P.n[0]) % P.n[1];
-        const int bz = key / (P.n[0] * P.n[1]);
+        int bx, by, bz;
+        key_cell(P, key, bx, by, bz);
+        // a stencil that does not wrap: row pointers and constant offsets
+        // (with key_cell's divisions: 64^3 cells x 96 directions 23.95 -> 23.43
+        // ms a step, 27 x 25 x 29 x 50 with two flavors 814 -> 771 us)
+        auto put = [&](auto at) {
 #pragma unroll
-        for (int kk = 0; kk < SWt::MZ; kk++)
+            for (int kk = 0; kk < SWt::MZ; kk++)
 #pragma unroll
-            for (int jj = 0; jj < SWt::MY; jj++)
+                for (int jj = 0; jj < SWt::MY; jj++)
 #pragma unroll
-                for (int ii = 0; ii < SWt::MX; ii++) {
-                    if (!SWt::on(P, ii, jj, kk)) continue;
-                    const int k = (kk * SWt::MY + jj) * SWt::MX + ii;
-                    const float a = (k & 1) ? acc[k / 2].y : acc[k / 2].x;
-                    atomic_add_mesh(&mesh[cell_of(P, bx, by, bz, ii, jj, kk) * NG + q], conv(a, 0));
-                }
+                    for (int ii = 0; ii < SWt::MX; ii++) {
+                        if (!SWt::on(P, ii, jj, kk)) continue;
+                        const int k = (kk * SWt::MY + jj) * SWt::MX + ii;
+                        const float a = (k & 1) ? acc[k / 2].y : acc[k / 2].x;
+                        atomic_add_mesh(at(ii, jj, kk), conv(a, 0));
+                    }
+        };
+        if (bx + P.w[0] <= P.n[0] && by + P.w[1] <= P.n[1] && bz + P.w[2] <= P.n[2]) {
+            T* const m0 = mesh + ((long long)key) * NG + q;
+            const long long sy = (long long)P.n[0] * NG, sz = sy * P.n[1];
+            put([&](int ii, int jj, int kk) { return m0 + kk * sz + jj * sy + ii * NG; });
+        } else {
+            put([&](int ii, int jj, int kk) { return &mesh[cell_of(P, bx, by, bz, ii, jj, kk) * NG + q]; });
+        }
         if constexpr (WITH_DIAG) {
             if (don) {
                 T* g = dg.diag + cell_of(P, bx, by, bz, di, dj, dk) * kDiagSlots;
@@ -679,9 +698,8 @@ __device__ __forceinline__ void tile_deposit_diag(const DevParams& P, T* diag, c
         float2 acc[NF];
         auto flush = [&](int key) {
             if (!on) return;
-            const int bx = key % P.n[0];
-            const int by = (key / P.n[0]) % P.n[1];
-            const int bz = key / (P.n[0] * P.n[1]);
+            int bx, by, bz;
+            key_cell(P, key, bx, by, bz);
             T* g = diag + cell_of(P, bx, by, bz, ii, jj, kk) * kDiagSlots;
 #pragma unroll
             for (int m = 0; m < NF; m++) {
@@ -728,9 +746,8 @@ __device__ __forceinline__ void tile_deposit_diag(const DevParams& P, T* diag, c
     const int voff = SP + (comb_layout ? Comb<NF>::NV + c : sp * NH + H::re(i, i));
     RunAcc<float, S, SP> acc;
     auto flush = [&](int key) {
-        const int bx = key % P.n[0];
-        const int by = (key / P.n[0]) % P.n[1];
-        const int bz = key / (P.n[0] * P.n[1]);
+        int bx, by, bz;
+        key_cell(P, key, bx, by, bz);
 #pragma unroll
         for (int kk = 0; kk < SWt::MZ; kk++)
 #pragma unroll
@@ -783,9 +800,8 @@ __device__ __forceinline__ void tile_deposit(const DevParams& P, T* mesh, const 
     const int voff = SP + NS + (dir > 0 ? dir - 1 : 0);
     RunAcc<R, SZ * SY * SX, SP> acc;
     auto flush = [&](int key) {
-        const int bx = key % P.n[0];
-        const int by = (key / P.n[0]) % P.n[1];
-        const int bz = key / (P.n[0] * P.n[1]);
+        int bx, by, bz;
+        key_cell(P, key, bx, by, bz);
 #pragma unroll
         for (int kk = 0; kk < SZ; kk++)
 #pragma unroll
