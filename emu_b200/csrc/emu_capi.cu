@@ -1189,7 +1189,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
     const int nk = ctx->mixed ? 8 : 4;
     // timed as a step inside a longer run: the stage-4 mesh stays in the
     // combined layout (DevParams::m4_reduced) unless the run ends here
-    if ((ctx->mixed && ctx->P.m4_reduced) || ctx->comb64) emu::launch_ctl_m4(ctx->ctl, 2, ctx->stream);
+    if (ctx->mixed && ctx->P.m4_reduced) emu::launch_ctl_m4(ctx->ctl, 2, ctx->stream);
     const bool resort_due = ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
     if (max_kernels < nk + (resort_due ? 1 : 0))
         return fail(ctx, EMU_ERR_ARG, "emu_profile_step: kernel_ms too small");

@@ -113,3 +113,19 @@ def test_end_time_clips_the_last_step():
         info = c.evolve(10, 0.0, end)
         assert info.steps_done == len(dts) and abs(info.time - end) <= 1e-12 * end
         assert colwise_rel(c.get_particles(), ref) < 1e-11
+
+
+def test_mesh_can_be_read_after_a_profiled_step():
+    p, parts = _make(3, (4, 5, 3), 2, 9, 0)
+    meshes = []
+    for profiled in (False, True):
+        with api.Context(p) as c:
+            c.load_particles(parts)
+            c.evolve_begin(0.0, float("inf"), 3)
+            c.evolve_steps(2 if profiled else 3)
+            if profiled:
+                c.profile_step()
+            meshes.append(c.get_mesh())
+    scale = np.abs(meshes[0]).reshape(3 + 72, -1)[3:].reshape(8, -1).max(axis=1)
+    err = np.abs(meshes[1] - meshes[0]).reshape(3 + 72, -1)[3:].reshape(8, -1).max(axis=1)
+    assert (err <= 1e-11 * scale).all()
