@@ -117,10 +117,18 @@ def large_state(p):
     return n_particles(p) * api.nreal(p.nflavors) * 8 > 2 * L2_BYTES
 
 
-def effective_resort(p):
+def effective_resort(p, multi=False):
+    """The re-sort interval that the automatic setting picks."""
     r = p.resort_interval
     if r < 0:
-        r = 1 if sum(1 for c in p.ncell if c > 1) == 3 and p.shape_order >= 2 else 16
+        cells = 1
+        for c in p.ncell:
+            cells *= p.shape_order + 1 if c > 1 else 1
+        fp64 = p.precision != api.PREC_MIXED and p.fused == 1 and not multi and not p.max_adaptive_speedup > 1.0
+        r = 1 if cells > (3 if fp64 else 9) else 16
+        # FP64 along z, at most 256 particles per SM: several steps a launch
+        if fp64 and p.ncell[0] == p.ncell[1] == 1 and n_particles(p) <= 256 * 148:
+            r = 32 if p.ncell[2] > 1 else 0
     return r
 
 
@@ -302,7 +310,7 @@ def run_reference(args):
            "n_gpus": ws, "steps": done, "warmup": args.warmup, "ms_per_step": el / done * 1e3,
            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
            "dtype": "f64", "data": "synthetic",
-           "config": config_dict(args.workload, p, desc, ws, multi, effective_resort(p)),
+           "config": config_dict(args.workload, p, desc, ws, multi, effective_resort(p, multi)),
            "cpu_baseline": {"value": value, "unit": "particle-steps/s", "cores": nthreads, "kind": kind,
                             "sample": "%d RK4 steps (after %d warm-up) of %s, FP64, %.1f s" % (
                                 done, args.warmup, sdesc, el)},
@@ -393,7 +401,7 @@ def run_emu(args):
         from emu_b200 import sharding
         recs = sharding.shard(all_recs, rank, ws)
     n = recs.shape[0]
-    eff_resort = effective_resort(p)
+    eff_resort = effective_resort(p, multi)
     stream = torch.cuda.Stream()
     flush = None if large_state(p) else torch.zeros((512 << 20) // 8, dtype=torch.float64, device="cuda")
     ctx = make_context(p, stream, multi, rank, ws)
@@ -435,14 +443,18 @@ def run_emu(args):
     serial_step = float(per_kernel.sum())
     scale = min(1.0, ms_per_step / serial_step) if serial_step > 0 else 1.0
     per_pstep = algorithmic_bytes_per_particle_step(nf, mixed)
-    coop = kms.shape[1] == 1
+    # (one kernel for a whole step, and an entry more for a re-sort)
+    coop = kms.shape[1] <= 2
     split = nf == 2 and p.ncell[0] == 1 and p.ncell[1] == 1 and not mixed   # species-split kernels
     if coop:
-        kernel = "k_rk4_step_coop%s<%d>" % ("_split" if split else "", nf)
+        kernel = ("k_steps_1d<%d>" if p.fused == 1 else "k_rk4_step_coop%s<%%d>" % ("_split" if split else "")) % nf
         stage_serial = float(kms[:, 0].mean())
         bytes_per_launch = per_pstep * n + mesh_bytes_per_step(p, nf)
     else:
-        kernel = "k_rk4_stage%s<%d>" % ("_mixed" if mixed else ("_split" if split else ""), nf)
+        # FP64 stages on combined meshes, unless sharded or with unfused or whole-step kernels
+        comb = not mixed and not multi and p.fused == 1 and not p.max_adaptive_speedup > 1.0
+        kernel = "k_stage64<%d>" % nf if comb else \
+            "k_rk4_stage%s<%d>" % ("_mixed" if mixed else ("_split" if split else ""), nf)
         stage_idx = [1, 3, 5, 7] if mixed else [0, 1, 2, 3]
         stage_serial = float(kms[:, stage_idx].mean())
         bytes_per_launch = (per_pstep * n + mesh_bytes_per_step(p, nf)) / 4.0

@@ -414,6 +414,10 @@ __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevStat
     deposit_comb64<NF, T, WX, WY, RW, false, true>(P, A.lm_out, sm.rec, sm.key, sm.starts, sm.v, sm.d);
 }
 
+// (16^3 cells x 48 directions, 10 steps recorded and swept: 62.1 -> 29.5 ms
+// when recompute and sweep moved to the combined meshes and the products of
+// emu_tile64.cuh, 23.7 with the commutator's closed-form VJP; bound by the
+// FP64 products and the registers of the sweep, three CTAs per SM)
 template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 3) k_adj_stage(DevParams P, DevState S, int s, double dt, AdjStagePtrs A)
 {

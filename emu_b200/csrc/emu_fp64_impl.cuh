@@ -87,6 +87,13 @@ __device__ __forceinline__ void sc_static64(const DevState& S, const DevState& D
 // added by the stages that read those anyway): 234 words of state per
 // particle and step where Y and the sum stored by every stage took 288, with
 // the same operations in the reference's order.
+// What bounds it: the phases of a tile add up (stage 1 at 32^3 cells x 96
+// directions, 650 us: base 254, interpolation 160, deposit 235; the matrix
+// instruction's floor is 185 us for each of the two products, 27 cells padded
+// to 28).  Stages 1-4 and the re-sort there: 637/690/865/772 + 471 us, where a
+// thread per particle on the full meshes took 3710/4057/4065/2321 + 2352; 90
+// x 77 cells x 60 directions: 2149 -> 445 us a step.  Four CTAs per SM: five
+// (677 us) spill, three (741) leave latency open.
 // SC (stage 4 before a re-sort): the new state and every unchanged field of
 // particle p go to slot inv[p] of D, the other particle buffer (keys by stage
 // 3 into kout, iout, the sort before this kernel, D's deposit after it).
@@ -365,7 +372,8 @@ __global__ void __launch_bounds__(kBlock, 4)
 // dt K_3, K_3 in S.fs), made only on the steps after
 // which it can be read (m4_full_step), and the note of which kind of step
 // this is (StepCtl::m4_full).  A CTA takes tiles of 128 particles in turn, so
-// that a step without it costs one small grid.
+// that a step without it costs one small grid.  (32^3 cells x 96 directions:
+// the last step of a call takes 1.2 ms longer than the others' 3.8.)
 template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 3)
     k_deposit_full64(DevParams P, DevState S, const double* __restrict__ f, double* __restrict__ mesh, StepCtl* ctl)

@@ -103,8 +103,11 @@ typedef struct emu_params {
     uint64_t seed;           /* counter-based RNG seed for sim types 4 and 5
                                 (the reference seeds from the clock, main.cpp:240) */
     int resort_interval;     /* steps between on-device cell re-sorts (0 = never,
-                                < 0 = automatic: every step for 3D stencils,
-                                every 16 steps otherwise; default -1) */
+                                < 0 = automatic: every step for 27-cell stencils
+                                and for FP64 stencils of more than 3 cells; FP64
+                                1D problems that run in one launch every 32
+                                steps, or never with one cell; every 16 steps
+                                otherwise; default -1) */
     int fused;               /* RK4 kernels: 1 (default) one fused kernel per stage, a CUDA
                                 graph per step; 2: one cooperative launch per step when the
                                 grid fits on the GPU at once (FP64), else as 1; 0: unfused */
@@ -200,8 +203,8 @@ int emu_evolve(emu_context* ctx, int nsteps, double start_time, double end_time,
  * many steps (each a CUDA graph launch, no host synchronisation); end =
  * synchronise and report.  Steps past max_steps or end_time do no work. */
 int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int max_steps);
-/* Mixed precision without the adaptive timestep branch (max_adaptive_speedup
- * <= 1): the steps of one call but the last (and the last of the run) keep
+/* Without the adaptive timestep branch (max_adaptive_speedup <= 1, mixed
+ * precision and FP64): the steps of one call but the last (and the last of the run) keep
  * their stage-4 mesh only in the layout stage 4 interpolates, plus the
  * diagonal N_ii that compute_dt reads, none of which a caller can read
  * before the call returns; the results do not depend on how a run is split
@@ -209,9 +212,9 @@ int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int m
 int emu_evolve_steps(emu_context* ctx, int nsteps);
 int emu_evolve_end(emu_context* ctx, emu_run_info* info);
 /* Limit of the bounded grid-barrier waits of this context's cooperative
- * kernels (the whole-step kernel of fused = 2 and the adjoint's segment
- * kernels), in polls of a 64 ns sleep; polls < 0 restores the default
- * (2^22).  A wait that runs out sets EMU_ERR_TIMEOUT in the run's status and
+ * kernels (the kernels that run several steps of small 1D problems, the
+ * whole-step kernel of fused = 2 and the adjoint's segment kernels), in
+ * polls; polls < 0 restores the default (2^22).  A wait that runs out sets EMU_ERR_TIMEOUT in the run's status and
  * lets the kernel finish (the step's results are then invalid); the next
  * emu_evolve_begin or emu_load_particles resets the barrier.  No
  * counterpart in the reference (its steps have no device-side waits);
@@ -225,7 +228,8 @@ int emu_flush_l2(emu_context* ctx, void* device_buffer, int64_t bytes);
  * context stream.
  * kernel_ms[i] receives the duration of kernel i in launch order (the RK
  * stages, with the mixed path's finalize kernel before each; stage 4 also
- * reduces compute_dt), then, when a re-sort follows the step, the whole
+ * reduces compute_dt; one kernel for a whole step of the FP64 1D problems
+ * that run in one launch), then, when a re-sort follows the step, the whole
  * re-sort (keys, radix sort, gather, and the deposit of the new state that
  * stage 4 then leaves out, as emu_evolve_steps does) as one more entry;
  * *nkernels their count (at most 9).  Call after emu_evolve_begin. */
