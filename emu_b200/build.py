@@ -29,8 +29,8 @@ SOURCES = ["emu_k_comb64_3.cu", "emu_k_comb64_2.cu", "emu_k_fp64_3.cu", "emu_k_m
            "emu_init.cpp"]
 # the device initial-condition generator must round like the host one
 EXTRA = {"emu_init_device.cu": ["-fmad=false"]}
-HEADERS = ["emu_device.cuh", "emu_kernels.cuh", "emu_kernels_impl.cuh", "emu_fp64.cuh", "emu_tile64.cuh", "emu_fp64_impl.cuh", "emu_context.cuh", "emu_adjoint.cuh", "emu_host.h",
-           "emu_init_record.h"]
+HEADERS = ["emu_device.cuh", "emu_kernels.cuh", "emu_kernels_impl.cuh", "emu_fp64.cuh", "emu_tile64.cuh", "emu_fp64_impl.cuh", "emu_context.cuh", "emu_adjoint.cuh", "emu_window.h",
+           "emu_host.h", "emu_init_record.h"]
 
 
 def _stale(out, deps):

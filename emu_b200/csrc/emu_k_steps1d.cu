@@ -3,6 +3,7 @@
 #include "emu_adjoint.cuh"
 #include "emu_fp64.cuh"
 #include "emu_kernels_impl.cuh"
+#include "emu_window.h"
 
 namespace emu {
 namespace {
@@ -119,7 +120,9 @@ __device__ __noinline__ void deposit_spread(int nz, double* mesh, const double* 
     using R = Rec1D<NF>;
     constexpr int NT = DepN<NF, D>::NT;
     const int lane = threadIdx.x & 31, row = lane >> 2, col = lane & 3;
-    for (int base = lo; base <= hi; base += 8) {
+    const int ntiles = cell_tiles(lo, hi);
+    for (int tile = 0; tile < ntiles; tile++) {
+        const int base = lo + 8 * tile;
         double a[4];
         bool any = false;
 #pragma unroll
@@ -279,8 +282,9 @@ __device__ __forceinline__ void place_particles(const DevParams& P, Place1D& L, 
     L.wide = L.win > kWin;
     r -= lo;
     L.ci0 = L.wide ? first : r;
-    L.wlo = mn - lo;
-    L.whi = mx - lo + P.w[2] - 1;
+    const CellRange own = warp_cells(mn, mx, lo, P.w[2]);
+    L.wlo = own.lo;
+    L.whi = own.hi;
     L.narrow = !L.wide && mx >= mn && L.whi - L.wlo < kNarrow;
     place_weights<NF>(L, rec, wrec, sp, r);
     if (L.narrow) {
@@ -590,7 +594,7 @@ __global__ void __launch_bounds__(MAXT, 1)
             }
 #pragma unroll
             for (int k = 0; k < KI; k++) mrow_of[k] = (L.c0 + 4 * k + col) % nz * MR;
-            place_weights<NF>(L, rec, wrec, sp, r - mn);
+            place_weights<NF>(L, rec, wrec, sp, any ? r - mn : 0);
         }
     };
     if constexpr (!ONE) {
