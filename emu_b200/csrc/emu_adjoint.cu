@@ -77,7 +77,7 @@ struct emu_adjoint {
     double *wf = nullptr, *lamtmp = nullptr, *wpos = nullptr, *wtime = nullptr;
     double* rows = nullptr;     // n x NS staging for host transfers
     unsigned* map[2] = {};      // recorded forward: slot -> slot at the segment start, through the re-sorts
-    bool final_mapped = false;  // perm slot nck: the map of the run's last segment (re-sorts in it)
+    bool final_mapped = false;  // perm slot nck: the map of the run's last segment (re-sorts in it), undone first
     // per-step mode with re-sorts: the backward's recompute re-sorts as the
     // forward did; second state buffers, the re-sort permutation of every
     // step of a sub-segment, the composed map of every sub-segment
@@ -1368,6 +1368,17 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     G.lamYd = a->lamYd;
     G.lamN = a->lamN;
 
+    // the static fields and the adjoint state through the composed map in a
+    // perm slot: back to the order before a segment's re-sorts
+    auto undo_sorts = [&](int slot) -> int {
+        emu::k_static_scatter<<<g, emu::kBlock, 0, st>>>(stat_view(a, w, S), stat_view(a, 1 - w, S),
+                                                         a->perm + (size_t)slot * cap, a->lamY0, a->lamtmp, NS + 2);
+        CU(cudaMemcpyAsync(a->lamY0, a->lamtmp, sizeof(double) * (size_t)(NS + 2) * cap, cudaMemcpyDeviceToDevice,
+                           st));
+        w = 1 - w;
+        return EMU_OK;
+    };
+    if (!rps && a->final_mapped && (r = undo_sorts(a->nck))) return r;
     for (int seg = a->nck - 1; seg >= 0; seg--) {
         const int k0 = seg * a->interval, k1 = std::min(k0 + a->interval, a->nsteps), len = k1 - k0;
         DevState W = stat_view(a, w, S);   // static fields in this segment's slot order
@@ -1621,15 +1632,8 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
                 }
             }
         }
-        if (!rps && seg > 0 && a->resorted[seg]) {
-            // undo the re-sorts of the previous segment (composed map)
-            const unsigned* perm = a->perm + (size_t)seg * cap;
-            emu::k_static_scatter<<<g, emu::kBlock, 0, st>>>(W, stat_view(a, 1 - w, S), perm, a->lamY0, a->lamtmp,
-                                                             NS + 2);
-            CU(cudaMemcpyAsync(a->lamY0, a->lamtmp, sizeof(double) * (size_t)(NS + 2) * cap, cudaMemcpyDeviceToDevice,
-                               st));
-            w = 1 - w;
-        }
+        // (the re-sorts of the segment before this one)
+        if (!rps && seg > 0 && a->resorted[seg] && (r = undo_sorts(seg))) return r;
     }
     CU(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
