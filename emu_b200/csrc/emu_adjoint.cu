@@ -56,6 +56,7 @@ struct emu_adjoint {
     // device) and the backward recomputes nothing; full_steps = capacity
     bool full = false;
     int full_steps = 0;
+    bool fits = false;          // the loaded particles' run can be recorded that way (adj_records)
     double t0 = 0.0;
     std::vector<double> dts;
     std::vector<char> resorted; // segment c began with a cell re-sort (permutation perm[c])
@@ -903,6 +904,13 @@ std::vector<int> rps_layout(int len, int B)
     return sb;
 }
 
+// a run of the loaded particles can be recorded whole (k_steps_1d, or
+// co-resident segments): depends on their number, not on the capacity
+bool adj_records(const emu_context* ctx)
+{
+    return ctx->steps1d || emu::adj_coop_fits(ctx->nf, ctx->P, ctx->S[ctx->cur].n);
+}
+
 // device arrays for a recorded run of nsteps with checkpoints every interval
 int ensure_adj(emu_context* ctx, int nsteps, int interval)
 {
@@ -911,7 +919,8 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
     const int nck = (nsteps + interval - 1) / interval;
     const long long nm = cmesh_elems(ctx);
     emu_adjoint* a = ctx->adj;
-    if (a && (a->cap != cap || a->NS != NS || a->ck_slots < nck || a->interval_cap < interval ||
+    const bool fits = adj_records(ctx);
+    if (a && (a->cap != cap || a->NS != NS || a->ck_slots < nck || a->interval_cap < interval || a->fits != fits ||
               (int)a->dts.size() < nsteps || (a->full && a->full_steps < nsteps))) {
         free_adj(a);
         a = ctx->adj = nullptr;
@@ -921,6 +930,7 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         ctx->adj = a;
         a->cap = cap;
         a->NS = NS;
+        a->fits = fits;
         a->dts.resize(std::max(nsteps, 1));
         a->ck_slots = std::max(nck, 1);
         a->interval_cap = interval;
@@ -938,8 +948,7 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
         const char* fenv = std::getenv("EMU_ADJOINT_FULL_STORE");
         // (the recorded forward takes dt from combined meshes: no adaptive
         // timestep there)
-        a->full = a->store && (!fenv || std::atoi(fenv) != 0) && !(ctx->prm.max_adaptive_speedup > 1.0) &&
-                  (ctx->steps1d || emu::adj_coop_fits(ctx->nf, ctx->P, ctx->S[ctx->cur].n)) &&
+        a->full = a->store && (!fenv || std::atoi(fenv) != 0) && !(ctx->prm.max_adaptive_speedup > 1.0) && fits &&
                   (size_t)nsteps * (per_step + sizeof(double) * slot) <= budget;
         a->full_steps = a->full ? nsteps : 0;
         const size_t st_steps = a->full ? (size_t)nsteps : a->store ? (size_t)interval : 1;
