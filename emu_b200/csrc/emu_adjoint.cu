@@ -1355,7 +1355,8 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     int w = 0;
     emu::k_static_scatter<<<g, emu::kBlock, 0, st>>>(S, stat_view(a, 0, S), nullptr, nullptr, nullptr, 0);
     CU(cudaMemsetAsync(a->lmesh[0], 0, sizeof(double) * nm, st));
-    emu::launch_ctl_set(ctx->ctl, 0.0, 0.0, INFINITY, INT_MAX, 0, st);
+    // (a sweep that timed out before this one does not end it)
+    emu::launch_ctl_set(ctx->ctl, 0.0, 0.0, INFINITY, INT_MAX, 1, st);
     if ((r = check_launch(ctx, "adjoint input"))) return r;
     const bool coop = a->store && emu::adj_coop_fits(nf, ctx->P, n);
     // per-step mode with re-sorts (the recomputes re-sort as the forward did)

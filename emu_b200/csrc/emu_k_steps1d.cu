@@ -179,7 +179,13 @@ __device__ __noinline__ void deposit_tiles(int ncells, double* mesh, int stride,
 
 // Grid barrier in two halves: arrivals counted up from 0 over the launch (the
 // last CTA to leave the kernel sets the count back).  The wait is bounded;
-// false: it gave up (ST_TIMEOUT is set, the CTA leaves the kernel).
+// false: it gave up (ST_TIMEOUT is set, the CTA goes to the kernel's end).
+__device__ __forceinline__ bool steps_timed_out(const StepCtl* ctl)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&ctl->status) : "memory");
+    return (v & ST_TIMEOUT) != 0;
+}
 __device__ __forceinline__ void steps_arrive(StepCtl* ctl)
 {
     __syncthreads();
@@ -881,9 +887,8 @@ __global__ void __launch_bounds__(MAXT, 1)
         last = last_next;
         if (done) break;
     }
-    if (!alive) return;
 
-    if (active) {
+    if (alive && active) {
 #pragma unroll
         for (int e = 0; e < NH; e++) S.f0[(sp * NH + e) * cap + p] = y0[e];
         if (sp == 0) {
@@ -901,14 +906,19 @@ __global__ void __launch_bounds__(MAXT, 1)
             cmesh[msize + i] = 0.0;
         }
     }
-    // the last CTA to leave writes the step control (all hold the same)
+    // the last CTA to leave writes the step control (all hold the same).  Every
+    // CTA comes by, also one that gave up a wait, so that the counts are right
+    // for the next launch; then the run ends with the steps before this launch
+    // (the launches queued behind it return at once)
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
             __threadfence();
             ctl->blocks_done = 0u;
             ctl->bar_count = 0u;
-            if (dt_mode == DT_ADVANCE) {
+            if (steps_timed_out(ctl)) {
+                ctl->done = 1;
+            } else if (dt_mode == DT_ADVANCE) {
                 ctl->t = t_run;
                 ctl->dt = dt;
                 ctl->step = step;
@@ -982,9 +992,10 @@ __global__ void __launch_bounds__(MAXT, 1)
         shape<double>(zpos(len - 1) * P.dxi[2], P.ord[2], first, L.wz);
         sref = wrapi(first, nz);
     }
-    __syncthreads();
+    // (a segment swept before this one in the same call gave up)
+    bool alive = __syncthreads_and(!steps_timed_out(ctl));
     unsigned nbar = 0;
-    for (int j = len - 1; j >= 0; j--) {
+    for (int j = len - 1; j >= 0 && alive; j--) {
         const double* const sst = A.rec.sst + j * A.rec.sst_stride;
         const double dt = A.dts[j];
         load(sst + 3 * (2 * NH) * cap, yn);   // Y_n
@@ -1060,10 +1071,13 @@ __global__ void __launch_bounds__(MAXT, 1)
                 load(s == 2 ? A.rec.seg + j * A.rec.seg_stride : sst + (s - 3) * (2 * NH) * cap, ys);   // Y_{s-1}
             }
             nbar++;
-            if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) return;
+            if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) {
+                alive = false;
+                break;
+            }
         }
     }
-    if (active) {
+    if (alive && active) {
 #pragma unroll
         for (int e = 0; e < NH; e++) A.lamY0[(sp * NH + e) * cap + p] = lamY[e];
         A.lamN[sp * cap + p] += dN;
