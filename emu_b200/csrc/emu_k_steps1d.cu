@@ -858,8 +858,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                 }
                 if (wait) {
                     nbar++;
-                    // (the caller's limit is for fused = 2 and the adjoint)
-                    if (!steps_wait(ctl, nbar * gridDim.x, REC ? P.wait_polls : kBarrierSpins)) {
+                    if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) {
                         alive = false;
                         break;
                     }

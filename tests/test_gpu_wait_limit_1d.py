@@ -30,6 +30,41 @@ def _clean(c, p, parts, n):
     assert colwise_rel(c.get_particles(), ref) < 1e-11
 
 
+@pytest.mark.parametrize("resort", [0, 1, 4])
+def test_steps(resort):
+    p = _params(resort)
+    parts = api.init_particles(p)
+    with api.Context(p) as c:
+        c.load_particles(parts)
+        c.set_wait_limit(0)
+        with pytest.raises(api.EmuError) as e:
+            c.evolve(9)
+        assert e.value.code & api.EMU_ERR_TIMEOUT
+        with pytest.raises(api.EmuError) as e:
+            c.step(1e-13)
+        assert e.value.code & api.EMU_ERR_TIMEOUT
+        c.set_wait_limit(-1)
+        _clean(c, p, parts, 9)
+
+
+def test_a_run_that_timed_out_takes_no_further_steps():
+    p = _params(2)
+    parts = api.init_particles(p)
+    with api.Context(p) as c:
+        c.load_particles(parts)
+        c.evolve_begin(0.0, float("inf"), 20)
+        c.evolve_steps(5)
+        c.synchronize()
+        c.set_wait_limit(0)
+        c.evolve_steps(6)
+        c.set_wait_limit(-1)
+        c.evolve_steps(4)
+        info = c.evolve_end()
+        assert info.status & api.EMU_ERR_TIMEOUT and info.steps_done == 5
+        assert info.time > 0.0
+        _clean(c, p, parts, 9)
+
+
 def test_recorded_run_and_sweep():
     p = _params(2)
     parts = api.init_particles(p)
