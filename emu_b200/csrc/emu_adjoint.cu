@@ -186,8 +186,9 @@ struct AdjFwdPtrs {
 // Stage recompute: K = RHS(Yin, M_s); s < 4: acc, Y_{s+1} = Y0 + a dt K and
 // its deposit; s == 4: Y_n = acc + b4 dt K, and the step's completion: Y_new =
 // Renormalize(Y_n), positions advanced and wrapped, the deposit of Y_new at
-// the new positions.  Same operations as the forward stage kernel.
-template <int NF, int WX, int WY, int WZ, int KS>
+// the new positions.  Same operations as the forward stage kernel.  LIVE: the
+// meshes are written in the same launch (see mesh_load).
+template <int NF, int WX, int WY, int WZ, int KS, bool LIVE>
 __device__ __forceinline__ void adj_fwd_body(const DevParams& P, const DevState& S, int s, double dt,
                                              const AdjFwdPtrs& A)
 {
@@ -211,7 +212,7 @@ __device__ __forceinline__ void adj_fwd_body(const DevParams& P, const DevState&
         vsc = S.vscale[p];
     }
     int slot = adj_tile<NF, T, WX, WY, WZ, RW>(P, sm, active, x, v, st);
-    interp64<NF, T, WX, WY, RW>(P, A.mesh_in, sm.rec, sm.key, sm.v);
+    interp64<NF, T, WX, WY, RW, false, LIVE>(P, A.mesh_in, sm.rec, sm.key, sm.v);
     __syncthreads();
     double* rec = sm.rec + slot * RW;
     double hs[NH], c[NV];
@@ -290,7 +291,7 @@ __device__ __forceinline__ void adj_fwd_body(const DevParams& P, const DevState&
 template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 4) k_adj_fwd_stage(DevParams P, DevState S, int s, double dt, AdjFwdPtrs A)
 {
-    adj_fwd_body<NF, WX, WY, WZ, KS>(P, S, s, dt, A);
+    adj_fwd_body<NF, WX, WY, WZ, KS, false>(P, S, s, dt, A);
 }
 
 struct AdjStagePtrs {
@@ -310,8 +311,8 @@ struct AdjStagePtrs {
 
 // One backward launch: (s < 4) finish stage s+1 by gathering its adjoint
 // mesh, (s >= 1) start stage s: commutator VJP and the scatter of lam_H.
-// s = 4 starts from the Renormalize VJP.
-template <int NF, int WX, int WY, int WZ, int KS>
+// s = 4 starts from the Renormalize VJP.  LIVE: as adj_fwd_body.
+template <int NF, int WX, int WY, int WZ, int KS, bool LIVE>
 __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevState& S, int s, double dt,
                                                const AdjStagePtrs& A)
 {
@@ -340,7 +341,7 @@ __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevStat
     if (s < 4) {
         // D^T (the transpose of the N / F deposit): G_c of nu; of nubar with
         // the opposite sign for real components
-        interp64<NF, T, WX, WY, RW, true>(P, A.lm_in, sm.rec, sm.key, sm.v);
+        interp64<NF, T, WX, WY, RW, true, LIVE>(P, A.lm_in, sm.rec, sm.key, sm.v);
         __syncthreads();
         adj_sums<NF, WP>(rec, 1.0, g);
         __syncthreads();
@@ -386,7 +387,7 @@ __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevStat
         }
     }
     if (s < 1) return;
-    interp64<NF, T, WX, WY, RW>(P, A.mesh_s, sm.rec, sm.key, sm.v);
+    interp64<NF, T, WX, WY, RW, false, LIVE>(P, A.mesh_s, sm.rec, sm.key, sm.v);
     __syncthreads();
     double hs[NH], c[NV];
     adj_sums<NF, WP>(rec, P.sqrt2GF_inv_vol, hs);
@@ -422,7 +423,7 @@ __device__ __forceinline__ void adj_stage_body(const DevParams& P, const DevStat
 template <int NF, int WX, int WY, int WZ, int KS>
 __global__ void __launch_bounds__(kBlock, 3) k_adj_stage(DevParams P, DevState S, int s, double dt, AdjStagePtrs A)
 {
-    adj_stage_body<NF, WX, WY, WZ, KS>(P, S, s, dt, A);
+    adj_stage_body<NF, WX, WY, WZ, KS, false>(P, S, s, dt, A);
 }
 
 // One checkpoint segment of len steps, stored step by step:
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_fwd_coop(DevParams P, Dev
             // next step's dt; M_4 is complete and every block holds this step's
             // dt, so it overlaps stage 4 and shares its barrier
             if (s == 4 && G.record) dt_reduce_comb64<NF>(P, seg_m(G, j, 3), ctl, reduce_blocks(P));
-            adj_fwd_body<NF, WX, WY, WZ, KS>(P, Q, s, dt, seg_fwd_ptrs(G, j, s, cap, next, more, G.record ? ctl : nullptr));
+            adj_fwd_body<NF, WX, WY, WZ, KS, true>(P, Q, s, dt, seg_fwd_ptrs(G, j, s, cap, next, more, G.record ? ctl : nullptr));
             grid_barrier(ctl, P.wait_polls);
         }
         if (G.record && __ldcg(&ctl->done) && more) break;   // (uniform: read after the barrier)
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_seg_bwd_coop(DevParams P, Dev
         const double dt = G.dts[G.k0 + j];
 #pragma unroll 1
         for (int s = 4; s >= 0; s--) {
-            adj_stage_body<NF, WX, WY, WZ, KS>(P, Q, s, dt, seg_stage_ptrs(G, j, s, cap));
+            adj_stage_body<NF, WX, WY, WZ, KS, true>(P, Q, s, dt, seg_stage_ptrs(G, j, s, cap));
             grid_barrier(ctl, P.wait_polls);
         }
     }

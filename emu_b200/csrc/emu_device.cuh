@@ -127,6 +127,17 @@ __device__ __forceinline__ void shape(double delta, int order, int& first, R w[3
     }
 }
 
+// A value of a mesh that this kernel only reads, or (LIVE) that other CTAs of
+// the same launch write before a grid barrier: the read-only path is for data
+// that stands for the whole kernel, a plain load is ordered by the barrier's
+// acquire.
+template <bool LIVE, class T>
+__device__ __forceinline__ T mesh_load(const T* m)
+{
+    if constexpr (LIVE) return *m;
+    else return __ldg(m);
+}
+
 __device__ __forceinline__ int wrapi(int a, int n)
 {
     int r = a % n;

@@ -42,7 +42,7 @@ __device__ __forceinline__ void dt_reduce_comb64(const DevParams& P, const doubl
             const double2* d = reinterpret_cast<const double2*>(mesh + c * kCombSlots<NF> + Comb<NF>::NG);
 #pragma unroll
             for (int i = 0; i < NF; i++) {
-                const double2 t = d[i];
+                const double2 t = __ldcg(d + i);
                 vm = fmax(vm, fmax(t.x, t.y));
             }
         }

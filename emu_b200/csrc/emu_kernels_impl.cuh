@@ -59,8 +59,8 @@ inline unsigned grid_for(long long n, int block = kBlock)
 // FP64 potential of one particle (Evolve.cpp:128-158 with the Vvac and
 // interpolate fills): V starts at the vacuum term and accumulates
 // coef*inside per stencil cell, nubar with the reference's sign rule.
-template <int NF, class SWt>
-__device__ __forceinline__ void potential_fp64(const DevParams& P, const double* __restrict__ mesh,
+template <int NF, class SWt, bool LIVE = false>
+__device__ __forceinline__ void potential_fp64(const DevParams& P, const double* mesh,
                                                const Stencil<double>& st, double vx, double vy, double vz,
                                                double vscale, double* V)
 {
@@ -73,14 +73,13 @@ __device__ __forceinline__ void potential_fp64(const DevParams& P, const double*
     }
     STENCIL_LOOP(SWt, {
         const long long cell = cell_of(P, st.b[0], st.b[1], st.b[2], ii, jj, kk);
-        const double* __restrict__ m = mesh + cell * ND;
+        const double* m = mesh + cell * ND;
         const double coef = ((P.sqrt2GF_inv_vol * st.wx[ii]) * st.wy[jj]) * st.wz[kk];
+        auto ld = [&](int k) { return mesh_load<LIVE>(m + k); };
 #pragma unroll
         for (int e = 0; e < NH; e++) {
-            const double SI = __ldg(m + e) - __ldg(m + 2 * NH + e) * vx - __ldg(m + 4 * NH + e) * vy -
-                              __ldg(m + 6 * NH + e) * vz;
-            const double Sb = __ldg(m + NH + e) - __ldg(m + 3 * NH + e) * vx - __ldg(m + 5 * NH + e) * vy -
-                              __ldg(m + 7 * NH + e) * vz;
+            const double SI = ld(e) - ld(2 * NH + e) * vx - ld(4 * NH + e) * vy - ld(6 * NH + e) * vz;
+            const double Sb = ld(NH + e) - ld(3 * NH + e) * vx - ld(5 * NH + e) * vy - ld(7 * NH + e) * vz;
             double inside = H::is_im(e) ? SI + Sb : SI - Sb;
             if (e == 0) inside = inside + P.matter;
             const double t = coef * inside;
@@ -563,9 +562,10 @@ __device__ __forceinline__ int tile_deposit_block_split(const DevParams& P, T* m
 // ===========================================================================
 // fused FP64 RK4 stage
 // ===========================================================================
-template <int NF, class SWt>
+// COOP: a stage of a whole-step launch (its meshes are written there too)
+template <int NF, class SWt, bool COOP = false>
 __device__ __forceinline__ void rk4_stage_body(const DevParams& P, const DevState& S, int s,
-                                               const double* __restrict__ mesh_in, double* __restrict__ mesh_out,
+                                               const double* mesh_in, double* __restrict__ mesh_out,
                                                double* mesh_zero, long long nzero, StepCtl* ctl, double dt,
                                                int dt_mode = -1)
 {
@@ -630,7 +630,7 @@ __device__ __forceinline__ void rk4_stage_body(const DevParams& P, const DevStat
             }
         }
         double V[NS];
-        potential_fp64<NF, SWt>(P, mesh_in, st, vx, vy, vz, vsc, V);
+        potential_fp64<NF, SWt, COOP>(P, mesh_in, st, vx, vy, vz, vsc, V);
         const double bw = dt * kRK4B[s - 1];
         const double aw = s < 4 ? dt * kRK4A[s] : 0.0;
         int stt = 0;
@@ -712,8 +712,8 @@ __device__ __forceinline__ void rk4_stage_body(const DevParams& P, const DevStat
 }
 
 // FP64 potential of one species (potential_fp64 restricted to species sp)
-template <int NF, class SWt>
-__device__ __forceinline__ void potential_fp64_sp(const DevParams& P, const double* __restrict__ mesh,
+template <int NF, class SWt, bool LIVE>
+__device__ __forceinline__ void potential_fp64_sp(const DevParams& P, const double* mesh,
                                                   const Stencil<double>& st, double vx, double vy, double vz,
                                                   double vscale, int sp, double* V)
 {
@@ -723,7 +723,7 @@ __device__ __forceinline__ void potential_fp64_sp(const DevParams& P, const doub
     for (int e = 0; e < NH; e++) V[e] = P.M2[sp][e] * vscale;
     STENCIL_LOOP(SWt, {
         const long long cell = cell_of(P, st.b[0], st.b[1], st.b[2], ii, jj, kk);
-        const double* __restrict__ m = mesh + cell * ND;
+        const double* m = mesh + cell * ND;
         const double coef = ((P.sqrt2GF_inv_vol * st.wx[ii]) * st.wy[jj]) * st.wz[kk];
         // the cell's 8 NH values (two flavors: 16-byte vector loads, every
         // group of NH = 4 starts on a 32-byte boundary)
@@ -731,13 +731,13 @@ __device__ __forceinline__ void potential_fp64_sp(const DevParams& P, const doub
         if constexpr (NH % 2 == 0) {
 #pragma unroll
             for (int k = 0; k < ND / 2; k++) {
-                const double2 v = __ldg(reinterpret_cast<const double2*>(m) + k);
+                const double2 v = mesh_load<LIVE>(reinterpret_cast<const double2*>(m) + k);
                 c[2 * k] = v.x;
                 c[2 * k + 1] = v.y;
             }
         } else {
 #pragma unroll
-            for (int k = 0; k < ND; k++) c[k] = __ldg(m + k);
+            for (int k = 0; k < ND; k++) c[k] = mesh_load<LIVE>(m + k);
         }
 #pragma unroll
         for (int e = 0; e < NH; e++) {
@@ -753,9 +753,9 @@ __device__ __forceinline__ void potential_fp64_sp(const DevParams& P, const doub
 
 // Species-split FP64 RK4 stage (1D stencils): thread t advances species
 // t / kBlock of particle t % kBlock; same arithmetic as rk4_stage_body.
-template <int NF, class SWt>
+template <int NF, class SWt, bool COOP = false>
 __device__ __forceinline__ void rk4_stage_body_split(const DevParams& P, const DevState& S, int s,
-                                                     const double* __restrict__ mesh_in, double* __restrict__ mesh_out,
+                                                     const double* mesh_in, double* __restrict__ mesh_out,
                                                      double* mesh_zero, long long nzero, StepCtl* ctl, double dt,
                                                      int dt_mode = -1)
 {
@@ -798,7 +798,7 @@ __device__ __forceinline__ void rk4_stage_body_split(const DevParams& P, const D
             a0[e] = s > 1 ? S.acc[o] : 0.0;
         }
         double V[NH], K[NH];
-        potential_fp64_sp<NF, SWt>(P, mesh_in, st, vx, vy, vz, vsc, sp, V);
+        potential_fp64_sp<NF, SWt, COOP>(P, mesh_in, st, vx, vy, vz, vsc, sp, V);
         commutator<NF, double>(V, f, K, P.inv_hbar);
         const double bw = dt * kRK4B[s - 1];
         const double aw = s < 4 ? dt * kRK4A[s] : 0.0;
@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_rk4_step_coop(DevParams P, DevSta
     double* const m[4] = {m0, m1, m2, m3};
 #pragma unroll 1
     for (int s = 1; s <= 4; s++) {
-        rk4_stage_body<NF, SWt>(P, S, s, m[s - 1], m[s % 4], m[(s + 1) % 4], nmesh, ctl, dt);
+        rk4_stage_body<NF, SWt, true>(P, S, s, m[s - 1], m[s % 4], m[(s + 1) % 4], nmesh, ctl, dt);
         if (s < 4) grid_barrier(ctl, P.wait_polls);
     }
     if (dt_mode == DT_ADVANCE) dt_reduce_and_finish<NF, double>(P, m3, ctl, DT_ADVANCE, reduce_blocks(P));
@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(2 * kBlock, 2) k_rk4_step_coop_split(DevParams
     double* const m[4] = {m0, m1, m2, m3};
 #pragma unroll 1
     for (int s = 1; s <= 4; s++) {
-        rk4_stage_body_split<NF, SWt>(P, S, s, m[s - 1], m[s % 4], m[(s + 1) % 4], nmesh, ctl, dt);
+        rk4_stage_body_split<NF, SWt, true>(P, S, s, m[s - 1], m[s % 4], m[(s + 1) % 4], nmesh, ctl, dt);
         if (s < 4) grid_barrier(ctl, P.wait_polls);
     }
     if (dt_mode == DT_ADVANCE) dt_reduce_and_finish<NF, double>(P, m3, ctl, DT_ADVANCE, reduce_blocks(P));

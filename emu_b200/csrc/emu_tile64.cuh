@@ -246,10 +246,10 @@ __device__ __forceinline__ void run_starts(const int* skey, unsigned* starts)
 // The interpolated, velocity-weighted sums u_j = G_0j - v . G_dj of the
 // warp's 32 slots, from the combined mesh, into the records' values
 // (rec + WP + j).  sv: v per slot and dimension, rows of VS.  PLUS: G_0 + v . G_d
-// (the transpose of a deposit, see emu_adjoint.cu).
-template <int NF, class T, int WX, int WY, int RW, bool PLUS = false>
-__device__ __forceinline__ void interp64(const DevParams& P, const double* __restrict__ mesh, double* srec,
-                                         const int* skey, const double* sv)
+// (the transpose of a deposit, see emu_adjoint.cu).  LIVE: see mesh_load.
+template <int NF, class T, int WX, int WY, int RW, bool PLUS = false, bool LIVE = false>
+__device__ __forceinline__ void interp64(const DevParams& P, const double* mesh, double* srec, const int* skey,
+                                         const double* sv)
 {
     constexpr int KS = T::KS, NT = T::NT, NV = T::NV, NCS = T::NCS, WP = T::WP, VS = T::VS;
     const int lane = threadIdx.x & 31, base = threadIdx.x & ~31, row = lane >> 2, col = lane & 3;
@@ -277,7 +277,7 @@ __device__ __forceinline__ void interp64(const DevParams& P, const double* __res
             if (!kc.inside) cell = kc.template wrapped<T, WX, WY>(P, 4 * k + col);
             const double* m = mesh + (long long)cell * NCS + q0;
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++) b[k][nt] = __ldg(m + 8 * nt);
+            for (int nt = 0; nt < NT; nt++) b[k][nt] = mesh_load<LIVE>(m + 8 * nt);
         }
 #pragma unroll
         for (int g = 0; g < 4; g++) {
