@@ -13,8 +13,10 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
+#include <iterator>
 #include <memory>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -37,15 +39,21 @@ bool is_pageable(const void* p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-int ensure_ring(emu_context* ctx)
+// the ring, whole or not at all (a copy then goes the plain way; the next one
+// asks again)
+bool ring_ready(emu_context* ctx)
 {
-    if (ctx->ring) return EMU_OK;
-    CU(emu_ctx::host_malloc(&ctx->ring, kChunk * kSlots));
-    for (int i = 0; i < kSlots; i++) {
-        const cudaError_t e = cudaEventCreateWithFlags(&ctx->ring_event[i], cudaEventDisableTiming);
-        if (e != cudaSuccess) return emu_ctx::fail(ctx, EMU_ERR_CUDA, std::string("ring event: ") + cudaGetErrorString(e));
+    if (ctx->ring) return true;
+    for (auto& e : ctx->ring_event)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) e = nullptr;
+    bool ok = std::all_of(std::begin(ctx->ring_event), std::end(ctx->ring_event), [](cudaEvent_t e) { return e; });
+    ok = ok && emu_ctx::host_malloc(&ctx->ring, kChunk * kSlots) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();
+        ctx->ring = nullptr;
+        emu_ctx::ring_free(ctx);
     }
-    return EMU_OK;
+    return ok;
 }
 
 // Chunks handed out in order; done[i]: chunk i has been moved.  The workers
@@ -56,11 +64,12 @@ struct Work {
     std::atomic<bool> stop{false};
     long long total = 0;
     std::unique_ptr<std::atomic<char>[]> done;
-    void start(long long n)
+    bool start(long long n)
     {
         total = n;
-        done.reset(new std::atomic<char>[(size_t)n]);
-        for (long long i = 0; i < n; i++) done[i].store(0, std::memory_order_relaxed);
+        done.reset(new (std::nothrow) std::atomic<char>[(size_t)n]);
+        for (long long i = 0; done && i < n; i++) done[i].store(0, std::memory_order_relaxed);
+        return done != nullptr;
     }
     void wait(long long i) const
     {
@@ -94,15 +103,17 @@ struct Workers {
     }
 };
 
-// start the workers; false when not one could be started
+// start the workers; false when not one could be started (nothing is thrown
+// through the C interface)
 template <class Move>
 bool start(Workers& ws, Move move)
 {
     const unsigned hc = std::max(2u, std::thread::hardware_concurrency());
     const int n = (int)std::min<unsigned>(kWorkers, hc / 2);
     try {
+        ws.t.reserve(n);
         for (int i = 0; i < n; i++) ws.t.emplace_back([&ws, move] { work_loop(ws.w, move); });
-    } catch (const std::system_error&) {
+    } catch (const std::exception&) {
     }
     return !ws.t.empty();
 }
@@ -128,18 +139,16 @@ int emu_ctx::copy_to_host(emu_context* ctx, void* dst, const void* src, size_t b
         CU(cudaStreamSynchronize(st));
         return EMU_OK;
     };
-    if (bytes < kStagedMin || !is_pageable(dst)) return plain();
+    if (bytes < kStagedMin || !is_pageable(dst) || !ring_ready(ctx)) return plain();
     int r;
-    if ((r = ensure_ring(ctx))) return r;
     char* const d = static_cast<char*>(dst);
     const char* const s = static_cast<const char*>(src);
     const long long n = (long long)((bytes + kChunk - 1) / kChunk);
     auto size = [=](long long i) { return std::min(kChunk, bytes - (size_t)i * kChunk); };
     Work w;
-    w.start(n);
+    if (!w.start(n)) return plain();
     char* const ring = ctx->ring;
     Workers ws{w, {}};
-    if (!start(ws, [=](long long i) { std::memcpy(d + i * kChunk, ring + (i % kSlots) * kChunk, size(i)); })) return plain();
     auto issue = [&](long long i) -> int {
         CU(cudaMemcpyAsync(ring + (i % kSlots) * kChunk, s + i * kChunk, size(i), cudaMemcpyDeviceToHost, st));
         CU(cudaEventRecord(ctx->ring_event[i % kSlots], st));
@@ -147,6 +156,9 @@ int emu_ctx::copy_to_host(emu_context* ctx, void* dst, const void* src, size_t b
     };
     for (long long i = 0; i < std::min<long long>(n, kSlots); i++)
         if ((r = issue(i))) return r;
+    // (the workers poll: none while the stream still works)
+    CU(cudaEventSynchronize(ctx->ring_event[0]));
+    if (!start(ws, [=](long long i) { std::memcpy(d + i * kChunk, ring + (i % kSlots) * kChunk, size(i)); })) return plain();
     for (long long i = 0; i < n; i++) {
         CU(cudaEventSynchronize(ctx->ring_event[i % kSlots]));
         w.ready.store(i + 1, std::memory_order_release);
@@ -169,16 +181,16 @@ int emu_ctx::copy_to_device(emu_context* ctx, void* dst, const void* src, size_t
         CU(cudaStreamSynchronize(st));
         return EMU_OK;
     };
-    if (bytes < kStagedMin || !is_pageable(src)) return plain();
-    int r;
-    if ((r = ensure_ring(ctx))) return r;
+    if (bytes < kStagedMin || !is_pageable(src) || !ring_ready(ctx)) return plain();
     char* const d = static_cast<char*>(dst);
     const char* const s = static_cast<const char*>(src);
     const long long n = (long long)((bytes + kChunk - 1) / kChunk);
     auto size = [=](long long i) { return std::min(kChunk, bytes - (size_t)i * kChunk); };
     Work w;
-    w.start(n);
+    if (!w.start(n)) return plain();
     char* const ring = ctx->ring;
+    // (the workers poll: none while the stream still works)
+    CU(cudaStreamSynchronize(st));
     Workers ws{w, {}};
     if (!start(ws, [=](long long i) { std::memcpy(ring + (i % kSlots) * kChunk, s + i * kChunk, size(i)); })) return plain();
     // chunk i is handed out (its slot's last copy has completed) kSlots / 2
