@@ -921,8 +921,8 @@ int ensure_adj(emu_context* ctx, int nsteps, int interval)
     const long long nm = cmesh_elems(ctx);
     emu_adjoint* a = ctx->adj;
     const bool fits = adj_records(ctx);
-    if (a && (a->cap != cap || a->NS != NS || a->ck_slots < nck || a->interval_cap < interval || a->fits != fits ||
-              (int)a->dts.size() < nsteps || (a->full && a->full_steps < nsteps))) {
+    if (a && (a->cap != cap || a->NS != NS || a->ck_slots < nck || a->interval_cap < interval ||
+              (int)a->dts.size() < nsteps || (a->full && (a->full_steps < nsteps || !fits)) || (fits && !a->fits))) {
         free_adj(a);
         a = ctx->adj = nullptr;
     }
@@ -1123,7 +1123,8 @@ int segment_sweep(emu_context* ctx, const DevState& W, const emu::SegPtrs& G, bo
 // cooperative launch that advances the segment with dt from the device step
 // control, storing Y_0 and x, the stage states and the meshes of every step
 // (what the backward would otherwise recompute), then the particle time and
-// the state after the segment back into the context.
+// the state after the segment back into the context.  When the 1D kernel's
+// launch is refused, ctx->steps1d is false on return and no step was taken.
 int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
 {
     const int NS = ctx->NS;
@@ -1160,6 +1161,7 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
             emu::Rec1DStore rec{G.seg, G.sst, G.mst, G.seg_stride, G.sst_stride, G.mst_stride};
             cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, S, ctx->cmesh, ctx->mesh[3], ctx->ctl, len,
                                                  emu::DT_ADVANCE, st, &rec);
+            if (emu_ctx::leave_steps_1d(ctx, e)) return EMU_OK;   // (refused: nothing has run)
             if (e != cudaSuccess)
                 return fail(ctx, EMU_ERR_CUDA, std::string("recorded segment: ") + cudaGetErrorString(e));
             continue;
@@ -1234,7 +1236,10 @@ int emu_adjoint_forward(emu_context* ctx, int nsteps, int checkpoint_interval, d
     // (only the last step's stage-4 mesh can be read)
     if (ctx->steps1d || ctx->comb64) emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
     if (a->full) {
+        const bool one_d = ctx->steps1d;
         if ((r = record_full(ctx, a, nsteps, checkpoint_interval))) return r;
+        if (one_d && !ctx->steps1d)   // (refused: again, laid out for the stage kernels)
+            return emu_adjoint_forward(ctx, nsteps, checkpoint_interval, start_time, dts, info);
     } else {
     // cell re-sorts on the step loop's schedule; the backward recomputes each
     // segment in its start order, so a segment's re-sorts are composed into

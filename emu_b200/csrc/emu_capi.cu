@@ -293,11 +293,35 @@ int ensure_cmesh(emu_context* ctx)
     return EMU_OK;
 }
 
-// nsteps steps of k_steps_1d (dt_mode as launch_steps_1d)
+// The automatic re-sort interval.  A 27-cell stencil loses its per-CTA cell
+// runs within a step or two once particles leave their cells, a 1D stencil
+// within several.  FP64 stages in a plane re-sort every step too, since the
+// re-sort is made by stage 4's stores (90 x 77 cells x 60 directions: 445 us
+// per step at 1, 457 at 2, 498 at 4, 577 at 16).  Several steps per launch: the
+// re-sort's own launches weigh more and a window a few cells wider costs
+// little (two flavors, 128 x 80: 15.5 us per step at 16, 14.3 at 32, 13.9 at
+// 64; 50 cells x 2 beams, whose warps outgrow the products past 40 steps:
+// 11.0, 10.5, 23.1); one cell needs none.
+void choose_resort(emu_context* ctx)
+{
+    if (ctx->auto_resort) {
+        const int cells = ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2];
+        ctx->prm.resort_interval = cells > (ctx->comb64 ? 3 : 9) ? 1 : 16;
+        if (ctx->steps1d) ctx->prm.resort_interval = ctx->P.ncells > 1 ? 32 : 0;
+    }
+    // with a re-sort after every step, the deposits of stages 1-3 see
+    // cell-sorted particles; otherwise every deposit ranks its keys
+    ctx->P.rank_stages = ctx->prm.resort_interval != 1;
+}
+
+// nsteps steps of k_steps_1d (dt_mode as launch_steps_1d).  When its grid is
+// refused (a stream that may not use every SM) nothing has run and ctx->steps1d
+// is false on return: the caller takes the steps with the stage kernels
 int run_steps_1d(emu_context* ctx, int nsteps, int dt_mode)
 {
     const cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, ctx->S[ctx->cur], ctx->cmesh, ctx->mesh[3], ctx->ctl,
                                                nsteps, dt_mode, ctx->stream);
+    if (emu_ctx::leave_steps_1d(ctx, e)) return EMU_OK;
     if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("cooperative steps: ") + cudaGetErrorString(e));
     ctx->cur_mesh = 3;
     return EMU_OK;
@@ -613,12 +637,25 @@ bool rk4_fused(const emu_context* ctx)
 }  // namespace
 
 // ===========================================================================
+bool emu_ctx::leave_steps_1d(emu_context* ctx, cudaError_t e)
+{
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported)
+        return false;
+    cudaGetLastError();
+    // (the meshes are as a step of the stage kernels leaves them)
+    ctx->steps1d = false;
+    ctx->comb64 = true;
+    choose_resort(ctx);
+    return true;
+}
+
 int emu_ctx::step_device(emu_context* ctx, bool last_stage_deposit)
 {
     int r;
     if (ctx->steps1d) {
-        return run_steps_1d(ctx, 1, emu::DT_ADVANCE);
-    } else if (ctx->coop) {
+        if ((r = run_steps_1d(ctx, 1, emu::DT_ADVANCE)) || ctx->steps1d) return r;
+    }
+    if (ctx->coop) {
         double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
         cudaError_t e = emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx), ctx->ctl,
                                                   emu::DT_ADVANCE, ctx->stream);
@@ -708,7 +745,8 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     // (a sharded run reduces every deposit between stages: per-stage kernels)
     ctx->coop = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 2 && rk4_fused(ctx) &&
                 emu::coop_step_fits(ctx->nf, ctx->P, n);
-    // fused == 1, 1D along z, the grid fits: several steps per launch
+    // fused == 1, 1D along z, the grid fits: several steps per launch (until a
+    // launch is refused, leave_steps_1d)
     ctx->steps1d = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                    emu::steps_1d_fit(ctx->nf, ctx->P, n);
     // any other FP64 RK4 context of one rank without the adaptive timestep:
@@ -716,24 +754,7 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     ctx->comb64 = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                   !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d;
     if ((ctx->steps1d || ctx->comb64) && (r = ensure_cmesh(ctx))) return r;
-    if (ctx->auto_resort) {
-        // a 27-cell stencil loses its per-CTA cell runs within a step or two
-        // once particles leave their cells, a 1D stencil within several.  FP64
-        // stages in a plane re-sort every step too, since the re-sort is made
-        // by stage 4's stores (90 x 77 cells x 60 directions: 445 us per step
-        // at 1, 457 at 2, 498 at 4, 577 at 16)
-        const int cells = ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2];
-        ctx->prm.resort_interval = cells > (ctx->comb64 ? 3 : 9) ? 1 : 16;
-        // several steps per launch: the re-sort's own launches weigh more and
-        // a window a few cells wider costs little (two flavors, 128 x 80: 15.5
-        // us per step at 16, 14.3 at 32, 13.9 at 64; 50 cells x 2 beams, whose
-        // warps outgrow the products past 40 steps: 11.0, 10.5, 23.1); one
-        // cell needs none
-        if (ctx->steps1d) ctx->prm.resort_interval = ctx->P.ncells > 1 ? 32 : 0;
-    }
-    // with a re-sort after every step, the deposits of stages 1-3 see
-    // cell-sorted particles; otherwise every deposit ranks its keys
-    ctx->P.rank_stages = ctx->prm.resort_interval != 1;
+    choose_resort(ctx);
     ctx->loaded = true;
     ctx->adj_valid = false;
     ctx->steps_since_sort = 0;
@@ -1029,10 +1050,10 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
     emu::launch_ctl_set(ctx->ctl, dt, 0.0, INFINITY, 1, 1, ctx->stream);
     if (rk4_fused(ctx)) {
         if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+        r = ctx->steps1d ? run_steps_1d(ctx, 1, -1) : EMU_OK;
         // (FP64 stages: a re-sort due after the step is made by its stage 4)
         fuse = ctx->comb64 && ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
-        if (ctx->steps1d) {
-            r = run_steps_1d(ctx, 1, -1);
+        if (r || ctx->steps1d) {
         } else if (ctx->coop) {
             double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
             cudaError_t e = emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx), ctx->ctl,
@@ -1088,19 +1109,18 @@ int emu_evolve_steps(emu_context* ctx, int nsteps)
     // caller can read after the call)
     if (((ctx->mixed && ctx->P.m4_reduced) || ctx->steps1d || ctx->comb64) && nsteps > 0)
         emu::launch_ctl_m4(ctx->ctl, nsteps, ctx->stream);
-    if (ctx->steps1d) {
+    int i = 0;
+    while (ctx->steps1d && i < nsteps) {
         // one launch up to the next re-sort
         const int ri = ctx->prm.resort_interval;
-        for (int i = 0; i < nsteps;) {
-            int len = std::min(nsteps - i, 256);
-            if (ri > 0) len = std::min(len, std::max(ri - ctx->steps_since_sort, 1));
-            if ((r = run_steps_1d(ctx, len, emu::DT_ADVANCE))) return r;
-            i += len;
-            if (ri > 0 && (ctx->steps_since_sort += len) >= ri && (r = resort(ctx))) return r;
-        }
-        return EMU_OK;
+        int len = std::min(nsteps - i, 256);
+        if (ri > 0) len = std::min(len, std::max(ri - ctx->steps_since_sort, 1));
+        if ((r = run_steps_1d(ctx, len, emu::DT_ADVANCE))) return r;
+        if (!ctx->steps1d) break;
+        i += len;
+        if (ri > 0 && (ctx->steps_since_sort += len) >= ri && (r = resort(ctx))) return r;
     }
-    for (int i = 0; i < nsteps; i++) {
+    for (; i < nsteps; i++) {
         // when a re-sort follows this step, its gather makes the deposit of
         // the new state (in cell order) instead of the last stage
         const bool resort_next =
@@ -1159,7 +1179,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
 {
     if (!ctx || !kernel_ms || !nkernels) return EMU_ERR_ARG;
     if (!rk4_fused(ctx)) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: requires fused RK4");
-    if (ctx->coop || ctx->steps1d) {
+    while (ctx->coop || ctx->steps1d) {
         // one cooperative kernel per step
         if (max_kernels < 1) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: kernel_ms too small");
         cudaEvent_t a, b;
@@ -1167,18 +1187,20 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
         CU(cudaEventCreate(&b));
         double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
         CU(cudaEventRecord(a, ctx->stream));
-        if (ctx->steps1d) {
+        const bool one_launch = ctx->steps1d;
+        if (one_launch) {
             if (int rs = run_steps_1d(ctx, 1, emu::DT_ADVANCE)) return rs;
         }
-        cudaError_t e = ctx->steps1d ? cudaSuccess
-                                     : emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx),
-                                                                 ctx->ctl, emu::DT_ADVANCE, ctx->stream);
+        cudaError_t e = one_launch ? cudaSuccess
+                                   : emu::launch_rk4_step_coop(ctx->nf, ctx->P, ctx->S[ctx->cur], m, mesh_elems(ctx),
+                                                               ctx->ctl, emu::DT_ADVANCE, ctx->stream);
         CU(cudaEventRecord(b, ctx->stream));
         if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("cooperative step: ") + cudaGetErrorString(e));
         CU(cudaEventSynchronize(b));
         CU(cudaEventElapsedTime(&kernel_ms[0], a, b));
         cudaEventDestroy(a);
         cudaEventDestroy(b);
+        if (one_launch && !ctx->steps1d) continue;   // (refused: the stage kernels)
         *nkernels = 1;
         ctx->cur_mesh = 3;
         int r;

@@ -129,6 +129,9 @@ void ring_free(emu_context* ctx);
 // last_stage_deposit = false leaves the deposit of the new state to a
 // re-sort with deposit that the caller makes next.
 int step_device(emu_context* ctx, bool last_stage_deposit = true);
+// after a launch of k_steps_1d: true when e says that its grid cannot be
+// co-resident, and the context goes on with the stage kernels from here
+bool leave_steps_1d(emu_context* ctx, cudaError_t e);
 // sum a deposited mesh (FP64, or int64 for the mixed path) over the ranks of
 // the attached communicator, enqueued on st; no-op without one
 int reduce_mesh(emu_context* ctx, void* mesh, bool int64, cudaStream_t st);
