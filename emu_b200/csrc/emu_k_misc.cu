@@ -16,6 +16,8 @@ namespace emu {
                                                      cudaStream_t);                                              \
     extern template void launch_deposit_full64_t<NF>(const DevParams&, const DevState&, const double*, double*,  \
                                                      StepCtl*, cudaStream_t);                                    \
+    extern template void launch_deposit_t<NF>(const DevParams&, const DevState&, const double*, double*, StepCtl*, \
+                                              cudaStream_t);                                                     \
     extern template void launch_rhs_t<NF>(const DevParams&, const DevState&, const double*, const double*,       \
                                           double*, cudaStream_t);                                                \
     extern template void launch_rk4_stage_mixed_t<NF>(const DevParams&, const DevState&, int, const float*,      \
@@ -90,9 +92,29 @@ void launch_deposit(int nf, const DevParams& P, const DevState& S, const double*
     launch_deposit_full64(nf, P, S, f, mesh, nullptr, st);
 }
 
+// The full deposit by lanes that sum a value each run by run (k_deposit), or by
+// matrix products (k_deposit_full64).  A product has eight columns of values
+// to a warp and costs the same for a run of one particle as of four, so short
+// runs lose: particles per cell below the line, each class's crossover (us a
+// call, run by run / products): 8^3 cells, three flavors, 4 per cell 101/141,
+// 16 64/65, 40 66/53, 24^3 at 8 167/171; the y-z plane of 90 x 77 cells at 4
+// 103/107, 8 98/77; CIC boxes 24^3 at 4 58/61, 8 72/54 (two flavors).  Along z
+// a run by run walk has three cells only: 1024 cells, three flavors, 96 per
+// cell 44/49, two 38/36.
+static bool deposit_run_by_run(int nf, const DevParams& P, long long n)
+{
+    if (P.w[0] == 1 && P.w[1] == 1 && P.w[2] == 3) return nf == 3 || n < 64 * P.ncells;
+    return n < (P.w[0] * P.w[1] * P.w[2] == 27 ? 12 : 6) * P.ncells;
+}
+
 void launch_deposit_full64(int nf, const DevParams& P, const DevState& S, const double* f, double* mesh, StepCtl* ctl,
                            cudaStream_t st)
 {
+    if (deposit_run_by_run(nf, P, S.n)) {
+        if (nf == 2) launch_deposit_t<2>(P, S, f, mesh, ctl, st);
+        else launch_deposit_t<3>(P, S, f, mesh, ctl, st);
+        return;
+    }
     if (nf == 2) launch_deposit_full64_t<2>(P, S, f, mesh, ctl, st);
     else launch_deposit_full64_t<3>(P, S, f, mesh, ctl, st);
 }

@@ -973,6 +973,48 @@ __global__ void __launch_bounds__(2 * kBlock, 2) k_rk4_step_coop_split(DevParams
 // ===========================================================================
 // unfused building blocks (FP64)
 // ===========================================================================
+// The full deposit, run by run (k_deposit_full64's other form, for particles in
+// short runs: see launch_deposit_full64).  ctl as there.
+template <int NF, int WX, int WY, int WZ>
+__global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, const double* __restrict__ f,
+                                                    double* __restrict__ mesh, StepCtl* ctl)
+{
+    using SWt = SW<WX, WY, WZ>;
+    constexpr int NH = NF * NF, NS = 2 * NH;
+    double dt = 0.0;
+    if (ctl) {
+        grid_dep_wait();
+        grid_dep_launch();
+        dt = ctl->dt;
+        const bool done = ctl->done, full = !done && m4_full_step(ctl);
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->m4_full = done ? 2 : full ? 1 : 0;
+        if (!full) return;
+    }
+    const long long ntile = (S.n + kBlock - 1) / kBlock;
+    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        const long long p = tile * kBlock + threadIdx.x;
+        const bool active = p < S.n;
+        Stencil<double> st{};
+        double fN[NS] = {};
+        double vx = 0, vy = 0, vz = 0;
+        if (active) {
+            make_stencil<double>(P, S.pos[0][p], S.pos[1][p], S.pos[2][p], st);
+            vx = S.vhat[0][p];
+            vy = S.vhat[1][p];
+            vz = S.vhat[2][p];
+#pragma unroll
+            for (int c = 0; c < NS; c++) {
+                double y = f[c * S.cap + p];
+                if (ctl) y = __dadd_rn(__dmul_rn(dt, S.fs[c * S.cap + p]), y);
+                fN[c] = y * S.Nn[c / NH][p];
+            }
+        }
+        tile_deposit_block<NF, SWt, double>(P, mesh, active, st, fN, vx, vy, vz,
+                                            [](double a, int) -> double { return a; }, true);
+        __syncthreads();   // (the next tile's ranks use the records' memory)
+    }
+}
+
 template <int NF, int WX, int WY, int WZ>
 __global__ void __launch_bounds__(kBlock) k_rhs(DevParams P, DevState S, const double* __restrict__ f,
                                                 const double* __restrict__ mesh, double* __restrict__ K)
@@ -2221,6 +2263,20 @@ void launch_gather_deposit_t(bool mixed, const DevParams& P, const DevState& src
             k_gather_deposit<NF, WXv, WYv, WZv, false><<<grid_for(src.n), kBlock, bytes, st>>>(P, src, dst, perm,
                                                                                               mesh, qmesh);
         }
+    });
+}
+
+template <int NF>
+void launch_deposit_t(const DevParams& P, const DevState& S, const double* f, double* mesh, StepCtl* ctl,
+                      cudaStream_t st)
+{
+    EMU_W_DISPATCH(P, {
+        constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
+        auto kern = k_deposit<NF, WXv, WYv, WZv>;
+        smem_optin(kern, bytes);
+        const unsigned grid = (unsigned)std::min<long long>(grid_for(S.n), 148 * 12);
+        if (ctl) launch_pdl(kern, grid, kBlock, bytes, st, P, S, f, mesh, ctl);
+        else kern<<<grid_for(S.n), kBlock, bytes, st>>>(P, S, f, mesh, (StepCtl*)nullptr);
     });
 }
 
