@@ -372,8 +372,9 @@ int deposit_current(emu_context* ctx)
 {
     const DevState& S = ctx->S[ctx->cur];
     int r;
+    const bool comb = ctx->steps1d || ctx->comb64;
     if ((r = zero_mesh(ctx, 0))) return r;
-    if ((r = zero_mesh(ctx, 1))) return r;
+    if (!comb && (r = zero_mesh(ctx, 1))) return r;
     if (ctx->mixed) {
         if ((r = deposit_full_q(ctx))) return r;
         emu::launch_full_to_comb(ctx->nf, ctx->P, ctx->qfull, ctx->qmesh[0], ctx->stream);
@@ -382,14 +383,26 @@ int deposit_current(emu_context* ctx)
         emu::launch_deposit(ctx->nf, ctx->P, S, S.f0, ctx->mesh[0], ctx->stream);
         if ((r = check_launch(ctx, "deposit"))) return r;
         if ((r = emu_ctx::reduce_mesh(ctx, ctx->mesh[0], false, ctx->stream))) return r;
-        if (ctx->steps1d || ctx->comb64) {
-            emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh, ctx->stream);
-            if ((r = check_launch(ctx, "combined mesh"))) return r;
-            CU(cudaMemsetAsync(ctx->cmesh + cmesh_elems(ctx), 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
-        }
     }
     ctx->cur_mesh = 0;
     ctx->fused_ready = true;
+    ctx->cmesh_ready = false;
+    return EMU_OK;
+}
+
+// the meshes that a fused step starts from: the deposit of the current state
+// and, for steps on combined meshes, that deposit in their layout (a load or
+// a deposit alone does without)
+int ready_meshes(emu_context* ctx)
+{
+    int r;
+    if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+    if ((ctx->steps1d || ctx->comb64) && !ctx->cmesh_ready) {
+        emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh, ctx->stream);
+        if ((r = check_launch(ctx, "combined mesh"))) return r;
+        CU(cudaMemsetAsync(ctx->cmesh + cmesh_elems(ctx), 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
+        ctx->cmesh_ready = true;
+    }
     return EMU_OK;
 }
 
@@ -1049,7 +1062,7 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
     bool fuse = false;
     emu::launch_ctl_set(ctx->ctl, dt, 0.0, INFINITY, 1, 1, ctx->stream);
     if (rk4_fused(ctx)) {
-        if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+        if ((r = ready_meshes(ctx))) return r;
         r = ctx->steps1d ? run_steps_1d(ctx, 1, -1) : EMU_OK;
         // (FP64 stages: a re-sort due after the step is made by its stage 4)
         fuse = ctx->comb64 && ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
@@ -1085,7 +1098,7 @@ int emu_evolve_begin(emu_context* ctx, double start_time, double end_time, int m
     if (!ctx->loaded) return fail(ctx, EMU_ERR_STATE, "emu_evolve: no particles loaded");
     if (!rk4_fused(ctx)) return fail(ctx, EMU_ERR_ARG, "emu_evolve: device-resident loop requires fused RK4");
     int r;
-    if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+    if ((r = ready_meshes(ctx))) return r;
     emu::launch_ctl_set(ctx->ctl, 0.0, start_time, end_time, max_steps, 1, ctx->stream);
     if (ctx->mixed) {
         // the full mesh of the current state (after steps the step's first

@@ -57,6 +57,7 @@ struct emu_context {
     size_t sort_tmp_bytes = 0;
     int cur_mesh = 0;
     bool fused_ready = false;
+    bool cmesh_ready = false;           // the current deposit is in cmesh too
     bool loaded = false;
     // step graphs per particle buffer and variant (0: the last stage deposits
     // the new state; 1: it does not, the re-sort gather that follows does)
