@@ -314,6 +314,28 @@ void choose_resort(emu_context* ctx)
     ctx->P.rank_stages = ctx->prm.resort_interval != 1;
 }
 
+// Single steps of a host at the automatic interval of 1 with stencils of 4 to 9
+// cells, two flavors and a grid of one wave of short runs: the re-sort's
+// launches weigh more there than the order they restore, so it waits until the
+// particles may have moved kMovedCells cells (0.025 cells a step, a re-sort
+// every step / then: 90 x 77 cells x 2 with CIC 231/198 us, with TSC 252/224,
+// 30 x 30 x 6 157/136, 16^3 x 6 with CIC 177/166; more particles or flavors
+// lose, 8 x 8 x 40 77/82, three flavors 99/114)
+constexpr double kMovedCells = 0.1;
+bool resort_by_motion(const emu_context* ctx)
+{
+    const long long n = ctx->S[ctx->cur].n;
+    return ctx->auto_resort && ctx->comb64 && ctx->prm.resort_interval == 1 && ctx->nf == 2 &&
+           ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2] <= 9 && n <= 148 * 4 * emu::kBlock && n <= 8 * ctx->P.ncells;
+}
+double cells_per_cm(const DevParams& P)
+{
+    double m = 0.0;
+    for (int d = 0; d < 3; d++)
+        if (P.n[d] > 1) m = std::max(m, P.dxi[d]);
+    return m;
+}
+
 // nsteps steps of k_steps_1d (dt_mode as launch_steps_1d).  When its grid is
 // refused (a stream that may not use every SM) nothing has run and ctx->steps1d
 // is false on return: the caller takes the steps with the stage kernels
@@ -576,6 +598,7 @@ int resort(emu_context* ctx, bool deposit = false)
         // (the step's stage 4 has made it, into the other buffer)
         ctx->cur = 1 - ctx->cur;
         ctx->steps_since_sort = 0;
+        ctx->moved = 0.0;
         ctx->adj_valid = false;
         return EMU_OK;
     }
@@ -603,6 +626,7 @@ int resort(emu_context* ctx, bool deposit = false)
     if ((r = check_launch(ctx, "resort"))) return r;
     ctx->cur = 1 - ctx->cur;
     ctx->steps_since_sort = 0;
+    ctx->moved = 0.0;
     ctx->adj_valid = false;   // slot order changed
     // the deposited meshes are order independent; stage 1 of the next step
     // reads the same mesh as before the re-sort
@@ -771,6 +795,7 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     ctx->loaded = true;
     ctx->adj_valid = false;
     ctx->steps_since_sort = 0;
+    ctx->moved = 0.0;
     // (asynchronous from here: the callers wait for what they need)
     return deposit_current(ctx);
 }
@@ -1059,13 +1084,18 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
     if (!ctx->loaded) return fail(ctx, EMU_ERR_STATE, "emu_step: no particles loaded");
     if (!(dt >= 0.0) || !std::isfinite(dt)) return fail(ctx, EMU_ERR_ARG, "emu_step: dt must be finite and >= 0");
     int r;
-    bool fuse = false;
+    bool fuse = false, lazy = false;
+    bool due = ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
     emu::launch_ctl_set(ctx->ctl, dt, 0.0, INFINITY, 1, 1, ctx->stream);
     if (rk4_fused(ctx)) {
         if ((r = ready_meshes(ctx))) return r;
         r = ctx->steps1d ? run_steps_1d(ctx, 1, -1) : EMU_OK;
+        lazy = resort_by_motion(ctx);
+        if (lazy) ctx->moved += dt * emu::kC * cells_per_cm(ctx->P);
+        due = lazy ? ctx->moved >= kMovedCells
+                   : ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
         // (FP64 stages: a re-sort due after the step is made by its stage 4)
-        fuse = ctx->comb64 && ctx->prm.resort_interval > 0 && ctx->steps_since_sort + 1 >= ctx->prm.resort_interval;
+        fuse = ctx->comb64 && due;
         if (r || ctx->steps1d) {
         } else if (ctx->coop) {
             double* const m[4] = {ctx->mesh[0], ctx->mesh[1], ctx->mesh[2], ctx->mesh[3]};
@@ -1074,9 +1104,12 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
             r = e == cudaSuccess ? EMU_OK : fail(ctx, EMU_ERR_CUDA, std::string("cooperative step: ") +
                                                                       cudaGetErrorString(e));
         } else {
+            const int ranks = ctx->P.rank_stages;
+            if (lazy) ctx->P.rank_stages = 1;   // (particles may have left their cells)
             r = ctx->mixed    ? enqueue_rk4_mixed(ctx, ctx->stream, false)
                 : ctx->comb64 ? enqueue_rk4_comb64(ctx, ctx->stream, false, !fuse)
                               : enqueue_rk4_fp64(ctx, ctx->stream, false);
+            ctx->P.rank_stages = ranks;
         }
         if (r) return r;
         if (ctx->mixed && (r = sum_full_parts(ctx))) return r;
@@ -1086,8 +1119,8 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
         if (ctx->mixed) return fail(ctx, EMU_ERR_ARG, "emu_step: the mixed path integrates with RK4 only");
         if ((r = step_generic(ctx, dt))) return r;
     }
-    if (++ctx->steps_since_sort >= ctx->prm.resort_interval && ctx->prm.resort_interval > 0)
-        if ((r = resort(ctx, fuse))) return r;
+    ctx->steps_since_sort++;
+    if (due && (r = resort(ctx, fuse))) return r;
     if ((r = sync_ctl(ctx))) return r;
     return status_of(ctx, bad);
 }

@@ -66,6 +66,7 @@ struct emu_context {
     DevState graph_S[2][2];
     DevState graph_D[2][2];             // and the other buffer (the mixed stage 4 re-sorts into it)
     int steps_since_sort = 0;
+    double moved = 0.0;                 // cells that single steps may have moved particles since then
     bool auto_resort = false;           // prm.resort_interval chosen at each load
     bool coop = false;                  // whole-step cooperative kernel (small FP64 problems)
     bool steps1d = false;               // several steps per cooperative launch (k_steps_1d)
