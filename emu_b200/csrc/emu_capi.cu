@@ -412,20 +412,26 @@ int deposit_current(emu_context* ctx)
     return EMU_OK;
 }
 
-// the meshes that a fused step starts from: the deposit of the current state
-// and, for steps on combined meshes, that deposit in their layout (a load or
+// for steps on combined meshes, the current deposit in their layout (a load or
 // a deposit alone does without)
-int ready_meshes(emu_context* ctx)
+int ready_cmesh(emu_context* ctx)
 {
     int r;
-    if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
-    if ((ctx->steps1d || ctx->comb64) && !ctx->cmesh_ready) {
+    if (ctx->fused_ready && (ctx->steps1d || ctx->comb64) && !ctx->cmesh_ready) {
         emu::launch_full_to_comb64(ctx->nf, ctx->P, ctx->mesh[0], ctx->cmesh, ctx->stream);
         if ((r = check_launch(ctx, "combined mesh"))) return r;
         CU(cudaMemsetAsync(ctx->cmesh + cmesh_elems(ctx), 0, sizeof(double) * cmesh_elems(ctx), ctx->stream));
         ctx->cmesh_ready = true;
     }
     return EMU_OK;
+}
+
+// the meshes that a fused step starts from
+int ready_meshes(emu_context* ctx)
+{
+    int r;
+    if (!ctx->fused_ready && (r = deposit_current(ctx))) return r;
+    return ready_cmesh(ctx);
 }
 
 // ---- step bodies -----------------------------------------------------------
@@ -1151,6 +1157,8 @@ int emu_evolve_steps(emu_context* ctx, int nsteps)
 {
     if (!ctx) return EMU_ERR_ARG;
     int r;
+    // (a run may go on over a load or a deposit)
+    if ((r = ready_cmesh(ctx))) return r;
     // the last of these steps deposits the full stage-4 mesh (the one a
     // caller can read after the call)
     if (((ctx->mixed && ctx->P.m4_reduced) || ctx->steps1d || ctx->comb64) && nsteps > 0)
@@ -1225,6 +1233,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
 {
     if (!ctx || !kernel_ms || !nkernels) return EMU_ERR_ARG;
     if (!rk4_fused(ctx)) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: requires fused RK4");
+    if (int rc = ready_cmesh(ctx)) return rc;
     while (ctx->coop || ctx->steps1d) {
         // one cooperative kernel per step
         if (max_kernels < 1) return fail(ctx, EMU_ERR_ARG, "emu_profile_step: kernel_ms too small");

@@ -56,3 +56,29 @@ def test_deposits_on_both_sides(case):
             c.step(dt)
             assert _close(c.get_mesh(), mesh, mag, nf * nf, 1e-11)
             assert colwise_rel(c.get_particles(), run) < 1e-11
+
+
+@pytest.mark.parametrize("nf,cells", [(2, (1, 1, 40)), (3, (1, 1, 12)), (2, (1, 5, 6)), (3, (3, 3, 4))])
+def test_a_run_goes_on_over_a_load_and_a_deposit(nf, cells):
+    L = tuple(0.5 * c if c > 1 else 1.0 for c in cells)
+    _, p, a = _case("x", nf, cells, 2, L, 9, 3, rho=2e9, maxError=1e-2)
+    b = a[::-1].copy()
+    b[:, 0:3] = a[:, 0:3]
+    b[:, 4:7] = a[:, 0:3]
+    o = Oracle(p)
+    with api.Context(p) as c:
+        c.load_particles(a)
+        c.evolve_begin(0.0, float("inf"), 9)
+        c.evolve_steps(3)
+        dt = c.evolve_end().dt_next
+        c.load_particles(b)
+        c.evolve_steps(1)
+        mesh = o.rk_step(b, dt)[0]
+        assert colwise_rel(c.get_particles(), b) < 1e-11
+        c.deposit()
+        c.evolve_steps(1)
+        # (the step's dt: of the mesh that the step before it left, the load's limit)
+        dt, _ = o.compute_dt(mesh, o.vvac_max(b))
+        o.rk_step(b, dt)
+        info = c.evolve_end()
+        assert info.steps_done == 5 and colwise_rel(c.get_particles(), b) < 1e-11
