@@ -315,18 +315,19 @@ void choose_resort(emu_context* ctx)
 }
 
 // Single steps of a host at the automatic interval of 1 with stencils of 4 to 9
-// cells, two flavors and a grid of one wave of short runs: the re-sort's
-// launches weigh more there than the order they restore, so it waits until the
-// particles may have moved kMovedCells cells (0.025 cells a step, a re-sort
-// every step / then: 90 x 77 cells x 2 with CIC 231/198 us, with TSC 252/224,
-// 30 x 30 x 6 157/136, 16^3 x 6 with CIC 177/166; more particles or flavors
-// lose, 8 x 8 x 40 77/82, three flavors 99/114)
+// cells, two flavors and a grid of one wave: the re-sort's launches weigh more
+// there than the order they restore, so it waits until the particles may have
+// moved kMovedCells cells (0.025 cells a step, a re-sort every step / then: 90
+// x 77 cells x 2 with CIC 231/198 us, with TSC 252/224, 30 x 30 x 6 157/136, x
+// 40 117/95, 16^3 x 6 with CIC 177/166).  Long runs in a few CTAs lose (8 x 8 x
+// 40 77/82), and three flavors (99/114).
 constexpr double kMovedCells = 0.1;
 bool resort_by_motion(const emu_context* ctx)
 {
     const long long n = ctx->S[ctx->cur].n;
     return ctx->auto_resort && ctx->comb64 && ctx->prm.resort_interval == 1 && ctx->nf == 2 &&
-           ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2] <= 9 && n <= 148 * 4 * emu::kBlock && n <= 8 * ctx->P.ncells;
+           ctx->P.w[0] * ctx->P.w[1] * ctx->P.w[2] <= 9 && n <= 148 * 4 * emu::kBlock &&
+           (n <= 8 * ctx->P.ncells || n > 4096);
 }
 double cells_per_cm(const DevParams& P)
 {
