@@ -348,8 +348,9 @@ __device__ __forceinline__ void deposit_runs64(const DevParams& P, const double*
 #pragma unroll
             for (int m = 0; m < MT; m++) c2[m][0] = c2[m][1] = 0.0;
         // slots 4 k .. 4 k + 3; masked: some belong to another run (their
-        // values count as zero; rows past the stencil's cells hold other words
-        // of the record and are not used)
+        // values and weights, which need not be finite, count as zero; rows
+        // past the stencil's cells hold other words of the record and are not
+        // used)
         auto step = [&](int k, bool masked) {
             const int s = 4 * k + col;
             const bool in = !masked || (s >= a && s < e);
@@ -362,7 +363,8 @@ __device__ __forceinline__ void deposit_runs64(const DevParams& P, const double*
             }
 #pragma unroll
             for (int m = 0; m < MT; m++) {
-                const double wgt = r[8 * m];
+                double wgt = r[8 * m];
+                if (!in) wgt = 0.0;
                 dmma(c[m][0], c[m][1], wgt, b);
                 if constexpr (DIAG)
                     if (m % dstep == dm) dmma(c2[m][0], c2[m][1], wgt, b2);
