@@ -693,13 +693,20 @@ __global__ void k_soa_to_rows(const long long* __restrict__ id, const double* __
     for (int c = 0; c < ncomp; c++) dst[r * ncomp + c] = src[c * cap + p];
 }
 
+// (an adjoint state that is not finite: noted in ctl)
 __global__ void k_rows_to_soa(const long long* __restrict__ id, const double* __restrict__ src, int ncomp,
-                              long long cap, long long n, double* __restrict__ dst)
+                              long long cap, long long n, double* __restrict__ dst, StepCtl* ctl)
 {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const long long r = id[p];
-    for (int c = 0; c < ncomp; c++) dst[c * cap + p] = src[r * ncomp + c];
+    bool odd = false;
+    for (int c = 0; c < ncomp; c++) {
+        const double x = src[r * ncomp + c];
+        odd = odd || not_finite<1>(&x);
+        dst[c * cap + p] = x;
+    }
+    if (odd) ctl->odd_lam = 1;
 }
 
 // ---- launchers ----------------------------------------------------------------
@@ -1348,12 +1355,14 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     const long long nm = cmesh_elems(ctx);
 
     // adjoint state of the final (renormalised) state, in the final slot order
+    // (a sweep that timed out before this one does not end it)
+    emu::launch_ctl_set(ctx->ctl, 0.0, 0.0, INFINITY, INT_MAX, 1, st);
     if ((r = emu_ctx::copy_to_device(ctx, a->rows, lam_f_final, sizeof(double) * (size_t)n * NS))) return r;
-    emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, NS, cap, n, a->lamY0);
+    emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, NS, cap, n, a->lamY0, ctx->ctl);
     CU(cudaStreamSynchronize(st));
     if (lam_N_final) {
         if ((r = emu_ctx::copy_to_device(ctx, a->rows, lam_N_final, sizeof(double) * (size_t)n * 2))) return r;
-        emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, 2, cap, n, a->lamN);
+        emu::k_rows_to_soa<<<g, emu::kBlock, 0, st>>>(S.id, a->rows, 2, cap, n, a->lamN, ctx->ctl);
     } else {
         CU(cudaMemsetAsync(a->lamN, 0, sizeof(double) * 2 * cap, st));
     }
@@ -1361,8 +1370,6 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     int w = 0;
     emu::k_static_scatter<<<g, emu::kBlock, 0, st>>>(S, stat_view(a, 0, S), nullptr, nullptr, nullptr, 0);
     CU(cudaMemsetAsync(a->lmesh[0], 0, sizeof(double) * nm, st));
-    // (a sweep that timed out before this one does not end it)
-    emu::launch_ctl_set(ctx->ctl, 0.0, 0.0, INFINITY, INT_MAX, 1, st);
     if ((r = check_launch(ctx, "adjoint input"))) return r;
     const bool coop = a->store && emu::adj_coop_fits(nf, ctx->P, n);
     // per-step mode with re-sorts (the recomputes re-sort as the forward did)

@@ -775,13 +775,13 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
         ctx->P.g_scale = gs[0];
         ctx->P.g_unscale = gu[0];
     }
-    emu::launch_cell_keys(ctx->P, ctx->aos, ctx->nreal, n, ctx->keys, ctx->idx, ctx->stream);
+    emu::launch_cell_keys(ctx->P, ctx->aos, ctx->nreal, n, ctx->keys, ctx->idx, ctx->ctl, ctx->stream);
     if ((r = sort_perm(ctx, n))) return r;
     ctx->cur = 0;
     DevState& S = ctx->S[0];
     S.n = n;
     ctx->S[1].n = n;
-    emu::launch_pack(ctx->nf, ctx->P, ctx->aos, ctx->idx2, n, S, ctx->stream);
+    emu::launch_pack(ctx->nf, ctx->P, ctx->aos, ctx->idx2, n, S, ctx->ctl, ctx->stream);
     if (ctx->mixed) emu::launch_mixed_shadow(ctx->nf, S, ctx->stream);
     if ((r = check_launch(ctx, "pack"))) return r;
     // (step graphs re-capture themselves when P or S differ from their capture)

@@ -127,6 +127,16 @@ __device__ __forceinline__ void shape(double delta, int order, int& first, R w[3
     }
 }
 
+// some of N values is a NaN or an infinity
+template <int N>
+__device__ __forceinline__ bool not_finite(const double* x)
+{
+    int m = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) m = max(m, __double2hiint(x[i]) & 0x7fffffff);
+    return m >= 0x7ff00000;
+}
+
 // A value of a mesh that this kernel only reads, or (LIVE) that other CTAs of
 // the same launch write before a grid barrier: the read-only path is for data
 // that stands for the whole kernel, a plain load is ordered by the barrier's

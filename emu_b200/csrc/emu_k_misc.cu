@@ -48,9 +48,9 @@ EMU_EXTERN(3)
 
 
 void launch_pack(int nf, const DevParams& P, const double* aos, const unsigned* perm, long long n, DevState S,
-                 cudaStream_t st)
+                 StepCtl* ctl, cudaStream_t st)
 {
-    EMU_NF_DISPATCH(nf, (k_pack<NFv><<<grid_for(n), kBlock, 0, st>>>(P, aos, perm, n, S)));
+    EMU_NF_DISPATCH(nf, (k_pack<NFv><<<grid_for(n), kBlock, 0, st>>>(P, aos, perm, n, S, ctl)));
 }
 
 void launch_unpack(int nf, const DevState& S, double* aos, cudaStream_t st)
@@ -64,9 +64,9 @@ void launch_unpack_rhs(int nf, const DevState& S, const double* K, double* aos, 
 }
 
 void launch_cell_keys(const DevParams& P, const double* aos, int nreal, long long n, unsigned* keys, unsigned* idx,
-                      cudaStream_t st)
+                      StepCtl* ctl, cudaStream_t st)
 {
-    k_cell_keys_aos<<<grid_for(n), kBlock, 0, st>>>(P, aos, nreal, n, keys, idx);
+    k_cell_keys_aos<<<grid_for(n), kBlock, 0, st>>>(P, aos, nreal, n, keys, idx, ctl);
 }
 
 void launch_state_keys(const DevParams& P, const DevState& S, unsigned* keys, unsigned* idx, cudaStream_t st)

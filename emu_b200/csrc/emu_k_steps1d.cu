@@ -177,6 +177,28 @@ __device__ __noinline__ void deposit_tiles(int ncells, double* mesh, int stride,
     }
 }
 
+// ONE: the same value by value, a thread per mesh value, over the particles
+// that touch the cell (CELLS, see k_steps_1d)
+template <int NF, int D>
+__device__ __noinline__ void deposit_cells(int ncells, double* mesh, int stride, const double* srec, const double* sfn)
+{
+    using R = Rec1D<NF>;
+    constexpr int NQ = 8 * DepN<NF, D>::NT, NS = 2 * NF * NF;
+    for (int i = threadIdx.x; i < ncells * NQ; i += blockDim.x) {
+        const int c = i / NQ, q = i - c * NQ;
+        double sum = 0.0;
+        for (int k = 0; k < kOnePart; k++) {
+            const double* r = srec + k * R::RW;
+            const double w = dep_weight_periodic<NF>(r, c, ncells);
+            if (w == 0.0) continue;
+            if constexpr (D == DEP_COMB) sum += w * (r[R::CV + q % R::NV] * r[R::V + q / R::NV]);
+            else if constexpr (D == DEP_DIAG) sum += w * (q < 2 * NF ? r[R::DG + (q < 2 * NF ? q : 0)] : 0.0);
+            else sum += w * (sfn[k * R::FW + q % NS] * r[R::V + q / NS]);
+        }
+        mesh[c * stride + q] = sum;
+    }
+}
+
 // Grid barrier in two halves: arrivals counted up from 0 over the launch (the
 // last CTA to leave the kernel sets the count back).  The wait is bounded;
 // false: it gave up (ST_TIMEOUT is set, the CTA goes to the kernel's end).
@@ -264,7 +286,7 @@ __device__ __forceinline__ void place_weights(Place1D& L, double* rec, const dou
 
 // stencil, window and weights at the position z (barrier inside).  sref: a
 // cell near the CTA's particles
-template <int NF>
+template <int NF, bool CELLS>
 __device__ __forceinline__ void place_particles(const DevParams& P, Place1D& L, double z, bool active, int sp, int sref,
                                                 int (*swin)[16], double* rec, const double* wrec)
 {
@@ -291,7 +313,7 @@ __device__ __forceinline__ void place_particles(const DevParams& P, Place1D& L, 
     const CellRange own = warp_cells(mn, mx, lo, P.w[2]);
     L.wlo = own.lo;
     L.whi = own.hi;
-    L.narrow = !L.wide && mx >= mn && L.whi - L.wlo < kNarrow;
+    L.narrow = !CELLS && !L.wide && mx >= mn && L.whi - L.wlo < kNarrow;
     place_weights<NF>(L, rec, wrec, sp, r);
     if (L.narrow) {
 #pragma unroll
@@ -461,16 +483,16 @@ __device__ __forceinline__ void deposit_1d(const Place1D& L, const double* srec,
         if (diag) deposit_spread<NF, DEP_DIAG, false>(nz, mesh, srec, sfn, r0, L.wlo, L.whi, L.c0);
     }
 }
-// and of a wide window, value by value: this thread's half of the pair's
+// value by value, cells first, first + 1, ..: this thread's half of the pair's
 template <int NF, bool MINUS>
-__device__ __forceinline__ void deposit_1d_wide(const DevParams& P, const Place1D& L, const double* rec, int sp,
-                                                double* mesh, bool diag)
+__device__ __forceinline__ void deposit_1d_cells(const DevParams& P, const Place1D& L, const double* rec, int sp,
+                                                 int first, double* mesh, bool diag)
 {
     using R = Rec1D<NF>;
     constexpr int NV = R::NV, HV = NV / 2, NG = R::NG, NCS = kCombSlots<NF>;
 #pragma unroll 1
     for (int i = 0; i < P.w[2]; i++) {
-        double* m = mesh + (L.ci0 + i) % P.n[2] * NCS;
+        double* m = mesh + (first + i) % P.n[2] * NCS;
         const double wi = i == 0 ? L.wz[0] : i == 1 ? L.wz[1] : L.wz[2];
         for (int d = 0; d < 4; d++) {
             const double wd = MINUS && d > 0 ? -(wi * rec[R::V + d]) : wi * rec[R::V + d];
@@ -486,10 +508,16 @@ __device__ __forceinline__ void deposit_1d_wide(const DevParams& P, const Place1
 // REC (not ONE): a recorded run (Rec1DStore): every step's state, stage states
 // and meshes are kept, the meshes where they are stored (zeroed; M_1 of the
 // first step deposited) instead of in cmesh; the last step's M_1 is not made.
-template <int NF, bool ONE, int MAXT, bool REC>
-__global__ void __launch_bounds__(MAXT, 1)
-    k_steps_1d(DevParams P, DevState S, double* __restrict__ cmesh, double* __restrict__ full, StepCtl* ctl,
-               int npart, int nsteps, int dt_mode, Rec1DStore store)
+// CELLS: a state with values that are not finite.  The products meet a warp's
+// other particles and cells with weight zero, which a finite value passes and
+// this would not; these states go cell by cell (scalar interpolation and
+// deposits), which takes such a value to the cells of its stencil only.
+// (A second body behind one look at ctl->odd: looks at every stage's values,
+// with the cell-by-cell code in their shadow, cost 1 to 4 % of a step.)
+template <int NF, bool ONE, bool REC, bool CELLS>
+__device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState& S, double* __restrict__ cmesh,
+                                              double* __restrict__ full, StepCtl* ctl, int npart, int nsteps,
+                                              int dt_mode, const Rec1DStore& store)
 {
     using H = Herm<NF>;
     using C = Comb<NF>;
@@ -513,7 +541,6 @@ __global__ void __launch_bounds__(MAXT, 1)
     __shared__ double sred[16];
     __shared__ int sref;
 
-    if (ctl->done) return;
     double t_run = ctl->t, dt = ctl->dt;
     const double end_time = ctl->end_time;
     int step = ctl->step, last = ctl->last, done = 0, st_dt = 0;
@@ -571,7 +598,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     auto locate = [&]() {
         if constexpr (!ONE) {
             // (cells relative to the first particle's at the launch)
-            place_particles<NF>(P, L, z, active, sp, sref, swin, rec, wrec);
+            place_particles<NF, CELLS>(P, L, z, active, sp, sref, swin, rec, wrec);
         } else {
             int first = 0;
             if (active) {
@@ -588,7 +615,7 @@ __global__ void __launch_bounds__(MAXT, 1)
                 scount[tid] = 0;
                 *reinterpret_cast<unsigned*>(srows[tid]) = 0x01010101u * kOnePart;
             }
-            L.narrow = __syncthreads_and(!any || mx - mn + P.w[2] <= kNarrow);
+            L.narrow = __syncthreads_and(!CELLS && (!any || mx - mn + P.w[2] <= kNarrow));
             L.c0 = any ? wrapi(ref + mn, nz) : 0;
             L.wlo = 0;
             L.whi = any ? mx - mn + P.w[2] - 1 : -1;
@@ -771,11 +798,15 @@ __global__ void __launch_bounds__(MAXT, 1)
                         if (q < NG) out[c * MR + q] = t2;
                         else sdiag[c * kDiagSlots + q - NG] = t2;
                     }
+                } else if constexpr (CELLS) {
+                    deposit_cells<NF, DEP_COMB>(ncells, out, MR, srec, sfn);
+                    if (diag) deposit_cells<NF, DEP_DIAG>(ncells, sdiag, kDiagSlots, srec, sfn);
+                    if (fdep) deposit_cells<NF, DEP_FULL>(ncells, full, ND, srec, sfn);
                 } else {
                     deposit_tiles<NF, DEP_COMB>(ncells, out, MR, srec, sfn);
                     if (diag) deposit_tiles<NF, DEP_DIAG>(ncells, sdiag, kDiagSlots, srec, sfn);
                 }
-                if (fdep) {
+                if (!CELLS && fdep) {
                     // (cells in place of rows relative to the warp's first)
                     if (L.narrow) {
                         __syncthreads();
@@ -799,16 +830,17 @@ __global__ void __launch_bounds__(MAXT, 1)
             } else {
                 if (!(REC && s == 4 && final_step)) {
                     __syncwarp();   // (a warp reads only its own records)
-                    if (!L.wide) {
+                    if (!CELLS && !L.wide) {
                         deposit_1d<NF, false>(L, srec, sfn, wrec, mesh_out, nz, diag);
                         if (fdep && L.whi >= L.wlo)
                             deposit_spread<NF, DEP_FULL, false>(nz, full, srec, sfn, warp * 16, L.wlo, L.whi, L.c0);
                     } else if (active) {
-                        deposit_1d_wide<NF, false>(P, L, rec, sp, mesh_out, diag);
+                        const int first = CELLS && !L.wide ? L.c0 + L.ci0 : L.ci0;
+                        deposit_1d_cells<NF, false>(P, L, rec, sp, first, mesh_out, diag);
                         if (fdep) {
 #pragma unroll 1
                             for (int i = 0; i < P.w[2]; i++) {
-                                double* m = full + (long long)((L.ci0 + i) % nz) * ND;
+                                double* m = full + (long long)((first + i) % nz) * ND;
                                 const double wi = i == 0 ? L.wz[0] : i == 1 ? L.wz[1] : L.wz[2];
                                 for (int d = 0; d < 4; d++)
                                     for (int e = 0; e < NH; e++)
@@ -890,6 +922,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (alive && active) {
 #pragma unroll
         for (int e = 0; e < NH; e++) S.f0[(sp * NH + e) * cap + p] = y0[e];
+        if (not_finite<NH>(y0)) ctl->odd = 1;
         if (sp == 0) {
             S.pos[0][p] = x;
             S.pos[1][p] = yy;
@@ -929,6 +962,16 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
 }
 
+template <int NF, bool ONE, int MAXT, bool REC>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_steps_1d(DevParams P, DevState S, double* __restrict__ cmesh, double* __restrict__ full, StepCtl* ctl,
+               int npart, int nsteps, int dt_mode, Rec1DStore store)
+{
+    if (ctl->done) return;
+    if (ctl->odd) steps_1d_body<NF, ONE, REC, true>(P, S, cmesh, full, ctl, npart, nsteps, dt_mode, store);
+    else steps_1d_body<NF, ONE, REC, false>(P, S, cmesh, full, ctl, npart, nsteps, dt_mode, store);
+}
+
 // The backward sweep over recorded steps of a 1D run (emu_adjoint.cu: the
 // discrete adjoint), last step first, in one cooperative launch with the
 // means of k_steps_1d: the adjoint state in registers, the windows of the
@@ -937,10 +980,11 @@ __global__ void __launch_bounds__(MAXT, 1)
 // (stage 0 only gathers).  The next stage's recorded mesh and state are
 // loaded between arrival and wait.  Two flavors, 128 x 80: a recorded step
 // 49 -> 17 us, a backward step 62 -> 22 us (against tiles of 128 particles
-// that reloaded their state and ranked their keys in every stage).
-template <int NF, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1)
-    k_adjoint_1d(DevParams P, DevState S, Adj1DStore A, StepCtl* ctl, int npart, int len)
+// that reloaded their state and ranked their keys in every stage).  CELLS: as
+// k_steps_1d, for a recorded state or an adjoint state that is not finite.
+template <int NF, bool CELLS>
+__device__ __forceinline__ void adjoint_1d_body(const DevParams& P, const DevState& S, const Adj1DStore& A, StepCtl* ctl,
+                                                int npart, int len)
 {
     using H = Herm<NF>;
     using C = Comb<NF>;
@@ -999,7 +1043,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         const double dt = A.dts[j];
         load(sst + 3 * (2 * NH) * cap, yn);   // Y_n
         load(sst + 2 * (2 * NH) * cap, ys);   // Y_4
-        place_particles<NF>(P, L, zpos(j), active, sp, sref, swin, rec, wrec);
+        place_particles<NF, CELLS>(P, L, zpos(j), active, sp, sref, swin, rec, wrec);
         stage_window<NF>(L, sm_fwd, stage_mesh(j, 4), nz);
         __syncthreads();
 #pragma unroll 1
@@ -1059,8 +1103,8 @@ __global__ void __launch_bounds__(MAXT, 1)
             }
             __syncwarp();
             double* const lm_out = A.lm + (s & 3) * A.lm_stride;
-            if (!L.wide) deposit_1d<NF, true>(L, srec, nullptr, wrec, lm_out, nz, false);
-            else if (active) deposit_1d_wide<NF, true>(P, L, rec, sp, lm_out, false);
+            if (!CELLS && !L.wide) deposit_1d<NF, true>(L, srec, nullptr, wrec, lm_out, nz, false);
+            else if (active) deposit_1d_cells<NF, true>(P, L, rec, sp, L.wide ? L.ci0 : L.c0 + L.ci0, lm_out, false);
             // the next stage's target (last read three stages ago)
             double* const lz = A.lm + ((s + 3) & 3) * A.lm_stride;
             for (int i = gtid; i < msize; i += nthreads) lz[i] = 0.0;
@@ -1089,6 +1133,14 @@ __global__ void __launch_bounds__(MAXT, 1)
             ctl->bar_count = 0u;
         }
     }
+}
+
+template <int NF, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_adjoint_1d(DevParams P, DevState S, Adj1DStore A, StepCtl* ctl, int npart, int len)
+{
+    if (ctl->odd | ctl->odd_lam) adjoint_1d_body<NF, true>(P, S, A, ctl, npart, len);
+    else adjoint_1d_body<NF, false>(P, S, A, ctl, npart, len);
 }
 
 // particles per CTA: spread over the SMs, whole warps of 16, at least 64 (a

@@ -112,6 +112,8 @@ struct StepCtl {
     // same; 2: the run had ended before the latest step)
     int m4_full_from;
     int m4_full;
+    int odd;        // the particles hold (or held, since their load) a value that is not finite
+    int odd_lam;    // and the adjoint state of the sweep in progress
 };
 
 enum DtMode : int { DT_QUERY = 0, DT_INIT = 1, DT_ADVANCE = 2 };
@@ -121,12 +123,14 @@ constexpr int kBlock = 128;
 constexpr long long kBarrierSpins = 1ll << 22;
 
 // launchers (all asynchronous on the given stream)
+// ctl: its word `odd` is set when the records call for it (launch_cell_keys
+// clears it)
 void launch_pack(int nf, const DevParams& P, const double* aos, const unsigned* perm, long long n, DevState S,
-                 cudaStream_t st);
+                 StepCtl* ctl, cudaStream_t st);
 void launch_unpack(int nf, const DevState& S, double* aos, cudaStream_t st);
 void launch_unpack_rhs(int nf, const DevState& S, const double* K, double* aos, cudaStream_t st);
 void launch_cell_keys(const DevParams& P, const double* aos, int nreal, long long n, unsigned* keys,
-                      unsigned* idx, cudaStream_t st);
+                      unsigned* idx, StepCtl* ctl, cudaStream_t st);
 void launch_deposit(int nf, const DevParams& P, const DevState& S, const double* f, double* mesh, cudaStream_t st);
 void launch_deposit_q(int nf, const DevParams& P, const DevState& S, const double* f, long long* mesh,
                       cudaStream_t st);

@@ -1829,7 +1829,7 @@ __global__ void __launch_bounds__(kBlock, WX == 1 && WY == 1 ? 5 : 4) k_rk4_stag
 // AoS records (rows of 3+nattribs) -> SoA, row perm[i] goes to slot i
 template <int NF>
 __global__ void k_pack(DevParams P, const double* __restrict__ aos, const unsigned* __restrict__ perm, long long n,
-                       DevState S)
+                       DevState S, StepCtl* ctl)
 {
     constexpr int NH = NF * NF, NA = 8 + 2 * (2 + NH), NR = 3 + NA;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1841,15 +1841,19 @@ __global__ void k_pack(DevParams P, const double* __restrict__ aos, const unsign
     S.time[i] = r[3 + 0];
     for (int d = 0; d < 4; d++) S.pup[d][i] = r[3 + 4 + d];
     const double pupt = r[3 + 7];
-    for (int d = 0; d < 3; d++) S.vhat[d][i] = r[3 + 4 + d] / pupt;
-    S.vscale[i] = P.c4 / (2. * pupt);
+    const double v[4] = {r[3 + 4] / pupt, r[3 + 5] / pupt, r[3 + 6] / pupt, P.c4 / (2. * pupt)};
+    for (int d = 0; d < 3; d++) S.vhat[d][i] = v[d];
+    S.vscale[i] = v[3];
+    bool odd = not_finite<4>(v);
     for (int sp = 0; sp < 2; sp++) {
         const int base = 3 + 8 + sp * (2 + NH);
         S.Nn[sp][i] = r[base];
         S.Ll[sp][i] = r[base + 1];
         for (int e = 0; e < NH; e++) S.f0[(sp * NH + e) * S.cap + i] = r[base + 2 + e];
+        odd = odd || not_finite<2 + NH>(r + base);
     }
     S.id[i] = row;
+    if (odd) ctl->odd = 1;
 }
 
 template <int NF>
@@ -1892,10 +1896,11 @@ __global__ void k_unpack_rhs(DevState S, const double* __restrict__ K, double* _
 }
 
 __global__ void k_cell_keys_aos(DevParams P, const double* __restrict__ aos, int nreal, long long n,
-                                unsigned* keys, unsigned* idx)
+                                unsigned* keys, unsigned* idx, StepCtl* ctl)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i == 0) ctl->odd = 0;
     Stencil<double> st;
     make_stencil<double>(P, aos[i * nreal + 0], aos[i * nreal + 1], aos[i * nreal + 2], st);
     keys[i] = (unsigned)stencil_key(P, st.b);
@@ -2102,6 +2107,7 @@ __global__ void k_ctl_set(StepCtl* ctl, double dt, double t, double end_time, in
     ctl->bar_gen = 0u;
     ctl->dt_hist = nullptr;
     ctl->m4_full_from = 0;
+    ctl->odd_lam = 0;
     if (reset_status) {
         ctl->status = 0;
         ctl->bad = LLONG_MAX;
