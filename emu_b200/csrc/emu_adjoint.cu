@@ -1166,7 +1166,7 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
         if (ctx->steps1d) {
             if ((r = deposit_comb_into(ctx, S, S.f0, G.mst))) return r;
             emu::Rec1DStore rec{G.seg, G.sst, G.mst, G.seg_stride, G.sst_stride, G.mst_stride};
-            cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, S, ctx->cmesh, ctx->mesh[3], ctx->ctl, len,
+            cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, S, ctx->cmesh, ctx->mesh[0], ctx->ctl, len,
                                                  emu::DT_ADVANCE, st, &rec);
             if (emu_ctx::leave_steps_1d(ctx, e)) return EMU_OK;   // (refused: nothing has run)
             if (e != cudaSuccess)
@@ -1184,16 +1184,18 @@ int record_full(emu_context* ctx, emu_adjoint* a, int nsteps, int interval)
                                cudaMemcpyDeviceToDevice, st));
         if ((r = check_launch(ctx, "recorded segment"))) return r;
     }
-    // the context as after the step loop: the new state's deposit in mesh 0,
-    // the last step's stage-4 mesh as the current mesh
-    ctx->cur_mesh = 3;
-    if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its combined mesh)
+    // the context as after the step loop: the last step's stage-4 mesh as the
+    // current mesh; unless that is its place, the new state's deposit in mesh 0
+    ctx->cur_mesh = stage4_mesh(ctx);
+    if (ctx->steps1d || ctx->comb64) ctx->fused_ready = false;   // (the next step deposits its meshes)
     if (ctx->steps1d) return EMU_OK;   // (its last step deposits the full stage-4 mesh)
     const DevState& S = ctx->S[ctx->cur];
     const int last = nsteps - (nseg - 1) * interval - 1;   // (the last step in its segment)
-    if ((r = deposit_into(ctx, S, S.f0, ctx->mesh[0]))) return r;
-    CU(cudaMemsetAsync(ctx->mesh[1], 0, sizeof(double) * mesh_elems(ctx), st));
-    return deposit_into(ctx, emu::seg_state(S, G, last), emu::seg_y(G, last, 4, cap), ctx->mesh[3]);
+    if (!ctx->comb64) {
+        if ((r = deposit_into(ctx, S, S.f0, ctx->mesh[0]))) return r;
+        CU(cudaMemsetAsync(ctx->mesh[1], 0, sizeof(double) * mesh_elems(ctx), st));
+    }
+    return deposit_into(ctx, emu::seg_state(S, G, last), emu::seg_y(G, last, 4, cap), ctx->mesh[ctx->cur_mesh]);
 }
 
 }  // namespace
@@ -1372,6 +1374,7 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     CU(cudaMemsetAsync(a->lmesh[0], 0, sizeof(double) * nm, st));
     if ((r = check_launch(ctx, "adjoint input"))) return r;
     const bool coop = a->store && emu::adj_coop_fits(nf, ctx->P, n);
+    ctx->fused_ready = false;   // (until the end: the recomputes use the context's meshes)
     // per-step mode with re-sorts (the recomputes re-sort as the forward did)
     const bool rps = !a->store && ctx->prm.resort_interval > 0 && a->gperm;
 
@@ -1669,11 +1672,14 @@ int emu_adjoint_backward(emu_context* ctx, const double* lam_f_final, const doub
     if ((r = emu_ctx::copy_to_host(ctx, lam_f0, a->rows, sizeof(double) * (size_t)n * NS))) return r;
     emu::k_soa_to_rows<<<g, emu::kBlock, 0, st>>>(W0.id, a->lamN, 2, cap, n, a->rows);
     if ((r = emu_ctx::copy_to_host(ctx, lam_N0, a->rows, sizeof(double) * (size_t)n * 2))) return r;
-    // the forward meshes were reused: restore the current state's deposit
+    // the forward meshes were reused: restore the current state's deposit (the
+    // combined meshes, in the same memory, are made from it when wanted)
     double* const* M = ctx->mesh;
     CU(cudaMemsetAsync(M[1], 0, sizeof(double) * mesh_elems(ctx), st));
     if ((r = deposit_into(ctx, S, S.f0, M[0]))) return r;
     ctx->cur_mesh = 0;
+    ctx->fused_ready = true;
+    ctx->cmesh_ready = false;
     CU(cudaStreamSynchronize(st));
     return check_launch(ctx, "adjoint output");
 }

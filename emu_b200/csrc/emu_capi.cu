@@ -287,12 +287,6 @@ long long qmesh_elems(const emu_context* c) { return c->P.ncells * (c->ND + emu:
 
 long long cmesh_elems(const emu_context* c) { return c->P.ncells * ((c->nf == 3 ? emu::Comb<3>::NG : emu::Comb<2>::NG) + emu::kDiagSlots); }
 
-int ensure_cmesh(emu_context* ctx)
-{
-    if (!ctx->cmesh) CU(emu_ctx::dev_malloc(&ctx->cmesh, sizeof(double) * 4 * cmesh_elems(ctx)));
-    return EMU_OK;
-}
-
 // The automatic re-sort interval.  A 27-cell stencil loses its per-CTA cell
 // runs within a step or two once particles leave their cells, a 1D stencil
 // within several.  FP64 stages in a plane re-sort every step too, since the
@@ -342,11 +336,11 @@ double cells_per_cm(const DevParams& P)
 // is false on return: the caller takes the steps with the stage kernels
 int run_steps_1d(emu_context* ctx, int nsteps, int dt_mode)
 {
-    const cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, ctx->S[ctx->cur], ctx->cmesh, ctx->mesh[3], ctx->ctl,
+    const cudaError_t e = emu::launch_steps_1d(ctx->nf, ctx->P, ctx->S[ctx->cur], ctx->cmesh, ctx->mesh[0], ctx->ctl,
                                                nsteps, dt_mode, ctx->stream);
     if (emu_ctx::leave_steps_1d(ctx, e)) return EMU_OK;
     if (e != cudaSuccess) return fail(ctx, EMU_ERR_CUDA, std::string("cooperative steps: ") + cudaGetErrorString(e));
-    ctx->cur_mesh = 3;
+    ctx->cur_mesh = stage4_mesh(ctx);
     return EMU_OK;
 }
 
@@ -453,7 +447,7 @@ int enqueue_rk4_fp64(emu_context* ctx, cudaStream_t st, bool with_dt, bool dep4 
 }
 
 // FP64 RK4 on combined meshes: stage s reads cmesh s-1, deposits cmesh s%4,
-// zeroes cmesh (s+1)%4; the full stage-4 mesh (mesh[3], on the steps after
+// zeroes cmesh (s+1)%4; the full stage-4 mesh (mesh[0], on the steps after
 // which it can be read) by a kernel between stages 3 and 4.  dep4 = false: a
 // re-sort follows, made by stage 4's stores (enqueue_sc_before), then the
 // deposit of the re-sorted state.  stage_event(i, end): before and after each
@@ -470,10 +464,10 @@ int enqueue_rk4_comb64(emu_context* ctx, cudaStream_t st, bool with_dt, bool dep
     for (int s = 1; s <= 3; s++) {
         const bool keys = s == 3 && !dep4;
         stage_event(s - 1, 0);
-        emu::launch_stage64(ctx->nf, ctx->P, S, s, cm(s - 1), cm(s), cm(s + 1), s == 2 ? ctx->mesh[3] : nullptr,
+        emu::launch_stage64(ctx->nf, ctx->P, S, s, cm(s - 1), cm(s), cm(s + 1), s == 2 ? ctx->mesh[0] : nullptr,
                             ctx->ctl, dt_mode, st, nullptr, nullptr, keys ? ctx->keys : nullptr,
                             keys ? ctx->idx : nullptr);
-        if (s == 3) emu::launch_deposit_full64(ctx->nf, ctx->P, S, S.f0, ctx->mesh[3], ctx->ctl, st);
+        if (s == 3) emu::launch_deposit_full64(ctx->nf, ctx->P, S, S.f0, ctx->mesh[0], ctx->ctl, st);
         stage_event(s - 1, 1);
     }
     if (dep4) {
@@ -722,7 +716,7 @@ int emu_ctx::step_device(emu_context* ctx, bool last_stage_deposit)
         if (!ctx->graph[c][v] && (r = build_graph(ctx, v))) return r;
         CU(cudaGraphLaunch(ctx->graph[c][v], ctx->stream));
     }
-    ctx->cur_mesh = ctx->mixed ? 1 : 3;
+    ctx->cur_mesh = ctx->mixed ? 1 : stage4_mesh(ctx);
     return EMU_OK;
 }
 
@@ -797,7 +791,6 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     // stage kernels on combined meshes
     ctx->comb64 = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                   !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d;
-    if ((ctx->steps1d || ctx->comb64) && (r = ensure_cmesh(ctx))) return r;
     choose_resort(ctx);
     ctx->loaded = true;
     ctx->adj_valid = false;
@@ -866,8 +859,12 @@ int emu_create(const emu_params* p, emu_context** out)
         if (!r && emu_ctx::dev_malloc(&ctx->gmesh, sizeof(float) * ctx->P.ncells * (ctx->nf == 3 ? emu::Comb<3>::NG : emu::Comb<2>::NG)) != cudaSuccess)
             r = EMU_ERR_NOMEM;
     } else {
-        for (int i = 0; i < 4 && !r; i++)
-            if (emu_ctx::dev_malloc(&ctx->mesh[i], sizeof(double) * me) != cudaSuccess) r = EMU_ERR_NOMEM;
+        static_assert(4 * (emu::Comb<2>::NG + emu::kDiagSlots) <= 3 * 8 * 4 &&
+                          4 * (emu::Comb<3>::NG + emu::kDiagSlots) <= 3 * 8 * 9,
+                      "the combined meshes fit in three full ones");
+        if (!r && emu_ctx::dev_malloc(&ctx->mesh[0], sizeof(double) * 4 * me) != cudaSuccess) r = EMU_ERR_NOMEM;
+        for (int i = 1; i < 4 && !r; i++) ctx->mesh[i] = ctx->mesh[0] + i * me;
+        ctx->cmesh = ctx->mesh[1];
     }
     if (!r && emu_ctx::dev_malloc(&ctx->planes, sizeof(double) * ctx->P.ncells * emu_ncomp(ctx->nf)) != cudaSuccess)
         r = EMU_ERR_NOMEM;
@@ -903,8 +900,7 @@ void emu_destroy(emu_context* ctx)
     for (int i = 0; i < 2; i++) if (ctx->pblock[i]) emu_ctx::dev_free(ctx->pblock[i]);
     if (ctx->tblock) emu_ctx::dev_free(ctx->tblock);
     if (ctx->S[0].kgen) emu_ctx::dev_free(ctx->S[0].kgen);
-    for (int i = 0; i < 4; i++) if (ctx->mesh[i]) emu_ctx::dev_free(ctx->mesh[i]);
-    if (ctx->cmesh) emu_ctx::dev_free(ctx->cmesh);
+    if (ctx->mesh[0]) emu_ctx::dev_free(ctx->mesh[0]);   // (one block)
     for (int i = 0; i < 2; i++) if (ctx->qmesh[i]) emu_ctx::dev_free(ctx->qmesh[i]);
     if (ctx->qfull) emu_ctx::dev_free(ctx->qfull);
     if (ctx->qfull_part) emu_ctx::dev_free(ctx->qfull_part);
@@ -1120,7 +1116,7 @@ int emu_step(emu_context* ctx, double dt, int64_t* bad)
         }
         if (r) return r;
         if (ctx->mixed && (r = sum_full_parts(ctx))) return r;
-        ctx->cur_mesh = ctx->mixed ? 1 : 3;
+        ctx->cur_mesh = ctx->mixed ? 1 : stage4_mesh(ctx);
         ctx->fused_ready = true;
     } else {
         if (ctx->mixed) return fail(ctx, EMU_ERR_ARG, "emu_step: the mixed path integrates with RK4 only");
@@ -1258,7 +1254,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
         cudaEventDestroy(b);
         if (one_launch && !ctx->steps1d) continue;   // (refused: the stage kernels)
         *nkernels = 1;
-        ctx->cur_mesh = 3;
+        ctx->cur_mesh = stage4_mesh(ctx);
         int r;
         if (ctx->prm.resort_interval > 0 && ++ctx->steps_since_sort >= ctx->prm.resort_interval)
             if ((r = resort(ctx))) return r;
@@ -1342,7 +1338,7 @@ int emu_profile_step(emu_context* ctx, float* kernel_ms, int max_kernels, int* n
     int r = check_launch(ctx, "profile step");
     if (r) return r;
     if (ctx->mixed && (r = sum_full_parts(ctx))) return r;
-    ctx->cur_mesh = ctx->mixed ? 1 : 3;
+    ctx->cur_mesh = ctx->mixed ? 1 : stage4_mesh(ctx);
     if (ctx->prm.resort_interval > 0) ctx->steps_since_sort++;
     if (sc) {
         if ((r = resort(ctx, true))) return r;   // (the buffers change places)

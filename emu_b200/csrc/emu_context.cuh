@@ -32,8 +32,9 @@ struct emu_context {
     double* mesh[4] = {nullptr, nullptr, nullptr, nullptr};
     // FP64 steps on combined meshes (steps1d, comb64): M_1..M_4 in the combined
     // layout with the diagonal slots (kCombSlots per cell), one after the
-    // other; mesh[0] and mesh[3] then hold the full deposit of a load and the
-    // full stage-4 mesh
+    // other, in the memory of mesh[1..3] (the four full meshes are one block);
+    // mesh[0] then holds the full deposit of a load, later the full stage-4
+    // mesh (stage4_mesh)
     double* cmesh = nullptr;
     long long* qmesh[2] = {nullptr, nullptr};
     // mixed path: the full 8 NF^2 mesh of the state at the last deposit
@@ -85,6 +86,9 @@ struct emu_context {
     cudaEvent_t ring_event[8] = {};
     std::string err;
 };
+
+// which full mesh holds the stage-4 mesh after an FP64 step
+inline int stage4_mesh(const emu_context* c) { return c->steps1d || c->comb64 ? 0 : 3; }
 
 namespace emu_ctx {
 
