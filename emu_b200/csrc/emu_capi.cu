@@ -331,6 +331,16 @@ double cells_per_cm(const DevParams& P)
     return m;
 }
 
+// Along z with TSC and two flavors, less than two particles a cell: the stage
+// kernels on full meshes, whose lanes walk such runs (and two threads a
+// particle), where a product holds one or two of eight particles (evolve and
+// single steps in us, full / combined meshes: 40,000 cells x 1 197/222 and
+// 205/265; x 2 of 20,000 134/129 and 143/161; CIC there 205/134)
+bool sparse_1d(const emu_context* ctx, long long n)
+{
+    return ctx->nf == 2 && ctx->P.w[0] == 1 && ctx->P.w[1] == 1 && ctx->P.w[2] == 3 && n < 2 * ctx->P.ncells;
+}
+
 // nsteps steps of k_steps_1d (dt_mode as launch_steps_1d).  When its grid is
 // refused (a stream that may not use every SM) nothing has run and ctx->steps1d
 // is false on return: the caller takes the steps with the stage kernels
@@ -788,9 +798,9 @@ int emu_ctx::load_from_aos(emu_context* ctx, int64_t n, double pupt_min, const d
     ctx->steps1d = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
                    emu::steps_1d_fit(ctx->nf, ctx->P, n);
     // any other FP64 RK4 context of one rank without the adaptive timestep:
-    // stage kernels on combined meshes
+    // stage kernels on combined meshes (almost any, see sparse_1d)
     ctx->comb64 = !ctx->mixed && !ctx->comm && !ctx->local && ctx->prm.fused == 1 && rk4_fused(ctx) &&
-                  !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d;
+                  !(ctx->prm.max_adaptive_speedup > 1.0) && !ctx->steps1d && !sparse_1d(ctx, n);
     choose_resort(ctx);
     ctx->loaded = true;
     ctx->adj_valid = false;
