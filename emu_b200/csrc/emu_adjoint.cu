@@ -18,8 +18,7 @@
 //   lam_K4 = b4 dt lam_n,  lam_Ks = b_s dt lam_n + a_{s+1} dt lam_Y{s+1}
 //   lam_Ys = C_Y^T(H_s) lam_Ks  +  N D^T( I^T( C_H^T(Y_s) lam_Ks ) )
 //   lam_Y0 = lam_n + sum_{s>=2} lam_Ys + lam_Y1,  lam_N += Y_s . D^T(...)
-// C_Y^T, C_H^T: the commutator is bilinear, so each adjoint component is the
-// commutator with a unit vector contracted with lam (exact).  I^T scatters
+// C_Y^T, C_H^T: two commutators (commutator_vjp, exact).  I^T scatters
 // like a deposit (same mesh layout, velocity sign flipped, factor
 // sqrt(2) G_F / V_cell); D^T gathers like an interpolation.  The
 // Renormalize adjoint replays its branches (trace fix, diagonal clamp,
@@ -28,8 +27,9 @@
 // Memory: checkpoints of (Y_0, x) every `interval` steps; a segment is
 // recomputed forward into per-step (Y_0, x) slots, then each step's stage
 // states Y_2..Y_4, Y_n and meshes M_1..M_4 are recomputed before its
-// backward.  Particles keep their slot order for the whole recorded run (no
-// re-sort).
+// backward.  A run recorded whole (record_full) is re-sorted at segment starts
+// only, any other on the step loop's schedule; the sweep undoes the composed
+// maps on the static fields and the adjoint state.
 #include "emu_adjoint.cuh"
 #include "emu_context.cuh"
 #include "emu_fp64_impl.cuh"

@@ -33,7 +33,7 @@ namespace {
 //   - stages are separated by a grid barrier (measured 2350 clocks with the
 //     mesh reductions it waits for; a kernel boundary cost about the same,
 //     plus the reload of the state).  What the next stage does not wait for
-//     (zeroing, the timestep) runs between arrival and wait;
+//     (zeroing) runs between arrival and wait;
 //   - compute_dt over the stage-4 mesh: each CTA reduces its share of the
 //     cells before it arrives at the step's last barrier.  (Every CTA all of
 //     them behind its arrival, as it was: 30,000 particles in 30,000 cells

@@ -119,7 +119,7 @@ struct StepCtl {
 enum DtMode : int { DT_QUERY = 0, DT_INIT = 1, DT_ADVANCE = 2 };
 
 constexpr int kBlock = 128;
-// default limit of a grid-barrier wait (polls of 64 ns sleeps, ~0.3 s or more)
+// default limit of a grid-barrier wait (polls, each a read through L2: seconds)
 constexpr long long kBarrierSpins = 1ll << 22;
 
 // launchers (all asynchronous on the given stream)

@@ -104,7 +104,9 @@ typedef struct emu_params {
                                 (the reference seeds from the clock, main.cpp:240) */
     int resort_interval;     /* steps between on-device cell re-sorts (0 = never,
                                 < 0 = automatic: every step for 27-cell stencils
-                                and for FP64 stencils of more than 3 cells; FP64
+                                and for FP64 stencils of more than 3 cells (single
+                                steps of small two-flavor problems: once the
+                                particles may have moved a tenth of a cell); FP64
                                 1D problems that run in one launch every 32
                                 steps, or never with one cell; every 16 steps
                                 otherwise; default -1) */
@@ -215,8 +217,9 @@ int emu_evolve_end(emu_context* ctx, emu_run_info* info);
  * kernels (the kernels that run several steps of small 1D problems, the
  * whole-step kernel of fused = 2 and the adjoint's segment kernels), in
  * polls; polls < 0 restores the default (2^22).  A wait that runs out sets EMU_ERR_TIMEOUT in the run's status and
- * lets the kernel finish (the step's results are then invalid); the next
- * emu_evolve_begin or emu_load_particles resets the barrier.  No
+ * lets the kernel finish (the step's results are then invalid; steps queued
+ * behind a launch of several steps are not taken); load the particles again
+ * before the next run.  No
  * counterpart in the reference (its steps have no device-side waits);
  * tests use a limit of 0 to make a wait run out. */
 int emu_set_wait_limit(emu_context* ctx, int64_t polls);
@@ -287,7 +290,8 @@ int emu_deposit_noalloc(const emu_params* p, const double* d_records, int64_t n,
  * emu_adjoint_forward: nsteps device-resident RK4 steps from the loaded
  * state with the configured timestep rule, recording every step's dt (into
  * dts when not NULL) and a checkpoint of (f, x) every checkpoint_interval
- * steps.  Particles keep their order (no re-sort) during a recorded run.
+ * steps.  Re-sorts of the run (at checkpoints, or on resort_interval's
+ * schedule) are undone by the backward sweep.
  * Requires precision FP64, integration_type 1, rk_type 4, fused >= 1.
  *
  * emu_adjoint_objective: J = sum over cells |N_emu|^2 / V_cell of the
