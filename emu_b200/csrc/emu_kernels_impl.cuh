@@ -974,15 +974,16 @@ __global__ void __launch_bounds__(2 * kBlock, 2) k_rk4_step_coop_split(DevParams
 // unfused building blocks (FP64)
 // ===========================================================================
 // The full deposit, run by run (k_deposit_full64's other form, for particles in
-// short runs: see launch_deposit_full64).  ctl as there.
-template <int NF, int WX, int WY, int WZ>
+// short runs: see launch_deposit_full64).  STEP: between stages 3 and 4 of a
+// step, as there (a block takes tiles in turn); else a tile a block.
+template <int NF, int WX, int WY, int WZ, bool STEP>
 __global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, const double* __restrict__ f,
                                                     double* __restrict__ mesh, StepCtl* ctl)
 {
     using SWt = SW<WX, WY, WZ>;
     constexpr int NH = NF * NF, NS = 2 * NH;
     double dt = 0.0;
-    if (ctl) {
+    if constexpr (STEP) {
         grid_dep_wait();
         grid_dep_launch();
         dt = ctl->dt;
@@ -990,7 +991,7 @@ __global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, con
         if (blockIdx.x == 0 && threadIdx.x == 0) ctl->m4_full = done ? 2 : full ? 1 : 0;
         if (!full) return;
     }
-    const long long ntile = (S.n + kBlock - 1) / kBlock;
+    const long long ntile = STEP ? (S.n + kBlock - 1) / kBlock : blockIdx.x + 1;
     for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
         const long long p = tile * kBlock + threadIdx.x;
         const bool active = p < S.n;
@@ -1005,13 +1006,14 @@ __global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, con
 #pragma unroll
             for (int c = 0; c < NS; c++) {
                 double y = f[c * S.cap + p];
-                if (ctl) y = __dadd_rn(__dmul_rn(dt, S.fs[c * S.cap + p]), y);
+                if constexpr (STEP) y = __dadd_rn(__dmul_rn(dt, S.fs[c * S.cap + p]), y);
                 fN[c] = y * S.Nn[c / NH][p];
             }
         }
         tile_deposit_block<NF, SWt, double>(P, mesh, active, st, fN, vx, vy, vz,
                                             [](double a, int) -> double { return a; }, true);
-        __syncthreads();   // (the next tile's ranks use the records' memory)
+        if constexpr (STEP) __syncthreads();   // (the next tile's ranks use the records' memory)
+        else break;
     }
 }
 
@@ -2278,11 +2280,16 @@ void launch_deposit_t(const DevParams& P, const DevState& S, const double* f, do
 {
     EMU_W_DISPATCH(P, {
         constexpr int bytes = tile_smem_bytes<NF, SW<WXv, WYv, WZv>, double>();
-        auto kern = k_deposit<NF, WXv, WYv, WZv>;
-        smem_optin(kern, bytes);
-        const unsigned grid = (unsigned)std::min<long long>(grid_for(S.n), 148 * 12);
-        if (ctl) launch_pdl(kern, grid, kBlock, bytes, st, P, S, f, mesh, ctl);
-        else kern<<<grid_for(S.n), kBlock, bytes, st>>>(P, S, f, mesh, (StepCtl*)nullptr);
+        const auto in_step = k_deposit<NF, WXv, WYv, WZv, true>;
+        const auto alone = k_deposit<NF, WXv, WYv, WZv, false>;
+        if (ctl) {
+            smem_optin(in_step, bytes);
+            launch_pdl(in_step, (unsigned)std::min<long long>(grid_for(S.n), 148 * 12), kBlock, bytes, st, P, S, f, mesh,
+                       ctl);
+        } else {
+            smem_optin(alone, bytes);
+            alone<<<grid_for(S.n), kBlock, bytes, st>>>(P, S, f, mesh, nullptr);
+        }
     });
 }
 
