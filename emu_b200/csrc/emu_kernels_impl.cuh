@@ -975,7 +975,9 @@ __global__ void __launch_bounds__(2 * kBlock, 2) k_rk4_step_coop_split(DevParams
 // ===========================================================================
 // The full deposit, run by run (k_deposit_full64's other form, for particles in
 // short runs: see launch_deposit_full64).  STEP: between stages 3 and 4 of a
-// step, as there (a block takes tiles in turn); else a tile a block.
+// step, as there (a block takes tiles in turn); else a tile a block (the loop
+// cost unfused steps up to 8 %: three flavors, 600 cells x 2, forward Euler 147
+// us with it, 135 without).
 template <int NF, int WX, int WY, int WZ, bool STEP>
 __global__ void __launch_bounds__(kBlock) k_deposit(DevParams P, DevState S, const double* __restrict__ f,
                                                     double* __restrict__ mesh, StepCtl* ctl)
