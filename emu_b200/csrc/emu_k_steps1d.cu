@@ -35,7 +35,8 @@ namespace {
 //     plus the reload of the state).  What the next stage does not wait for
 //     (zeroing) runs between arrival and wait;
 //   - compute_dt over the stage-4 mesh: each CTA reduces its share of the
-//     cells before it arrives at the step's last barrier.  (Every CTA all of
+//     cells before it arrives at the step's last barrier (before it leaves, in
+//     the last step of a launch).  (Every CTA all of
 //     them behind its arrival, as it was: 30,000 particles in 30,000 cells
 //     67 against 48 us a step, in 400,000 cells 557 against 136; the same to
 //     300 cells.)
@@ -645,6 +646,7 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
     const double dt_fac = stupid_factor<NF>(P), dt_vmin = P.cell_volume * P.Ye * P.rho / kMp;
     bool alive = true;
     unsigned nbar = 0;
+    int slot = 0;  // of the control's vmax_bits: the step's largest number
     int cur = 0;   // ONE: which half of smesh holds the stage mesh
 
     for (int it = 0; it < nsteps && alive; it++) {
@@ -872,7 +874,9 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
                         atomicMax(&ctl->vmax_bits[it & 1], (unsigned long long)__double_as_longlong(vm));
                     }
                 }
-                const bool wait = s < 4 || dt_mode == DT_ADVANCE || !final_step;
+                // (the launch's last step ends without a barrier: the last CTA to
+                // leave finds the next timestep)
+                const bool wait = s < 4 || !(final_step || (dt_mode == DT_ADVANCE && (last || step + 1 >= max_step)));
                 if (wait) steps_arrive(ctl);
                 // the mesh deposited two stages on (its last readers are past
                 // the previous barrier)
@@ -891,8 +895,12 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
                     }
                 }
                 if (s == 4 && dt_mode == DT_ADVANCE) {
-                    const double vm = __longlong_as_double((long long)__ldcg(&ctl->vmax_bits[it & 1]));
-                    dt_next = next_dt_stupid(P, fmax(P.flavor_cfl_factor > 0.0 ? vm : 0.0, dt_vmin), dt_fac, st_dt);
+                    slot = it & 1;
+                    dt_next = -INFINITY;
+                    if (wait) {
+                        const double vm = __longlong_as_double((long long)__ldcg(&ctl->vmax_bits[slot]));
+                        dt_next = next_dt_stupid(P, fmax(P.flavor_cfl_factor > 0.0 ? vm : 0.0, dt_vmin), dt_fac, st_dt);
+                    }
                 } else if (s == 2 && gtid == 0) {
                     ctl->vmax_bits[(it + 1) & 1] = 0ull;   // (every CTA has read the last step's)
                 }
@@ -949,6 +957,15 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
             __threadfence();
             ctl->blocks_done = 0u;
             ctl->bar_count = 0u;
+            if (!ONE && dt_mode == DT_ADVANCE) {
+                const double vm = __longlong_as_double((long long)__ldcg(&ctl->vmax_bits[slot]));
+                dt = next_dt_stupid(P, fmax(P.flavor_cfl_factor > 0.0 ? vm : 0.0, dt_vmin), dt_fac, st_dt);
+                if (end_time - t_run < dt) {
+                    dt = end_time - t_run;
+                    last = 1;
+                }
+                if (st_dt) done = 1;
+            }
             ctl->vmax_bits[0] = ctl->vmax_bits[1] = 0ull;
             if (steps_timed_out(ctl)) {
                 ctl->done = 1;
