@@ -205,12 +205,26 @@ __device__ __noinline__ void deposit_cells(int ncells, double* mesh, int stride,
 
 // Grid barrier in two halves: arrivals counted up from 0 over the launch (the
 // last CTA to leave the kernel sets the count back).  The wait is bounded;
-// false: it gave up (ST_TIMEOUT is set, the CTA goes to the kernel's end).
+// false: it gave up (ST_TIMEOUT is set; steps_gave_up).
 __device__ __forceinline__ bool steps_timed_out(const StepCtl* ctl)
 {
     int v;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&ctl->status) : "memory");
     return (v & ST_TIMEOUT) != 0;
+}
+// A CTA leaves after a wait that gave up (thread 0): the last one of all sets
+// the counts back for the next launch and ends the run (the launches queued
+// behind this one return at once)
+__device__ __noinline__ void steps_gave_up(StepCtl* ctl)
+{
+    __threadfence();
+    if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        ctl->blocks_done = 0u;
+        ctl->bar_count = 0u;
+        ctl->vmax_bits[0] = ctl->vmax_bits[1] = 0ull;
+        ctl->done = 1;
+    }
 }
 __device__ __forceinline__ void steps_arrive(StepCtl* ctl)
 {
@@ -218,23 +232,32 @@ __device__ __forceinline__ void steps_arrive(StepCtl* ctl)
     if (threadIdx.x == 0)
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
 }
-__device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target, long long polls)
+// (A limit that is not a constant in the poll's loop cost 0.05 us a barrier:
+// the first polls go without, a limit below them takes the slow loop at once.)
+constexpr int kFirstPolls = 1 << 16;
+__device__ __noinline__ int steps_wait_slow(StepCtl* ctl, unsigned target, long long polls)
+{
+    for (long long it = 0;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->bar_count) : "memory");
+        if (v >= target) return 1;
+        if (++it > polls) {
+            atomicOr(&ctl->status, ST_TIMEOUT);
+            return 0;
+        }
+    }
+}
+__device__ __forceinline__ bool steps_wait(StepCtl* ctl, unsigned target, bool patient, long long polls)
 {
     __shared__ int ok;
     if (threadIdx.x == 0) {
-        int good = 1;
-        unsigned v;
-        long long it = 0;
-        for (;;) {
+        int it = patient ? 0 : kFirstPolls;
+        for (; it < kFirstPolls; it++) {
+            unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->bar_count) : "memory");
             if (v >= target) break;
-            if (++it > polls) {
-                atomicOr(&ctl->status, ST_TIMEOUT);
-                good = 0;
-                break;
-            }
         }
-        ok = good;
+        ok = it < kFirstPolls ? 1 : steps_wait_slow(ctl, target, patient ? polls - kFirstPolls : polls);
     }
     __syncthreads();
     return ok != 0;
@@ -644,12 +667,12 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
     __syncthreads();
     locate();
     const double dt_fac = stupid_factor<NF>(P), dt_vmin = P.cell_volume * P.Ye * P.rho / kMp;
-    bool alive = true;
+    const bool patient = P.wait_polls >= kFirstPolls;
     unsigned nbar = 0;
     int slot = 0;  // of the control's vmax_bits: the step's largest number
     int cur = 0;   // ONE: which half of smesh holds the stage mesh
 
-    for (int it = 0; it < nsteps && alive; it++) {
+    for (int it = 0; it < nsteps; it++) {
         if (hist && gtid == 0) hist[step] = dt;
         const bool want_full = step >= full_from || last || step + 1 >= max_step;
         const bool final_step = it + 1 == nsteps;
@@ -889,9 +912,9 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
                 }
                 if (wait) {
                     nbar++;
-                    if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) {
-                        alive = false;
-                        break;
+                    if (!steps_wait(ctl, nbar * gridDim.x, patient, P.wait_polls)) {
+                        if (tid == 0) steps_gave_up(ctl);
+                        return;
                     }
                 }
                 if (s == 4 && dt_mode == DT_ADVANCE) {
@@ -928,7 +951,7 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
         if (done) break;
     }
 
-    if (alive && active) {
+    if (active) {
 #pragma unroll
         for (int e = 0; e < NH; e++) S.f0[(sp * NH + e) * cap + p] = y0[e];
         if (not_finite<NH>(y0)) ctl->odd = 1;
@@ -947,10 +970,8 @@ __device__ __forceinline__ void steps_1d_body(const DevParams& P, const DevState
             cmesh[msize + i] = 0.0;
         }
     }
-    // the last CTA to leave writes the step control (all hold the same).  Every
-    // CTA comes by, also one that gave up a wait, so that the counts are right
-    // for the next launch; then the run ends with the steps before this launch
-    // (the launches queued behind it return at once)
+    // the last CTA to leave writes the step control (all hold the same), unless
+    // another gave up a wait: then the run ends with the steps before this launch
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(&ctl->blocks_done, 1u) == gridDim.x - 1) {
@@ -1054,10 +1075,14 @@ __device__ __forceinline__ void adjoint_1d_body(const DevParams& P, const DevSta
         shape<double>(zpos(len - 1) * P.dxi[2], P.ord[2], first, L.wz);
         sref = wrapi(first, nz);
     }
-    // (a segment swept before this one in the same call gave up)
-    bool alive = __syncthreads_and(!steps_timed_out(ctl));
+    if (!__syncthreads_and(!steps_timed_out(ctl))) {
+        // (a segment swept before this one in the same call gave up)
+        if (tid == 0) steps_gave_up(ctl);
+        return;
+    }
+    const bool patient = P.wait_polls >= kFirstPolls;
     unsigned nbar = 0;
-    for (int j = len - 1; j >= 0 && alive; j--) {
+    for (int j = len - 1; j >= 0; j--) {
         const double* const sst = A.rec.sst + j * A.rec.sst_stride;
         const double dt = A.dts[j];
         load(sst + 3 * (2 * NH) * cap, yn);   // Y_n
@@ -1133,13 +1158,13 @@ __device__ __forceinline__ void adjoint_1d_body(const DevParams& P, const DevSta
                 load(s == 2 ? A.rec.seg + j * A.rec.seg_stride : sst + (s - 3) * (2 * NH) * cap, ys);   // Y_{s-1}
             }
             nbar++;
-            if (!steps_wait(ctl, nbar * gridDim.x, P.wait_polls)) {
-                alive = false;
-                break;
+            if (!steps_wait(ctl, nbar * gridDim.x, patient, P.wait_polls)) {
+                if (tid == 0) steps_gave_up(ctl);
+                return;
             }
         }
     }
-    if (alive && active) {
+    if (active) {
 #pragma unroll
         for (int e = 0; e < NH; e++) A.lamY0[(sp * NH + e) * cap + p] = lamY[e];
         A.lamN[sp * cap + p] += dN;
